@@ -21,7 +21,7 @@
 
 #include <cooperative_groups.h>
 
-#include "tpk_common.cuh"
+#include "fps_common.cuh"
 
 namespace cg = cooperative_groups;
 
@@ -29,42 +29,18 @@ namespace tpk
 {
 TPK_DEFINE_STATUS_WORD()
 
+// fps_rounds.cu
+bool fps_rounds_fits(int n);
+int fps_rounds(int b, int n, int m, int log2bs, const float* xyz, int32_t* idxs, float* new_xyz, cudaStream_t stream);
+
 namespace
 {
 
 constexpr int kFpsMaxThreads = 512;
 constexpr int kFpsMaxRanks = 16;
 constexpr int kFpsMaxPpt = 32;
-constexpr unsigned long long kWaitLimitNs = 1000000000ull;  // give up a wait after one second
 constexpr int kMsgBytes = 20;  // {key_hi, key_lo, x, y} + {z}
 
-__device__ __forceinline__ uint32_t smem_u32(const void* p)
-{
-    return static_cast<uint32_t>(__cvta_generic_to_shared(p));
-}
-__device__ __forceinline__ uint32_t cluster_ctarank()
-{
-    uint32_t r;
-    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-    return r;
-}
-__device__ __forceinline__ uint32_t cluster_nctarank()
-{
-    uint32_t r;
-    asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(r));
-    return r;
-}
-__device__ __forceinline__ uint32_t mapa_cluster(uint32_t addr, uint32_t rank)
-{
-    uint32_t r;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
-    return r;
-}
-__device__ __forceinline__ void cluster_sync_all()
-{
-    asm volatile("barrier.cluster.arrive.release.aligned;\n\t"
-                 "barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
 // Remote store that signals the destination CTA's mbarrier with the bytes written.
 __device__ __forceinline__ void st_async_msg(uint32_t addr_a, uint32_t addr_z, uint32_t mbar,
                                              uint32_t hi, uint32_t lo, float x, float y, float z)
@@ -77,58 +53,6 @@ __device__ __forceinline__ void st_async_msg(uint32_t addr_a, uint32_t addr_z, u
                      "r"(addr_z), "r"(__float_as_uint(z)), "r"(mbar)
                  : "memory");
 }
-__device__ __forceinline__ void mbar_init(uint32_t mbar, uint32_t count)
-{
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(mbar), "r"(count) : "memory");
-}
-__device__ __forceinline__ void mbar_arrive_expect_tx(uint32_t mbar, uint32_t bytes)
-{
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(mbar), "r"(bytes)
-                 : "memory");
-}
-__device__ __forceinline__ bool mbar_try_wait(uint32_t mbar, uint32_t parity)
-{
-    uint32_t ok;
-    asm volatile("{\n\t.reg .pred p;\n\t"
-                 "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
-                 "selp.u32 %0, 1, 0, p;\n\t}"
-                 : "=r"(ok)
-                 : "r"(mbar), "r"(parity)
-                 : "memory");
-    return ok != 0;
-}
-
-__device__ __forceinline__ unsigned long long global_timer_ns()
-{
-    unsigned long long t;
-    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-    return t;
-}
-
-// Waits for the phase with the given parity; false if it has not completed within
-// kWaitLimitNs (the clock is read only every 256 unsuccessful polls).
-__device__ __forceinline__ bool mbar_wait_bounded(uint32_t mbar, uint32_t parity)
-{
-    unsigned long long t0 = 0;
-    for (unsigned it = 1;; ++it)
-    {
-        if (mbar_try_wait(mbar, parity)) return true;
-        if ((it & 255u) == 0u)
-        {
-            const unsigned long long now = global_timer_ns();
-            if (t0 == 0)
-                t0 = now;
-            else if (now - t0 > kWaitLimitNs)
-                return false;
-        }
-    }
-}
-
-__device__ __forceinline__ uint32_t bitrev_low(uint32_t v, int bits)
-{
-    return bits == 0 ? 0u : (__brev(v) >> (32 - bits));
-}
-
 // Winner of one arg-max stage: key = bits of the running minimum (negative: no
 // candidate), k = index of the point in its cloud, (x, y, z) = its coordinates.
 struct Msg
@@ -138,14 +62,6 @@ struct Msg
 };
 
 constexpr int fps_max_threads(int ppt) { return ppt <= 16 ? 512 : 128; }
-
-// Tie rank of point k: the reference's strided scan + tree keeps, among equal maxima,
-// the smallest bit-reversed (k mod bs), then the smallest (k div bs).
-__device__ __forceinline__ uint32_t fps_rank(int k, int log2bs)
-{
-    const uint32_t u = static_cast<uint32_t>(k);
-    return (bitrev_low(u & ((1u << log2bs) - 1u), log2bs) << 22) | (u >> log2bs);
-}
 
 // Lane holding the largest key among the lanes of the warp.  One redux and one ballot
 // when that key is unique (the usual case); ranks are only computed and reduced when
@@ -172,48 +88,10 @@ __device__ __forceinline__ int warp_argmax(int key, int k, int log2bs)
 //      then polls its own CTA's barrier (with a time limit) and reduces the messages.
 // The round loop is unrolled by two so that the double-buffered message slots and
 // barriers have compile-time addresses.  A CTA has at least two warps.
-// packed pairs of floats for the two-wide FP32 instructions of sm_100
-__device__ __forceinline__ unsigned long long pack2(float lo, float hi)
-{
-    unsigned long long r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
-    return r;
-}
-__device__ __forceinline__ void unpack2(unsigned long long v, float& lo, float& hi)
-{
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
-}
-__device__ __forceinline__ unsigned long long add2(unsigned long long a, unsigned long long b)
-{
-    unsigned long long r;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-__device__ __forceinline__ unsigned long long mul2(unsigned long long a, unsigned long long b)
-{
-    unsigned long long r;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-__device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigned long long b, unsigned long long c)
-{
-    unsigned long long r;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-    return r;
-}
-
-//
-// SORTED: the points come from a spatially sorted copy (x, y, z, original index) and a
-// warp owns a contiguous run of it, i.e. a compact region of space.  A warp whose
-// bounding box is farther from the newest sample than its largest running minimum
-// cannot change any of its minima, so it skips the update and sends last round's winner
-// again.  In the late rounds, which are most of them, a sample only reaches a few warps.
-// The result does not depend on the order of the copy: ties are decided by the rank of
-// the original index at every level.
-template <int PPT, bool CLUSTERED, bool SORTED>
+template <int PPT, bool CLUSTERED>
 __global__ void __launch_bounds__(fps_max_threads(PPT), 1)
     fps_onchip_kernel(int n, int m, int log2bs, int flat, const float* __restrict__ xyz_all,
-                      const float4* __restrict__ sorted_all, int32_t* __restrict__ idxs_all)
+                      int32_t* __restrict__ idxs_all)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -251,39 +129,13 @@ __global__ void __launch_bounds__(fps_max_threads(PPT), 1)
     };
 
     float px[PPT], py[PPT], pz[PPT], md[PPT];
-    // bounding box of the warp's points (SORTED only)
-    float bminx = CUDART_INF_F, bminy = CUDART_INF_F, bminz = CUDART_INF_F;
-    float bmaxx = -CUDART_INF_F, bmaxy = -CUDART_INF_F, bmaxz = -CUDART_INF_F;
 #pragma unroll
     for (int p = 0; p < PPT; ++p)
     {
-        int k = point_index(p);
+        const int k = point_index(p);
         float x = 0.f, y = 0.f, z = 0.f;
         bool valid = false;
-        if (SORTED)
-        {
-            // slot of the sorted copy: warp-contiguous, lanes interleaved
-            const int slot = ((rank * nwarps + warp) * PPT + p) * 32 + lane;
-            k = n;
-            if (slot < n)
-            {
-                const float4 v = __ldg(sorted_all + static_cast<size_t>(cloud) * n + slot);
-                x = v.x;
-                y = v.y;
-                z = v.z;
-                k = __float_as_int(v.w);
-                const float mag = sumsq_abc(x, y, z);
-                valid = !(static_cast<double>(mag) <= 1e-3);
-                // fminf/fmaxf drop NaN: such a point never changes its minimum anyway
-                bminx = fminf(bminx, x);
-                bminy = fminf(bminy, y);
-                bminz = fminf(bminz, z);
-                bmaxx = fmaxf(bmaxx, x);
-                bmaxy = fmaxf(bmaxy, y);
-                bmaxz = fmaxf(bmaxz, z);
-            }
-        }
-        else if (k < n)
+        if (k < n)
         {
             x = __ldg(xyz + 3 * static_cast<size_t>(k) + 0);
             y = __ldg(xyz + 3 * static_cast<size_t>(k) + 1);
@@ -299,24 +151,6 @@ __global__ void __launch_bounds__(fps_max_threads(PPT), 1)
         // w carries the point's index so that the winner's message needs no index arithmetic
         sxyz[p * nthreads + tid] = make_float4(x, y, z, __int_as_float(k));
     }
-
-    if (SORTED)
-    {
-#pragma unroll
-        for (int o = 16; o >= 1; o >>= 1)
-        {
-            bminx = fminf(bminx, __shfl_xor_sync(kFullMask, bminx, o));
-            bminy = fminf(bminy, __shfl_xor_sync(kFullMask, bminy, o));
-            bminz = fminf(bminz, __shfl_xor_sync(kFullMask, bminz, o));
-            bmaxx = fmaxf(bmaxx, __shfl_xor_sync(kFullMask, bmaxx, o));
-            bmaxy = fmaxf(bmaxy, __shfl_xor_sync(kFullMask, bmaxy, o));
-            bmaxz = fmaxf(bmaxz, __shfl_xor_sync(kFullMask, bmaxz, o));
-        }
-    }
-    // SORTED: the warp's winner of the last round it updated in, and the bound a sample's
-    // squared distance to the box must exceed for the warp to skip (infinite: never skip)
-    Msg wm = {INT_MIN, 0, 0.f, 0.f, 0.f};
-    float skip_above = CUDART_INF_F;
 
     float cx = 0.f, cy = 0.f, cz = 0.f;
     if (n > 0)
@@ -366,22 +200,7 @@ __global__ void __launch_bounds__(fps_max_threads(PPT), 1)
         if (CLUSTERED && tid == 0)
             mbar_arrive_expect_tx(smem_u32(mbar + PAR), static_cast<uint32_t>(nslots * kMsgBytes));
 
-        bool active = true;
-        if (SORTED)
-        {
-            // squared distance from the sample to the warp's box; a computed distance is at
-            // least this bound less a few ulp, far inside the margin taken here
-            const float ex = fmaxf(fmaxf(bminx - cx, cx - bmaxx), 0.f);
-            const float ey = fmaxf(fmaxf(bminy - cy, cy - bmaxy), 0.f);
-            const float ez = fmaxf(fmaxf(bminz - cz, cz - bmaxz), 0.f);
-            const float lb = __fmaf_rn(ez, ez, __fmaf_rn(ex, ex, __fmul_rn(ey, ey)));
-            // the operands are the same in every lane; the vote makes the branch provably
-            // uniform for the warp-wide instructions inside it
-            active = __any_sync(kFullMask, !(__fmul_rn(lb, 0.9999f) > skip_above)) != 0;
-        }
         Msg msg;
-        if (active)
-        {
         // ---- every point: distance to the newest sample, running minimum, thread maximum
         if constexpr (PPT >= 2)
         {
@@ -425,23 +244,7 @@ __global__ void __launch_bounds__(fps_max_threads(PPT), 1)
         uint32_t eq = 0;
 #pragma unroll
         for (int p = 0; p < PPT; ++p) eq |= (md[p] == best) ? (1u << p) : 0u;
-        int bp = __ffs(eq) - 1;
-        if (SORTED && key == wkey && wkey >= 0 && (eq & (eq - 1u)) != 0u)
-        {
-            // several of this lane's points tie: the original index decides (no layout rule
-            // in a sorted copy).  Plain per-lane code, no warp-wide instruction.
-            uint32_t best_rank = 0xFFFFFFFFu;
-            for (uint32_t e = eq; e != 0u; e &= e - 1u)
-            {
-                const int p = __ffs(e) - 1;
-                const uint32_t r = fps_rank(__float_as_int(my_xyz[p * nthreads].w), log2bs);
-                if (r < best_rank)
-                {
-                    best_rank = r;
-                    bp = p;
-                }
-            }
-        }
+        const int bp = __ffs(eq) - 1;
         const float4 mine = my_xyz[bp * nthreads];
         uint32_t ball = __ballot_sync(kFullMask, key == wkey);
         if (__popc(ball) > 1 && wkey >= 0)
@@ -451,19 +254,13 @@ __global__ void __launch_bounds__(fps_max_threads(PPT), 1)
             ball = __ballot_sync(kFullMask, key == wkey && r == wr);
         }
         const int src1 = __ffs(ball) - 1;
-        if (SORTED || (CLUSTERED && flat))
+        if (CLUSTERED && flat)
         {
             msg.key = wkey;
             msg.k = __shfl_sync(kFullMask, __float_as_int(mine.w), src1);
             msg.x = __shfl_sync(kFullMask, mine.x, src1);
             msg.y = __shfl_sync(kFullMask, mine.y, src1);
             msg.z = __shfl_sync(kFullMask, mine.z, src1);
-            if (SORTED)
-            {
-                wm = msg;
-                // no skipping on tiny bounds, where a computed distance may have lost precision
-                skip_above = fmaxf(__int_as_float(wkey), 1.0e-30f);
-            }
         }
         else if (lane == src1)
         {
@@ -471,18 +268,6 @@ __global__ void __launch_bounds__(fps_max_threads(PPT), 1)
                                                  __float_as_uint(mine.x), __float_as_uint(mine.y));
             wmsg_z[PAR * 32 + warp] = mine.z;
         }
-        }  // active
-        else
-        {
-            msg = wm;
-        }
-        if (SORTED && !(CLUSTERED && flat) && lane == 0)
-        {
-            wmsg_a[PAR * 32 + warp] = make_uint4(static_cast<uint32_t>(msg.key), static_cast<uint32_t>(msg.k),
-                                                 __float_as_uint(msg.x), __float_as_uint(msg.y));
-            wmsg_z[PAR * 32 + warp] = msg.z;
-        }
-
         // ---- stage 2: the CTA's best point
         if (!(CLUSTERED && flat))
         {
@@ -558,467 +343,6 @@ __global__ void __launch_bounds__(fps_max_threads(PPT), 1)
     if (CLUSTERED) cluster_sync_all();
 }
 
-// ---------------------------------------------------------------- several samples per exchange
-//
-// The sorted kernel above pays one arg-max exchange per sample.  This kernel takes up to eight
-// samples out of one exchange, exactly:
-//
-//   Every warp publishes its best point e1 = {key, index, x, y, z} and the KEY of its second
-//   best point (key2).  Every warp then sorts the warps' best points (key, then tie rank of the
-//   index) and accepts the longest prefix t0, t1, ... in which every t_i
-//     (a) is untouched by the samples accepted before it: !(dist(t_i, t_j) < md(t_i)) for all
-//         j < i, evaluated with the update's own arithmetic, so its running minimum - its key -
-//         is what the sequential algorithm would see after applying t_0..t_{i-1};
-//     (b) beats everything a warp that already gave a sample still holds: key(t_i) > key2 of
-//         those warps (running minima only shrink, so key2 bounds the warp's leftovers);
-//     (c) has a positive key (the list is sorted by key, then by the tie rank of the index, so
-//         equal keys come in the reference's order);
-//     (d) follows only samples with finite coordinates: a sample's own minimum must drop to
-//         zero when it is applied, or the reference would pick it again (a warp publishes such
-//         a point with the largest key2 there is, so test (b) covers it).
-//   Points of warps that gave no sample are bounded by that warp's e1, which sorts after t_i.
-//   So t_i is the largest running minimum that remains after t_0..t_{i-1} were applied: the
-//   sample the reference picks next.  Cutting the prefix early is always allowed, which is
-//   what makes the conservative tests (b) and (c) safe.
-//
-// Late in a run the largest running minima sit in different holes of the cloud, so almost
-// every candidate passes: about five samples per exchange at 16384 points, with the update,
-// the warp arg-max and the cluster exchange paid once for all of them.  Applying several
-// samples is one pass over the warp's points with a minimum per sample in reach; the order
-// of the minima does not matter.  With 16 or more points per lane a warp's points are four groups
-// with a bounding box each, and a sample only updates the groups it can reach (under half the
-// groups of the warps it reaches at all): 12 % faster at 32768 points per cloud and with 64
-// clouds resident, no change at 16 clouds of 16384, where the update is not what the exchange
-// waits for.  Requires the sorted copy and at most 32 warps per cloud.
-constexpr int kFpsBatchMax = 8;       // samples per exchange
-constexpr int kBatchMsgBytes = 24;    // {x, y, z, key2} + key + index
-
-// One warp's entry into a peer's tables: coordinates and key2 (what the acceptance test reads
-// with one load), the key into a compact table of its own (the ranking reads 32 keys with eight
-// loads), and the point's index.
-__device__ __forceinline__ void st_async_batch(uint32_t addr_c, uint32_t addr_key, uint32_t addr_k, uint32_t mbar,
-                                               const uint4& c, uint32_t key, uint32_t k)
-{
-    asm volatile(
-        "st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%1, %2, %3, %4}, [%5];" ::
-            "r"(addr_c), "r"(c.x), "r"(c.y), "r"(c.z), "r"(c.w), "r"(mbar)
-        : "memory");
-    asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.b32 [%0], %1, [%2];" ::
-                     "r"(addr_key), "r"(key), "r"(mbar)
-                 : "memory");
-    asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.b32 [%0], %1, [%2];" ::
-                     "r"(addr_k), "r"(k), "r"(mbar)
-                 : "memory");
-}
-
-template <int PPT, int MAXT, bool CLUSTERED>
-__global__ void __launch_bounds__(MAXT, 1)
-    fps_batched_kernel(int n, int m, int log2bs, const float* __restrict__ xyz_all,
-                       const float4* __restrict__ sorted_all, int32_t* __restrict__ idxs_all)
-{
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int nthreads = blockDim.x, nwarps = nthreads >> 5;
-    const int nranks = CLUSTERED ? static_cast<int>(cluster_nctarank()) : 1;
-    const int rank = CLUSTERED ? static_cast<int>(cluster_ctarank()) : 0;
-    const int cloud = blockIdx.x / nranks;
-    const int gtid = rank * nthreads + tid;
-    const int nslots = nranks * nwarps;  // at most 32: one slot per warp of the cluster
-    const int my_slot = rank * nwarps + warp;
-
-    // shared memory: slot tables of both parities (32 x {16, 4, 4} B each), 2 mbarriers, per warp
-    // the sorted candidates of an exchange (8 x 24 B) and the warp's own entry, then the CTA's points
-    uint4* tab_c = reinterpret_cast<uint4*>(smem_raw);        // [2][32] {x, y, z, key2}
-    int* tab_key = reinterpret_cast<int*>(tab_c + 64);        // [2][32] key
-    int* tab_k = tab_key + 64;                                // [2][32] index of the point
-    uint64_t* mbar = reinterpret_cast<uint64_t*>(tab_k + 64);
-    uint4* sort_c = reinterpret_cast<uint4*>(mbar + 2);       // [16 warps][8] {x, y, z, key2}
-    uint2* sort_k = reinterpret_cast<uint2*>(sort_c + 16 * kFpsBatchMax);  // [16 warps][8] {key, index}
-    uint4* own_c = reinterpret_cast<uint4*>(sort_k + 16 * kFpsBatchMax);   // [16 warps]
-    uint2* own_k = reinterpret_cast<uint2*>(own_c + 16);                   // [16 warps] {key, index}
-    float4* sxyz = reinterpret_cast<float4*>(own_k + 16);
-    uint4* my_sort_c = sort_c + warp * kFpsBatchMax;
-    uint2* my_sort_k = sort_k + warp * kFpsBatchMax;
-
-    const float* xyz = xyz_all + static_cast<size_t>(cloud) * n * 3;
-    int32_t* idxs = idxs_all + static_cast<size_t>(cloud) * m;
-
-    float px[PPT], py[PPT], pz[PPT], md[PPT];
-    // The warp's points in NG groups of GP * 32 consecutive points of the sorted copy (compact in
-    // space), each with its bounding box: a sample only updates the groups it can reach.
-    constexpr int NG = PPT >= 16 ? 4 : 1;  // measured: no gain below 16 points per lane
-    constexpr int GP = PPT / NG;
-    float gmin[NG][3], gmax[NG][3];
-#pragma unroll
-    for (int g = 0; g < NG; ++g)
-#pragma unroll
-        for (int a = 0; a < 3; ++a)
-        {
-            gmin[g][a] = CUDART_INF_F;
-            gmax[g][a] = -CUDART_INF_F;
-        }
-#pragma unroll
-    for (int p = 0; p < PPT; ++p)
-    {
-        // slot of the sorted copy: warp-contiguous, lanes interleaved
-        const int slot = ((rank * nwarps + warp) * PPT + p) * 32 + lane;
-        float x = 0.f, y = 0.f, z = 0.f;
-        int k = n;
-        bool valid = false;
-        if (slot < n)
-        {
-            const float4 v = __ldg(sorted_all + static_cast<size_t>(cloud) * n + slot);
-            x = v.x;
-            y = v.y;
-            z = v.z;
-            k = __float_as_int(v.w);
-            const float mag = sumsq_abc(x, y, z);
-            valid = !(static_cast<double>(mag) <= 1e-3);
-            gmin[p / GP][0] = fminf(gmin[p / GP][0], x);
-            gmin[p / GP][1] = fminf(gmin[p / GP][1], y);
-            gmin[p / GP][2] = fminf(gmin[p / GP][2], z);
-            gmax[p / GP][0] = fmaxf(gmax[p / GP][0], x);
-            gmax[p / GP][1] = fmaxf(gmax[p / GP][1], y);
-            gmax[p / GP][2] = fmaxf(gmax[p / GP][2], z);
-        }
-        px[p] = x;
-        py[p] = y;
-        pz[p] = z;
-        md[p] = valid ? 1e10f : -1.0f;  // negative: never a candidate (fminf keeps it negative)
-        sxyz[p * nthreads + tid] = make_float4(x, y, z, __int_as_float(k));
-    }
-    // lane l keeps the box of group l % NG: in the reach test below it answers for that group
-    // and for sample l / NG of the list
-    float bminx = CUDART_INF_F, bminy = CUDART_INF_F, bminz = CUDART_INF_F;
-    float bmaxx = -CUDART_INF_F, bmaxy = -CUDART_INF_F, bmaxz = -CUDART_INF_F;
-#pragma unroll
-    for (int g = 0; g < NG; ++g)
-    {
-#pragma unroll
-        for (int a = 0; a < 3; ++a)
-#pragma unroll
-            for (int o = 16; o >= 1; o >>= 1)
-            {
-                gmin[g][a] = fminf(gmin[g][a], __shfl_xor_sync(kFullMask, gmin[g][a], o));
-                gmax[g][a] = fmaxf(gmax[g][a], __shfl_xor_sync(kFullMask, gmax[g][a], o));
-            }
-        if (lane % NG == g)
-        {
-            bminx = gmin[g][0];
-            bminy = gmin[g][1];
-            bminz = gmin[g][2];
-            bmaxx = gmax[g][0];
-            bmaxy = gmax[g][1];
-            bmaxz = gmax[g][2];
-        }
-    }
-    if (gtid == 0 && m > 0) idxs[0] = 0;
-    // the list of samples to apply next (the same in every warp), in the warp's sort scratch:
-    // at first the cloud's point 0
-    if (lane == 0)
-    {
-        float cx = 0.f, cy = 0.f, cz = 0.f;
-        if (n > 0)
-        {
-            cx = __ldg(xyz + 0);
-            cy = __ldg(xyz + 1);
-            cz = __ldg(xyz + 2);
-        }
-        my_sort_c[0] = make_uint4(__float_as_uint(cx), __float_as_uint(cy), __float_as_uint(cz), 0u);
-        my_sort_k[0] = make_uint2(0u, 0u);
-        own_c[warp] = make_uint4(0u, 0u, 0u, 0x80000000u);
-        own_k[warp] = make_uint2(0x80000000u, 0u);
-    }
-    // slots no warp owns sort behind every real entry (key INT_MIN), in both tables
-    if (tid < 64 && (tid & 31) >= nslots)
-    {
-        tab_c[tid] = make_uint4(0u, 0u, 0u, 0x80000000u);
-        tab_key[tid] = static_cast<int>(0x80000000u);
-        tab_k[tid] = 0;
-    }
-    if (CLUSTERED)
-    {
-        if (tid == 0)
-        {
-            mbar_init(smem_u32(mbar + 0), 1);
-            mbar_init(smem_u32(mbar + 1), 1);
-            asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-        }
-        cluster_sync_all();
-    }
-    else
-    {
-        __syncthreads();
-    }
-    // remote addresses of this warp's slot in CTA `lane` of the cluster, parity 0; parity 1 lies
-    // 32 entries (one barrier) further in the same shared window
-    uint32_t rem_c = 0, rem_key = 0, rem_k = 0, rem_bar = 0;
-    if (CLUSTERED && lane < nranks)
-    {
-        rem_c = mapa_cluster(smem_u32(tab_c + my_slot), lane);
-        rem_key = mapa_cluster(smem_u32(tab_key + my_slot), lane);
-        rem_k = mapa_cluster(smem_u32(tab_k + my_slot), lane);
-        rem_bar = mapa_cluster(smem_u32(mbar), lane);
-    }
-    const float4* my_xyz = sxyz + tid;
-    // the warp's entry of the last exchange it recomputed lives in own_c / own_k; infinite bound:
-    // the first pass never skips
-    float skip_above = CUDART_INF_F;
-    bool failed = false;
-    int nb = 1;   // samples to apply
-    int j = 1;    // next output position
-
-    for (int exch = 0; j < m; ++exch)
-    {
-        const int par = exch & 1;
-        // (the CTA's last warp arms the barrier: in the middle CTA of a cluster warp 0 holds the
-        // middle of the Morton order, the warp almost every sample reaches and every exchange waits for)
-        if (CLUSTERED && tid == nthreads - 32)
-            mbar_arrive_expect_tx(smem_u32(mbar + par), static_cast<uint32_t>(nslots * kBatchMsgBytes));
-
-        // ---- 1. apply the samples to the groups of points they can reach
-        // lane l tests sample l / NG against the box of group l % NG: one vote for all samples and
-        // groups.  Every lane holds all candidates of the list (loads in flight together; entries
-        // beyond nb are stale and unused).
-        uint4 sc[kFpsBatchMax];
-#pragma unroll
-        for (int i = 0; i < kFpsBatchMax; ++i) sc[i] = my_sort_c[i];
-        bool in_reach = false;
-        {
-            const int ts = lane / NG;
-            const uint4 sl = my_sort_c[ts < kFpsBatchMax ? ts : 0];
-            const float cx = __uint_as_float(sl.x), cy = __uint_as_float(sl.y), cz = __uint_as_float(sl.z);
-            const float ex = fmaxf(fmaxf(bminx - cx, cx - bmaxx), 0.f);
-            const float ey = fmaxf(fmaxf(bminy - cy, cy - bmaxy), 0.f);
-            const float ez = fmaxf(fmaxf(bminz - cz, cz - bmaxz), 0.f);
-            const float lb = __fmaf_rn(ez, ez, __fmaf_rn(ex, ex, __fmul_rn(ey, ey)));
-            // out of reach: farther from the group's box than the largest running minimum of the
-            // whole warp (a bound for the group's own)
-            in_reach = ts < nb && !(__fmul_rn(lb, 0.9999f) > skip_above);
-        }
-        const uint32_t todo = __ballot_sync(kFullMask, in_reach);
-        const bool touched = todo != 0u;
-#pragma unroll
-        for (int i = 0; i < kFpsBatchMax; ++i)
-        {
-            const uint32_t groups = (todo >> (i * NG)) & ((1u << NG) - 1u);  // warp-uniform
-            if (groups != 0u)
-            {
-                const float cx = __uint_as_float(sc[i].x), cy = __uint_as_float(sc[i].y), cz = __uint_as_float(sc[i].z);
-                if constexpr (PPT >= 2)
-                {
-                    const unsigned long long ncx = pack2(-cx, -cx), ncy = pack2(-cy, -cy), ncz = pack2(-cz, -cz);
-#pragma unroll
-                    for (int g = 0; g < NG; ++g)
-                    {
-                        if ((groups >> g) & 1u)
-                        {
-#pragma unroll
-                            for (int p = g * GP; p < (g + 1) * GP; p += 2)
-                            {
-                                const unsigned long long dx = add2(pack2(px[p], px[p + 1]), ncx);
-                                const unsigned long long dy = add2(pack2(py[p], py[p + 1]), ncy);
-                                const unsigned long long dz = add2(pack2(pz[p], pz[p + 1]), ncz);
-                                float d0, d1;
-                                unpack2(fma2(dz, dz, fma2(dx, dx, mul2(dy, dy))), d0, d1);
-                                md[p] = fminf(d0, md[p]);
-                                md[p + 1] = fminf(d1, md[p + 1]);
-                            }
-                        }
-                    }
-                }
-                else
-                {
-                    md[0] = fminf(sumsq_abc(px[0] - cx, py[0] - cy, pz[0] - cz), md[0]);
-                }
-            }
-        }
-        if (touched)
-        {
-            // ---- the warp's best point (ties: rank of the original index) and the key of its second best
-            float red[PPT];
-#pragma unroll
-            for (int p = 0; p < PPT; ++p) red[p] = md[p];
-#pragma unroll
-            for (int w = PPT / 2; w >= 1; w >>= 1)
-#pragma unroll
-                for (int p = 0; p < w; ++p) red[p] = fmaxf(red[p], red[p + w]);
-            const float best = red[0];
-            const int key = __float_as_int(best);
-            const int wkey = __reduce_max_sync(kFullMask, key);
-            uint32_t eq = 0;
-#pragma unroll
-            for (int p = 0; p < PPT; ++p) eq |= (md[p] == best) ? (1u << p) : 0u;
-            int bp = __ffs(eq) - 1;
-            if (key == wkey && wkey >= 0 && (eq & (eq - 1u)) != 0u)
-            {
-                uint32_t best_rank = 0xFFFFFFFFu;
-                for (uint32_t e = eq; e != 0u; e &= e - 1u)
-                {
-                    const int p = __ffs(e) - 1;
-                    const uint32_t r = fps_rank(__float_as_int(my_xyz[p * nthreads].w), log2bs);
-                    if (r < best_rank)
-                    {
-                        best_rank = r;
-                        bp = p;
-                    }
-                }
-            }
-            if (bp < 0) bp = 0;
-            const float4 mine = my_xyz[bp * nthreads];
-            const bool mine_finite = sumsq_abc(mine.x - mine.x, mine.y - mine.y, mine.z - mine.z) == 0.f;
-            // second best of the warp: a lane that holds the best counts the best of its other
-            // points (the vote below does not wait for this reduction, nor it for the vote)
-            float alt = -2.0f;
-#pragma unroll
-            for (int p = 0; p < PPT; ++p) alt = fmaxf(alt, p == bp ? -2.0f : md[p]);
-            int key2 = __reduce_max_sync(kFullMask, __float_as_int(key == wkey ? alt : best));
-            uint32_t ball = __ballot_sync(kFullMask, key == wkey);
-            if (__popc(ball) > 1 && wkey >= 0)
-            {
-                key2 = wkey;  // another lane holds an equal minimum
-                const uint32_t r = key == wkey ? fps_rank(__float_as_int(mine.w), log2bs) : 0xFFFFFFFFu;
-                const uint32_t wr = __reduce_min_sync(kFullMask, r);
-                ball = __ballot_sync(kFullMask, key == wkey && r == wr);
-            }
-            const int h1 = __ffs(ball) - 1;
-            // the holder publishes through shared memory: every warp-wide instruction on this path
-            // costs about a hundred cycles, a store and a load do not
-            if (lane == h1)
-            {
-                // (d): a point with a non-finite coordinate does not drop to zero when it becomes a
-                // sample (inf - inf and NaN leave its minimum where it is) and the reference then
-                // picks it again; the largest key2 there is stops every later candidate
-                if (!mine_finite) key2 = 0x7fffffff;
-                own_c[warp] = make_uint4(__float_as_uint(mine.x), __float_as_uint(mine.y), __float_as_uint(mine.z),
-                                         static_cast<uint32_t>(key2));
-                own_k[warp] = make_uint2(static_cast<uint32_t>(wkey), __float_as_uint(mine.w));
-            }
-            __syncwarp();
-            // no skipping on tiny bounds, where a computed distance may have lost precision
-            skip_above = fmaxf(__int_as_float(wkey), 1.0e-30f);
-        }
-        // ---- 2. publish the warp's entry to every CTA of the cluster
-        if (CLUSTERED)
-        {
-            if (lane < nranks)
-            {
-                const uint4 oc = own_c[warp];
-                const uint2 ok2 = own_k[warp];
-                st_async_batch(rem_c + par * 32 * 16, rem_key + par * 32 * 4, rem_k + par * 32 * 4, rem_bar + par * 8, oc,
-                               ok2.x, ok2.y);
-            }
-            const uint32_t parity = static_cast<uint32_t>(exch >> 1) & 1u;
-            if (!failed && !mbar_wait_bounded(smem_u32(mbar + par), parity))
-            {
-                if (lane == 0) atomicOr(&g_dev_status, kStatusWaitAbandoned);
-                failed = true;
-            }
-        }
-        else
-        {
-            if (lane == 0)
-            {
-                const uint2 ok2 = own_k[warp];
-                tab_c[par * 32 + my_slot] = own_c[warp];
-                tab_key[par * 32 + my_slot] = static_cast<int>(ok2.x);
-                tab_k[par * 32 + my_slot] = static_cast<int>(ok2.y);
-            }
-            __syncthreads();
-        }
-        // ---- 3. the samples this exchange yields (every warp computes the same list)
-        // Position of every slot's entry in the exact order of the picks: key descending, then the
-        // tie rank of the point's index, then the slot.  Every lane walks the 32 keys of the table
-        // (broadcast loads, no warp-wide instruction; unowned slots hold INT_MIN).
-        const uint4 ec = tab_c[par * 32 + lane];
-        const int key_l = tab_key[par * 32 + lane];
-        const int k_l = tab_k[par * 32 + lane];
-        int4 kq[8];
-#pragma unroll
-        for (int q = 0; q < 8; ++q) kq[q] = reinterpret_cast<const int4*>(tab_key + par * 32)[q];
-        // integer arithmetic on the comparison results, no short-circuit operators: the compiler
-        // turns those into a branch per step, which costs more than the step
-        int pos = 0, same = 0;
-#pragma unroll
-        for (int q = 0; q < 8; ++q)
-        {
-            const int ks[4] = {kq[q].x, kq[q].y, kq[q].z, kq[q].w};
-#pragma unroll
-            for (int c = 0; c < 4; ++c)
-            {
-                pos += ks[c] > key_l ? 1 : 0;
-                same += ks[c] == key_l ? 1 : 0;
-            }
-        }
-        const bool tie = same > 1;  // the lane's own slot is the one match; without ties pos is exact
-        if (tie && key_l >= 0)  // rare: equal keys of real entries, the ranks of the indices decide
-        {
-            const uint32_t rl = fps_rank(k_l, log2bs);
-            pos = 0;
-            for (int s = 0; s < 32; ++s)
-            {
-                const int ks = tab_key[par * 32 + s];
-                bool before = ks > key_l;
-                if (ks == key_l && s != lane)
-                {
-                    const uint32_t rs = fps_rank(tab_k[par * 32 + s], log2bs);
-                    before = rs < rl || (rs == rl && s < lane);
-                }
-                pos += before ? 1 : 0;
-            }
-        }
-        __syncwarp();  // the list of the previous exchange has been read by every lane
-        if (lane < nslots && pos < kFpsBatchMax)
-        {
-            my_sort_c[pos] = ec;
-            my_sort_k[pos] = make_uint2(static_cast<uint32_t>(key_l), static_cast<uint32_t>(k_l));
-        }
-        __syncwarp();
-        const int ncand = nslots < kFpsBatchMax ? nslots : kFpsBatchMax;
-        // every lane runs the test (lanes without a candidate on entry 0): no branch, and the
-        // loads do not wait for one another
-        bool ok;
-        {
-            const int tl = lane < ncand ? lane : 0;
-            const uint4 tc = my_sort_c[tl];
-            const float tx = __uint_as_float(tc.x), ty = __uint_as_float(tc.y), tz = __uint_as_float(tc.z);
-            const int tkey = static_cast<int>(my_sort_k[tl].x);
-            const float tmd = __int_as_float(tkey);
-            uint4 ss[kFpsBatchMax - 1];
-#pragma unroll
-            for (int s = 0; s < kFpsBatchMax - 1; ++s) ss[s] = my_sort_c[s < ncand ? s : 0];
-            // (c) a positive key: at zero every remaining point coincides with a sample, samples of
-            // this exchange included, and only the first pick of an exchange knows their order
-            int okw = (tkey > 0 ? 1 : 0) & (lane < ncand ? 1 : 0);
-#pragma unroll
-            for (int s = 0; s < kFpsBatchMax - 1; ++s)
-            {
-                const float sx = __uint_as_float(ss[s].x), sy = __uint_as_float(ss[s].y), sz = __uint_as_float(ss[s].z);
-                // (a) untouched by sample s, with the update's arithmetic (x + (-c) rounds like x - c)
-                const float d = sumsq_abc(tx - sx, ty - sy, tz - sz);
-                // (b) above whatever the warp that gave sample s still holds; (d) is folded into key2
-                const int pass = (d < tmd ? 0 : 1) & (tkey > static_cast<int>(ss[s].w) ? 1 : 0);
-                okw &= (s >= lane ? 1 : 0) | pass;
-            }
-            ok = okw != 0 || lane == 0;  // the first pick of an exchange is exact by construction
-        }
-        const uint32_t okmask = __ballot_sync(kFullMask, ok);
-        nb = __ffs(~okmask) - 1;  // length of the accepted prefix (lane 0 always accepts)
-        if (nb > m - j) nb = m - j;
-        if (gtid == 0)
-        {
-            for (int i = 0; i < nb; ++i)
-            {
-                const uint2 sk = my_sort_k[i];
-                idxs[j + i] = static_cast<int>(sk.x) >= 0 ? static_cast<int>(sk.y) : 0;
-            }
-        }
-        j += nb;
-    }
-    // no CTA may leave while a peer can still write into its shared memory
-    if (CLUSTERED) cluster_sync_all();
-}
-
 // ---------------------------------------------------------------- spatial sort
 //
 // Copy of every cloud in Morton order of a 2^bits-per-axis grid over its bounding box,
@@ -1026,15 +350,6 @@ __global__ void __launch_bounds__(MAXT, 1)
 // in shared memory.  The order inside a cell is whatever the atomics give; the sampling
 // kernel's result does not depend on it.
 constexpr int kSortThreads = 1024;
-
-__device__ __forceinline__ uint32_t spread3(uint32_t v)
-{
-    v = (v | (v << 16)) & 0x030000FFu;
-    v = (v | (v << 8)) & 0x0300F00Fu;
-    v = (v | (v << 4)) & 0x030C30C3u;
-    v = (v | (v << 2)) & 0x09249249u;
-    return v;
-}
 
 __global__ void __launch_bounds__(kSortThreads)
     fps_sort_kernel(int n, int bits, const float* __restrict__ xyz_all, float4* __restrict__ sorted_all)
@@ -1835,11 +1150,11 @@ bool fps_pick_config(int n, int m, FpsConfig* out)
     return true;
 }
 
-template <int PPT, bool CLUSTERED, bool SORTED>
-int fps_launch_t(const FpsConfig& c, int b, int n, int m, int log2bs, const float* xyz,
-                 const float4* sorted, int32_t* idxs, cudaStream_t stream)
+template <int PPT, bool CLUSTERED>
+int fps_launch_t(const FpsConfig& c, int b, int n, int m, int log2bs, const float* xyz, int32_t* idxs,
+                 cudaStream_t stream)
 {
-    auto kernel = fps_onchip_kernel<PPT, CLUSTERED, SORTED>;
+    auto kernel = fps_onchip_kernel<PPT, CLUSTERED>;
     prefer_max_shared(kernel);
     const size_t smem = fps_smem_bytes(c);
     cudaError_t err;
@@ -1878,7 +1193,7 @@ int fps_launch_t(const FpsConfig& c, int b, int n, int m, int log2bs, const floa
     // test hook "fps_tree" selects the three-stage exchange
     const int flat = (c.nranks > 1 && c.nranks * (c.nthreads / 32) <= 32 && !test_path("fps_tree")) ? 1 : 0;
     count_launches(1);
-    err = cudaLaunchKernelEx(&cfg, kernel, n, m, log2bs, flat, xyz, sorted, idxs);
+    err = cudaLaunchKernelEx(&cfg, kernel, n, m, log2bs, flat, xyz, idxs);
     if (err != cudaSuccess)
     {
         set_error("fps launch (cluster %d x %d threads x %d points): %s", c.nranks, c.nthreads,
@@ -1888,139 +1203,36 @@ int fps_launch_t(const FpsConfig& c, int b, int n, int m, int log2bs, const floa
     return TPK_OK;
 }
 
-size_t fps_batched_smem_bytes(const FpsConfig& c)
-{
-    // slot tables (2 x 32 x 24 B), 2 mbarriers, per-warp sort scratch (16 x 8 x 24 B) and own entry
-    // (16 x 24 B), coordinates
-    return 2 * 32 * 24 + 16 + 16 * kFpsBatchMax * 24 + 16 * 24 + static_cast<size_t>(c.ppt) * c.nthreads * 4 * sizeof(float);
-}
-
-template <int PPT, int MAXT, bool CLUSTERED>
-int fps_launch_batched_t(const FpsConfig& c, int b, int n, int m, int log2bs, const float* xyz, const float4* sorted,
-                         int32_t* idxs, cudaStream_t stream)
-{
-    auto kernel = fps_batched_kernel<PPT, MAXT, CLUSTERED>;
-    prefer_max_shared(kernel);
-    const size_t smem = fps_batched_smem_bytes(c);
-    cudaError_t err;
-    if (smem > kDynSmemOptIn)
-    {
-        err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-        if (err != cudaSuccess)
-        {
-            set_error("fps: shared memory attribute: %s", cudaGetErrorString(err));
-            return TPK_ERR_CUDA;
-        }
-    }
-    if (c.nranks > 8)
-    {
-        err = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-        if (err != cudaSuccess)
-        {
-            set_error("fps: cluster size attribute: %s", cudaGetErrorString(err));
-            return TPK_ERR_CUDA;
-        }
-    }
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(static_cast<unsigned>(b) * c.nranks, 1, 1);
-    cfg.blockDim = dim3(c.nthreads, 1, 1);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = c.nranks;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    count_launches(1);
-    err = cudaLaunchKernelEx(&cfg, kernel, n, m, log2bs, xyz, sorted, idxs);
-    if (err != cudaSuccess)
-    {
-        set_error("fps launch (several samples per exchange, cluster %d x %d threads x %d points): %s", c.nranks,
-                  c.nthreads, c.ppt, cudaGetErrorString(err));
-        return TPK_ERR_CUDA;
-    }
-    return TPK_OK;
-}
-
 template <bool CLUSTERED>
-int fps_launch_batched(const FpsConfig& c, int b, int n, int m, int log2bs, const float* xyz, const float4* sorted,
-                       int32_t* idxs, cudaStream_t stream)
-{
-    // Blocks of four warps get their own build: with 512 threads as the bound the compiler has
-    // 128 registers, too few to keep the loads of a merge in flight together.  The lean build
-    // stays for batches whose CTAs only fit the GPU at once with it (measured on 64 clouds).
-    const bool roomy = c.nthreads <= 128 && static_cast<long long>(b) * c.nranks <= 2ll * num_sms();
-#define TPK_FPS_BATCHED_CASE(P)                                                                                      \
-    case P:                                                                                                          \
-        return roomy                                                                                                 \
-                   ? fps_launch_batched_t<P, 128, CLUSTERED>(c, b, n, m, log2bs, xyz, sorted, idxs, stream)          \
-                   : fps_launch_batched_t<P, fps_max_threads(P), CLUSTERED>(c, b, n, m, log2bs, xyz, sorted, idxs, stream)
-    switch (c.ppt)
-    {
-        TPK_FPS_BATCHED_CASE(1);
-        TPK_FPS_BATCHED_CASE(2);
-        TPK_FPS_BATCHED_CASE(4);
-        TPK_FPS_BATCHED_CASE(8);
-        TPK_FPS_BATCHED_CASE(16);
-        TPK_FPS_BATCHED_CASE(32);
-    default: break;
-    }
-#undef TPK_FPS_BATCHED_CASE
-    set_error("fps: unsupported points per thread %d", c.ppt);
-    return TPK_ERR_UNSUPPORTED;
-}
-
-// The kernel with several samples per exchange takes clusters of at most 32 warps (one slot per
-// warp) and 16 warps per CTA; test hook "fps_single" keeps the one-sample-per-exchange kernel.
-bool fps_wants_batched(const FpsConfig& c)
-{
-    return c.nranks * (c.nthreads / 32) <= 32 && c.nthreads / 32 <= 16 && !test_path("fps_single");
-}
-
-// Cluster shape for that kernel: eight CTAs of four warps fill the 32 slots with the fewest
-// warps per SM (measured best from 4096 to 32768 points per cloud, for 16 and for 64 clouds).
-// Larger clouds keep the shape fps_pick_config chose, and with it the one-sample kernel.
-void fps_batched_config(int n, FpsConfig* c)
-{
-    char text[8];
-    if (test_value("fps_config", text, sizeof(text)) || test_path("fps_single")) return;
-    FpsConfig e;
-    e.nranks = 8;
-    e.nthreads = 128;
-    e.ppt = round_up_pow2((n + 1023) / 1024);
-    if (fps_config_ok(e, n)) *c = e;
-}
-
-template <bool CLUSTERED, bool SORTED>
-int fps_launch_s(const FpsConfig& c, int b, int n, int m, int log2bs, const float* xyz,
-                 const float4* sorted, int32_t* idxs, cudaStream_t stream)
+int fps_launch_s(const FpsConfig& c, int b, int n, int m, int log2bs, const float* xyz, int32_t* idxs,
+                 cudaStream_t stream)
 {
     switch (c.ppt)
     {
-    case 1: return fps_launch_t<1, CLUSTERED, SORTED>(c, b, n, m, log2bs, xyz, sorted, idxs, stream);
-    case 2: return fps_launch_t<2, CLUSTERED, SORTED>(c, b, n, m, log2bs, xyz, sorted, idxs, stream);
-    case 4: return fps_launch_t<4, CLUSTERED, SORTED>(c, b, n, m, log2bs, xyz, sorted, idxs, stream);
-    case 8: return fps_launch_t<8, CLUSTERED, SORTED>(c, b, n, m, log2bs, xyz, sorted, idxs, stream);
-    case 16: return fps_launch_t<16, CLUSTERED, SORTED>(c, b, n, m, log2bs, xyz, sorted, idxs, stream);
-    case 32: return fps_launch_t<32, CLUSTERED, SORTED>(c, b, n, m, log2bs, xyz, sorted, idxs, stream);
+    case 1: return fps_launch_t<1, CLUSTERED>(c, b, n, m, log2bs, xyz, idxs, stream);
+    case 2: return fps_launch_t<2, CLUSTERED>(c, b, n, m, log2bs, xyz, idxs, stream);
+    case 4: return fps_launch_t<4, CLUSTERED>(c, b, n, m, log2bs, xyz, idxs, stream);
+    case 8: return fps_launch_t<8, CLUSTERED>(c, b, n, m, log2bs, xyz, idxs, stream);
+    case 16: return fps_launch_t<16, CLUSTERED>(c, b, n, m, log2bs, xyz, idxs, stream);
+    case 32: return fps_launch_t<32, CLUSTERED>(c, b, n, m, log2bs, xyz, idxs, stream);
     default: break;
     }
     set_error("fps: unsupported points per thread %d", c.ppt);
     return TPK_ERR_UNSUPPORTED;
 }
 
-// Which kernel family a call takes.  The sorted copy pays when a cloud has enough chunks for
-// most of them to be skipped and enough rounds to earn back the sort.  Test hooks:
-// "fps_global" (large-cloud kernels on any cloud), "fps_unsorted" (no sorted copy anywhere),
-// "fps_sorted" (sorted copy whatever the size).
+// Which kernel family a call takes.  One sample per exchange costs 0.26 us a sample on clouds of up
+// to 1024 points, 0.6 us at 16384; the rounds cost a sort and 20 to 60 rounds of 1.7 us and more,
+// whatever the number of samples (256 -> 64: 22 us against 41; 1024 -> 256: 67 against 70;
+// 2048 -> 512: 140 against 115).
+// Test hooks: "fps_global" (large-cloud kernels on any cloud), "fps_unsorted" (one sample per
+// exchange, no sorted copy anywhere), "fps_sorted" (the rounds whatever the size).
 enum FpsPath
 {
-    kFpsOnchip,        // cluster per cloud, registers, no scratch
-    kFpsOnchipSorted,  // cluster per cloud on the sorted copy (16 B/point)
-    kFpsPruned,        // large clouds on the sorted copy (20 B/point)
-    kFpsGlobal         // large clouds, unsorted (4 B/point)
+    kFpsOnchip,  // cluster per cloud, registers, one sample per exchange
+    kFpsRounds,  // cluster per cloud, rounds of independent samples (fps_rounds.cu)
+    kFpsPruned,  // large clouds on the sorted copy (20 B/point)
+    kFpsGlobal   // large clouds, unsorted (4 B/point)
 };
 
 FpsPath fps_pick_path(int n, int m, FpsConfig* c)
@@ -2029,8 +1241,8 @@ FpsPath fps_pick_path(int n, int m, FpsConfig* c)
         return (static_cast<long long>(n) <= kFpsPrunedMaxPoints && !test_path("fps_unsorted")) ? kFpsPruned
                                                                                                   : kFpsGlobal;
     if (test_path("fps_unsorted")) return kFpsOnchip;
-    const bool worth = test_path("fps_sorted") || (n >= 4096 && m >= 128);
-    return worth ? kFpsOnchipSorted : kFpsOnchip;
+    const bool rounds = test_path("fps_sorted") || (n > 1100 && m >= 48);
+    return rounds && fps_rounds_fits(n) ? kFpsRounds : kFpsOnchip;
 }
 
 }  // namespace
@@ -2043,18 +1255,21 @@ extern "C" int64_t tpk_fps_scratch_bytes(int b, int n, int m)
     switch (tpk::fps_pick_path(n, m, &c))
     {
     case tpk::kFpsOnchip: return 0;
-    // optional: the spatially sorted copy, (x, y, z, index) per point
-    case tpk::kFpsOnchipSorted: return static_cast<int64_t>(b) * n * 16;
+    // accepted and not used: the kernel sorts on chip (part of the interface since a kernel took a
+    // sorted copy of clouds of this size from here)
+    case tpk::kFpsRounds: return n >= 4096 && m >= 128 ? static_cast<int64_t>(b) * n * 16 : 0;
     // large clouds: the running minimum, one float per point, behind the sorted copy if one is used
     case tpk::kFpsPruned: return static_cast<int64_t>(b) * n * 20;
     default: return static_cast<int64_t>(b) * n * 4;
     }
 }
 
-extern "C" int tpk_furthest_point_sampling(int b, int n, int m, const float* xyz, void* scratch,
-                                           int64_t scratch_bytes, int32_t* idxs, void* stream)
+// new_xyz (optional): coordinates of the samples; *wrote_xyz tells whether the kernel wrote them
+static int fps_run(int b, int n, int m, const float* xyz, void* scratch, int64_t scratch_bytes, int32_t* idxs,
+                   float* new_xyz, bool* wrote_xyz, void* stream)
 {
     using namespace tpk;
+    *wrote_xyz = false;
     TPK_REQUIRE(b >= 0 && n >= 0 && m >= 0, "fps: negative size (b=%d n=%d m=%d)", b, n, m);
     if (b == 0 || m == 0) return TPK_OK;
     TPK_REQUIRE(n > 0, "fps: cannot sample %d points from an empty cloud", m);
@@ -2088,20 +1303,20 @@ extern "C" int tpk_furthest_point_sampling(int b, int n, int m, const float* xyz
         }
         return fps_launch_global(b, n, m, log2bs, xyz, static_cast<float*>(scratch), idxs, s);
     }
-    if (path != kFpsOnchip && scratch != nullptr && (reinterpret_cast<uintptr_t>(scratch) & 15u) == 0)
+    if (path == kFpsRounds)
     {
-        float4* sorted = static_cast<float4*>(scratch);
-        const int rc = fps_launch_sort(b, n, xyz, sorted, s);
-        if (rc != TPK_OK) return rc;
-        fps_batched_config(n, &c);
-        if (fps_wants_batched(c))
-            return c.nranks > 1 ? fps_launch_batched<true>(c, b, n, m, log2bs, xyz, sorted, idxs, s)
-                                : fps_launch_batched<false>(c, b, n, m, log2bs, xyz, sorted, idxs, s);
-        return c.nranks > 1 ? fps_launch_s<true, true>(c, b, n, m, log2bs, xyz, sorted, idxs, s)
-                            : fps_launch_s<false, true>(c, b, n, m, log2bs, xyz, sorted, idxs, s);
+        *wrote_xyz = true;
+        return fps_rounds(b, n, m, log2bs, xyz, idxs, new_xyz, s);
     }
-    return c.nranks > 1 ? fps_launch_s<true, false>(c, b, n, m, log2bs, xyz, nullptr, idxs, s)
-                        : fps_launch_s<false, false>(c, b, n, m, log2bs, xyz, nullptr, idxs, s);
+    return c.nranks > 1 ? fps_launch_s<true>(c, b, n, m, log2bs, xyz, idxs, s)
+                        : fps_launch_s<false>(c, b, n, m, log2bs, xyz, idxs, s);
+}
+
+extern "C" int tpk_furthest_point_sampling(int b, int n, int m, const float* xyz, void* scratch,
+                                           int64_t scratch_bytes, int32_t* idxs, void* stream)
+{
+    bool wrote_xyz;
+    return fps_run(b, n, m, xyz, scratch, scratch_bytes, idxs, nullptr, &wrote_xyz, stream);
 }
 
 // Coordinates of the samples, new_xyz[b, j, :] = xyz[b, idxs[b, j], :].  A separate pass of a
@@ -2131,8 +1346,9 @@ extern "C" int tpk_furthest_point_sampling_xyz(int b, int n, int m, const float*
                                                void* stream)
 {
     using namespace tpk;
-    const int rc = tpk_furthest_point_sampling(b, n, m, xyz, scratch, scratch_bytes, idxs, stream);
-    if (rc != TPK_OK || new_xyz == nullptr || b == 0 || m == 0) return rc;
+    bool wrote_xyz;
+    const int rc = fps_run(b, n, m, xyz, scratch, scratch_bytes, idxs, new_xyz, &wrote_xyz, stream);
+    if (rc != TPK_OK || new_xyz == nullptr || b == 0 || m == 0 || wrote_xyz) return rc;
     const long long total = static_cast<long long>(b) * m;
     const long long grid = (total + 255) / 256;
     TPK_REQUIRE(grid < (1ll << 31), "fps: too many samples");

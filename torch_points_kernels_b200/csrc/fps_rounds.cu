@@ -1,0 +1,1095 @@
+// Furthest point sampling by rounds of independent samples (sm_100a).
+//
+// The sequential algorithm picks the point with the largest running minimum, lowers the minima
+// around it, and starts over: m - 1 dependent steps.  Most of them do not depend on each other.
+// Write V(t) for the pair (running minimum of t, tie rank of t), ordered as the algorithm
+// orders its picks.  If no point u with V(u) above V(t) lies within its own running minimum of t,
+//
+//     there is no u with V(u) > V(t) and dist(u, t) < minimum(u),
+//
+// then t is a sample, its minimum at the moment it is picked is the one it has now, and picking it
+// early changes nothing for the points picked before it: minima only shrink, so whatever is picked
+// before t has a V above V(t) today already, does not touch t (dist >= its minimum >= that of t)
+// and is not touched by t.  All such points are taken in one round.  The order is recovered at the
+// end: running minima at pick time never increase along the sequence, so the samples sorted by V
+// are the sequence, and it is complete once m - 1 samples lie above every minimum that is left.
+//
+// A round only looks at the active points, those whose minimum is at least a fraction f of the
+// largest one.  16384 points, 4096 samples: 62 rounds with f = 0.8 (a CPU model of this scheme)
+// instead of 4095 dependent steps, with about 170 active points and 76 samples per round.
+//
+// One cluster of CTAs per cloud; a CTA holds its share of the points, in the order of a Hilbert curve, in
+// registers (PPT per lane).  A round is
+//   1. every warp lists its active points in the entry tables of all CTAs of the cluster and
+//      drops the lanes' best points that the strongest few of them block; cluster barrier;
+//   2. every point that is left is checked against all entries by one warp; what passes is a
+//      sample and goes to the sample tables of all CTAs; cluster barrier;
+//   3. every warp applies the samples that reach its bounding box.
+// The curve is Hilbert's because a run of it is connected: of 128 points in Morton order some lie
+// on both sides of an octant's face, and the warp with the worst box was reached by 42 samples per
+// round (7 to 10 in Hilbert order, mean 4.5), which is what the others waited for.
+// What bounds it is the latency of a round (two exchanges between the CTAs and the three dependent
+// phases, 9000 cycles at 16384 points and eight CTAs), not bandwidth or arithmetic.  Measured, B200,
+// one sample per dependent step before: 16384 -> 4096 one cloud 0.97 ms before, 0.29 now; 16 clouds
+// 1.08 and 0.40; 131072 -> 8192 7.3 and 0.94; a lattice of 20^3 (ties everywhere) 17.0 and 2.0.
+#include <climits>
+#include <cstdlib>
+#include <math_constants.h>
+
+#include <cooperative_groups.h>
+
+#include "fps_common.cuh"
+
+namespace cg = cooperative_groups;
+
+namespace tpk
+{
+TPK_DEFINE_STATUS_WORD()
+
+namespace
+{
+
+constexpr int kRoundsMaxRanks = 16;
+constexpr int kRoundsThreads = 512;
+constexpr int kRoundsStrongest = 4;  // of a warp's points, compared with its others before they go out
+constexpr int kRoundsBuckets = 4096;     // final order: 32 octaves of the minimum, 128 buckets each
+constexpr int kRoundsBucketShift = 16;   // 2^23 float images per octave / 128
+constexpr uint32_t kNoRank = 0xFFFFFFFFu;
+
+// Offsets into dynamic shared memory.  The sort of the points uses all of it before the rounds
+// begin; the list of the CTA's own samples outlives the tables of the rounds.
+struct RoundsLayout
+{
+    int per_warp;          // points per warp: chunk c of the sorted points goes to CTA c mod nranks
+    int share;             // points per CTA, per_warp * warps
+    int cap_entries;       // active points a CTA may list per round
+    int cap_picks;         // samples a CTA may take per round
+    int cells;             // cells of the spatial sort
+    int stage, hist, base, start;             // sort
+    int own, entries, picks, surv, surv_idx, mine_ent, mine_idx, mine_pick;  // rounds
+    int f_hist, f_base, f_start, f_sorted;    // final order
+    int bytes;
+};
+
+// What a CTA tells the others at the first barrier of a round.
+struct RoundsNote
+{
+    int entries;  // active points (may exceed the capacity: the round is repeated with fewer)
+    int top;      // largest running minimum, as the integer image of the float
+    int above;    // own samples above the largest minimum of the previous round
+    int pad;
+};
+
+__device__ __forceinline__ int ordered_image(float v)
+{
+    const int b = __float_as_int(v);
+    return b >= 0 ? b : b ^ 0x7FFFFFFF;
+}
+__device__ __forceinline__ float from_ordered(int o) { return __int_as_float(o >= 0 ? o : o ^ 0x7FFFFFFF); }
+
+// 16 bytes of shared memory of CTA r of the cluster.
+template <bool CLUSTERED>
+__device__ __forceinline__ int4 load_cluster(const int* p, int r)
+{
+    if constexpr (!CLUSTERED) return *reinterpret_cast<const int4*>(p);
+    int4 v;
+    asm volatile("ld.shared::cluster.v4.b32 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+                 : "r"(mapa_cluster(smem_u32(p), r))
+                 : "memory");
+    return v;
+}
+template <bool CLUSTERED>
+__device__ __forceinline__ void store_cluster(int* p, int r, int4 v)
+{
+    if constexpr (!CLUSTERED)
+        *reinterpret_cast<int4*>(p) = v;
+    else
+        asm volatile("st.shared::cluster.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(mapa_cluster(smem_u32(p), r)), "r"(v.x),
+                     "r"(v.y), "r"(v.z), "r"(v.w)
+                     : "memory");
+}
+
+template <int PPT, int NR>  // points per lane, CTAs per cloud
+__global__ void __launch_bounds__(kRoundsThreads, 1)
+    fps_rounds_kernel(int n, int m, int log2bs, int bits, RoundsLayout lay, const float* __restrict__ xyz_all,
+                      int32_t* __restrict__ idxs_all, float* __restrict__ new_xyz_all)
+{
+    extern __shared__ __align__(16) unsigned char smem[];
+    __shared__ RoundsNote s_note[2][kRoundsMaxRanks];  // by parity of the round: a fast CTA may be one round ahead
+    __shared__ int s_npicks_of[kRoundsMaxRanks];
+    __shared__ float s_box_of[kRoundsMaxRanks][8];
+    __shared__ float4 s_top_of[kRoundsMaxRanks];
+    __shared__ uint32_t s_toprank_of[kRoundsMaxRanks];
+    __shared__ int s_topidx_of[kRoundsMaxRanks];
+    __shared__ int s_scan[32];
+    __shared__ int s_slice_of[kRoundsMaxRanks];
+    __shared__ int s_box[6];
+    __shared__ int s_bad;
+    __shared__ int s_count[2], s_surv[2], s_npicks[2], s_max[2], s_above[2];  // by parity of the round
+    __shared__ __align__(8) uint64_t s_mbar[8];  // notes, entries, sample counts, samples: two of each
+    __shared__ uint32_t s_top;
+
+    constexpr int THREADS = kRoundsThreads, NW = THREADS / 32;
+    constexpr bool CLUSTERED = NR > 1;
+    constexpr int nranks = NR, lg_ranks = NR == 1 ? 0 : (NR == 2 ? 1 : (NR == 4 ? 2 : (NR == 8 ? 3 : 4)));
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int rank = CLUSTERED ? static_cast<int>(cluster_ctarank()) : 0;
+    const int cloud = blockIdx.x / nranks;
+    const float* xyz = xyz_all + static_cast<size_t>(cloud) * n * 3;
+    int32_t* idxs = idxs_all + static_cast<size_t>(cloud) * m;
+    float* new_xyz = new_xyz_all ? new_xyz_all + static_cast<size_t>(cloud) * m * 3 : nullptr;
+    const int per_warp = lay.per_warp;
+
+    // address of a variable of CTA r of the cluster
+    auto at_rank = [&](auto* p, int r) {
+        if constexpr (CLUSTERED)
+            return cg::this_cluster().map_shared_rank(p, static_cast<unsigned>(r));
+        else
+            return p;
+    };
+    auto sync_all = [&]() {
+        if constexpr (CLUSTERED)
+            cluster_sync_all();
+        else
+            __syncthreads();
+    };
+    auto block_scan_excl = [&](int v, int& total) -> int {  // all threads; uses s_scan
+        int incl = v;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1)
+        {
+            const int t = __shfl_up_sync(kFullMask, incl, o);
+            if (lane >= o) incl += t;
+        }
+        __syncthreads();
+        if (lane == 31) s_scan[warp] = incl;
+        __syncthreads();
+        if (warp == 0)
+        {
+            int w = lane < NW ? s_scan[lane] : 0;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1)
+            {
+                const int t = __shfl_up_sync(kFullMask, w, o);
+                if (lane >= o) w += t;
+            }
+            s_scan[lane] = w;
+        }
+        __syncthreads();
+        total = s_scan[31];
+        return (warp ? s_scan[warp - 1] : 0) + incl - v;
+    };
+    // hist: this CTA's counts of `cells` bins (complete in every CTA, cluster barrier passed).
+    // start[c] = first position of bin c over all CTAs, base[c] = what the CTAs before this one
+    // have in the bin.  A CTA adds up its part of the bins over all CTAs and hands the results back.
+    auto bin_positions = [&](int* hist, int* base, int* start, int cells) {
+        const int slice = cells / nranks;  // a multiple of four
+        const int c0 = rank * slice;
+        int before = 0;  // of the bins of this slice that earlier passes covered
+        for (int b = 0; b < slice; b += 4 * THREADS)
+        {
+            const int c = c0 + b + 4 * tid;
+            const bool in = b + 4 * tid < slice;
+            int4 tot = make_int4(0, 0, 0, 0);
+            if (in)
+            {
+                constexpr int BATCH = nranks < 4 ? nranks : 4;  // loads from so many CTAs in flight together
+#pragma unroll
+                for (int r0 = 0; r0 < nranks; r0 += BATCH)
+                {
+                    int4 v[BATCH];
+#pragma unroll
+                    for (int r = 0; r < BATCH; ++r) v[r] = load_cluster<CLUSTERED>(hist + c, r0 + r);
+#pragma unroll
+                    for (int r = 0; r < BATCH; ++r)
+                    {
+                        store_cluster<CLUSTERED>(base + c, r0 + r, tot);
+                        tot.x += v[r].x;
+                        tot.y += v[r].y;
+                        tot.z += v[r].z;
+                        tot.w += v[r].w;
+                    }
+                }
+            }
+            int total;
+            const int run = before + block_scan_excl(tot.x + tot.y + tot.z + tot.w, total);
+            before += total;
+            if (in)
+                *reinterpret_cast<int4*>(start + c) =
+                    make_int4(run, run + tot.x, run + tot.x + tot.y, run + tot.x + tot.y + tot.z);
+        }
+        if (nranks > 1)
+        {
+            if (tid < nranks) at_rank(&s_slice_of[0], tid)[rank] = before;
+            sync_all();
+            int offset = 0;
+#pragma unroll
+            for (int r = 0; r < nranks; ++r) offset += r < rank ? s_slice_of[r] : 0;
+            for (int c = c0 + 4 * tid; c < c0 + slice; c += 4 * THREADS)
+            {
+                int4 v = *reinterpret_cast<int4*>(start + c);
+                v = make_int4(v.x + offset, v.y + offset, v.z + offset, v.w + offset);
+#pragma unroll
+                for (int r = 0; r < nranks; ++r) store_cluster<CLUSTERED>(start + c, r, v);
+            }
+        }
+        sync_all();
+    };
+
+    // ------------------------------------------------ load, box, spatial sort across the cluster
+    float px[PPT], py[PPT], pz[PPT], md[PPT];
+    int pi[PPT];
+    if (tid < 3) s_box[tid] = INT_MAX;
+    if (tid >= 3 && tid < 6) s_box[tid] = INT_MIN;
+    if (tid == 0)
+    {
+        s_bad = 0;
+        for (int i = 0; i < 2; ++i)
+        {
+            s_count[i] = 0;
+            s_surv[i] = 0;
+            s_npicks[i] = 0;
+            s_max[i] = INT_MIN;
+            s_above[i] = 0;
+        }
+        if constexpr (CLUSTERED)
+        {
+            for (int i = 0; i < 8; ++i) mbar_init(smem_u32(&s_mbar[i]), 1);
+            asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        }
+        s_top = kNoRank;
+    }
+    int* hist = reinterpret_cast<int*>(smem + lay.hist);
+    int* base = reinterpret_cast<int*>(smem + lay.base);
+    int* start = reinterpret_cast<int*>(smem + lay.start);
+    for (int c = tid; c < lay.cells; c += THREADS) hist[c] = 0;
+    __syncthreads();
+    const int raw_share = (n + nranks - 1) / nranks;
+    const int raw0 = rank * raw_share;
+    const int nlocal = max(0, min(raw_share, n - raw0));
+    {
+        float lo[3] = {CUDART_INF_F, CUDART_INF_F, CUDART_INF_F};
+        float hi[3] = {-CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F};
+        bool bad = false;
+#pragma unroll
+        for (int g = 0; g < PPT; ++g)
+        {
+            const int k = g * THREADS + tid;
+            pi[g] = -1;
+            px[g] = py[g] = pz[g] = 0.f;
+            if (k < nlocal)
+            {
+                const float* src = xyz + 3 * static_cast<size_t>(raw0 + k);
+                pi[g] = raw0 + k;
+                px[g] = __ldg(src + 0);
+                py[g] = __ldg(src + 1);
+                pz[g] = __ldg(src + 2);
+                if (fabsf(px[g]) < 1.0e18f && fabsf(py[g]) < 1.0e18f && fabsf(pz[g]) < 1.0e18f)
+                {
+                    lo[0] = fminf(lo[0], px[g]);
+                    hi[0] = fmaxf(hi[0], px[g]);
+                    lo[1] = fminf(lo[1], py[g]);
+                    hi[1] = fmaxf(hi[1], py[g]);
+                    lo[2] = fminf(lo[2], pz[g]);
+                    hi[2] = fmaxf(hi[2], pz[g]);
+                }
+                else
+                    bad = true;  // not finite, or too large to square
+            }
+        }
+#pragma unroll
+        for (int a = 0; a < 3; ++a)
+        {
+            const int l = __reduce_min_sync(kFullMask, ordered_image(lo[a]));
+            const int h = __reduce_max_sync(kFullMask, ordered_image(hi[a]));
+            if (lane == 0)
+            {
+                atomicMin(&s_box[a], l);
+                atomicMax(&s_box[3 + a], h);
+            }
+        }
+        if (__any_sync(kFullMask, bad) && lane == 0) s_bad = 1;
+        __syncthreads();
+        for (int i = tid; i < nranks * 7; i += THREADS)
+        {
+            const int r = i / 7, a = i - r * 7;
+            at_rank(&s_box_of[0][0], r)[rank * 8 + a] = a < 6 ? from_ordered(s_box[a]) : static_cast<float>(s_bad);
+        }
+        sync_all();
+    }
+    bool sequential = false;
+    {
+        float lo[3] = {CUDART_INF_F, CUDART_INF_F, CUDART_INF_F};
+        float ext = 0.f;
+#pragma unroll
+        for (int a = 0; a < 3; ++a)
+        {
+            float h = -CUDART_INF_F;
+            for (int r = 0; r < nranks; ++r)
+            {
+                lo[a] = fminf(lo[a], s_box_of[r][a]);
+                h = fmaxf(h, s_box_of[r][3 + a]);
+            }
+            ext = fmaxf(ext, h - lo[a]);
+        }
+        for (int r = 0; r < nranks; ++r) sequential |= s_box_of[r][6] != 0.f;
+        const float qmax = static_cast<float>((1 << bits) - 1);
+        const float inv_h = (ext > 0.f && ext < CUDART_INF_F) ? static_cast<float>(1 << bits) * 0.999999f / ext : 0.f;
+        // fmaxf drops NaN, the clamp takes care of infinities: any cell is a correct cell
+        auto cell_of = [&](float x, float y, float z) -> int {
+            const uint32_t qx = static_cast<uint32_t>(fminf(fmaxf((x - lo[0]) * inv_h, 0.f), qmax));
+            const uint32_t qy = static_cast<uint32_t>(fminf(fmaxf((y - lo[1]) * inv_h, 0.f), qmax));
+            const uint32_t qz = static_cast<uint32_t>(fminf(fmaxf((z - lo[2]) * inv_h, 0.f), qmax));
+            return static_cast<int>(hilbert3(qx, qy, qz, bits));
+        };
+        int cell[PPT];
+#pragma unroll
+        for (int g = 0; g < PPT; ++g)
+        {
+            cell[g] = cell_of(px[g], py[g], pz[g]);
+            if (pi[g] >= 0) atomicAdd(&hist[cell[g]], 1);
+        }
+        sync_all();
+        bin_positions(hist, base, start, lay.cells);
+        float4* stage = reinterpret_cast<float4*>(smem + lay.stage);
+        int pos[PPT];
+#pragma unroll
+        for (int g = 0; g < PPT; ++g)
+            if (pi[g] >= 0) pos[g] = start[cell[g]] + atomicAdd(&base[cell[g]], 1);
+#pragma unroll
+        for (int g = 0; g < PPT; ++g)
+            if (pi[g] >= 0)
+            {
+                const int chunk = pos[g] / per_warp;
+                at_rank(stage, chunk & (nranks - 1))[(chunk >> lg_ranks) * per_warp + pos[g] - chunk * per_warp] =
+                    make_float4(px[g], py[g], pz[g], __int_as_float(pi[g]));
+            }
+        sync_all();
+        // A warp owns per_warp consecutive points.  Neighbouring chunks go to different CTAs: the
+        // active points of a round lie close together, and a round lasts as long as its busiest CTA.
+        const int left = n - (warp * nranks + rank) * per_warp;
+#pragma unroll
+        for (int g = 0; g < PPT; ++g)
+        {
+            const int o = g * 32 + lane, p = warp * per_warp + o;
+            pi[g] = -1;
+            px[g] = py[g] = pz[g] = 0.f;
+            md[g] = -1.0f;  // never a candidate, never updated
+            if (o < per_warp && o < left)
+            {
+                const float4 v = stage[p];
+                px[g] = v.x;
+                py[g] = v.y;
+                pz[g] = v.z;
+                pi[g] = __float_as_int(v.w);
+                if (!(static_cast<double>(sumsq_abc(v.x, v.y, v.z)) <= 1e-3)) md[g] = 1e10f;
+            }
+        }
+    }
+    // bounding box of the warp's candidates and the largest of their minima (integer image)
+    float wlo[3], whi[3];
+    int wmax = INT_MIN;
+    {
+        float lo[3] = {CUDART_INF_F, CUDART_INF_F, CUDART_INF_F}, hi[3] = {-CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F};
+#pragma unroll
+        for (int g = 0; g < PPT; ++g)
+        {
+            wmax = max(wmax, __float_as_int(md[g]));
+            const bool in = md[g] >= 0.f && fabsf(px[g]) < 1.0e18f && fabsf(py[g]) < 1.0e18f && fabsf(pz[g]) < 1.0e18f;
+            lo[0] = in ? fminf(lo[0], px[g]) : lo[0];
+            hi[0] = in ? fmaxf(hi[0], px[g]) : hi[0];
+            lo[1] = in ? fminf(lo[1], py[g]) : lo[1];
+            hi[1] = in ? fmaxf(hi[1], py[g]) : hi[1];
+            lo[2] = in ? fminf(lo[2], pz[g]) : lo[2];
+            hi[2] = in ? fmaxf(hi[2], pz[g]) : hi[2];
+        }
+#pragma unroll
+        for (int a = 0; a < 3; ++a)
+        {
+            wlo[a] = from_ordered(__reduce_min_sync(kFullMask, ordered_image(lo[a])));
+            whi[a] = from_ordered(__reduce_max_sync(kFullMask, ordered_image(hi[a])));
+        }
+        wmax = __reduce_max_sync(kFullMask, wmax);
+    }
+    // coordinates as pairs of points for the two-wide FP32 instructions
+    unsigned long long qx[PPT / 2], qy[PPT / 2], qz[PPT / 2];
+#pragma unroll
+    for (int g = 0; g < PPT / 2; ++g)
+    {
+        qx[g] = pack2(px[2 * g], px[2 * g + 1]);
+        qy[g] = pack2(py[2 * g], py[2 * g + 1]);
+        qz[g] = pack2(pz[2 * g], pz[2 * g + 1]);
+    }
+    auto coords = [&](int g, float& x, float& y, float& z) {
+        float o;
+        if (g & 1)
+        {
+            unpack2(qx[g / 2], o, x);
+            unpack2(qy[g / 2], o, y);
+            unpack2(qz[g / 2], o, z);
+        }
+        else
+        {
+            unpack2(qx[g / 2], x, o);
+            unpack2(qy[g / 2], y, o);
+            unpack2(qz[g / 2], z, o);
+        }
+    };
+
+    // Tables that all CTAs fill: item p of CTA r at r * capacity + p, the capacity one more than a
+    // multiple of eight.  Lane l reads items l / nranks, ... of CTA l mod nranks: no bank conflicts.
+    const int from = lane & (nranks - 1);
+    // Applies the samples of a table: `mine` of this lane's CTA, `places` = nranks * the most of any CTA.
+    auto apply = [&](const float4* list, int cap, int places, int mine) {
+        bool touched = false;
+        for (int i0 = 0; i0 < places; i0 += 32)
+        {
+            bool reach = false;
+            if ((i0 + lane) >> lg_ranks < mine)
+            {
+                const float4 s = list[from * cap + ((i0 + lane) >> lg_ranks)];
+                // same expression and rounding as a point's distance: never above that of a point in the box
+                reach = sumsq_abc(fmaxf(fmaxf(wlo[0] - s.x, s.x - whi[0]), 0.f), fmaxf(fmaxf(wlo[1] - s.y, s.y - whi[1]), 0.f),
+                                  fmaxf(fmaxf(wlo[2] - s.z, s.z - whi[2]), 0.f)) < __int_as_float(wmax);
+            }
+            uint32_t todo = __ballot_sync(kFullMask, reach);
+            touched |= todo != 0u;
+            while (todo != 0u)
+            {
+                // two samples at a time: one load latency and one chain of arithmetic for both
+                const int a = __ffs(todo) - 1;
+                todo &= todo - 1u;
+                const int b = todo != 0u ? __ffs(todo) - 1 : a;
+                todo &= todo - 1u;
+                const float4 s = list[(a & (nranks - 1)) * cap + ((i0 + a) >> lg_ranks)];
+                const float4 t = list[(b & (nranks - 1)) * cap + ((i0 + b) >> lg_ranks)];
+                const unsigned long long sx = pack2(-s.x, -s.x), sy = pack2(-s.y, -s.y), sz = pack2(-s.z, -s.z);
+                const unsigned long long tx = pack2(-t.x, -t.x), ty = pack2(-t.y, -t.y), tz = pack2(-t.z, -t.z);
+#pragma unroll
+                for (int g = 0; g < PPT / 2; ++g)
+                {
+                    const unsigned long long ax = add2(qx[g], sx), ay = add2(qy[g], sy), az = add2(qz[g], sz);
+                    const unsigned long long bx = add2(qx[g], tx), by = add2(qy[g], ty), bz = add2(qz[g], tz);
+                    const unsigned long long da = fma2(az, az, fma2(ax, ax, mul2(ay, ay)));
+                    const unsigned long long db = fma2(bz, bz, fma2(bx, bx, mul2(by, by)));
+                    float d0, d1, e0, e1;
+                    unpack2(da, d0, d1);
+                    unpack2(db, e0, e1);
+                    md[2 * g] = fminf(md[2 * g], fminf(d0, e0));
+                    md[2 * g + 1] = fminf(md[2 * g + 1], fminf(d1, e1));
+                }
+            }
+        }
+        if (touched)
+        {
+            int k = __float_as_int(md[0]);
+#pragma unroll
+            for (int g = 1; g < PPT; ++g) k = max(k, __float_as_int(md[g]));
+            wmax = __reduce_max_sync(kFullMask, k);
+        }
+    };
+    // The point with the largest V, M its minimum: everyone learns it; returns the CTA that holds it.
+    // Its coordinates are in s_top_of, its index in s_topidx_of of that CTA's slot.
+    auto find_top = [&](int top) -> int {
+        bool have = false;
+        if (wmax == top)
+        {
+            uint32_t mine = kNoRank;
+#pragma unroll
+            for (int g = 0; g < PPT; ++g)
+                if (__float_as_int(md[g]) == top) mine = min(mine, fps_rank(pi[g], log2bs));
+            have = mine != kNoRank;
+            if (have) atomicMin(&s_top, mine);
+        }
+        __syncthreads();
+        const uint32_t best = s_top;
+        if (best == kNoRank && tid < nranks) at_rank(&s_toprank_of[0], tid)[rank] = kNoRank;
+        if (have)
+        {
+#pragma unroll
+            for (int g = 0; g < PPT; ++g)
+                if (__float_as_int(md[g]) == top && fps_rank(pi[g], log2bs) == best)
+#pragma unroll 1
+                    for (int r = 0; r < nranks; ++r)
+                    {
+                        float x, y, z;
+                        coords(g, x, y, z);
+                        at_rank(&s_top_of[0], r)[rank] = make_float4(x, y, z, 0.f);
+                        at_rank(&s_topidx_of[0], r)[rank] = pi[g];
+                        at_rank(&s_toprank_of[0], r)[rank] = best;
+                    }
+        }
+        __syncthreads();
+        if (tid == 0) s_top = kNoRank;
+        sync_all();
+        int w = 0;
+        for (int r = 1; r < nranks; ++r)
+            if (s_toprank_of[r] < s_toprank_of[w]) w = r;
+        return w;
+    };
+
+    int2* own = reinterpret_cast<int2*>(smem + lay.own);  // this CTA's samples: (minimum, index)
+    float4* entries = reinterpret_cast<float4*>(smem + lay.entries);
+    float4* picks = reinterpret_cast<float4*>(smem + lay.picks);
+    float4* surv = reinterpret_cast<float4*>(smem + lay.surv);
+    int* surv_idx = reinterpret_cast<int*>(smem + lay.surv_idx);
+    // (a cloud in one CTA needs no exchange: its own lists are the tables)
+    float4* mine_ent = CLUSTERED ? reinterpret_cast<float4*>(smem + lay.mine_ent) : entries;
+    int* mine_idx = reinterpret_cast<int*>(smem + lay.mine_idx);  // read by the others where minima tie
+    float4* mine_pick = CLUSTERED ? reinterpret_cast<float4*>(smem + lay.mine_pick) : picks;
+
+    // sample 0 is point 0, candidate or not: the first pending sample (every thread writes the same value)
+    if (rank == 0 && tid == 0)
+    {
+        idxs[0] = 0;
+        if (new_xyz)
+            for (int a = 0; a < 3; ++a) new_xyz[a] = __ldg(xyz + a);
+    }
+    s_top_of[0] = make_float4(__ldg(xyz), __ldg(xyz + 1), __ldg(xyz + 2), 0.f);
+    sync_all();  // the staged points have been read everywhere: the tables may be written
+
+    // samples to apply at the head of the next round: a table filled by all CTAs, or one sample
+    const float4* pending = s_top_of;
+    int places = 1, my_places = lane == 0 ? 1 : 0;
+    int tau_key = INT_MAX;               // active: minimum above this image, or
+    uint32_t tau_rank = kNoRank - 1u;    // equal to it and tie rank at most this one
+    uint32_t rank_limit = kNoRank - 1u;
+    float gap = 0.05f;  // 1 - f
+    bool overflow_before = false;
+    int top_before = INT_MAX, first_top = 0, top = 0;
+    int taken = 0;  // samples so far, without the first
+    int fill = 0;   // index of every sample after the last one that changed a minimum
+    auto set_tau = [&]() {
+        // at least 1: a minimum of zero is a point that coincides with a sample
+        // ... and towards the end not below what the last sample will have (its minimum falls at most
+        // as fast as 1 / samples: planar clouds): samples beyond m are taken for nothing
+        const float part = fminf(static_cast<float>(taken) / static_cast<float>(m), 1.0f);
+        const float f = fmaxf(1.0f - gap, 0.9f * part);
+        tau_key = max(1, min(top, __float_as_int(f * __int_as_float(top))));
+        tau_rank = tau_key == top ? rank_limit : kNoRank - 1u;
+        top_before = top;
+    };
+    bool failed = false;  // a bounded wait ran out
+    int nown = 0;
+    uint32_t nexch = 0;  // exchanges of samples so far
+    for (uint32_t round = 0;; ++round)
+    {
+        const int par = round & 1u;
+        RoundsNote* notes = s_note[par];
+        // ---- 3 of the round before: apply its samples
+        apply(pending, lay.cap_picks, places, my_places);
+        // ---- 1: active points to every CTA of the cluster
+        if (!sequential && wmax >= tau_key)
+        {
+            uint32_t act[PPT];
+            int nact = 0;
+            int bk = -1, bi = 0;
+            float bx = 0.f, by = 0.f, bz = 0.f;
+#pragma unroll
+            for (int g = 0; g < PPT; ++g)
+            {
+                const int k = __float_as_int(md[g]);
+                const bool a = k > tau_key || (k == tau_key && fps_rank(pi[g], log2bs) <= tau_rank);
+                act[g] = __ballot_sync(kFullMask, a);
+                nact += __popc(act[g]);
+                if (a && (k > bk || (k == bk && fps_rank(pi[g], log2bs) < fps_rank(bi, log2bs))))
+                {
+                    bk = k;
+                    bi = pi[g];
+                    coords(g, bx, by, bz);
+                }
+            }
+            if (nact > 0)
+            {
+                int pos = 0;
+                if (lane == 0) pos = atomicAdd(&s_count[par], nact);
+                pos = __shfl_sync(kFullMask, pos, 0);
+#pragma unroll
+                for (int g = 0; g < PPT; ++g)
+                    if (act[g] != 0u)
+                    {
+                        const int p = pos + __popc(act[g] & ((1u << lane) - 1u));
+                        if ((act[g] >> lane & 1u) && p < lay.cap_entries)
+                        {
+                            float x, y, z;
+                            coords(g, x, y, z);
+                            mine_ent[p] = make_float4(x, y, z, md[g]);
+                            mine_idx[p] = pi[g];
+                        }
+                        pos += __popc(act[g]);
+                    }
+                // the strongest few of the lanes' best points against the others
+                bool open = bk >= 0;
+                uint32_t rest = __ballot_sync(kFullMask, open);
+                for (int step = 0; step < kRoundsStrongest && (rest & (rest - 1u)) != 0u; ++step)
+                {
+                    const bool in = rest >> lane & 1u;
+                    const int uk = __reduce_max_sync(kFullMask, in ? bk : -1);
+                    const int src = __ffs(__ballot_sync(kFullMask, in && bk == uk)) - 1;
+                    const float ux = __shfl_sync(kFullMask, bx, src), uy = __shfl_sync(kFullMask, by, src),
+                                uz = __shfl_sync(kFullMask, bz, src);
+                    // (a lane with the same minimum may come first by its rank: it stays open)
+                    if (in && bk < uk && sumsq_abc(ux - bx, uy - by, uz - bz) < __int_as_float(uk)) open = false;
+                    rest = __ballot_sync(kFullMask, in && open && lane != src);
+                }
+                const uint32_t left = __ballot_sync(kFullMask, open);
+                int sp = 0;
+                if (lane == 0) sp = atomicAdd(&s_surv[par], __popc(left));
+                sp = __shfl_sync(kFullMask, sp, 0) + __popc(left & ((1u << lane) - 1u));
+                if (open)
+                {
+                    surv[sp] = make_float4(bx, by, bz, __int_as_float(bk));
+                    surv_idx[sp] = bi;
+                }
+            }
+        }
+        if constexpr (CLUSTERED) fence_async_smem();  // the bulk copies read what this thread listed
+        if (lane == 0) atomicMax(&s_max[par], wmax);
+        if (!sequential && taken >= m - 1)
+        {
+            // enough samples: are m - 1 of them above all that is left?
+            int above = 0;
+            for (int i = tid; i < nown; i += THREADS) above += own[i].x > top_before ? 1 : 0;
+            above = __reduce_add_sync(kFullMask, above);
+            if (lane == 0 && above) atomicAdd(&s_above[par], above);
+        }
+        __syncthreads();
+        const int nsurv = s_surv[par];
+        const int nlisted = min(s_count[par], lay.cap_entries);
+        if (tid == 0)
+        {
+            // the other round's counters: read by everyone before the barrier above, used after the next one
+            s_count[par ^ 1] = 0;
+            s_surv[par ^ 1] = 0;
+            s_npicks[par ^ 1] = 0;
+            s_max[par ^ 1] = INT_MIN;
+            s_above[par ^ 1] = 0;
+        }
+        if constexpr (CLUSTERED)
+        {
+            // A note to every CTA, then the list in one bulk copy each; the note says how many bytes
+            // to wait for.  (Stores of single entries cost the receiver some cycles each: 3400 cycles
+            // per round at 276 entries and eight CTAs, with a cluster barrier or with st.async.)
+            const uint32_t mnote = smem_u32(&s_mbar[par]), ment = smem_u32(&s_mbar[2 + par]);
+            if (tid == 0) mbar_arrive_expect_tx(mnote, nranks * 16);
+            if (tid < nranks)
+            {
+                st_async_v4(mapa_cluster(smem_u32(&notes[rank]), tid), mapa_cluster(mnote, tid), s_count[par], s_max[par],
+                            s_above[par], 0);
+                if (nlisted > 0)
+                    bulk_to_cta(mapa_cluster(smem_u32(entries + rank * lay.cap_entries), tid), smem_u32(mine_ent),
+                                nlisted * 16, mapa_cluster(ment, tid));
+            }
+            bool ok = mbar_wait_bounded(mnote, round >> 1 & 1u);
+            int bytes = 0;
+            for (int r = 0; r < nranks; ++r) bytes += 16 * min(notes[r].entries, lay.cap_entries);
+            if (tid == 0) mbar_arrive_expect_tx(ment, bytes);
+            ok = ok && mbar_wait_bounded(ment, round >> 1 & 1u);
+            if (!__syncthreads_and(ok ? 1 : 0))
+            {
+                failed = true;
+                break;
+            }
+        }
+        else
+        {
+            if (tid == 0)
+            {
+                notes[0].entries = s_count[par];
+                notes[0].top = s_max[par];
+                notes[0].above = s_above[par];
+            }
+            __syncthreads();
+        }
+        int nentries = 0, above = 0, longest = 0;
+        bool overflow = false;
+        top = INT_MIN;
+        for (int r = 0; r < nranks; ++r)
+        {
+            nentries += notes[r].entries;
+            longest = max(longest, notes[r].entries);
+            top = max(top, notes[r].top);
+            above += notes[r].above;
+        }
+        overflow = longest > lay.cap_entries;
+        if (round == 0) first_top = top;
+        bool alone = overflow;  // take the first point in the order, nothing else
+        if (sequential)
+        {
+            if (top < 0 || taken >= m - 1) break;
+            alone = true;
+        }
+        else if (top <= 0 || (taken >= m - 1 && above >= m - 1))
+        {
+            if (top != 0 || taken >= m - 1) break;
+            alone = true;  // only points that coincide with a sample are left: the first of them, from now on
+        }
+        if (alone)
+        {
+            const int w = find_top(top);
+            const int k = s_topidx_of[w];
+            if (top == 0 && !sequential)
+            {
+                fill = k;
+                break;
+            }
+            taken += 1;
+            if (rank == w && !sequential)
+            {
+                if (tid == 0) own[nown] = make_int2(top, k);
+                nown += 1;
+            }
+            if (rank == 0 && tid == 0 && sequential)
+            {
+                idxs[taken] = k;
+                if (new_xyz)
+                    for (int a = 0; a < 3; ++a)
+                        new_xyz[3 * static_cast<size_t>(taken) + a] = __ldg(xyz + 3 * static_cast<size_t>(k) + a);
+            }
+            pending = s_top_of + w;
+            places = 1;
+            my_places = lane == 0 ? 1 : 0;
+        }
+        else
+            places = 0;
+        if (nentries == 0 || overflow || sequential)
+        {
+            // a lower threshold where nothing was listed, a higher one where it was too much
+            if (overflow)
+            {
+                if (tau_key >= top) rank_limit >>= 1;  // ties: list the first of them by rank
+                gap = overflow_before ? 0.f : 0.5f * gap;
+            }
+            else if (tau_key == top)
+                rank_limit = rank_limit * 2u + 1u;
+            overflow_before = overflow;
+            set_tau();
+            __syncthreads();  // list of own samples, counters
+            continue;
+        }
+        overflow_before = false;
+
+        // ---- 2: what no active point precedes and touches is a sample
+        const int my_entries = notes[from].entries;
+        constexpr int Q = 2;  // points a warp checks side by side
+        for (int s0 = warp * Q; s0 < nsurv; s0 += NW * Q)
+        {
+            float4 t[Q];
+            bool b[Q];
+            int same = 0;
+#pragma unroll
+            for (int q = 0; q < Q; ++q)
+            {
+                t[q] = surv[min(s0 + q, nsurv - 1)];
+                b[q] = false;
+            }
+            for (int at0 = lane; at0 < longest << lg_ranks; at0 += 128)
+            {
+                float4 e[4];
+#pragma unroll
+                for (int u = 0; u < 4; ++u)
+                {
+                    // beyond the list: an entry that touches nothing
+                    const int p = (at0 + 32 * u) >> lg_ranks;
+                    e[u] = entries[from * lay.cap_entries + min(p, lay.cap_entries - 1)];
+                    if (p >= my_entries) e[u].w = -1.0f;
+                }
+#pragma unroll
+                for (int u = 0; u < 4; ++u)
+#pragma unroll
+                    for (int q = 0; q < Q; ++q)
+                    {
+                        const bool near = sumsq_abc(e[u].x - t[q].x, e[u].y - t[q].y, e[u].z - t[q].z) < e[u].w;
+                        b[q] |= near && e[u].w > t[q].w;
+                        same += near && e[u].w == t[q].w ? 1 : 0;
+                    }
+            }
+            // every point meets itself; more than that is a tie to be decided by rank
+            uint32_t free_of = 0;
+#pragma unroll
+            for (int q = 0; q < Q; ++q)
+                if (!__any_sync(kFullMask, b[q]) && s0 + q < nsurv) free_of |= 1u << q;
+            if (__reduce_add_sync(kFullMask, same) > Q)
+#pragma unroll
+                for (int q = 0; q < Q; ++q)
+                    if (free_of >> q & 1u)
+                    {
+                        const uint32_t tr = fps_rank(surv_idx[s0 + q], log2bs);
+                        bool first = true;
+#pragma unroll 1
+                        for (int at = lane; at < longest << lg_ranks; at += 32)
+                        {
+                            if (at >> lg_ranks >= my_entries) continue;
+                            const float4 e = entries[from * lay.cap_entries + (at >> lg_ranks)];
+                            if (e.w == t[q].w && sumsq_abc(e.x - t[q].x, e.y - t[q].y, e.z - t[q].z) < e.w &&
+                                fps_rank(at_rank(mine_idx, from)[at >> lg_ranks], log2bs) < tr)
+                                first = false;
+                        }
+                        if (!__all_sync(kFullMask, first)) free_of &= ~(1u << q);
+                    }
+            if (free_of != 0u)
+            {
+                int p = 0;
+                if (lane == 0) p = atomicAdd(&s_npicks[par], __popc(free_of));
+                p = __shfl_sync(kFullMask, p, 0);
+                // beyond the capacity: it is still the first of its neighbourhood next round
+                if (lane < Q && (free_of >> lane & 1u))
+                {
+                    p += __popc(free_of & ((1u << lane) - 1u));
+                    if (p < lay.cap_picks)
+                    {
+                        const float4 v = surv[s0 + lane];
+                        mine_pick[p] = v;
+                        own[nown + p] = make_int2(__float_as_int(v.w), surv_idx[s0 + lane]);
+                    }
+                }
+            }
+        }
+        if constexpr (CLUSTERED) fence_async_smem();
+        __syncthreads();
+        const int np = min(s_npicks[par], lay.cap_picks);
+        nown += np;
+        if constexpr (CLUSTERED)
+        {
+            const uint32_t mcnt = smem_u32(&s_mbar[4 + (nexch & 1u)]), mpick = smem_u32(&s_mbar[6 + (nexch & 1u)]);
+            if (tid == 0) mbar_arrive_expect_tx(mcnt, nranks * 4);
+            if (tid < nranks) st_async_b32(mapa_cluster(smem_u32(&s_npicks_of[rank]), tid), mapa_cluster(mcnt, tid), np);
+            if (tid < nranks && np > 0)
+                bulk_to_cta(mapa_cluster(smem_u32(picks + rank * lay.cap_picks), tid), smem_u32(mine_pick), np * 16,
+                            mapa_cluster(mpick, tid));
+            bool ok = mbar_wait_bounded(mcnt, nexch >> 1 & 1u);
+            int bytes = 0;
+            for (int r = 0; r < nranks; ++r) bytes += 16 * s_npicks_of[r];
+            if (tid == 0) mbar_arrive_expect_tx(mpick, bytes);
+            ok = ok && mbar_wait_bounded(mpick, nexch >> 1 & 1u);
+            ++nexch;
+            if (!__syncthreads_and(ok ? 1 : 0))
+            {
+                failed = true;
+                break;
+            }
+        }
+        else
+        {
+            if (tid == 0) s_npicks_of[0] = np;
+            __syncthreads();
+        }
+        int most = 0;
+        for (int r = 0; r < nranks; ++r)
+        {
+            taken += s_npicks_of[r];
+            most = max(most, s_npicks_of[r]);
+        }
+        pending = picks;
+        places = most << lg_ranks;
+        my_places = s_npicks_of[from];
+        // more active points per round mean fewer rounds, but longer ones
+        if (nentries < 160)
+            gap = fminf(fmaxf(gap * 1.25f, 1.0e-3f), 0.5f);
+        else if (nentries > 384)
+            gap *= nentries > 768 ? 0.5f : 0.8f;
+        if (rank_limit < (kNoRank >> 1) && nentries * 4 < lay.cap_entries) rank_limit = rank_limit * 2u + 1u;
+        set_tau();
+    }
+
+    if (failed)
+    {
+        if (tid == 0) atomicOr(&g_dev_status, kStatusWaitAbandoned);
+        if constexpr (CLUSTERED) cluster_sync_all();
+        return;
+    }
+    // ------------------------------------------------ the samples in order
+    int* f_hist = reinterpret_cast<int*>(smem + lay.f_hist);
+    int* f_base = reinterpret_cast<int*>(smem + lay.f_base);
+    int* f_start = reinterpret_cast<int*>(smem + lay.f_start);
+    int2* f_sorted = reinterpret_cast<int2*>(smem + lay.f_sorted);
+    // (one sample after the other: they are in place already)
+    const int listed = sequential ? 0 : taken;
+    for (int c = tid; c < kRoundsBuckets; c += THREADS) f_hist[c] = 0;
+    __syncthreads();
+    auto bucket_of = [&](int key) { return max(0, min(kRoundsBuckets - 1, (first_top - key) >> kRoundsBucketShift)); };
+    const int mine = nown;
+    for (int i = tid; i < mine; i += THREADS) atomicAdd(&f_hist[bucket_of(own[i].x)], 1);
+    sync_all();
+    bin_positions(f_hist, f_base, f_start, kRoundsBuckets);
+    const int part = max(1, (listed + nranks - 1) / nranks);
+    for (int i = tid; i < mine; i += THREADS)
+    {
+        const int2 e = own[i];
+        const int b = bucket_of(e.x);
+        const int pos = f_start[b] + atomicAdd(&f_base[b], 1);
+        const int owner = pos / part;
+        at_rank(f_sorted, owner)[pos - owner * part] = e;
+    }
+    sync_all();
+    for (int i = rank * part + tid; i < min(listed, (rank + 1) * part); i += THREADS)
+    {
+        const int2 e = f_sorted[i - rank * part];
+        const int b = bucket_of(e.x);
+        const int lo = f_start[b], hi = b + 1 < kRoundsBuckets ? f_start[b + 1] : listed;
+        int before = lo;
+        if (lo >= m - 1) continue;
+        for (int q = lo / part; q * part < hi; ++q)
+        {
+            const int2* src = at_rank(f_sorted, q);
+            const int a = max(lo - q * part, 0), z = min(hi - q * part, part);
+            for (int j = a; j < z; ++j)
+            {
+                const int2 o = src[j];
+                before += o.x > e.x || (o.x == e.x && fps_rank(o.y, log2bs) < fps_rank(e.y, log2bs)) ? 1 : 0;
+            }
+        }
+        if (before < m - 1)
+        {
+            idxs[before + 1] = e.y;
+            if (new_xyz)
+                for (int a = 0; a < 3; ++a)
+                    new_xyz[3 * static_cast<size_t>(before + 1) + a] = __ldg(xyz + 3 * static_cast<size_t>(e.y) + a);
+        }
+    }
+    for (int j = taken + 1 + rank * THREADS + tid; j < m; j += nranks * THREADS)
+    {
+        idxs[j] = fill;
+        if (new_xyz)
+            for (int a = 0; a < 3; ++a) new_xyz[3 * static_cast<size_t>(j) + a] = __ldg(xyz + 3 * static_cast<size_t>(fill) + a);
+    }
+    if constexpr (CLUSTERED) cluster_sync_all();  // shared memory stays until every CTA has read it
+}
+
+template <int PPT, int NR>
+int launch_rounds(int b, int n, int m, int log2bs, int bits, const RoundsLayout& lay, const float* xyz, int32_t* idxs,
+                  float* new_xyz, cudaStream_t stream)
+{
+    auto kernel = fps_rounds_kernel<PPT, NR>;
+    prefer_max_shared(kernel);
+    cudaError_t err = cudaSuccess;
+    if (static_cast<size_t>(lay.bytes) > kDynSmemOptIn)
+        err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, lay.bytes);
+    if (err == cudaSuccess && NR > 8)
+        err = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    if (err != cudaSuccess)
+    {
+        set_error("fps: kernel attribute: %s", cudaGetErrorString(err));
+        return TPK_ERR_CUDA;
+    }
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(static_cast<unsigned>(b) * NR, 1, 1);
+    cfg.blockDim = dim3(kRoundsThreads, 1, 1);
+    cfg.dynamicSmemBytes = lay.bytes;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = NR;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = NR > 1 ? 1 : 0;
+    count_launches(1);
+    err = cudaLaunchKernelEx(&cfg, kernel, n, m, log2bs, bits, lay, xyz, idxs, new_xyz);
+    if (err != cudaSuccess)
+    {
+        set_error("fps launch (rounds, cluster %d x %d points per lane): %s", NR, PPT, cudaGetErrorString(err));
+        return TPK_ERR_CUDA;
+    }
+    return TPK_OK;
+}
+
+}  // namespace
+
+// Largest cloud the kernel takes: 16 CTAs of 512 threads with 16 points each.
+bool fps_rounds_fits(int n) { return n <= kRoundsMaxRanks * 512 * 16; }
+
+int fps_rounds(int b, int n, int m, int log2bs, const float* xyz, int32_t* idxs, float* new_xyz, cudaStream_t stream)
+{
+    // A round costs about 3300 + (points per CTA) in some unit, 1024 points being as good as fewer, and
+    // 148, 72, 32, 15, 7 clusters of 1, 2, 4, 8, 16 such CTAs run at once (measured, 512 threads with
+    // 128 registers: one CTA per SM).  16384 -> 4096, us: 8 CTAs 290 up to 15 clouds and 545 for 16,
+    // 4 CTAs 400 up to 32 clouds; 4096 -> 1024: 140 with 8 or 4 CTAs, 178 with 2, 228 with 1.
+    static const int kAtOnce[5] = {148, 72, 32, 15, 7};
+    int nranks = 0;
+    double least = 0.;
+    for (int l = 0; l < 5; ++l)
+    {
+        const int per_cta = (n + (1 << l) - 1) >> l;
+        if (per_cta > kRoundsThreads * (l == 4 ? 16 : 8)) continue;
+        const int waves = (b + kAtOnce[l] - 1) / kAtOnce[l];
+        const double cost = waves * (3300. + (per_cta > 1024 ? per_cta : 1024)) * (l == 4 ? 1.3 : 1.);
+        if (nranks == 0 || cost < least * 0.97)
+        {
+            nranks = 1 << l;
+            least = cost;
+        }
+    }
+    char text[64];
+    if (test_value("fps_config", text, sizeof(text)))
+    {
+        // test hook "fps_config=nranks:...": another cluster size for the same cloud
+        const int r = atoi(text);
+        if (r >= 1 && r <= kRoundsMaxRanks && (r & (r - 1)) == 0 && n <= r * kRoundsThreads * (r == 16 ? 16 : 8)) nranks = r;
+    }
+    const int threads = kRoundsThreads;
+    RoundsLayout lay = {};
+    lay.per_warp = (n + nranks * (threads / 32) - 1) / (nranks * (threads / 32));
+    lay.share = lay.per_warp * (threads / 32);
+    const int ppt = (lay.per_warp + 31) / 32;
+    int bits = 2;
+    while (bits < 4 && (4 << (3 * bits)) < n) ++bits;  // about four points per cell, at most 16^3 cells
+    lay.cells = 1 << (3 * bits);
+    lay.cap_entries = (nranks == 1 ? 2048 : (nranks == 2 ? 1024 : (nranks == 4 ? 512 : (nranks == 8 ? 384 : 256)))) + 1;
+    lay.cap_picks = (nranks >= 16 ? 64 : 1024 / nranks) + 1;
+    int at = 0;
+    auto take = [&](int bytes) {
+        const int o = at;
+        at += (bytes + 15) / 16 * 16;
+        return o;
+    };
+    lay.stage = take(lay.share * 16);
+    lay.hist = take(lay.cells * 4);
+    lay.base = take(lay.cells * 4);
+    lay.start = take(lay.cells * 4);
+    int most = at;
+    at = 0;
+    lay.own = take(lay.share * 8);
+    const int after_own = at;
+    lay.entries = take(nranks * lay.cap_entries * 16);
+    lay.picks = take(nranks * lay.cap_picks * 16);
+    lay.surv = take(threads * 16);
+    lay.surv_idx = take(threads * 4);
+    lay.mine_idx = take(lay.cap_entries * 4);
+    if (nranks > 1)
+    {
+        lay.mine_ent = take(lay.cap_entries * 16);
+        lay.mine_pick = take(lay.cap_picks * 16);
+    }
+    most = at > most ? at : most;
+    at = after_own;
+    lay.f_hist = take(kRoundsBuckets * 4);
+    lay.f_base = take(kRoundsBuckets * 4);
+    lay.f_start = take(kRoundsBuckets * 4);
+    lay.f_sorted = take(lay.share * 8);
+    most = at > most ? at : most;
+    lay.bytes = most;
+#define TPK_ROUNDS(P, R) \
+    if (nranks == R && ppt <= P) return launch_rounds<P, R>(b, n, m, log2bs, bits, lay, xyz, idxs, new_xyz, stream)
+    TPK_ROUNDS(2, 1);
+    TPK_ROUNDS(4, 1);
+    TPK_ROUNDS(8, 1);
+    TPK_ROUNDS(2, 2);
+    TPK_ROUNDS(4, 2);
+    TPK_ROUNDS(8, 2);
+    TPK_ROUNDS(2, 4);
+    TPK_ROUNDS(4, 4);
+    TPK_ROUNDS(8, 4);
+    TPK_ROUNDS(2, 8);
+    TPK_ROUNDS(4, 8);
+    TPK_ROUNDS(8, 8);
+    TPK_ROUNDS(4, 16);
+    TPK_ROUNDS(8, 16);
+    TPK_ROUNDS(16, 16);
+#undef TPK_ROUNDS
+    set_error("fps: unsupported cluster of %d with %d points per lane", nranks, ppt);
+    return TPK_ERR_UNSUPPORTED;
+}
+
+}  // namespace tpk
