@@ -168,6 +168,15 @@ def test_fps_scratch_kernel_tie_break_and_skip_rule(n, sorted_copy, monkeypatch)
     np.testing.assert_array_equal(npy(tpk.furthest_point_sample(cu(x), mm)), orc.fps(x, mm))
 
 
+@pytest.mark.parametrize("family", ["fps_sorted", "fps_sorted,fps_global", "fps_unsorted"])
+def test_fps_coordinates_too_large_for_a_box(family, monkeypatch):
+    data.use_paths(monkeypatch, family)
+    x = data.unit_ball(1, 3000, seed=9).numpy().copy()
+    x[0, 700] = (2e18, 0.0, 1.0)
+    x[0, 1700] = (-3e18, 1.0, 1.0)
+    np.testing.assert_array_equal(npy(tpk.furthest_point_sample(cu(x), 90)), orc.fps(x, 90))
+
+
 @pytest.mark.parametrize("B,N,m,env", [(3, 1000, 200, None), (2, 16384, 700, None), (2, 16384, 700, "fps_unsorted"),
                                        (1, 150000, 40, None), (1, 150000, 40, "fps_unsorted"), (4, 257, 257, None)])
 def test_fps_returns_sampled_coordinates(B, N, m, env, monkeypatch):

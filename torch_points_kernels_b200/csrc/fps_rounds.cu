@@ -450,7 +450,8 @@ __global__ void __launch_bounds__(kRoundsThreads, 1)
             {
                 const float4 s = list[from * cap + ((i0 + lane) >> lg_ranks)];
                 // same expression and rounding as a point's distance: never above that of a point in the box
-                reach = sumsq_abc(fmaxf(fmaxf(wlo[0] - s.x, s.x - whi[0]), 0.f), fmaxf(fmaxf(wlo[1] - s.y, s.y - whi[1]), 0.f),
+                // (which leaves out coordinates of 1e18 and more: then every warp is in reach)
+                reach = sequential || sumsq_abc(fmaxf(fmaxf(wlo[0] - s.x, s.x - whi[0]), 0.f), fmaxf(fmaxf(wlo[1] - s.y, s.y - whi[1]), 0.f),
                                   fmaxf(fmaxf(wlo[2] - s.z, s.z - whi[2]), 0.f)) < __int_as_float(wmax);
             }
             uint32_t todo = __ballot_sync(kFullMask, reach);
