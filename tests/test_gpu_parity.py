@@ -168,6 +168,24 @@ def test_fps_scratch_kernel_tie_break_and_skip_rule(n, sorted_copy, monkeypatch)
     np.testing.assert_array_equal(npy(tpk.furthest_point_sample(cu(x), mm)), orc.fps(x, mm))
 
 
+@pytest.mark.parametrize("n,m,ranks", [(1500, 1500, 8), (33000, 9000, 16), (33000, 3000, 1), (70001, 2000, 1),
+                                       (140000, 700, 1), (140000, 5000, 2)])
+@pytest.mark.parametrize("kind", ["mixture", "lattice"])
+def test_fps_large_rounds_every_chunk_size(n, m, ranks, kind, monkeypatch):
+    """One, two and four points per lane, one and several groups of chunks per warp, chunks as entries
+    and points as entries, lists that overflow (ties), samples up to the last point."""
+    data.use_paths(monkeypatch, "fps_global", "fps_config=%d" % ranks)
+    if kind == "lattice":
+        x = np.random.default_rng(n).integers(1, 40, (1, n, 3)).astype(np.float32) / 8
+        m = min(m, 1000)
+    else:
+        x = data.gaussian_mixture(1, n, seed=n).numpy()
+    got, xyz = tpk.furthest_point_sample(cu(x), m, return_xyz=True)
+    np.testing.assert_array_equal(npy(got), orc.fps(x, m))
+    np.testing.assert_array_equal(npy(xyz), np.take_along_axis(x, npy(got).astype(np.int64)[..., None], 1))
+    assert _lib.device_status() == 0
+
+
 @pytest.mark.parametrize("family", ["fps_sorted", "fps_sorted,fps_global", "fps_unsorted"])
 def test_fps_coordinates_too_large_for_a_box(family, monkeypatch):
     data.use_paths(monkeypatch, family)

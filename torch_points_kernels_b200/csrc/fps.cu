@@ -33,6 +33,11 @@ TPK_DEFINE_STATUS_WORD()
 bool fps_rounds_fits(int n);
 int fps_rounds(int b, int n, int m, int log2bs, const float* xyz, int32_t* idxs, float* new_xyz, cudaStream_t stream);
 
+// fps_large.cu
+bool fps_large_fits(long long n);
+int fps_large(int b, int n, int m, int log2bs, const float* xyz, void* scratch, int32_t* idxs, float* new_xyz,
+              cudaStream_t stream);
+
 namespace
 {
 
@@ -343,163 +348,6 @@ __global__ void __launch_bounds__(fps_max_threads(PPT), 1)
     if (CLUSTERED) cluster_sync_all();
 }
 
-// ---------------------------------------------------------------- spatial sort
-//
-// Copy of every cloud in Morton order of a 2^bits-per-axis grid over its bounding box,
-// as (x, y, z, original index): one CTA per cloud, counting sort with the cell counters
-// in shared memory.  The order inside a cell is whatever the atomics give; the sampling
-// kernel's result does not depend on it.
-constexpr int kSortThreads = 1024;
-
-__global__ void __launch_bounds__(kSortThreads)
-    fps_sort_kernel(int n, int bits, const float* __restrict__ xyz_all, float4* __restrict__ sorted_all)
-{
-    extern __shared__ int cnt[];  // 8^bits counters
-    __shared__ float s_min[3][kSortThreads / 32], s_max[3][kSortThreads / 32];
-    __shared__ int s_warp[kSortThreads / 32];
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const float* xyz = xyz_all + static_cast<size_t>(blockIdx.x) * n * 3;
-    float4* sorted = sorted_all + static_cast<size_t>(blockIdx.x) * n;
-    const int ncell = 1 << (3 * bits);
-
-    float mn[3] = {CUDART_INF_F, CUDART_INF_F, CUDART_INF_F};
-    float mx[3] = {-CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F};
-    for (int k = tid; k < n; k += kSortThreads)
-    {
-#pragma unroll
-        for (int a = 0; a < 3; ++a)
-        {
-            const float v = __ldg(xyz + 3 * static_cast<size_t>(k) + a);
-            if (fabsf(v) < 1.0e18f)  // the box of the finite coordinates
-            {
-                mn[a] = fminf(mn[a], v);
-                mx[a] = fmaxf(mx[a], v);
-            }
-        }
-    }
-#pragma unroll
-    for (int a = 0; a < 3; ++a)
-    {
-#pragma unroll
-        for (int o = 16; o >= 1; o >>= 1)
-        {
-            mn[a] = fminf(mn[a], __shfl_xor_sync(kFullMask, mn[a], o));
-            mx[a] = fmaxf(mx[a], __shfl_xor_sync(kFullMask, mx[a], o));
-        }
-        if (lane == 0)
-        {
-            s_min[a][warp] = mn[a];
-            s_max[a][warp] = mx[a];
-        }
-    }
-    for (int c = tid; c < ncell; c += kSortThreads) cnt[c] = 0;
-    __syncthreads();
-    float ext = 0.f;
-#pragma unroll
-    for (int a = 0; a < 3; ++a)
-    {
-        float lo = s_min[a][0], hi = s_max[a][0];
-        for (int w = 1; w < kSortThreads / 32; ++w)
-        {
-            lo = fminf(lo, s_min[a][w]);
-            hi = fmaxf(hi, s_max[a][w]);
-        }
-        mn[a] = lo;
-        ext = fmaxf(ext, hi - lo);
-    }
-    const float qmax = static_cast<float>((1 << bits) - 1);
-    const float inv_h = (ext > 0.f && ext < CUDART_INF_F) ? static_cast<float>(1 << bits) * 0.999999f / ext : 0.f;
-    auto cell_of_point = [&](float x, float y, float z) -> int {
-        // fmaxf drops NaN, the clamp takes care of infinities: any cell is a correct cell
-        const uint32_t qx = static_cast<uint32_t>(fminf(fmaxf((x - mn[0]) * inv_h, 0.f), qmax));
-        const uint32_t qy = static_cast<uint32_t>(fminf(fmaxf((y - mn[1]) * inv_h, 0.f), qmax));
-        const uint32_t qz = static_cast<uint32_t>(fminf(fmaxf((z - mn[2]) * inv_h, 0.f), qmax));
-        return static_cast<int>(spread3(qx) | (spread3(qy) << 1) | (spread3(qz) << 2));
-    };
-
-    for (int k = tid; k < n; k += kSortThreads)
-    {
-        const float x = __ldg(xyz + 3 * static_cast<size_t>(k) + 0);
-        const float y = __ldg(xyz + 3 * static_cast<size_t>(k) + 1);
-        const float z = __ldg(xyz + 3 * static_cast<size_t>(k) + 2);
-        atomicAdd(&cnt[cell_of_point(x, y, z)], 1);
-    }
-    __syncthreads();
-
-    // exclusive prefix sum of the counters: a run of cells per thread, then the runs' totals
-    const int per = ncell >= kSortThreads ? ncell / kSortThreads : 1;
-    const int c0 = tid * per;
-    int sum = 0;
-    if (c0 < ncell)
-        for (int c = c0; c < c0 + per; ++c) sum += cnt[c];
-    int incl = sum;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1)
-    {
-        const int t = __shfl_up_sync(kFullMask, incl, o);
-        if (lane >= o) incl += t;
-    }
-    if (lane == 31) s_warp[warp] = incl;
-    __syncthreads();
-    if (warp == 0)
-    {
-        int w = s_warp[lane];
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1)
-        {
-            const int t = __shfl_up_sync(kFullMask, w, o);
-            if (lane >= o) w += t;
-        }
-        s_warp[lane] = w;
-    }
-    __syncthreads();
-    int run = (warp ? s_warp[warp - 1] : 0) + incl - sum;
-    if (c0 < ncell)
-        for (int c = c0; c < c0 + per; ++c)
-        {
-            const int v = cnt[c];
-            cnt[c] = run;
-            run += v;
-        }
-    __syncthreads();
-
-    for (int k = tid; k < n; k += kSortThreads)
-    {
-        const float x = __ldg(xyz + 3 * static_cast<size_t>(k) + 0);
-        const float y = __ldg(xyz + 3 * static_cast<size_t>(k) + 1);
-        const float z = __ldg(xyz + 3 * static_cast<size_t>(k) + 2);
-        const int pos = atomicAdd(&cnt[cell_of_point(x, y, z)], 1);
-        sorted[pos] = make_float4(x, y, z, __int_as_float(k));
-    }
-}
-
-// about four points per cell, at most 32^3 cells (128 KB of counters)
-int fps_sort_bits(int n)
-{
-    int bits = 1;
-    while (bits < 5 && (1ll << (3 * bits)) * 4 < n) ++bits;
-    return bits;
-}
-
-int fps_launch_sort(int b, int n, const float* xyz, float4* sorted, cudaStream_t stream)
-{
-    const int bits = fps_sort_bits(n);
-    const size_t smem = sizeof(int) << (3 * bits);
-    prefer_max_shared(fps_sort_kernel);
-    if (smem > kDynSmemOptIn)
-    {
-        cudaError_t err = cudaFuncSetAttribute(fps_sort_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                               static_cast<int>(smem));
-        if (err != cudaSuccess)
-        {
-            set_error("fps sort: shared memory attribute: %s", cudaGetErrorString(err));
-            return TPK_ERR_CUDA;
-        }
-    }
-    count_launches(1), fps_sort_kernel<<<b, kSortThreads, smem, stream>>>(n, bits, xyz, sorted);
-    return check_launch("fps sort");
-}
-
 // ---------------------------------------------------------------- large clouds
 //
 // Clouds too large for the register-resident kernel: one 16-CTA cluster of 512-thread
@@ -689,317 +537,6 @@ __global__ void __launch_bounds__(kFpsBigThreads, 1)
     cluster_sync_all();
 }
 
-// ---------------------------------------------------------------- large clouds, sorted
-//
-// The same clouds on a spatially sorted copy.  The copy is cut into chunks of 128
-// consecutive points (a compact region each); lane c of a warp keeps, in registers, the
-// bounding box of the warp's chunk c, the chunk's largest running minimum and the point
-// that holds it.  A round tests every chunk's box against the new sample: a chunk farther
-// away than its largest minimum cannot change and is skipped.  The few chunks in reach are
-// updated by their whole warp (four points per lane: coordinates from the sorted copy,
-// minima from scratch, written back only where they changed).  Late rounds touch a few
-// kilobytes per cloud instead of the whole cloud.
-constexpr int kFpsChunk = 128;  // points per chunk: 32 lanes x 4
-
-template <int CPL>  // chunks per lane: a warp owns 32 * CPL chunks
-__global__ void __launch_bounds__(kFpsBigThreads, 1)
-    fps_pruned_kernel(int n, int m, int log2bs, const float* __restrict__ xyz_all,
-                      const float4* __restrict__ sorted_all, float* __restrict__ temp_all,
-                      int32_t* __restrict__ idxs_all)
-{
-    __shared__ __align__(16) uint4 wmsg_a[64];
-    __shared__ __align__(16) uint4 cmsg_a[64];
-    __shared__ float wmsg_z[64];
-    __shared__ float cmsg_z[64];
-    __shared__ __align__(8) uint64_t mbar[2];
-
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int nwarps = kFpsBigThreads / 32;
-    const int nranks = static_cast<int>(cluster_nctarank());
-    const int rank = static_cast<int>(cluster_ctarank());
-    const int cloud = blockIdx.x / nranks;
-    const int gtid = rank * kFpsBigThreads + tid;
-
-    const float* xyz = xyz_all + static_cast<size_t>(cloud) * n * 3;
-    const float4* sorted = sorted_all + static_cast<size_t>(cloud) * n;
-    float* temp = temp_all + static_cast<size_t>(cloud) * n;
-    int32_t* idxs = idxs_all + static_cast<size_t>(cloud) * m;
-
-    // Chunk (slot s, lane c) of warp w is chunk (s * 32 + c) * total_warps + w of the cloud:
-    // neighbouring chunks belong to different warps, so the handful of chunks a sample
-    // reaches are updated side by side instead of one after the other.
-    const long long gwarp = static_cast<long long>(rank) * nwarps + warp;
-    const long long total_warps = static_cast<long long>(nranks) * nwarps;
-    float bmin[CPL][3], bmax[CPL][3], cmax[CPL], bx[CPL], by[CPL], bz[CPL];
-    int bk[CPL];
-#pragma unroll
-    for (int s = 0; s < CPL; ++s)
-    {
-        float kmin[3] = {CUDART_INF_F, CUDART_INF_F, CUDART_INF_F};
-        float kmax[3] = {-CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F};
-        cmax[s] = -1.0f;
-        bk[s] = 0;
-        bx[s] = by[s] = bz[s] = 0.f;
-        for (int c = 0; c < 32; ++c)
-        {
-            const long long base = (static_cast<long long>(s * 32 + c) * total_warps + gwarp) * kFpsChunk;
-            if (base >= n) break;  // warp-uniform
-            float lo[3] = {CUDART_INF_F, CUDART_INF_F, CUDART_INF_F};
-            float hi[3] = {-CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F};
-            bool any_valid = false;
-#pragma unroll
-            for (int u = 0; u < kFpsChunk / 32; ++u)
-            {
-                const long long p = base + u * 32 + lane;
-                if (p < n)
-                {
-                    const float4 v = __ldg(sorted + p);
-                    const float mag = sumsq_abc(v.x, v.y, v.z);
-                    const bool valid = !(static_cast<double>(mag) <= 1e-3);
-                    temp[p] = valid ? 1e10f : -1.0f;
-                    any_valid |= valid;
-                    // fminf/fmaxf drop NaN: such a point never changes its minimum anyway
-                    lo[0] = fminf(lo[0], v.x);
-                    lo[1] = fminf(lo[1], v.y);
-                    lo[2] = fminf(lo[2], v.z);
-                    hi[0] = fmaxf(hi[0], v.x);
-                    hi[1] = fmaxf(hi[1], v.y);
-                    hi[2] = fmaxf(hi[2], v.z);
-                }
-            }
-#pragma unroll
-            for (int a = 0; a < 3; ++a)
-#pragma unroll
-                for (int o = 16; o >= 1; o >>= 1)
-                {
-                    lo[a] = fminf(lo[a], __shfl_xor_sync(kFullMask, lo[a], o));
-                    hi[a] = fmaxf(hi[a], __shfl_xor_sync(kFullMask, hi[a], o));
-                }
-            const bool chunk_valid = __any_sync(kFullMask, any_valid) != 0;
-            if (lane == c)
-            {
-#pragma unroll
-                for (int a = 0; a < 3; ++a)
-                {
-                    kmin[a] = lo[a];
-                    kmax[a] = hi[a];
-                }
-                cmax[s] = chunk_valid ? 1e10f : -1.0f;  // every chunk with a candidate is updated in round 1
-            }
-        }
-#pragma unroll
-        for (int a = 0; a < 3; ++a)
-        {
-            bmin[s][a] = kmin[a];
-            bmax[s][a] = kmax[a];
-        }
-    }
-
-    float cx = __ldg(xyz + 0), cy = __ldg(xyz + 1), cz = __ldg(xyz + 2);
-    if (gtid == 0 && m > 0) idxs[0] = 0;
-    if (tid == 0)
-    {
-        mbar_init(smem_u32(mbar + 0), 1);
-        mbar_init(smem_u32(mbar + 1), 1);
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    }
-    cluster_sync_all();
-
-    uint32_t rem_a[2] = {0, 0}, rem_z[2] = {0, 0}, rem_bar[2] = {0, 0};
-    if (warp == 0 && lane < nranks)
-    {
-#pragma unroll
-        for (int par = 0; par < 2; ++par)
-        {
-            rem_a[par] = mapa_cluster(smem_u32(cmsg_a + par * 32 + rank), lane);
-            rem_z[par] = mapa_cluster(smem_u32(cmsg_z + par * 32 + rank), lane);
-            rem_bar[par] = mapa_cluster(smem_u32(mbar + par), lane);
-        }
-    }
-    bool failed = false;
-    Msg wm = {INT_MIN, 0, 0.f, 0.f, 0.f};  // the warp's winner, recomputed when a chunk of it changed
-
-    for (int j = 1; j < m; ++j)
-    {
-        const int par = j & 1;
-        if (tid == 0)
-            mbar_arrive_expect_tx(smem_u32(mbar + par), static_cast<uint32_t>(nranks * kMsgBytes));
-
-        // ---- chunks in reach of the new sample
-        bool touched = false;
-#pragma unroll
-        for (int s = 0; s < CPL; ++s)
-        {
-            const float ex = fmaxf(fmaxf(bmin[s][0] - cx, cx - bmax[s][0]), 0.f);
-            const float ey = fmaxf(fmaxf(bmin[s][1] - cy, cy - bmax[s][1]), 0.f);
-            const float ez = fmaxf(fmaxf(bmin[s][2] - cz, cz - bmax[s][2]), 0.f);
-            const float lb = __fmaf_rn(ez, ez, __fmaf_rn(ex, ex, __fmul_rn(ey, ey)));
-            // a computed distance is at least this bound less a few ulp; no skipping on tiny
-            // bounds, where it may have lost precision.  A chunk without candidates
-            // (largest minimum -1) is skipped whenever the bound is positive or its box is empty.
-            const bool in_reach = !(__fmul_rn(lb, 0.9999f) > fmaxf(cmax[s], 1.0e-30f));
-            uint32_t todo = __ballot_sync(kFullMask, in_reach);
-            touched |= todo != 0u;
-            while (todo != 0u)  // warp-uniform
-            {
-                const int c = __ffs(todo) - 1;
-                todo &= todo - 1u;
-                const long long base = (static_cast<long long>(s * 32 + c) * total_warps + gwarp) * kFpsChunk;
-                float4 v[kFpsChunk / 32];
-                float t[kFpsChunk / 32];
-#pragma unroll
-                for (int u = 0; u < kFpsChunk / 32; ++u)
-                {
-                    const long long p = base + u * 32 + lane;
-                    const bool ok = p < n;
-                    v[u] = ok ? __ldg(sorted + p) : make_float4(0.f, 0.f, 0.f, 0.f);
-                    t[u] = ok ? temp[p] : -1.0f;
-                }
-                float best = -1.0f, mx = 0.f, my = 0.f, mz = 0.f;
-                int mk = 0;
-                uint32_t mrank = 0xFFFFFFFFu;
-#pragma unroll
-                for (int u = 0; u < kFpsChunk / 32; ++u)
-                {
-                    const float d = fminf(sumsq_abc(v[u].x - cx, v[u].y - cy, v[u].z - cz), t[u]);
-                    if (d < t[u]) temp[base + u * 32 + lane] = d;
-                    // among equal minima the original index decides (tie rank)
-                    const int k = __float_as_int(v[u].w);
-                    bool better = d > best;
-                    if (d == best && d >= 0.f)
-                    {
-                        if (mrank == 0xFFFFFFFFu) mrank = fps_rank(mk, log2bs);
-                        better = fps_rank(k, log2bs) < mrank;
-                    }
-                    if (better)
-                    {
-                        best = d;
-                        mk = k;
-                        mx = v[u].x;
-                        my = v[u].y;
-                        mz = v[u].z;
-                        mrank = 0xFFFFFFFFu;
-                    }
-                }
-                const int key = __float_as_int(best);
-                const int src = warp_argmax(key, mk, log2bs);
-                const int wkey = __shfl_sync(kFullMask, key, src);
-                const int wk = __shfl_sync(kFullMask, mk, src);
-                const float wx = __shfl_sync(kFullMask, mx, src);
-                const float wy = __shfl_sync(kFullMask, my, src);
-                const float wz = __shfl_sync(kFullMask, mz, src);
-                if (lane == c)
-                {
-                    cmax[s] = __int_as_float(wkey);
-                    bk[s] = wk;
-                    bx[s] = wx;
-                    by[s] = wy;
-                    bz[s] = wz;
-                }
-            }
-        }
-
-        // ---- stage 1: the warp's winner over its chunks (unchanged if no chunk was touched)
-        if (touched)  // warp-uniform
-        {
-            float best = cmax[0], x1 = bx[0], y1 = by[0], z1 = bz[0];
-            int k1 = bk[0];
-#pragma unroll
-            for (int s = 1; s < CPL; ++s)
-            {
-                bool better = cmax[s] > best;
-                if (cmax[s] == best && best >= 0.f) better = fps_rank(bk[s], log2bs) < fps_rank(k1, log2bs);
-                if (better)
-                {
-                    best = cmax[s];
-                    k1 = bk[s];
-                    x1 = bx[s];
-                    y1 = by[s];
-                    z1 = bz[s];
-                }
-            }
-            const int key = __float_as_int(best);
-            const int src = warp_argmax(key, k1, log2bs);
-            wm.key = __shfl_sync(kFullMask, key, src);
-            wm.k = __shfl_sync(kFullMask, k1, src);
-            wm.x = __shfl_sync(kFullMask, x1, src);
-            wm.y = __shfl_sync(kFullMask, y1, src);
-            wm.z = __shfl_sync(kFullMask, z1, src);
-        }
-        if (lane == 0)
-        {
-            wmsg_a[par * 32 + warp] = make_uint4(static_cast<uint32_t>(wm.key), static_cast<uint32_t>(wm.k),
-                                                 __float_as_uint(wm.x), __float_as_uint(wm.y));
-            wmsg_z[par * 32 + warp] = wm.z;
-        }
-        __syncthreads();
-
-        // ---- stage 2: CTA
-        Msg msg;
-        {
-            int key2 = INT_MIN, k2 = 0;
-            float x2 = 0.f, y2 = 0.f, z2 = 0.f;
-            if (lane < nwarps)
-            {
-                const uint4 a = wmsg_a[par * 32 + lane];
-                key2 = static_cast<int>(a.x);
-                k2 = static_cast<int>(a.y);
-                x2 = __uint_as_float(a.z);
-                y2 = __uint_as_float(a.w);
-                z2 = wmsg_z[par * 32 + lane];
-            }
-            const int src = warp_argmax(key2, k2, log2bs);
-            msg.key = __shfl_sync(kFullMask, key2, src);
-            msg.k = __shfl_sync(kFullMask, k2, src);
-            msg.x = __shfl_sync(kFullMask, x2, src);
-            msg.y = __shfl_sync(kFullMask, y2, src);
-            msg.z = __shfl_sync(kFullMask, z2, src);
-        }
-
-        // ---- stage 3: cluster
-        if (nranks > 1)
-        {
-            if (warp == 0 && lane < nranks)
-                st_async_msg(rem_a[par], rem_z[par], rem_bar[par], static_cast<uint32_t>(msg.key),
-                             static_cast<uint32_t>(msg.k), msg.x, msg.y, msg.z);
-            // a warp whose wait ran out records it and stops waiting but keeps taking part
-            // in every barrier and exchange (see the on-chip kernel)
-            const uint32_t parity = static_cast<uint32_t>((j - 1) >> 1) & 1u;
-            if (!failed && !mbar_wait_bounded(smem_u32(mbar + par), parity))
-            {
-                if (lane == 0) atomicOr(&g_dev_status, kStatusWaitAbandoned);
-                failed = true;
-            }
-            int key3 = INT_MIN, k3 = 0;
-            if (lane < nranks)
-            {
-                const uint2 a = *reinterpret_cast<const uint2*>(cmsg_a + par * 32 + lane);
-                key3 = static_cast<int>(a.x);
-                k3 = static_cast<int>(a.y);
-            }
-            const int src = warp_argmax(key3, k3, log2bs);
-            const uint4 win = cmsg_a[par * 32 + src];
-            msg.key = static_cast<int>(win.x);
-            msg.k = static_cast<int>(win.y);
-            msg.x = __uint_as_float(win.z);
-            msg.y = __uint_as_float(win.w);
-            msg.z = cmsg_z[par * 32 + src];
-        }
-        else if (tid == 0)
-        {
-            // one-CTA cluster: nobody completes the transaction count, do it locally
-            asm volatile("mbarrier.complete_tx.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(mbar + par)),
-                         "r"(static_cast<uint32_t>(nranks * kMsgBytes))
-                         : "memory");
-        }
-        cx = msg.x;
-        cy = msg.y;
-        cz = msg.z;
-        if (gtid == 0) idxs[j] = msg.key >= 0 ? msg.k : 0;
-    }
-    cluster_sync_all();
-}
-
 int fps_launch_global(int b, int n, int m, int log2bs, const float* xyz, float* temp,
                       int32_t* idxs, cudaStream_t stream)
 {
@@ -1031,57 +568,6 @@ int fps_launch_global(int b, int n, int m, int log2bs, const float* xyz, float* 
         return TPK_ERR_CUDA;
     }
     return TPK_OK;
-}
-
-// Largest cloud the sorted large-cloud kernel takes: 256 warps x 32 lanes x 4 chunks x 128 points.
-constexpr long long kFpsPrunedMaxPoints = 256ll * 32 * 4 * kFpsChunk;
-
-template <int CPL>
-int fps_launch_pruned_t(int b, int n, int m, int log2bs, const float* xyz, const float4* sorted, float* temp,
-                        int32_t* idxs, cudaStream_t stream)
-{
-    auto kernel = fps_pruned_kernel<CPL>;
-    prefer_max_shared(kernel);
-    cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-    if (err != cudaSuccess)
-    {
-        set_error("fps: cluster size attribute: %s", cudaGetErrorString(err));
-        return TPK_ERR_CUDA;
-    }
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(static_cast<unsigned>(b) * kFpsBigRanks, 1, 1);
-    cfg.blockDim = dim3(kFpsBigThreads, 1, 1);
-    cfg.dynamicSmemBytes = 0;
-    cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = kFpsBigRanks;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    count_launches(1);
-    err = cudaLaunchKernelEx(&cfg, kernel, n, m, log2bs, xyz, sorted, temp, idxs);
-    if (err != cudaSuccess)
-    {
-        set_error("fps launch (large clouds, sorted): %s", cudaGetErrorString(err));
-        return TPK_ERR_CUDA;
-    }
-    return TPK_OK;
-}
-
-// scratch: the sorted copy (16 bytes per point), then the running minima (4 bytes per point)
-int fps_launch_pruned(int b, int n, int m, int log2bs, const float* xyz, void* scratch, int32_t* idxs,
-                      cudaStream_t stream)
-{
-    float4* sorted = static_cast<float4*>(scratch);
-    float* temp = reinterpret_cast<float*>(sorted + static_cast<size_t>(b) * n);
-    const int rc = fps_launch_sort(b, n, xyz, sorted, stream);
-    if (rc != TPK_OK) return rc;
-    const long long per_lane = (static_cast<long long>(n) + 256ll * 32 * kFpsChunk - 1) / (256ll * 32 * kFpsChunk);
-    if (per_lane <= 1) return fps_launch_pruned_t<1>(b, n, m, log2bs, xyz, sorted, temp, idxs, stream);
-    if (per_lane <= 2) return fps_launch_pruned_t<2>(b, n, m, log2bs, xyz, sorted, temp, idxs, stream);
-    return fps_launch_pruned_t<4>(b, n, m, log2bs, xyz, sorted, temp, idxs, stream);
 }
 
 struct FpsConfig
@@ -1231,15 +717,14 @@ enum FpsPath
 {
     kFpsOnchip,  // cluster per cloud, registers, one sample per exchange
     kFpsRounds,  // cluster per cloud, rounds of independent samples (fps_rounds.cu)
-    kFpsPruned,  // large clouds on the sorted copy (20 B/point)
+    kFpsLarge,   // large clouds: rounds on a sorted copy in scratch (20 B/point, fps_large.cu)
     kFpsGlobal   // large clouds, unsorted (4 B/point)
 };
 
 FpsPath fps_pick_path(int n, int m, FpsConfig* c)
 {
     if (test_path("fps_global") || !fps_pick_config(n, m, c))
-        return (static_cast<long long>(n) <= kFpsPrunedMaxPoints && !test_path("fps_unsorted")) ? kFpsPruned
-                                                                                                  : kFpsGlobal;
+        return fps_large_fits(n) && !test_path("fps_unsorted") ? kFpsLarge : kFpsGlobal;
     if (test_path("fps_unsorted")) return kFpsOnchip;
     const bool rounds = test_path("fps_sorted") || (n > 1100 && m >= 48);
     return rounds && fps_rounds_fits(n) ? kFpsRounds : kFpsOnchip;
@@ -1259,7 +744,7 @@ extern "C" int64_t tpk_fps_scratch_bytes(int b, int n, int m)
     // sorted copy of clouds of this size from here)
     case tpk::kFpsRounds: return n >= 4096 && m >= 128 ? static_cast<int64_t>(b) * n * 16 : 0;
     // large clouds: the running minimum, one float per point, behind the sorted copy if one is used
-    case tpk::kFpsPruned: return static_cast<int64_t>(b) * n * 20;
+    case tpk::kFpsLarge: return static_cast<int64_t>(b) * n * 20;
     default: return static_cast<int64_t>(b) * n * 4;
     }
 }
@@ -1289,17 +774,18 @@ static int fps_run(int b, int n, int m, const float* xyz, void* scratch, int64_t
     }
     FpsConfig c;
     const FpsPath path = fps_pick_path(n, m, &c);
-    if (path == kFpsPruned || path == kFpsGlobal)
+    if (path == kFpsLarge || path == kFpsGlobal)
     {
         if (scratch == nullptr)
         {
             set_error("fps: clouds of %d points need tpk_fps_scratch_bytes() bytes of scratch", n);
             return TPK_ERR_SCRATCH;
         }
-        if (path == kFpsPruned)
+        if (path == kFpsLarge)
         {
             TPK_REQUIRE((reinterpret_cast<uintptr_t>(scratch) & 15u) == 0, "fps: scratch must be 16-byte aligned");
-            return fps_launch_pruned(b, n, m, log2bs, xyz, scratch, idxs, s);
+            *wrote_xyz = true;
+            return fps_large(b, n, m, log2bs, xyz, scratch, idxs, new_xyz, s);
         }
         return fps_launch_global(b, n, m, log2bs, xyz, static_cast<float*>(scratch), idxs, s);
     }

@@ -1,0 +1,1111 @@
+// Furthest point sampling of clouds that do not fit the register files of a cluster (sm_100a).
+//
+// Rounds of independent samples, as in fps_rounds.cu: a point t that no point u with a larger
+// running minimum (or an equal one and a smaller tie rank) touches, dist(u, t) < minimum(u), is a
+// sample whatever the sequence does before it, and the samples sorted by (minimum, rank) at the
+// moment they were picked are the sequence.  Here the points lie in global memory, in the order of
+// a Hilbert curve, in chunks of 32 * P points with a bounding box and the largest minimum of each
+// in shared memory; a warp owns a run of chunks.  A round is
+//   1. every warp applies the samples of the last round to the chunks that they reach, and lists
+//      what is active (minimum at least a fraction of the largest); cluster barrier;
+//   2. every CTA reads all lists; the candidates, shared out over the warps of the cluster, are
+//      checked against all entries; what passes is a sample; cluster barrier.
+// An entry is a point, or, as long as there are few samples and a chunk is small against their
+// distances, a whole chunk: (box, largest minimum) stands for its points, its first point is the
+// candidate.  A box reaches at least as far as its points, so this only delays a sample.
+// With points alone a list of a few thousand entries holds the neighbourhoods of one or two
+// maxima when a million points have a hundred samples.
+//
+// What bounds it is the latency of a round: two cluster barriers, the dependent loads of chunks from
+// L2, the check of the entries.  Measured, B200, one sample per exchange over the cluster before:
+// 8 clouds of 1048576 -> 65536 252 ms before, 20.2 now; 1048576 -> 16384 30.7 and 6.7;
+// 2 x 200000 -> 5000 8.5 and 2.4; a lattice of 64^3 -> 3000 (ties everywhere) 6.4 and 1.9.
+//
+// A sample's minimum is kept where it was: -minimum at its place, which no distance lowers and no
+// test takes for a candidate.  Points that are never candidates hold minus infinity.
+#include <climits>
+#include <cstdlib>
+#include <math_constants.h>
+
+#include <cooperative_groups.h>
+
+#include "fps_common.cuh"
+
+namespace cg = cooperative_groups;
+
+namespace tpk
+{
+namespace
+{
+
+constexpr int kLargeThreads = 1024;
+constexpr int kLargeWarps = kLargeThreads / 32;
+constexpr int kLargeMaxRanks = 16;
+constexpr int kLargeEntries = 4096;      // active points (half as many chunks) of a round
+constexpr int kLargeOwnEntries = 1024;   // of one CTA
+constexpr int kLargePicks = 2048;        // samples of a round
+constexpr int kLargeBuckets = 4096;
+constexpr int kLargeBucketShift = 16;    // while sampling: 128 buckets per octave, 32 octaves
+constexpr uint32_t kLargeNoRank = 0xFFFFFFFFu;
+constexpr int kMaxSmemBytes = 227 * 1024;
+
+struct LargeLayout
+{
+    int run;        // chunks of a warp
+    int groups;     // of up to 32 chunks of a warp
+    int cap_picks;  // samples a CTA may take per round
+    int meta, gbox, table, table_pos, own, own_pos, picks, mine_pick, hist, hits;
+    int f_hist, f_base, f_start;
+    int bytes;
+};
+
+__device__ __forceinline__ int ordered_image(float v)
+{
+    const int b = __float_as_int(v);
+    return b >= 0 ? b : b ^ 0x7FFFFFFF;
+}
+__device__ __forceinline__ float from_ordered(int o) { return __int_as_float(o >= 0 ? o : o ^ 0x7FFFFFFF); }
+
+// ---------------------------------------------------------------- order of the points
+//
+// Counting sort by cells of a 2^bits-per-axis grid along a Hilbert curve, all clouds at once, the
+// counters (and the box) in the part of the scratch where the running minima will be.
+
+struct SortBox
+{
+    float lo[3], inv_h, qmax;
+};
+
+__device__ __forceinline__ SortBox sort_box(const int* box, int bits)
+{
+    SortBox s;
+    float ext = 0.f;
+#pragma unroll
+    for (int a = 0; a < 3; ++a)
+    {
+        s.lo[a] = from_ordered(box[a]);
+        ext = fmaxf(ext, from_ordered(box[3 + a]) - s.lo[a]);
+    }
+    s.qmax = static_cast<float>((1 << bits) - 1);
+    s.inv_h = (ext > 0.f && ext < CUDART_INF_F) ? static_cast<float>(1 << bits) * 0.999999f / ext : 0.f;
+    return s;
+}
+__device__ __forceinline__ int sort_cell(const SortBox& s, int bits, float x, float y, float z)
+{
+    // fmaxf drops NaN, the clamp takes care of infinities: any cell is a correct cell
+    const uint32_t qx = static_cast<uint32_t>(fminf(fmaxf((x - s.lo[0]) * s.inv_h, 0.f), s.qmax));
+    const uint32_t qy = static_cast<uint32_t>(fminf(fmaxf((y - s.lo[1]) * s.inv_h, 0.f), s.qmax));
+    const uint32_t qz = static_cast<uint32_t>(fminf(fmaxf((z - s.lo[2]) * s.inv_h, 0.f), s.qmax));
+    return static_cast<int>(hilbert3(qx, qy, qz, bits));
+}
+
+__global__ void __launch_bounds__(256) large_clear_kernel(int n, int cells, int* __restrict__ counters)
+{
+    int* cnt = counters + static_cast<size_t>(blockIdx.y) * n;
+    for (int c = blockIdx.x * 256 + threadIdx.x; c < cells + 6; c += gridDim.x * 256)
+        cnt[c] = c < cells ? 0 : (c < cells + 3 ? INT_MAX : INT_MIN);
+}
+
+__global__ void __launch_bounds__(256) large_box_kernel(int n, int cells, const float* __restrict__ xyz_all, int* __restrict__ counters)
+{
+    const float* xyz = xyz_all + static_cast<size_t>(blockIdx.y) * n * 3;
+    int* box = counters + static_cast<size_t>(blockIdx.y) * n + cells;
+    __shared__ int s_box[6];
+    const int tid = threadIdx.x;
+    if (tid < 6) s_box[tid] = tid < 3 ? INT_MAX : INT_MIN;
+    __syncthreads();
+    int lo[3] = {INT_MAX, INT_MAX, INT_MAX}, hi[3] = {INT_MIN, INT_MIN, INT_MIN};
+    for (int k = blockIdx.x * 256 + tid; k < n; k += gridDim.x * 256)
+#pragma unroll
+        for (int a = 0; a < 3; ++a)
+        {
+            const float v = __ldg(xyz + 3 * static_cast<size_t>(k) + a);
+            if (fabsf(v) < 1.0e18f)
+            {
+                lo[a] = min(lo[a], ordered_image(v));
+                hi[a] = max(hi[a], ordered_image(v));
+            }
+        }
+#pragma unroll
+    for (int a = 0; a < 3; ++a)
+    {
+        const int l = __reduce_min_sync(kFullMask, lo[a]), h = __reduce_max_sync(kFullMask, hi[a]);
+        if ((tid & 31) == 0)
+        {
+            atomicMin(&s_box[a], l);
+            atomicMax(&s_box[3 + a], h);
+        }
+    }
+    __syncthreads();
+    if (tid < 3) atomicMin(&box[tid], s_box[tid]);
+    if (tid >= 3 && tid < 6) atomicMax(&box[tid], s_box[tid]);
+}
+
+// Counts the points of the cells, or (PLACE) puts the points to their places.
+template <bool PLACE>
+__global__ void __launch_bounds__(256)
+    large_cells_kernel(int n, int bits, const float* __restrict__ xyz_all, int* __restrict__ counters, float4* __restrict__ sorted_all)
+{
+    const float* xyz = xyz_all + static_cast<size_t>(blockIdx.y) * n * 3;
+    int* cnt = counters + static_cast<size_t>(blockIdx.y) * n;
+    float4* sorted = sorted_all + static_cast<size_t>(blockIdx.y) * n;
+    const SortBox s = sort_box(cnt + (1 << (3 * bits)), bits);
+    for (int k = blockIdx.x * 256 + threadIdx.x; k < n; k += gridDim.x * 256)
+    {
+        const float x = __ldg(xyz + 3 * static_cast<size_t>(k) + 0);
+        const float y = __ldg(xyz + 3 * static_cast<size_t>(k) + 1);
+        const float z = __ldg(xyz + 3 * static_cast<size_t>(k) + 2);
+        int* c = cnt + sort_cell(s, bits, x, y, z);
+        if constexpr (PLACE)
+            sorted[atomicAdd(c, 1)] = make_float4(x, y, z, __int_as_float(k));
+        else
+            atomicAdd(c, 1);
+    }
+}
+
+// Counters to first positions; one CTA per cloud.  cells: 8^bits, at least 64.
+__global__ void __launch_bounds__(1024) large_scan_kernel(int n, int cells, int* __restrict__ counters)
+{
+    int* cnt = counters + static_cast<size_t>(blockIdx.x) * n;
+    __shared__ int s_warp[33];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    constexpr int V = 8;
+    int before = 0;
+    for (int c0 = 0; c0 < cells; c0 += 1024 * V)
+    {
+        const int c = c0 + tid * V;
+        int v[V], sum = 0;
+#pragma unroll
+        for (int i = 0; i < V; ++i)
+        {
+            v[i] = c + i < cells ? cnt[c + i] : 0;
+            sum += v[i];
+        }
+        int incl = sum;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1)
+        {
+            const int t = __shfl_up_sync(kFullMask, incl, o);
+            if (lane >= o) incl += t;
+        }
+        if (lane == 31) s_warp[warp] = incl;
+        __syncthreads();
+        if (warp == 0)
+        {
+            int w = s_warp[lane];
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1)
+            {
+                const int t = __shfl_up_sync(kFullMask, w, o);
+                if (lane >= o) w += t;
+            }
+            s_warp[lane] = w;
+        }
+        __syncthreads();
+        int run = before + (warp ? s_warp[warp - 1] : 0) + incl - sum;
+#pragma unroll
+        for (int i = 0; i < V; ++i)
+        {
+            if (c + i < cells) cnt[c + i] = run;
+            run += v[i];
+        }
+        before += s_warp[31];
+        __syncthreads();
+    }
+}
+
+// Clouds too small to be worth a grid: as they are.
+__global__ void __launch_bounds__(256) large_copy_kernel(int n, const float* __restrict__ xyz_all, float4* __restrict__ sorted_all)
+{
+    const float* xyz = xyz_all + static_cast<size_t>(blockIdx.y) * n * 3;
+    for (int k = blockIdx.x * 256 + threadIdx.x; k < n; k += gridDim.x * 256)
+        sorted_all[static_cast<size_t>(blockIdx.y) * n + k] =
+            make_float4(__ldg(xyz + 3 * static_cast<size_t>(k)), __ldg(xyz + 3 * static_cast<size_t>(k) + 1),
+                        __ldg(xyz + 3 * static_cast<size_t>(k) + 2), __int_as_float(k));
+}
+
+// ---------------------------------------------------------------- sampling
+
+struct LargeNote
+{
+    int entries, top, above, picks;
+};
+
+template <int P>  // points per lane of a chunk
+__global__ void __launch_bounds__(kLargeThreads, 1)
+    fps_large_kernel(int n, int m, int log2bs, int nranks, LargeLayout lay, const float* __restrict__ xyz_all,
+                     float4* __restrict__ sorted_all, float* __restrict__ temp_all, int32_t* __restrict__ idxs_all,
+                     float* __restrict__ new_xyz_all)
+{
+    extern __shared__ __align__(16) unsigned char smem[];
+    __shared__ LargeNote s_note[2];               // by parity of the round: read by the other CTAs
+    __shared__ LargeNote s_notes[kLargeMaxRanks];  // of all CTAs
+    __shared__ int s_scan[32];
+    __shared__ unsigned long long s_top;
+    __shared__ unsigned long long s_tops[kLargeMaxRanks];
+    __shared__ int s_bad;
+
+    constexpr int CHUNK = 32 * P;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int rank = static_cast<int>(cluster_ctarank());
+    const int cloud = blockIdx.x / nranks;
+    const float* xyz = xyz_all + static_cast<size_t>(cloud) * n * 3;
+    float4* sorted = sorted_all + static_cast<size_t>(cloud) * n;
+    float* temp = temp_all + static_cast<size_t>(cloud) * n;
+    int32_t* idxs = idxs_all + static_cast<size_t>(cloud) * m;
+    float* new_xyz = new_xyz_all ? new_xyz_all + static_cast<size_t>(cloud) * m * 3 : nullptr;
+
+    const int run = lay.run;
+    const int nmeta = run * kLargeWarps;
+    float* meta = reinterpret_cast<float*>(smem + lay.meta);  // lo x y z, hi x y z, key: nmeta each
+    int* ckey = reinterpret_cast<int*>(meta + 6 * nmeta);
+    float* gbox = reinterpret_cast<float*>(smem + lay.gbox);
+    float4* table = reinterpret_cast<float4*>(smem + lay.table);
+    int* table_pos = reinterpret_cast<int*>(smem + lay.table_pos);
+    float4* own = reinterpret_cast<float4*>(smem + lay.own);
+    int* own_pos = reinterpret_cast<int*>(smem + lay.own_pos);
+    float4* picks = reinterpret_cast<float4*>(smem + lay.picks);
+    float4* mine_pick = reinterpret_cast<float4*>(smem + lay.mine_pick);
+    int* hist = reinterpret_cast<int*>(smem + lay.hist);
+    uint16_t* hits = reinterpret_cast<uint16_t*>(smem + lay.hits) + warp * 32;
+
+    auto at_rank = [&](auto* p, int r) { return cg::this_cluster().map_shared_rank(p, static_cast<unsigned>(r)); };
+    // Neighbouring runs belong to different CTAs: a round lasts as long as its busiest CTA.
+    const long long first = static_cast<long long>(warp * nranks + rank) * run * CHUNK;
+    auto chunk_base = [&](int c) { return first + static_cast<long long>(c) * CHUNK; };
+    auto index_at = [&](int pos) { return __float_as_int(__ldg(&sorted[pos].w)); };
+    auto box_dist = [&](const float (&b)[6], float x, float y, float z) {
+        // same expression and rounding as a point's distance: never above that of a point in the box
+        return sumsq_abc(fmaxf(fmaxf(b[0] - x, x - b[3]), 0.f), fmaxf(fmaxf(b[1] - y, y - b[4]), 0.f),
+                         fmaxf(fmaxf(b[2] - z, z - b[5]), 0.f));
+    };
+
+    // ------------------------------------------------ boxes, minima
+    if (tid == 0)
+    {
+        s_bad = 0;
+        for (int i = 0; i < 2; ++i) s_note[i] = LargeNote{0, INT_MIN, 0, 0};
+    }
+    for (int i = tid; i < kLargeBuckets; i += kLargeThreads) hist[i] = 0;
+    __syncthreads();
+    bool bad = false;
+    for (int g = 0; g < lay.groups; ++g)
+    {
+        const int left = min(32, run - 32 * g);
+        float glo[3] = {CUDART_INF_F, CUDART_INF_F, CUDART_INF_F}, ghi[3] = {-CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F};
+        for (int c = 0; c < left; ++c)
+        {
+            const long long base = chunk_base(32 * g + c);
+            float lo[3] = {CUDART_INF_F, CUDART_INF_F, CUDART_INF_F}, hi[3] = {-CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F};
+            int key = INT_MIN;
+            float4 v[P];
+#pragma unroll
+            for (int u = 0; u < P; ++u)
+                if (base + u * 32 + lane < n) v[u] = __ldg(sorted + base + u * 32 + lane);
+#pragma unroll
+            for (int u = 0; u < P; ++u)
+            {
+                const long long p = base + u * 32 + lane;
+                if (p >= n) continue;
+                const bool in = !(static_cast<double>(sumsq_abc(v[u].x, v[u].y, v[u].z)) <= 1e-3);
+                const float first_min = in ? 1e10f : -CUDART_INF_F;
+                __stcg(temp + p, first_min);
+                key = max(key, __float_as_int(first_min));
+                if (!in) continue;
+                if (fabsf(v[u].x) < 1.0e18f && fabsf(v[u].y) < 1.0e18f && fabsf(v[u].z) < 1.0e18f)
+                {
+                    lo[0] = fminf(lo[0], v[u].x);
+                    hi[0] = fmaxf(hi[0], v[u].x);
+                    lo[1] = fminf(lo[1], v[u].y);
+                    hi[1] = fmaxf(hi[1], v[u].y);
+                    lo[2] = fminf(lo[2], v[u].z);
+                    hi[2] = fmaxf(hi[2], v[u].z);
+                }
+                else
+                    bad = true;  // not finite, or too large to square
+            }
+            const int at = warp * run + 32 * g + c;
+#pragma unroll
+            for (int a = 0; a < 3; ++a)
+            {
+                const float l = from_ordered(__reduce_min_sync(kFullMask, ordered_image(lo[a])));
+                const float h = from_ordered(__reduce_max_sync(kFullMask, ordered_image(hi[a])));
+                glo[a] = fminf(glo[a], l);
+                ghi[a] = fmaxf(ghi[a], h);
+                if (lane == 0)
+                {
+                    meta[a * nmeta + at] = l;
+                    meta[(3 + a) * nmeta + at] = h;
+                }
+            }
+            key = __reduce_max_sync(kFullMask, key);
+            if (lane == 0) ckey[at] = key;
+        }
+        if (lane < 3)
+        {
+            gbox[(warp * lay.groups + g) * 8 + lane] = lane == 0 ? glo[0] : (lane == 1 ? glo[1] : glo[2]);
+            gbox[(warp * lay.groups + g) * 8 + 3 + lane] = lane == 0 ? ghi[0] : (lane == 1 ? ghi[1] : ghi[2]);
+        }
+    }
+    if (__any_sync(kFullMask, bad) && lane == 0) s_bad = 1;
+    cluster_sync_all();
+    bool sequential = false;  // one sample per round, every chunk in reach: coordinates that are not finite
+    for (int r = 0; r < nranks; ++r) sequential |= *at_rank(&s_bad, r) != 0;
+
+    // Lowers the minima of chunk c (of group g) by the samples hits[bit] of a mask; returns its key.
+    auto lower_chunk = [&](long long base, uint32_t mask) -> int {
+        float4 v[P];
+        float d0[P], md[P];
+#pragma unroll
+        for (int u = 0; u < P; ++u)
+        {
+            const long long p = base + u * 32 + lane;
+            d0[u] = -CUDART_INF_F;
+            v[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (p < n)
+            {
+                v[u] = __ldg(sorted + p);
+                d0[u] = __ldcg(temp + p);
+            }
+            md[u] = d0[u];
+        }
+        while (mask != 0u)
+        {
+            const float4 s = picks[hits[__ffs(mask) - 1]];
+            mask &= mask - 1u;
+#pragma unroll
+            for (int u = 0; u < P; ++u) md[u] = fminf(md[u], sumsq_abc(v[u].x - s.x, v[u].y - s.y, v[u].z - s.z));
+        }
+        int key = INT_MIN;
+#pragma unroll
+        for (int u = 0; u < P; ++u)
+        {
+            const long long p = base + u * 32 + lane;
+            if (p < n && md[u] != d0[u]) __stcg(temp + p, md[u]);
+            key = max(key, __float_as_int(md[u]));
+        }
+        return __reduce_max_sync(kFullMask, key);
+    };
+    // Applies the first `count` samples of the table.
+    auto apply = [&](int count) {
+        for (int g = 0; g < lay.groups; ++g)
+        {
+            const bool in = 32 * g + lane < run;
+            const int at = warp * run + 32 * g + lane;
+            int key = in ? ckey[at] : INT_MIN;
+            const int gkey = __reduce_max_sync(kFullMask, key);
+            if (gkey <= 0) continue;
+            float box[6], gb[6];
+#pragma unroll
+            for (int a = 0; a < 6; ++a)
+            {
+                box[a] = in ? meta[a * nmeta + at] : 0.f;
+                gb[a] = gbox[(warp * lay.groups + g) * 8 + a];
+            }
+            auto flush = [&](int nh) {
+                __syncwarp();
+                uint32_t mask = 0;
+                if (key > 0)
+                    for (int h = 0; h < nh; ++h)
+                    {
+                        const float4 s = picks[hits[h]];
+                        if (sequential || box_dist(box, s.x, s.y, s.z) < __int_as_float(key)) mask |= 1u << h;
+                    }
+                uint32_t todo = __ballot_sync(kFullMask, mask != 0u);
+                while (todo != 0u)
+                {
+                    const int c = __ffs(todo) - 1;
+                    todo &= todo - 1u;
+                    const int k = lower_chunk(chunk_base(32 * g + c), __shfl_sync(kFullMask, mask, c));
+                    if (lane == c) key = k;
+                }
+                __syncwarp();
+            };
+            int nh = 0;
+            for (int i0 = 0; i0 < count; i0 += 32)
+            {
+                bool reach = false;
+                if (i0 + lane < count)
+                {
+                    const float4 s = picks[i0 + lane];
+                    reach = sequential || box_dist(gb, s.x, s.y, s.z) < __int_as_float(gkey);
+                }
+                const uint32_t b = __ballot_sync(kFullMask, reach);
+                if (b == 0u) continue;
+                if (nh + __popc(b) > 32)
+                {
+                    flush(nh);
+                    nh = 0;
+                }
+                if (reach) hits[nh + __popc(b & ((1u << lane) - 1u))] = static_cast<uint16_t>(i0 + lane);
+                nh += __popc(b);
+            }
+            if (nh > 0) flush(nh);
+            if (in) ckey[at] = key;
+        }
+        __syncwarp();
+    };
+    // The first point in the order of V among those with the given image of the minimum (zero: samples,
+    // whose minimum is zero, included): (rank, place), the same in all CTAs; all ones if there is none.
+    auto find_top = [&](int top) -> unsigned long long {
+        if (tid == 0) s_top = ~0ull;
+        __syncthreads();
+        for (int g = 0; g < lay.groups; ++g)
+        {
+            const bool in = 32 * g + lane < run;
+            const int key = in ? ckey[warp * run + 32 * g + lane] : INT_MIN;
+            // (a chunk of samples only has a negative key: look at all of them for zeros)
+            uint32_t todo = __ballot_sync(kFullMask, in && (top > 0 ? key == top : true));
+            while (todo != 0u)
+            {
+                const int c = __ffs(todo) - 1;
+                todo &= todo - 1u;
+                const long long base = chunk_base(32 * g + c);
+                for (int u = 0; u < P; ++u)
+                {
+                    const long long p = base + u * 32 + lane;
+                    if (p >= n) continue;
+                    const int k = __float_as_int(__ldcg(temp + p));
+                    const bool zero_like = k == 0 || (k < 0 && k != __float_as_int(-CUDART_INF_F));
+                    if (top > 0 ? k == top : zero_like)
+                        atomicMin(&s_top, static_cast<unsigned long long>(fps_rank(index_at(static_cast<int>(p)), log2bs)) << 32 |
+                                              static_cast<unsigned long long>(p));
+                }
+            }
+        }
+        cluster_sync_all();
+        if (tid < nranks) s_tops[tid] = *at_rank(&s_top, tid);
+        __syncthreads();
+        unsigned long long best = ~0ull;
+        for (int r = 0; r < nranks; ++r) best = s_tops[r] < best ? s_tops[r] : best;
+        cluster_sync_all();  // everyone has read
+        return best;
+    };
+    int first_top = 0;
+    auto bucket_of = [&](int key) { return max(0, min(kLargeBuckets - 1, (first_top - key) >> kLargeBucketShift)); };
+
+    // sample 0 is point 0, candidate or not
+    if (tid == 0)
+    {
+        picks[0] = make_float4(__ldg(xyz), __ldg(xyz + 1), __ldg(xyz + 2), 0.f);
+        if (rank == 0)
+        {
+            idxs[0] = 0;
+            if (new_xyz)
+                for (int a = 0; a < 3; ++a) new_xyz[a] = __ldg(xyz + a);
+        }
+    }
+    int pending = 1;
+    int tau_key = INT_MAX;
+    uint32_t rank_limit = kLargeNoRank - 1u, tau_rank = rank_limit;
+    float gap = 0.25f;
+    bool overflow_before = false;
+    // chunks stand for their points while there are few samples
+    const int nchunks = static_cast<int>((static_cast<long long>(n) + CHUNK - 1) / CHUNK);
+    bool by_chunk = true;
+    int top = 0, top_before = INT_MAX, taken = 0, fill = 0;
+    auto set_tau = [&]() {
+        // towards the end not below what the last sample will have: samples beyond m are taken for nothing
+        const float part = fminf(static_cast<float>(taken) / static_cast<float>(m), 1.0f);
+        const float f = fmaxf(1.0f - gap, 0.9f * part);
+        tau_key = max(1, min(top, __float_as_int(f * __int_as_float(top))));
+        tau_rank = tau_key == top ? rank_limit : kLargeNoRank - 1u;
+        top_before = top;
+    };
+    __syncthreads();
+    for (uint32_t round = 0;; ++round)
+    {
+        const int par = round & 1u;
+        // ---- 1: samples of the round before, then the active points or chunks
+        if (pending > 0) apply(pending);
+        int wmax = INT_MIN;
+        for (int g = 0; g < lay.groups; ++g)
+        {
+            const bool in = 32 * g + lane < run;
+            const int at = warp * run + 32 * g + lane;
+            const int key = in ? ckey[at] : INT_MIN;
+            wmax = max(wmax, key);
+            if (sequential) continue;
+            uint32_t todo = __ballot_sync(kFullMask, key >= tau_key);
+            if (by_chunk && todo != 0u)
+            {
+                int pos = 0;
+                if (lane == 0) pos = atomicAdd(&s_note[par].entries, __popc(todo));
+                pos = __shfl_sync(kFullMask, pos, 0);
+                while (todo != 0u)
+                {
+                    const int c = __ffs(todo) - 1;
+                    todo &= todo - 1u;
+                    if (pos >= kLargeOwnEntries / 2) break;
+                    const long long base = chunk_base(32 * g + c);
+                    const int ck = __shfl_sync(kFullMask, key, c);
+                    unsigned long long best = ~0ull;
+                    int held = 0;
+#pragma unroll
+                    for (int u = 0; u < P; ++u)
+                    {
+                        const long long p = base + u * 32 + lane;
+                        if (p < n && __float_as_int(__ldcg(temp + p)) == ck)
+                        {
+                            held += 1;
+                            const unsigned long long v = static_cast<unsigned long long>(fps_rank(index_at(static_cast<int>(p)), log2bs)) << 32 |
+                                                         static_cast<unsigned long long>(p);
+                            best = v < best ? v : best;
+                        }
+                    }
+                    // the first of the points that hold the chunk's largest minimum
+                    const uint32_t hi = __reduce_min_sync(kFullMask, static_cast<uint32_t>(best >> 32));
+                    const uint32_t who = __ballot_sync(kFullMask, held > 0 && static_cast<uint32_t>(best >> 32) == hi);
+                    if (who != 0u && lane == __ffs(who) - 1)
+                    {
+                        const int a = warp * run + 32 * g + c;
+                        own[pos] = make_float4(meta[a], meta[nmeta + a], meta[2 * nmeta + a], __int_as_float(ck));
+                        own[kLargeOwnEntries / 2 + pos] = make_float4(meta[3 * nmeta + a], meta[4 * nmeta + a], meta[5 * nmeta + a], 0.f);
+                        own_pos[pos] = static_cast<int>(best & 0xFFFFFFFFull);
+                    }
+                    ++pos;
+                }
+            }
+            else
+                while (todo != 0u)
+                {
+                    const int c = __ffs(todo) - 1;
+                    todo &= todo - 1u;
+                    const long long base = chunk_base(32 * g + c);
+                    float md[P];
+                    uint32_t act[P];
+                    int nact = 0;
+#pragma unroll
+                    for (int u = 0; u < P; ++u)
+                    {
+                        const long long p = base + u * 32 + lane;
+                        md[u] = p < n ? __ldcg(temp + p) : -CUDART_INF_F;
+                    }
+#pragma unroll
+                    for (int u = 0; u < P; ++u)
+                    {
+                        const int k = __float_as_int(md[u]);
+                        bool a = k >= tau_key;
+                        if (a && k == tau_key && tau_rank != kLargeNoRank - 1u)
+                            a = fps_rank(index_at(static_cast<int>(base + u * 32 + lane)), log2bs) <= tau_rank;
+                        act[u] = __ballot_sync(kFullMask, a);
+                        nact += __popc(act[u]);
+                    }
+                    if (nact == 0) continue;
+                    int pos = 0;
+                    if (lane == 0) pos = atomicAdd(&s_note[par].entries, nact);
+                    pos = __shfl_sync(kFullMask, pos, 0);
+#pragma unroll
+                    for (int u = 0; u < P; ++u)
+                    {
+                        const int p = pos + __popc(act[u] & ((1u << lane) - 1u));
+                        if ((act[u] >> lane & 1u) && p < kLargeOwnEntries)
+                        {
+                            const float4 v = __ldg(sorted + base + u * 32 + lane);
+                            own[p] = make_float4(v.x, v.y, v.z, md[u]);
+                            own_pos[p] = static_cast<int>(base + u * 32 + lane);
+                        }
+                        pos += __popc(act[u]);
+                    }
+                }
+        }
+        wmax = __reduce_max_sync(kFullMask, wmax);
+        if (lane == 0) atomicMax(&s_note[par].top, wmax);
+        if (!sequential && taken >= m - 1)
+        {
+            // enough samples: are m - 1 of them above all that is left?
+            const int last = bucket_of(top_before);
+            int above = 0;
+            for (int c = tid; c < last; c += kLargeThreads) above += hist[c];
+            above = __reduce_add_sync(kFullMask, above);
+            if (lane == 0 && above) atomicAdd(&s_note[par].above, above);
+        }
+        cluster_sync_all();
+        if (tid < nranks) s_notes[tid] = *at_rank(&s_note[par], tid);
+        if (tid == 0) s_note[par ^ 1] = LargeNote{0, INT_MIN, 0, 0};  // read by everyone before this barrier
+        __syncthreads();
+        int nentries = 0, above = 0, longest = 0, before = 0;
+        const int from = warp & (nranks - 1);
+        top = INT_MIN;
+        for (int r = 0; r < nranks; ++r)
+        {
+            before += r < from ? s_notes[r].entries : 0;
+            nentries += s_notes[r].entries;
+            longest = max(longest, s_notes[r].entries);
+            top = max(top, s_notes[r].top);
+            above += s_notes[r].above;
+        }
+        const int cap = by_chunk ? kLargeEntries / 2 : kLargeEntries;
+        const int cap_own = by_chunk ? kLargeOwnEntries / 2 : kLargeOwnEntries;
+        const bool overflow = longest > cap_own || nentries > cap;
+        if (round == 0) first_top = top;
+        bool alone = overflow;  // take the first point in the order, nothing else
+        if (sequential)
+        {
+            if (top < 0 || taken >= m - 1) break;
+            alone = true;
+        }
+        else if (taken >= m - 1 && (above >= m - 1 || top <= 0))
+            break;
+        else if (top <= 0)
+        {
+            // only points that coincide with a sample are left: the first of them, from now on
+            const unsigned long long w = find_top(0);
+            if (w != ~0ull) fill = index_at(static_cast<int>(w & 0xFFFFFFFFull));
+            break;
+        }
+        if (alone)
+        {
+            unsigned long long w;
+            if (sequential && top == 0)
+                w = find_top(0);  // (no sample is marked: the zeros themselves)
+            else
+                w = find_top(top);
+            const int pos = static_cast<int>(w & 0xFFFFFFFFull);
+            taken += 1;
+            if (tid == 0)
+            {
+                const float4 v = __ldg(sorted + pos);
+                picks[0] = v;
+                const int k = __float_as_int(v.w);
+                if (sequential)
+                {
+                    if (rank == 0)
+                    {
+                        idxs[taken] = k;
+                        if (new_xyz)
+                            for (int a = 0; a < 3; ++a)
+                                new_xyz[3 * static_cast<size_t>(taken) + a] = __ldg(xyz + 3 * static_cast<size_t>(k) + a);
+                    }
+                }
+                else if (s_tops[rank] == w)
+                {
+                    __stcg(temp + pos, -__int_as_float(top));
+                    atomicAdd(&hist[bucket_of(top)], 1);
+                }
+            }
+            pending = 1;
+        }
+        else
+            pending = 0;
+        if (nentries == 0 || overflow || sequential)
+        {
+            if (overflow)
+            {
+                if (tau_key >= top)
+                {
+                    if (by_chunk)
+                        by_chunk = false;  // ties: points can be told apart by rank
+                    else
+                        rank_limit >>= 1;
+                }
+                gap = overflow_before ? 0.f : 0.5f * gap;
+            }
+            else if (tau_key == top)
+                rank_limit = rank_limit * 2u + 1u;
+            overflow_before = overflow;
+            set_tau();
+            __syncthreads();
+            continue;
+        }
+        overflow_before = false;
+        {
+            // the lists of all CTAs: warps share out a CTA's list
+            const int count = s_notes[from].entries, step = kLargeThreads / nranks;
+            const float4* src = at_rank(own, from);
+            const int* src_pos = at_rank(own_pos, from);
+            for (int i = (warp / nranks) * 32 + lane; i < count; i += step)
+            {
+                table[before + i] = src[i];
+                if (by_chunk) table[kLargeEntries / 2 + before + i] = src[kLargeOwnEntries / 2 + i];
+                table_pos[before + i] = src_pos[i];
+            }
+        }
+        __syncthreads();
+
+        // ---- 2: what no active point precedes and touches is a sample
+        constexpr int Q = 2;  // candidates a warp checks side by side
+        for (int q0 = (warp * nranks + rank) * Q; q0 < nentries; q0 += nranks * kLargeWarps * Q)
+        {
+            float4 t[Q];
+            int tpos[Q];
+            bool blocked[Q];
+            int same = 0;
+#pragma unroll
+            for (int q = 0; q < Q; ++q)
+            {
+                const int e = min(q0 + q, nentries - 1);
+                tpos[q] = table_pos[e];
+                t[q] = table[e];
+                if (by_chunk)
+                {
+                    const float4 v = __ldg(sorted + tpos[q]);
+                    t[q] = make_float4(v.x, v.y, v.z, t[q].w);
+                }
+                blocked[q] = false;
+            }
+            for (int at0 = 0; at0 < nentries; at0 += 128)
+            {
+#pragma unroll
+                for (int u = 0; u < 4; ++u)
+                {
+                    const int at = at0 + 32 * u + lane;
+                    float4 e = table[min(at, nentries - 1)];
+                    if (at >= nentries) e.w = -1.0f;  // touches nothing
+                    if (by_chunk)
+                    {
+                        const float4 h = table[kLargeEntries / 2 + min(at, nentries - 1)];
+                        const float box[6] = {e.x, e.y, e.z, h.x, h.y, h.z};
+#pragma unroll
+                        for (int q = 0; q < Q; ++q)
+                        {
+                            const bool near = box_dist(box, t[q].x, t[q].y, t[q].z) < e.w;
+                            blocked[q] |= near && e.w > t[q].w;
+                            same += near && e.w == t[q].w ? 1 : 0;
+                        }
+                    }
+                    else
+#pragma unroll
+                        for (int q = 0; q < Q; ++q)
+                        {
+                            const bool near = sumsq_abc(e.x - t[q].x, e.y - t[q].y, e.z - t[q].z) < e.w;
+                            blocked[q] |= near && e.w > t[q].w;
+                            same += near && e.w == t[q].w ? 1 : 0;
+                        }
+                }
+                bool all = true;
+#pragma unroll
+                for (int q = 0; q < Q; ++q) all &= __any_sync(kFullMask, blocked[q]) != 0;
+                if (all) break;
+            }
+            uint32_t free_of = 0;
+#pragma unroll
+            for (int q = 0; q < Q; ++q)
+                if (!__any_sync(kFullMask, blocked[q]) && q0 + q < nentries) free_of |= 1u << q;
+            if (free_of == 0u) continue;
+            // every candidate meets itself; more than that is a tie to be decided by rank
+            if (__reduce_add_sync(kFullMask, same) > Q)
+#pragma unroll
+                for (int q = 0; q < Q; ++q)
+                    if (free_of >> q & 1u)
+                    {
+                        const uint32_t tr = fps_rank(index_at(tpos[q]), log2bs);
+                        bool is_first = true;
+                        for (int at = lane; at < nentries; at += 32)
+                        {
+                            const float4 e = table[at];
+                            if (e.w != t[q].w) continue;
+                            float d;
+                            if (by_chunk)
+                            {
+                                const float4 h = table[kLargeEntries / 2 + at];
+                                const float box[6] = {e.x, e.y, e.z, h.x, h.y, h.z};
+                                d = box_dist(box, t[q].x, t[q].y, t[q].z);
+                            }
+                            else
+                                d = sumsq_abc(e.x - t[q].x, e.y - t[q].y, e.z - t[q].z);
+                            if (d < e.w && fps_rank(index_at(table_pos[at]), log2bs) < tr) is_first = false;
+                        }
+                        if (!__all_sync(kFullMask, is_first)) free_of &= ~(1u << q);
+                    }
+#pragma unroll
+            for (int q = 0; q < Q; ++q)
+                if (lane == q && (free_of >> q & 1u))
+                {
+                    const int p = atomicAdd(&s_note[par].picks, 1);
+                    // beyond the capacity: it is still the first of its neighbourhood next round
+                    if (p < lay.cap_picks)
+                    {
+                        mine_pick[p] = t[q];
+                        __stcg(temp + tpos[q], -t[q].w);
+                        atomicAdd(&hist[bucket_of(__float_as_int(t[q].w))], 1);
+                    }
+                }
+        }
+        cluster_sync_all();
+        if (tid < nranks) s_notes[tid].picks = min(at_rank(&s_note[par], tid)->picks, lay.cap_picks);
+        __syncthreads();
+        int total = 0;
+        before = 0;
+        for (int r = 0; r < nranks; ++r)
+        {
+            before += r < from ? s_notes[r].picks : 0;
+            total += s_notes[r].picks;
+        }
+        {
+            const int count = s_notes[from].picks, step = kLargeThreads / nranks;
+            const float4* src = at_rank(mine_pick, from);
+            for (int i = (warp / nranks) * 32 + lane; i < count; i += step) picks[before + i] = src[i];
+        }
+        pending = total;
+        taken += total;
+        // more active entries per round mean fewer rounds, but longer ones
+        if (nentries < 512)
+            gap = fminf(fmaxf(gap * 1.25f, 1.0e-3f), 0.5f);
+        else if (nentries > 1024)
+            gap *= nentries > 1536 ? 0.5f : 0.8f;
+        if (rank_limit < (kLargeNoRank >> 1) && nentries * 4 < kLargeEntries) rank_limit = rank_limit * 2u + 1u;
+        if (by_chunk && taken > nchunks / 4) by_chunk = false;
+        set_tau();
+        __syncthreads();
+    }
+
+    // ------------------------------------------------ the samples in order
+    if (!sequential)
+    {
+        int* f_hist = reinterpret_cast<int*>(smem + lay.f_hist);
+        int* f_base = reinterpret_cast<int*>(smem + lay.f_base);
+        int* f_start = reinterpret_cast<int*>(smem + lay.f_start);
+        int* slots = reinterpret_cast<int*>(temp);
+        cluster_sync_all();  // the tables have been read everywhere
+        for (int c = tid; c < kLargeBuckets; c += kLargeThreads) f_hist[c] = 0;
+        __syncthreads();
+        // buckets over the images that samples can have
+        int shift = 0;
+        const int low = max(0, top);
+        while ((max(first_top - low, 0) >> shift) >= kLargeBuckets - 1) ++shift;
+        auto bucket = [&](int key) { return max(0, min(kLargeBuckets - 1, (first_top - key) >> shift)); };
+        // a warp moves its samples to the front of its run, as (image of the minimum, index)
+        int mine = 0;
+        for (int c = 0; c < run; ++c)
+        {
+            const long long base = chunk_base(c);
+            if (base >= n) break;
+            int key[P], idx[P];
+            bool is[P];
+#pragma unroll
+            for (int u = 0; u < P; ++u)
+            {
+                const long long p = base + u * 32 + lane;
+                const float md = p < n ? __ldcg(temp + p) : 0.f;
+                is[u] = md < 0.f && md != -CUDART_INF_F;
+                key[u] = __float_as_int(-md);
+                idx[u] = is[u] ? __float_as_int(__ldcg(&sorted[p].w)) : 0;
+            }
+            __syncwarp();
+#pragma unroll
+            for (int u = 0; u < P; ++u)
+            {
+                const uint32_t b = __ballot_sync(kFullMask, is[u]);
+                if (is[u])
+                {
+                    __stcg(reinterpret_cast<int2*>(sorted + first + mine + __popc(b & ((1u << lane) - 1u))), make_int2(key[u], idx[u]));
+                    atomicAdd(&f_hist[bucket(key[u])], 1);
+                }
+                mine += __popc(b);
+            }
+            __syncwarp();
+        }
+        cluster_sync_all();
+        // first place of every bucket over all CTAs, and what the CTAs before this one have in it
+        {
+            constexpr int PER = kLargeBuckets / kLargeThreads;
+            int sum = 0, tot[PER];
+#pragma unroll
+            for (int i = 0; i < PER; ++i)
+            {
+                tot[i] = 0;
+                int mine_before = 0;
+                for (int r = 0; r < nranks; ++r)
+                {
+                    const int v = at_rank(f_hist, r)[tid * PER + i];
+                    mine_before += r < rank ? v : 0;
+                    tot[i] += v;
+                }
+                f_base[tid * PER + i] = mine_before;
+                sum += tot[i];
+            }
+            int incl = sum;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1)
+            {
+                const int t = __shfl_up_sync(kFullMask, incl, o);
+                if (lane >= o) incl += t;
+            }
+            if (lane == 31) s_scan[warp] = incl;
+            __syncthreads();
+            int at = incl - sum;
+            for (int w = 0; w < warp; ++w) at += s_scan[w];
+#pragma unroll
+            for (int i = 0; i < PER; ++i)
+            {
+                f_start[tid * PER + i] = at;
+                at += tot[i];
+            }
+            __syncthreads();
+        }
+        for (int i = lane; i < mine; i += 32)
+        {
+            const int2 e = __ldcg(reinterpret_cast<const int2*>(sorted + first + i));
+            const int b = bucket(e.x);
+            __stcg(slots + f_start[b] + atomicAdd(&f_base[b], 1), static_cast<int>(first) + i);
+        }
+        cluster_sync_all();
+        for (int i = rank * kLargeThreads + tid; i < taken; i += nranks * kLargeThreads)
+        {
+            const int2 e = __ldcg(reinterpret_cast<const int2*>(sorted + __ldcg(slots + i)));
+            const int b = bucket(e.x);
+            const int lo = f_start[b], hi = b + 1 < kLargeBuckets ? f_start[b + 1] : taken;
+            if (lo >= m - 1) continue;
+            int place = lo;
+#pragma unroll 4
+            for (int j = lo; j < hi; ++j)
+            {
+                const int2 o = __ldcg(reinterpret_cast<const int2*>(sorted + __ldcg(slots + j)));
+                place += o.x > e.x || (o.x == e.x && fps_rank(o.y, log2bs) < fps_rank(e.y, log2bs)) ? 1 : 0;
+            }
+            if (place < m - 1)
+            {
+                idxs[place + 1] = e.y;
+                if (new_xyz)
+                    for (int a = 0; a < 3; ++a)
+                        new_xyz[3 * static_cast<size_t>(place + 1) + a] = __ldg(xyz + 3 * static_cast<size_t>(e.y) + a);
+            }
+        }
+    }
+    for (int j = taken + 1 + rank * kLargeThreads + tid; j < m; j += nranks * kLargeThreads)
+    {
+        idxs[j] = fill;
+        if (new_xyz)
+            for (int a = 0; a < 3; ++a) new_xyz[3 * static_cast<size_t>(j) + a] = __ldg(xyz + 3 * static_cast<size_t>(fill) + a);
+    }
+    cluster_sync_all();  // shared memory stays until every CTA has read it
+}
+
+LargeLayout large_layout(int n, int nranks, int p)
+{
+    LargeLayout lay = {};
+    const long long nchunks = (static_cast<long long>(n) + 32 * p - 1) / (32 * p);
+    const int warps = nranks * kLargeWarps;
+    lay.run = static_cast<int>((nchunks + warps - 1) / warps);
+    lay.groups = (lay.run + 31) / 32;
+    lay.cap_picks = kLargePicks / nranks < 512 ? kLargePicks / nranks : 512;
+    long long at = 0;
+    auto take = [&](long long bytes) {
+        const long long o = at;
+        at += (bytes + 15) / 16 * 16;
+        return static_cast<int>(o);
+    };
+    lay.meta = take(static_cast<long long>(lay.run) * kLargeWarps * 28);
+    lay.gbox = take(static_cast<long long>(lay.groups) * kLargeWarps * 32);
+    lay.hist = take(kLargeBuckets * 4);
+    lay.hits = take(kLargeWarps * 64);
+    lay.own = take(kLargeOwnEntries * 16);
+    lay.own_pos = take(kLargeOwnEntries * 4);
+    lay.mine_pick = take(lay.cap_picks * 16);
+    lay.picks = take(kLargePicks * 16);
+    lay.table = take(kLargeEntries * 16);
+    lay.table_pos = take(kLargeEntries * 4);
+    // the final order takes the place of the entry table
+    lay.f_hist = lay.table;
+    lay.f_base = lay.table + kLargeBuckets * 4;
+    lay.f_start = lay.table + kLargeBuckets * 8;
+    lay.bytes = at > INT_MAX ? INT_MAX : static_cast<int>(at);
+    return lay;
+}
+
+template <int P>
+int launch_large(int b, int n, int m, int log2bs, int nranks, const LargeLayout& lay, const float* xyz, float4* sorted,
+                 float* temp, int32_t* idxs, float* new_xyz, cudaStream_t stream)
+{
+    auto kernel = fps_large_kernel<P>;
+    prefer_max_shared(kernel);
+    cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, lay.bytes);
+    if (err == cudaSuccess) err = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    if (err != cudaSuccess)
+    {
+        set_error("fps: kernel attribute: %s", cudaGetErrorString(err));
+        return TPK_ERR_CUDA;
+    }
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(static_cast<unsigned>(b) * nranks, 1, 1);
+    cfg.blockDim = dim3(kLargeThreads, 1, 1);
+    cfg.dynamicSmemBytes = lay.bytes;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = nranks;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    count_launches(1);
+    err = cudaLaunchKernelEx(&cfg, kernel, n, m, log2bs, nranks, lay, xyz, sorted, temp, idxs, new_xyz);
+    if (err != cudaSuccess)
+    {
+        set_error("fps launch (large clouds, cluster %d x %d points per lane): %s", nranks, P, cudaGetErrorString(err));
+        return TPK_ERR_CUDA;
+    }
+    return TPK_OK;
+}
+
+int sort_points(int b, int n, const float* xyz, float4* sorted, int* counters, cudaStream_t stream)
+{
+    // about four points per cell and at most 64^3 cells; the counters need 6 words more
+    int bits = 2;
+    while (bits < 6 && (32ll << (3 * bits)) <= n) ++bits;
+    const unsigned blocks = static_cast<unsigned>(n < 256 * 4 ? 1 : (n / (256 * 4) < 592 ? n / (256 * 4) : 592));
+    for (int b0 = 0; b0 < b; b0 += 65535)
+    {
+        const unsigned nb = static_cast<unsigned>(b - b0 < 65535 ? b - b0 : 65535);
+        const float* x = xyz + static_cast<size_t>(b0) * n * 3;
+        float4* s = sorted + static_cast<size_t>(b0) * n;
+        int* c = counters + static_cast<size_t>(b0) * n;
+        const dim3 grid(blocks, nb);
+        if (n < 512)
+        {
+            count_launches(1), large_copy_kernel<<<grid, 256, 0, stream>>>(n, x, s);
+            continue;
+        }
+        const int cells = 1 << (3 * bits);
+        count_launches(1), large_clear_kernel<<<dim3(blocks < 64 ? blocks : 64, nb), 256, 0, stream>>>(n, cells, c);
+        count_launches(1), large_box_kernel<<<grid, 256, 0, stream>>>(n, cells, x, c);
+        count_launches(1), large_cells_kernel<false><<<grid, 256, 0, stream>>>(n, bits, x, c, s);
+        count_launches(1), large_scan_kernel<<<nb, 1024, 0, stream>>>(n, cells, c);
+        count_launches(1), large_cells_kernel<true><<<grid, 256, 0, stream>>>(n, bits, x, c, s);
+    }
+    return check_launch("fps sort");
+}
+
+}  // namespace
+
+// scratch: the sorted copy (16 bytes per point), then the running minima (4 bytes per point)
+int fps_large(int b, int n, int m, int log2bs, const float* xyz, void* scratch, int32_t* idxs, float* new_xyz,
+              cudaStream_t stream)
+{
+    float4* sorted = static_cast<float4*>(scratch);
+    float* temp = reinterpret_cast<float*>(sorted + static_cast<size_t>(b) * n);
+    const int rc = sort_points(b, n, xyz, sorted, reinterpret_cast<int*>(temp), stream);
+    if (rc != TPK_OK) return rc;
+    // Seven clusters of 16 such CTAs run at once, 15 of eight.
+    int nranks = b <= 7 ? 16 : 8;
+    char text[64];
+    if (test_value("fps_config", text, sizeof(text)))
+    {
+        // test hook "fps_config=nranks:...": another cluster size for the same cloud
+        const int r = atoi(text);
+        if (r >= 1 && r <= kLargeMaxRanks && (r & (r - 1)) == 0) nranks = r;
+    }
+    // the smallest chunks of which a warp has at most 32
+    auto chunk_of = [&](int ranks) {
+        int p = 1;
+        while (p < 4 && (static_cast<long long>(n) + 32 * p - 1) / (32 * p) > 32ll * kLargeWarps * ranks) p *= 2;
+        return p;
+    };
+    int p = chunk_of(nranks);
+    LargeLayout lay = large_layout(n, nranks, p);
+    if (lay.bytes > kMaxSmemBytes - 2048)
+    {
+        nranks = kLargeMaxRanks;
+        p = chunk_of(nranks);
+        lay = large_layout(n, nranks, p);
+    }
+    if (p == 1) return launch_large<1>(b, n, m, log2bs, nranks, lay, xyz, sorted, temp, idxs, new_xyz, stream);
+    if (p == 2) return launch_large<2>(b, n, m, log2bs, nranks, lay, xyz, sorted, temp, idxs, new_xyz, stream);
+    return launch_large<4>(b, n, m, log2bs, nranks, lay, xyz, sorted, temp, idxs, new_xyz, stream);
+}
+
+// Largest cloud: 512 warps with 64 chunks of 128 points each.
+bool fps_large_fits(long long n) { return n <= 512ll * 64 * 128; }
+
+}  // namespace tpk
