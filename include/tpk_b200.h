@@ -393,6 +393,17 @@ TPK_API int tpk_gridding_f64(int b, int n_pts, float min_x, float max_x, float m
                              int32_t* grid_pt_indexes, void* stream);
 
 /*
+ * The same with a mask: points with keep (b,n_pts) uint8 zero are padding.  Their indexes are -1 and
+ * their weights 0: they add nothing to the grid and get no gradient.  keep may be NULL.
+ */
+TPK_API int tpk_gridding_keep_f32(int b, int n_pts, float min_x, float max_x, float min_y, float max_y,
+                                  float min_z, float max_z, const float* ptcloud, const uint8_t* keep, float* grid,
+                                  float* grid_pt_weights, int32_t* grid_pt_indexes, void* stream);
+TPK_API int tpk_gridding_keep_f64(int b, int n_pts, float min_x, float max_x, float min_y, float max_y,
+                                  float min_z, float max_z, const double* ptcloud, const uint8_t* keep, double* grid,
+                                  double* grid_pt_weights, int32_t* grid_pt_indexes, void* stream);
+
+/*
  * grad_ptcloud (b,n_pts,3) from grad_grid (b,n_grid_vertices): per axis the sum over the eight
  * vertices of +-grad * (the other two weights), in the reference's order (bit-identical).
  * Replaces gridding_grad_kernel_warpper, cuda/src/gridding_gpu.cu:306-333 (kernel :199-304).
@@ -429,6 +440,32 @@ TPK_API int tpk_cubic_feature_sampling_grad_f32(int b, int n_pts, int channels, 
 TPK_API int tpk_cubic_feature_sampling_grad_f64(int b, int n_pts, int channels, int scale, int neighborhood_size,
                                                 const double* grad_point_features, const int32_t* grid_pt_indexes,
                                                 double* grad_ptcloud, double* grad_cubic_features, void* stream);
+
+/*
+ * Both with scratch for a copy of the map that has the channel fastest; without scratch (NULL), or
+ * where the size is 0, the map is read in place.  TPK_ERR_SCRATCH if the buffer is shorter than
+ * tpk_cubic_feature_sampling_scratch_bytes() (itemsize 4 for f32, 8 for f64).
+ */
+TPK_API int64_t tpk_cubic_feature_sampling_scratch_bytes(int b, int n_pts, int channels, int scale, int neighborhood_size,
+                                                         int itemsize);
+TPK_API int tpk_cubic_feature_sampling_ws_f32(int b, int n_pts, int channels, int scale, int neighborhood_size,
+                                              const float* ptcloud, const float* cubic_features, float* point_features,
+                                              int32_t* grid_pt_indexes, void* scratch, int64_t scratch_bytes,
+                                              void* stream);
+TPK_API int tpk_cubic_feature_sampling_ws_f64(int b, int n_pts, int channels, int scale, int neighborhood_size,
+                                              const double* ptcloud, const double* cubic_features, double* point_features,
+                                              int32_t* grid_pt_indexes, void* scratch, int64_t scratch_bytes,
+                                              void* stream);
+TPK_API int tpk_cubic_feature_sampling_grad_ws_f32(int b, int n_pts, int channels, int scale,
+                                                   int neighborhood_size, const float* grad_point_features,
+                                                   const int32_t* grid_pt_indexes, float* grad_ptcloud,
+                                                   float* grad_cubic_features, void* scratch,
+                                                   int64_t scratch_bytes, void* stream);
+TPK_API int tpk_cubic_feature_sampling_grad_ws_f64(int b, int n_pts, int channels, int scale,
+                                                   int neighborhood_size, const double* grad_point_features,
+                                                   const int32_t* grid_pt_indexes, double* grad_ptcloud,
+                                                   double* grad_cubic_features, void* scratch,
+                                                   int64_t scratch_bytes, void* stream);
 
 /* ------------------------------------------- clustering and instance metrics ---- */
 

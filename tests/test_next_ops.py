@@ -226,6 +226,60 @@ def test_cubic_feature_sampling_matches_oracle_and_reference(B, n, c, scale, ns,
 
 
 @pytest.mark.gpu
+def test_gridding_padding_as_if_it_were_not_there():
+    """A padded batch against its clouds one by one without the padding: grids up to the order of the
+    additions (eight per point: 1e-6), gradients bit for bit, no gradient for padding."""
+    from torch_points_kernels_b200 import _lib, gridding
+
+    g = data.gen(8)
+    p = torch.rand(3, 700, 3, generator=g) * 1.7 - 0.9
+    p[0, ::3] = 0
+    p[2] = 0  # nothing but padding
+    p[1, 5] = torch.tensor([0.5, -0.25, -0.25])  # the sum is zero: padding as well
+    x = _cu(p).requires_grad_(True)
+    gg = _cu(torch.randn(3, 16 ** 3, generator=g))
+    grid = gridding.gridding(x, 8)
+    grid.backward(gg)
+    for b in range(3):
+        keep = p[b].sum(dim=1) != 0
+        y = _cu(p[b][keep] * 8)[None].requires_grad_(True)
+        one = gridding.GriddingFunction.apply(y, 8)
+        one.backward(gg[b:b + 1])
+        torch.testing.assert_close(grid[b], one[0], rtol=1e-6, atol=1e-6)
+        want = torch.zeros(700, 3)
+        want[keep] = y.grad[0].cpu() * 8
+        np.testing.assert_array_equal(x.grad[b].cpu().numpy(), want.numpy())
+    assert gridding.gridding(_cu(torch.zeros(0, 5, 3)), 4).shape == (1, 512)
+    assert _lib.device_status() == 0
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
+@pytest.mark.parametrize("B,n,c,scale,ns,offset", [(2, 400, 32, 10, 1, 0), (1, 300, 5, 9, 1, 0), (3, 200, 36, 7, 2, 0),
+                                                   (2, 173, 8, 11, 1, 1), (1, 1, 64, 2, 1, 0), (2, 100, 4, 33, 1, 0)])
+def test_cubic_feature_sampling_by_rows_matches_in_place(B, n, c, scale, ns, offset, dtype, monkeypatch):
+    """The copy with the channel fastest against the map read in place: values bit for bit, sums of a
+    vertex's points up to their order (at most a few hundred terms of order one)."""
+    from torch_points_kernels_b200.cubic_feature_sampling import CubicFeatureSamplingFunction
+
+    g = data.gen(n + c)
+    p = _cu((torch.rand(B, n, 3, generator=g) * (scale + 2) - 1).to(dtype))
+    cf = _cu(torch.randn(B, c, scale, scale, scale, generator=g).to(dtype))
+    size = B * n * (2 * ns) ** 3 * c
+    gout = _cu(torch.randn(size + offset, generator=g).to(dtype))[offset:].view(B, n, (2 * ns) ** 3, c)  # unaligned rows
+    got = []
+    for path in (None, "cubic_in_place"):
+        data.use_paths(monkeypatch, path)
+        f = cf.clone().requires_grad_(True)
+        out = CubicFeatureSamplingFunction.apply(p, f, ns)
+        out.backward(gout)
+        got.append((out.detach(), f.grad))
+    assert torch.equal(got[0][0], got[1][0])
+    tol = 1e-5 if dtype == torch.float32 else 1e-13
+    torch.testing.assert_close(got[0][1], got[1][1], rtol=tol, atol=10 * tol)
+
+
+@pytest.mark.gpu
 def test_grnet_float64_gradchecks():
     """The reference's own tests: test/test_gridding.py:21-31, test/test_cubic_feature_sampling.py:20-55."""
     from torch.autograd import gradcheck

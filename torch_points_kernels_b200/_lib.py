@@ -48,12 +48,18 @@ _SIGNATURES = {
     "tpk_chamfer_dist_grad_f64": [_c_int, _c_int, _ptr, _c_int, _ptr, _ptr, _ptr, _ptr, _ptr, _ptr, _ptr, _ptr],
     "tpk_gridding_f32": [_c_int, _c_int, _c_f32, _c_f32, _c_f32, _c_f32, _c_f32, _c_f32, _ptr, _ptr, _ptr, _ptr, _ptr],
     "tpk_gridding_f64": [_c_int, _c_int, _c_f32, _c_f32, _c_f32, _c_f32, _c_f32, _c_f32, _ptr, _ptr, _ptr, _ptr, _ptr],
+    "tpk_gridding_keep_f32": [_c_int, _c_int, _c_f32, _c_f32, _c_f32, _c_f32, _c_f32, _c_f32, _ptr, _ptr, _ptr, _ptr, _ptr, _ptr],
+    "tpk_gridding_keep_f64": [_c_int, _c_int, _c_f32, _c_f32, _c_f32, _c_f32, _c_f32, _c_f32, _ptr, _ptr, _ptr, _ptr, _ptr, _ptr],
     "tpk_gridding_grad_f32": [_c_int, _c_int, _c_i64, _ptr, _ptr, _ptr, _ptr, _ptr],
     "tpk_gridding_grad_f64": [_c_int, _c_int, _c_i64, _ptr, _ptr, _ptr, _ptr, _ptr],
     "tpk_cubic_feature_sampling_f32": [_c_int, _c_int, _c_int, _c_int, _c_int, _ptr, _ptr, _ptr, _ptr, _ptr],
     "tpk_cubic_feature_sampling_f64": [_c_int, _c_int, _c_int, _c_int, _c_int, _ptr, _ptr, _ptr, _ptr, _ptr],
     "tpk_cubic_feature_sampling_grad_f32": [_c_int, _c_int, _c_int, _c_int, _c_int, _ptr, _ptr, _ptr, _ptr, _ptr],
     "tpk_cubic_feature_sampling_grad_f64": [_c_int, _c_int, _c_int, _c_int, _c_int, _ptr, _ptr, _ptr, _ptr, _ptr],
+    "tpk_cubic_feature_sampling_ws_f32": [_c_int, _c_int, _c_int, _c_int, _c_int, _ptr, _ptr, _ptr, _ptr, _ptr, _c_i64, _ptr],
+    "tpk_cubic_feature_sampling_ws_f64": [_c_int, _c_int, _c_int, _c_int, _c_int, _ptr, _ptr, _ptr, _ptr, _ptr, _c_i64, _ptr],
+    "tpk_cubic_feature_sampling_grad_ws_f32": [_c_int, _c_int, _c_int, _c_int, _c_int, _ptr, _ptr, _ptr, _ptr, _ptr, _c_i64, _ptr],
+    "tpk_cubic_feature_sampling_grad_ws_f64": [_c_int, _c_int, _c_int, _c_int, _c_int, _ptr, _ptr, _ptr, _ptr, _ptr, _c_i64, _ptr],
     "tpk_sa_group": [_c_int, _c_int, _c_int, _c_int, _c_f32, _c_int, _ptr, _ptr, _ptr, _ptr, _ptr, _ptr, _ptr, _c_i64, _ptr],
     "tpk_grow_labels_step": [_c_i64, _c_int, _ptr, _ptr, _ptr, _c_int, _ptr],
     "tpk_instance_iou": [_c_int, _c_i64, _c_i64, _c_i64, _ptr, _ptr, _ptr, _ptr, _ptr, _ptr, _ptr, _ptr, _ptr],
@@ -63,7 +69,8 @@ EXPORTS = sorted(list(_SIGNATURES) + ["tpk_version", "tpk_last_error", "tpk_devi
                                        "tpk_fps_static_capacity", "tpk_ball_query_dense_scratch_bytes",
                                        "tpk_three_nn_scratch_bytes", "tpk_chamfer_dist_scratch_bytes",
                                        "tpk_ball_query_partial_dense_scratch_bytes", "tpk_knn_dense_scratch_bytes", "tpk_sa_group_scratch_bytes",
-                                       "tpk_knn_partial_dense_scratch_bytes", "tpk_grouping_grad_scratch_bytes"])
+                                       "tpk_knn_partial_dense_scratch_bytes", "tpk_cubic_feature_sampling_scratch_bytes",
+                                       "tpk_grouping_grad_scratch_bytes"])
 
 
 def lib():
@@ -105,6 +112,8 @@ def lib():
         handle.tpk_sa_group_scratch_bytes.restype = _c_i64
         handle.tpk_grouping_grad_scratch_bytes.argtypes = [_c_int, _c_int, _c_int, _c_int, _c_int]
         handle.tpk_grouping_grad_scratch_bytes.restype = _c_i64
+        handle.tpk_cubic_feature_sampling_scratch_bytes.argtypes = [_c_int] * 6
+        handle.tpk_cubic_feature_sampling_scratch_bytes.restype = _c_i64
         handle.tpk_fps_static_capacity.argtypes = []
         handle.tpk_fps_static_capacity.restype = _c_i64
         _lib = handle

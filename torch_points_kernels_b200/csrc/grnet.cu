@@ -14,6 +14,7 @@
 // One deliberate difference: the reference writes outside its tensors when a point lies
 // outside the grid (no bounds check on the eight vertex indices).  Here a vertex outside the
 // grid gets index -1 and contributes nothing, forward and backward.
+#include <climits>
 #include <type_traits>
 
 #include "tpk_common.cuh"
@@ -72,11 +73,18 @@ __device__ __forceinline__ T vertex_weight(T x, int x0)
 template <class T>
 __global__ void __launch_bounds__(kGrThreads)
     gridding_kernel(long long total, int n_pts, long long n_grid_vertices, float min_x, float min_y, float min_z, int len_x,
-                    int len_y, int len_z, const T* __restrict__ ptcloud, T* __restrict__ grid,
-                    T* __restrict__ grid_pt_weights, int* __restrict__ grid_pt_indexes)
+                    int len_y, int len_z, const T* __restrict__ ptcloud, const uint8_t* __restrict__ keep,
+                    T* __restrict__ grid, T* __restrict__ grid_pt_weights, int* __restrict__ grid_pt_indexes)
 {
     const long long t = static_cast<long long>(blockIdx.x) * kGrThreads + threadIdx.x;
     if (t >= total) return;
+    if (keep != nullptr && keep[t] == 0)
+    {
+        // padding: as if the point were not there
+        for (int v = 0; v < 8; ++v) grid_pt_indexes[8 * t + v] = -1;
+        for (int v = 0; v < 24; ++v) grid_pt_weights[24 * t + v] = static_cast<T>(0);
+        return;
+    }
     const long long cloud = t / n_pts;
     const T px = ptcloud[3 * t + 0], py = ptcloud[3 * t + 1], pz = ptcloud[3 * t + 2];
     int lo[3], up[3];
@@ -201,6 +209,88 @@ __global__ void __launch_bounds__(kGrThreads)
     atomicAdd(grad_cubic_features + (cloud * channels + k) * cub_scale + vertex, grad_point_features[t]);
 }
 
+// ---- through a copy of the map with the channel fastest
+//
+// The map has one plane of scale^3 values per channel, a row of the output all channels of a vertex:
+// read in place, every value is a 32-byte sector of its own (58.7 M of them for 16 clouds of 2048
+// points and maps of 32, 64 and 128 channels), and every addition of the gradient an atomic on one.
+// A tiled transposition is two coalesced passes over the map, after which a row is contiguous: 16
+// bytes per thread and load, or per vector reduction.
+
+// out[batch][c][r] = in[batch][r][c]; one 32 x 32 tile per CTA step.
+template <class T>
+__global__ void __launch_bounds__(kGrThreads)
+    transpose_kernel(long long tiles, int rows, int cols, int tiles_r, int tiles_c, const T* __restrict__ in, T* __restrict__ out)
+{
+    __shared__ T tile[32][33];
+    const int lane = threadIdx.x & 31, line = threadIdx.x >> 5;
+    for (long long t = blockIdx.x; t < tiles; t += gridDim.x)
+    {
+        const long long batch = t / (static_cast<long long>(tiles_r) * tiles_c);
+        const int rest = static_cast<int>(t - batch * tiles_r * tiles_c);
+        const int r0 = rest / tiles_c * 32, c0 = rest % tiles_c * 32;
+        const T* src = in + batch * rows * cols;
+        T* dst = out + batch * rows * cols;
+#pragma unroll
+        for (int i = 0; i < 32; i += kGrThreads / 32)
+            if (r0 + line + i < rows && c0 + lane < cols)
+                tile[line + i][lane] = __ldg(src + static_cast<long long>(r0 + line + i) * cols + c0 + lane);
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < 32; i += kGrThreads / 32)
+            if (c0 + line + i < cols && r0 + lane < rows)
+                dst[static_cast<long long>(c0 + line + i) * rows + r0 + lane] = tile[lane][line + i];
+        __syncthreads();
+    }
+}
+
+template <class T>
+void transpose(int b, int rows, int cols, const T* in, T* out, cudaStream_t s)
+{
+    const int tr = (rows + 31) / 32, tc = (cols + 31) / 32;
+    const long long tiles = static_cast<long long>(b) * tr * tc;
+    const unsigned g = static_cast<unsigned>(tiles < num_sms() * 64ll ? tiles : num_sms() * 64ll);
+    count_launches(1), transpose_kernel<T><<<g, kGrThreads, 0, s>>>(tiles, rows, cols, tr, tc, in, out);
+}
+
+// V: what a thread moves, T or four of it (channels a multiple of four, everything 16-byte aligned).
+template <class V>
+__global__ void __launch_bounds__(kGrThreads)
+    cubic_gather_rows_kernel(long long total, long long per_cloud, int row, long long cub_scale, const V* __restrict__ rows,
+                             const int* __restrict__ grid_pt_indexes, V* __restrict__ point_features)
+{
+    const long long t = static_cast<long long>(blockIdx.x) * kGrThreads + threadIdx.x;
+    if (t >= total) return;
+    const long long pv = t / row;
+    const int vertex = __ldg(grid_pt_indexes + pv);
+    V v = {};
+    if (vertex >= 0 && vertex < cub_scale) v = __ldg(rows + (pv / per_cloud * cub_scale + vertex) * row + (t - pv * row));
+    point_features[t] = v;
+}
+
+template <class V>
+__global__ void __launch_bounds__(kGrThreads)
+    cubic_scatter_rows_kernel(long long total, long long per_cloud, int row, long long cub_scale,
+                              const V* __restrict__ grad_point_features, const int* __restrict__ grid_pt_indexes,
+                              V* __restrict__ rows)
+{
+    const long long t = static_cast<long long>(blockIdx.x) * kGrThreads + threadIdx.x;
+    if (t >= total) return;
+    const long long pv = t / row;
+    const int vertex = __ldg(grid_pt_indexes + pv);
+    if (vertex < 0 || vertex >= cub_scale) return;
+    atomicAdd(rows + (pv / per_cloud * cub_scale + vertex) * row + (t - pv * row), __ldg(grad_point_features + t));
+}
+
+// Where the copy pays: two passes over the map against what the rows save.
+bool cubic_by_rows(int n_pts, int nvert, int channels, long long cub_scale)
+{
+    if (test_path("cubic_in_place")) return false;
+    return channels >= 4 && static_cast<long long>(n_pts) * nvert * 3 > cub_scale;
+}
+
+inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
+
 int grid_blocks(long long total, unsigned* out, const char* what)
 {
     const long long g = (total + kGrThreads - 1) / kGrThreads;
@@ -215,7 +305,7 @@ int grid_blocks(long long total, unsigned* out, const char* what)
 
 template <class T>
 int gridding_impl(int b, int n_pts, float min_x, float max_x, float min_y, float max_y, float min_z, float max_z,
-                  const T* ptcloud, T* grid, T* grid_pt_weights, int32_t* grid_pt_indexes, cudaStream_t s)
+                  const T* ptcloud, const uint8_t* keep, T* grid, T* grid_pt_weights, int32_t* grid_pt_indexes, cudaStream_t s)
 {
     TPK_REQUIRE(b >= 0 && n_pts >= 0, "gridding: negative size");
     const int len_x = static_cast<int>(max_x - min_x + 1), len_y = static_cast<int>(max_y - min_y + 1),
@@ -238,7 +328,7 @@ int gridding_impl(int b, int n_pts, float min_x, float max_x, float min_y, float
     const int rc = grid_blocks(total, &g, "gridding");
     if (rc != TPK_OK) return rc;
     count_launches(1), gridding_kernel<T><<<g, kGrThreads, 0, s>>>(total, n_pts, nv, min_x, min_y, min_z, len_x, len_y, len_z,
-                                                                ptcloud, grid, grid_pt_weights, grid_pt_indexes);
+                                                                ptcloud, keep, grid, grid_pt_weights, grid_pt_indexes);
     return check_launch("gridding");
 }
 
@@ -258,9 +348,29 @@ int gridding_grad_impl(int b, int n_pts, int64_t n_grid_vertices, const T* grid_
     return check_launch("gridding_grad");
 }
 
+// Bytes of the copy, 0 where the map is read in place.
+int64_t rows_scratch(int b, int n_pts, int channels, int scale, int neighborhood_size, int itemsize)
+{
+    if (b <= 0 || n_pts <= 0 || channels <= 0 || scale <= 0 || neighborhood_size < 1 || neighborhood_size > 8) return 0;
+    const long long cub = static_cast<long long>(scale) * scale * scale;
+    const int nvert = 8 * neighborhood_size * neighborhood_size * neighborhood_size;
+    if (cub > INT_MAX || !cubic_by_rows(n_pts, nvert, channels, cub)) return 0;
+    return static_cast<int64_t>(b) * channels * cub * itemsize;
+}
+
+template <class T>
+int check_rows_scratch(int b, int n_pts, int channels, int scale, int neighborhood_size, int64_t bytes)
+{
+    const int64_t need = rows_scratch(b, n_pts, channels, scale, neighborhood_size, sizeof(T));
+    if (bytes >= need) return TPK_OK;
+    set_error("cubic_feature_sampling: scratch of %lld bytes given, %lld needed", static_cast<long long>(bytes),
+              static_cast<long long>(need));
+    return TPK_ERR_SCRATCH;
+}
+
 template <class T>
 int cubic_impl(int b, int n_pts, int channels, int scale, int neighborhood_size, const T* ptcloud, const T* cubic_features,
-               T* point_features, int32_t* grid_pt_indexes, cudaStream_t s)
+               T* point_features, int32_t* grid_pt_indexes, T* scratch, int64_t scratch_bytes, cudaStream_t s)
 {
     TPK_REQUIRE(b >= 0 && n_pts >= 0 && channels >= 0 && scale > 0 && neighborhood_size >= 1 && neighborhood_size <= 8,
                 "cubic_feature_sampling: size out of range");
@@ -273,31 +383,63 @@ int cubic_impl(int b, int n_pts, int channels, int scale, int neighborhood_size,
     int rc = grid_blocks(pts, &g, "cubic_feature_sampling");
     if (rc != TPK_OK) return rc;
     count_launches(1), cubic_index_kernel<T><<<g, kGrThreads, 0, s>>>(pts, scale, neighborhood_size - 1, nvert, ptcloud, grid_pt_indexes);
+    const long long cub = static_cast<long long>(scale) * scale * scale;
+    if (scratch != nullptr)
+    {
+        rc = check_rows_scratch<T>(b, n_pts, channels, scale, neighborhood_size, scratch_bytes);
+        if (rc != TPK_OK) return rc;
+        if (rows_scratch(b, n_pts, channels, scale, neighborhood_size, sizeof(T)) > 0)
+        {
+            const long long total = pts * nvert * channels, per_cloud = static_cast<long long>(n_pts) * nvert;
+            const bool four = std::is_same<T, float>::value && channels % 4 == 0 && aligned16(scratch) && aligned16(point_features);
+            rc = grid_blocks(four ? total / 4 : total, &g, "cubic_feature_sampling");
+            if (rc != TPK_OK) return rc;
+            transpose(b, channels, static_cast<int>(cub), cubic_features, scratch, s);
+            count_launches(1);
+            if (four)
+                cubic_gather_rows_kernel<float4><<<g, kGrThreads, 0, s>>>(total / 4, per_cloud, channels / 4, cub,
+                                                                        reinterpret_cast<const float4*>(scratch), grid_pt_indexes,
+                                                                        reinterpret_cast<float4*>(point_features));
+            else
+                cubic_gather_rows_kernel<T><<<g, kGrThreads, 0, s>>>(total, per_cloud, channels, cub, scratch, grid_pt_indexes,
+                                                                   point_features);
+            return check_launch("cubic_feature_sampling");
+        }
+    }
     if (channels > 0)
     {
         const long long total = pts * nvert * channels;
         rc = grid_blocks(total, &g, "cubic_feature_sampling");
         if (rc != TPK_OK) return rc;
         count_launches(1), cubic_gather_kernel<T><<<g, kGrThreads, 0, s>>>(total, n_pts, nvert, channels,
-                                                                        static_cast<long long>(scale) * scale * scale,
-                                                                        cubic_features, grid_pt_indexes, point_features);
+                                                                        cub, cubic_features, grid_pt_indexes, point_features);
     }
     return check_launch("cubic_feature_sampling");
 }
 
 template <class T>
 int cubic_grad_impl(int b, int n_pts, int channels, int scale, int neighborhood_size, const T* grad_point_features,
-                    const int32_t* grid_pt_indexes, T* grad_ptcloud, T* grad_cubic_features, cudaStream_t s)
+                    const int32_t* grid_pt_indexes, T* grad_ptcloud, T* grad_cubic_features, T* scratch, int64_t scratch_bytes,
+                    cudaStream_t s)
 {
     TPK_REQUIRE(b >= 0 && n_pts >= 0 && channels >= 0 && scale > 0 && neighborhood_size >= 1 && neighborhood_size <= 8,
                 "cubic_feature_sampling_grad: size out of range");
     if (b == 0) return TPK_OK;
     const long long cub = static_cast<long long>(scale) * scale * scale;
+    const int nvert = 8 * neighborhood_size * neighborhood_size * neighborhood_size;
+    bool by_rows = false;
+    if (scratch != nullptr)
+    {
+        const int rc = check_rows_scratch<T>(b, n_pts, channels, scale, neighborhood_size, scratch_bytes);
+        if (rc != TPK_OK) return rc;
+        by_rows = rows_scratch(b, n_pts, channels, scale, neighborhood_size, sizeof(T)) > 0;
+    }
+    T* sums = by_rows ? scratch : grad_cubic_features;
     cudaError_t err = cudaSuccess;
     // the coordinates get no gradient: floor and ceil are flat (cubic_feature_sampling_gpu.cu:139-144)
     if (grad_ptcloud && n_pts > 0) err = cudaMemsetAsync(grad_ptcloud, 0, sizeof(T) * static_cast<size_t>(b) * n_pts * 3, s);
-    if (err == cudaSuccess && grad_cubic_features && channels > 0)
-        err = cudaMemsetAsync(grad_cubic_features, 0, sizeof(T) * static_cast<size_t>(b) * channels * cub, s);
+    if (err == cudaSuccess && sums && channels > 0)
+        err = cudaMemsetAsync(sums, 0, sizeof(T) * static_cast<size_t>(b) * channels * cub, s);
     if (err != cudaSuccess)
     {
         set_error("cubic_feature_sampling_grad: memset: %s", cudaGetErrorString(err));
@@ -305,11 +447,26 @@ int cubic_grad_impl(int b, int n_pts, int channels, int scale, int neighborhood_
     }
     if (n_pts == 0 || channels == 0) return TPK_OK;
     TPK_REQUIRE(grad_point_features && grid_pt_indexes && grad_cubic_features, "cubic_feature_sampling_grad: NULL pointer");
-    const int nvert = 8 * neighborhood_size * neighborhood_size * neighborhood_size;
     const long long total = static_cast<long long>(b) * n_pts * nvert * channels;
+    const long long per_cloud = static_cast<long long>(n_pts) * nvert;
+    const bool four = by_rows && std::is_same<T, float>::value && channels % 4 == 0 && aligned16(scratch) &&
+                      aligned16(grad_point_features);
     unsigned g;
-    const int rc = grid_blocks(total, &g, "cubic_feature_sampling_grad");
+    const int rc = grid_blocks(four ? total / 4 : total, &g, "cubic_feature_sampling_grad");
     if (rc != TPK_OK) return rc;
+    if (by_rows)
+    {
+        count_launches(1);
+        if (four)
+            cubic_scatter_rows_kernel<float4><<<g, kGrThreads, 0, s>>>(total / 4, per_cloud, channels / 4, cub,
+                                                                     reinterpret_cast<const float4*>(grad_point_features),
+                                                                     grid_pt_indexes, reinterpret_cast<float4*>(scratch));
+        else
+            cubic_scatter_rows_kernel<T><<<g, kGrThreads, 0, s>>>(total, per_cloud, channels, cub, grad_point_features,
+                                                                grid_pt_indexes, scratch);
+        transpose(b, static_cast<int>(cub), channels, scratch, grad_cubic_features, s);
+        return check_launch("cubic_feature_sampling_grad");
+    }
     count_launches(1), cubic_scatter_kernel<T><<<g, kGrThreads, 0, s>>>(total, n_pts, nvert, channels, cub, grad_point_features,
                                                                      grid_pt_indexes, grad_cubic_features);
     return check_launch("cubic_feature_sampling_grad");
@@ -323,8 +480,15 @@ int cubic_grad_impl(int b, int n_pts, int channels, int scale, int neighborhood_
                                          float max_z, const T* ptcloud, T* grid, T* grid_pt_weights,                  \
                                          int32_t* grid_pt_indexes, void* stream)                                       \
     {                                                                                                                   \
-        return tpk::gridding_impl<T>(b, n_pts, min_x, max_x, min_y, max_y, min_z, max_z, ptcloud, grid, grid_pt_weights, \
-                                     grid_pt_indexes, static_cast<cudaStream_t>(stream));                              \
+        return tpk::gridding_impl<T>(b, n_pts, min_x, max_x, min_y, max_y, min_z, max_z, ptcloud, nullptr, grid,       \
+                                     grid_pt_weights, grid_pt_indexes, static_cast<cudaStream_t>(stream));             \
+    }                                                                                                                   \
+    extern "C" int tpk_gridding_keep_##SUFFIX(int b, int n_pts, float min_x, float max_x, float min_y, float max_y,     \
+                                              float min_z, float max_z, const T* ptcloud, const uint8_t* keep, T* grid, \
+                                              T* grid_pt_weights, int32_t* grid_pt_indexes, void* stream)              \
+    {                                                                                                                   \
+        return tpk::gridding_impl<T>(b, n_pts, min_x, max_x, min_y, max_y, min_z, max_z, ptcloud, keep, grid,          \
+                                     grid_pt_weights, grid_pt_indexes, static_cast<cudaStream_t>(stream));             \
     }                                                                                                                   \
     extern "C" int tpk_gridding_grad_##SUFFIX(int b, int n_pts, int64_t n_grid_vertices, const T* grid_pt_weights,      \
                                               const int32_t* grid_pt_indexes, const T* grad_grid, T* grad_ptcloud,     \
@@ -338,7 +502,17 @@ int cubic_grad_impl(int b, int n_pts, int channels, int scale, int neighborhood_
                                                        int32_t* grid_pt_indexes, void* stream)                         \
     {                                                                                                                   \
         return tpk::cubic_impl<T>(b, n_pts, channels, scale, neighborhood_size, ptcloud, cubic_features, point_features, \
-                                  grid_pt_indexes, static_cast<cudaStream_t>(stream));                                 \
+                                  grid_pt_indexes, nullptr, 0, static_cast<cudaStream_t>(stream));                     \
+    }                                                                                                                   \
+    extern "C" int tpk_cubic_feature_sampling_ws_##SUFFIX(int b, int n_pts, int channels, int scale,                    \
+                                                          int neighborhood_size, const T* ptcloud,                     \
+                                                          const T* cubic_features, T* point_features,                  \
+                                                          int32_t* grid_pt_indexes, void* scratch,                     \
+                                                          int64_t scratch_bytes, void* stream)                         \
+    {                                                                                                                   \
+        return tpk::cubic_impl<T>(b, n_pts, channels, scale, neighborhood_size, ptcloud, cubic_features, point_features, \
+                                  grid_pt_indexes, static_cast<T*>(scratch), scratch_bytes,                            \
+                                  static_cast<cudaStream_t>(stream));                                                  \
     }                                                                                                                   \
     extern "C" int tpk_cubic_feature_sampling_grad_##SUFFIX(int b, int n_pts, int channels, int scale,                  \
                                                             int neighborhood_size, const T* grad_point_features,       \
@@ -346,10 +520,26 @@ int cubic_grad_impl(int b, int n_pts, int channels, int scale, int neighborhood_
                                                             T* grad_cubic_features, void* stream)                      \
     {                                                                                                                   \
         return tpk::cubic_grad_impl<T>(b, n_pts, channels, scale, neighborhood_size, grad_point_features,              \
-                                       grid_pt_indexes, grad_ptcloud, grad_cubic_features,                             \
+                                       grid_pt_indexes, grad_ptcloud, grad_cubic_features, nullptr, 0,                 \
                                        static_cast<cudaStream_t>(stream));                                             \
+    }                                                                                                                   \
+    extern "C" int tpk_cubic_feature_sampling_grad_ws_##SUFFIX(int b, int n_pts, int channels, int scale,               \
+                                                               int neighborhood_size, const T* grad_point_features,    \
+                                                               const int32_t* grid_pt_indexes, T* grad_ptcloud,        \
+                                                               T* grad_cubic_features, void* scratch,                  \
+                                                               int64_t scratch_bytes, void* stream)                    \
+    {                                                                                                                   \
+        return tpk::cubic_grad_impl<T>(b, n_pts, channels, scale, neighborhood_size, grad_point_features,              \
+                                       grid_pt_indexes, grad_ptcloud, grad_cubic_features, static_cast<T*>(scratch),   \
+                                       scratch_bytes, static_cast<cudaStream_t>(stream));                              \
     }
 
 TPK_GRNET_ENTRY(f32, float)
 TPK_GRNET_ENTRY(f64, double)
 #undef TPK_GRNET_ENTRY
+
+extern "C" int64_t tpk_cubic_feature_sampling_scratch_bytes(int b, int n_pts, int channels, int scale, int neighborhood_size,
+                                                            int itemsize)
+{
+    return tpk::rows_scratch(b, n_pts, channels, scale, neighborhood_size, itemsize);
+}

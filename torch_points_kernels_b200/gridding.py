@@ -15,10 +15,11 @@ def _suffix(t, what):
 
 
 class GriddingFunction(torch.autograd.Function):
-    """grid = gridding(ptcloud) on the cube [-scale, scale - 1]^3; ptcloud is in grid units."""
+    """grid = gridding(ptcloud) on the cube [-scale, scale - 1]^3; ptcloud is in grid units.  Points
+    whose place in keep (bool, (B, n_pts)) is False are padding."""
 
     @staticmethod
-    def forward(ctx, ptcloud, scale):
+    def forward(ctx, ptcloud, scale, keep=None):
         sfx = _suffix(ptcloud, "ptcloud")
         ptcloud = ptcloud.contiguous()
         b, n = ptcloud.shape[0], ptcloud.shape[1]
@@ -27,9 +28,9 @@ class GriddingFunction(torch.autograd.Function):
         weights = torch.empty((b, n, 8, 3), dtype=ptcloud.dtype, device=ptcloud.device)
         indexes = torch.empty((b, n, 8), dtype=torch.int32, device=ptcloud.device)
         with torch.cuda.device(ptcloud.device):
-            _lib.call("tpk_gridding_" + sfx, b, n, float(-scale), float(scale - 1), float(-scale), float(scale - 1),
-                      float(-scale), float(scale - 1), _lib.ptr(ptcloud), _lib.ptr(grid), _lib.ptr(weights),
-                      _lib.ptr(indexes), _lib.stream_of(ptcloud))
+            _lib.call("tpk_gridding_keep_" + sfx, b, n, float(-scale), float(scale - 1), float(-scale), float(scale - 1),
+                      float(-scale), float(scale - 1), _lib.ptr(ptcloud), _lib.ptr(keep), _lib.ptr(grid),
+                      _lib.ptr(weights), _lib.ptr(indexes), _lib.stream_of(ptcloud))
         ctx.save_for_backward(weights, indexes)
         return grid
 
@@ -43,7 +44,7 @@ class GriddingFunction(torch.autograd.Function):
         with torch.cuda.device(weights.device):
             _lib.call("tpk_gridding_grad_" + sfx, b, n, grad_grid.shape[1], _lib.ptr(weights), _lib.ptr(indexes),
                       _lib.ptr(grad_grid), _lib.ptr(grad_ptcloud), _lib.stream_of(weights))
-        return grad_ptcloud, None
+        return grad_ptcloud, None, None
 
 
 def gridding(ptcloud, scale):
@@ -67,11 +68,7 @@ def gridding(ptcloud, scale):
         raise ValueError("The input point cloud should be of size (B, n_pts, 3)")
 
     ptcloud = ptcloud * scale
-    grids = []
-    # points whose coordinates sum to zero are padding and are dropped, cloud by cloud
-    # (reference: gridding.py:54-60)
-    for p in torch.split(ptcloud, 1, dim=0):
-        non_zeros = torch.sum(p, dim=2).ne(0)
-        p = p[non_zeros].unsqueeze(dim=0)
-        grids.append(GriddingFunction.apply(p, scale))
-    return torch.cat(grids, dim=0).contiguous()
+    if ptcloud.shape[0] == 0:
+        ptcloud = ptcloud.reshape(1, 0, 3)  # one empty grid
+    # points whose coordinates sum to zero are padding (reference: gridding.py:54-60)
+    return GriddingFunction.apply(ptcloud, scale, torch.sum(ptcloud, dim=2).ne(0))
