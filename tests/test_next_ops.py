@@ -280,6 +280,29 @@ def test_cubic_feature_sampling_by_rows_matches_in_place(B, n, c, scale, ns, off
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("ignore,min_size", [([0], 4), ([], 1), ([3, 1], 2), ([0, 1, 2, 3, 7], 1)])
+def test_region_grow_is_the_search_of_every_label(ignore, min_size):
+    import torch_points_kernels_b200 as tpk
+
+    g = data.gen(17)
+    n = 6000
+    pos = _cu(torch.rand(n, 3, generator=g))
+    labels = _cu(torch.tensor([0, 1, 2, 3, 7])[torch.randint(0, 5, (n,), generator=g)])
+    batch = _cu(torch.sort(torch.tensor([0, 2, 3])[torch.randint(0, 3, (n,), generator=g)]).values)
+    labels[batch == 2] = 7  # a sample with one label only
+    got = tpk.region_grow(pos, labels, batch, ignore_labels=ignore, nsample=8, radius=0.06, min_cluster_size=min_size)
+    want = []
+    for l in torch.unique(labels).tolist():
+        if l in ignore:
+            continue
+        at = (labels == l).nonzero()[:, 0]
+        inner = torch.unique(batch[at], return_inverse=True)[1]
+        for c in tpk.grow_proximity(pos[at], inner, nsample=8, radius=0.06, min_cluster_size=min_size):
+            want.append(at[torch.tensor(c, device=at.device)].tolist())
+    assert [c.tolist() for c in got] == want
+
+
+@pytest.mark.gpu
 def test_grnet_float64_gradchecks():
     """The reference's own tests: test/test_gridding.py:21-31, test/test_cubic_feature_sampling.py:20-55."""
     from torch.autograd import gradcheck

@@ -80,33 +80,23 @@ def region_grow(
     assert pos.dim() == 2
     assert pos.shape[0] == labels.shape[0]
 
-    unique_labels = torch.unique(labels)
-    clusters = []
-    ind = torch.arange(0, pos.shape[0], device=pos.device)
-    for l in unique_labels:
-        if l in ignore_labels:
-            continue
-
-        # Build clusters for a given label (ignore other points)
-        label_mask = labels == l
-        local_ind = ind[label_mask]
-
-        # Remap batch to a continuous sequence (batch is sorted, so is the remapped vector)
-        label_batch = batch[label_mask]
-        remaped_batch = torch.unique(label_batch, return_inverse=True)[1]
-
-        # Cluster
-        label_clusters = grow_proximity(
-            pos[label_mask, :],
-            remaped_batch,
-            nsample=nsample,
-            radius=radius,
-            min_cluster_size=min_cluster_size,
-        )
-
-        # Remap indices to original coordinates
-        for cluster in label_clusters:
-            cluster = torch.tensor(cluster, device=pos.device)
-            clusters.append(local_ind[cluster])
-
-    return clusters
+    unique_labels, label_rank = torch.unique(labels, return_inverse=True)
+    kept = [not (l in ignore_labels) for l in unique_labels.cpu()]
+    if not any(kept):
+        return []
+    # One search and one labelling for all labels: the points ordered by label (original order inside a
+    # label), every (label, sample) pair a segment of its own.  Lists, seeds and the order of the clusters
+    # are those of a search per label, because the order inside a segment is the same.
+    rank_h = torch.tensor([sum(kept[:i]) if k else -1 for i, k in enumerate(kept)])
+    rank = rank_h.to(pos.device)[label_rank]
+    ind = (rank >= 0).nonzero()[:, 0]
+    ind = ind[torch.sort(rank[ind], stable=True).indices]
+    sample = batch[ind].long()
+    segment = torch.unique(rank[ind] * (sample.max() + 1) + sample, return_inverse=True)[1]
+    local_pos = pos[ind].float().contiguous()
+    neighbours = ball_query_partial_dense(radius, nsample, local_pos, local_pos, segment, segment)[0]
+    seeds = cluster_labels(neighbours)
+    seeds, order = torch.sort(seeds, stable=True)  # members ascending inside a cluster
+    counts = torch.unique_consecutive(seeds, return_counts=True)[1].tolist()
+    clusters = torch.split(ind[order], counts)
+    return [c for c in clusters if c.shape[0] >= min_cluster_size]
