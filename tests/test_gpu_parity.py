@@ -186,6 +186,43 @@ def test_fps_large_rounds_every_chunk_size(n, m, ranks, kind, monkeypatch):
     assert _lib.device_status() == 0
 
 
+@pytest.mark.parametrize("n,m,ns,r", [(1, 3, 2, 0.5), (5, 1, 9, 3.0), (127, 33, 8, 0.4), (1025, 70, 32, 0.3), (1027, 70, 3, 0.6),
+                                      (4097, 5, 64, 0.2), (1536, 40, 1, 0.01)])
+@pytest.mark.parametrize("per_warp", ["1", "2", "4"])
+def test_ball_query_warp_scan_matches_oracle(n, m, ns, r, per_warp, monkeypatch):
+    """Clouds that begin at every offset from a 16-byte boundary, heads, tails, full and empty balls,
+    coordinates that are not finite."""
+    data.use_paths(monkeypatch, "ball_warp_scan", "ball_warp_scan_q=" + per_warp)
+    x = data.unit_ball(4, n, seed=n).numpy().copy()
+    y = data.unit_ball(4, m, seed=n + 1).numpy().copy()
+    x[1, n // 2, 1] = np.nan
+    y[2, 0, 0] = np.inf
+    idx, dist = tpk.ball_query(r, ns, cu(x), cu(y), mode="dense")
+    oi, od = orc.ball_query_dense(r, ns, x, y)
+    np.testing.assert_array_equal(npy(idx), oi)
+    np.testing.assert_array_equal(npy(dist).view(np.int32), od.view(np.int32))
+    assert _lib.device_status() == 0
+
+
+@pytest.mark.parametrize("spread", [0.0, 0.02, 1.0])
+def test_ball_query_crowded_centres_are_scanned(spread, monkeypatch):
+    """What the grids leave over (more candidates than they take): dense and packed against the scan alone."""
+    g = data.gen(3)
+    x = torch.randn(2, 40000, 3, generator=g)
+    x[:, ::2] = x[:, :1] + spread * x[:, ::2]  # half of the points in one place
+    y = x[:, ::37].contiguous()
+    seg_x, seg_y = (torch.arange(2).repeat_interleave(k) for k in (40000, y.shape[1]))
+    got = []
+    for path in ("ball_query_no_warp_scan", "ball_query_global_grid", "ball_query_scan"):
+        data.use_paths(monkeypatch, path, "ball_query_no_warp_scan")
+        got.append(tpk.ball_query(0.3, 20, cu(x), cu(y), mode="dense") +
+                   tpk.ball_query(0.3, 20, cu(x.view(-1, 3)), cu(y.view(-1, 3)), mode="partial_dense", batch_x=cu(seg_x),
+                                  batch_y=cu(seg_y)))
+    for other in got[1:]:
+        for a, b in zip(got[0], other):
+            assert torch.equal(a, b)
+
+
 @pytest.mark.parametrize("family", ["fps_sorted", "fps_sorted,fps_global", "fps_unsorted"])
 def test_fps_coordinates_too_large_for_a_box(family, monkeypatch):
     data.use_paths(monkeypatch, family)

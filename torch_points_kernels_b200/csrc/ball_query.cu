@@ -34,6 +34,14 @@ bool sg_ball_query_fits(int b, int n, int nsample);
 int sg_ball_query(int b, int n, int m, float radius, int nsample, const float* new_xyz, const float* xyz,
                   int64_t* idx, float* dist, unsigned char* need, cudaStream_t s);
 
+// ball_scan.cu
+bool ball_scan_wanted(int b, int n, int m);
+int ball_scan_dense(int b, int n, int m, float radius, int nsample, const float* new_xyz, const float* xyz, int64_t* idx,
+                    float* dist, const unsigned char* need, cudaStream_t s);
+int ball_scan_partial(long long size_x, long long size_y, float radius, int nsample, const float* x, const float* y,
+                      const int64_t* batch_x, const int64_t* batch_y, int64_t* idx, float* dist, const unsigned char* need,
+                      cudaStream_t s);
+
 namespace
 {
 
@@ -272,6 +280,8 @@ extern "C" int tpk_ball_query_dense(int b, int n, int m, float radius, int nsamp
     if (b == 0 || m == 0 || nsample == 0) return TPK_OK;
     TPK_REQUIRE(new_xyz && idx && dist && (xyz || n == 0), "ball_query_dense: NULL pointer");
     cudaStream_t s = static_cast<cudaStream_t>(stream);
+    if (!test_path("ball_query_scan") && ball_scan_wanted(b, n, m))
+        return ball_scan_dense(b, n, m, radius, nsample, new_xyz, xyz, idx, dist, nullptr, s);
     int threads, q;
     pick_shape(static_cast<long long>(b) * m, &threads, &q);
     const int tiles = (m + threads * q - 1) / (threads * q);
@@ -330,6 +340,7 @@ extern "C" int tpk_ball_query_dense_ws(int b, int n, int m, float radius, int ns
     TPK_REQUIRE(new_xyz && xyz && idx && dist, "ball_query_dense: NULL pointer");
     TPK_REQUIRE((reinterpret_cast<uintptr_t>(scratch) & 255u) == 0, "ball_query_dense: scratch must be 256-byte aligned");
     cudaStream_t s = static_cast<cudaStream_t>(stream);
+    if (ball_scan_wanted(b, n, m)) return ball_scan_dense(b, n, m, radius, nsample, new_xyz, xyz, idx, dist, nullptr, s);
     const unsigned char* need = nullptr;
     int rc;
     if (use_smem_grid(b, n, nsample))
@@ -351,6 +362,7 @@ extern "C" int tpk_ball_query_dense_ws(int b, int n, int m, float radius, int ns
     }
     if (rc != TPK_OK) return rc;
     // centres the grid left over (dense neighbourhoods, degenerate clouds): index-order scan
+    if (need != nullptr) return ball_scan_dense(b, n, m, radius, nsample, new_xyz, xyz, idx, dist, need, s);
     int threads, q;
     pick_shape(static_cast<long long>(b) * m, &threads, &q);
     const int tiles = (m + threads * q - 1) / (threads * q);
@@ -425,5 +437,5 @@ extern "C" int tpk_ball_query_partial_dense_ws(int64_t size_x, int64_t size_y, f
     const int rc = hash_grid_ball_query(size_x, size_y, radius, nsample, x, y, batch_x, batch_y, idx, dist, scratch, &need, s);
     if (rc != TPK_OK) return rc;
     // queries the grid left over (crowded neighbourhoods, non-finite coordinates): index-order scan
-    return launch_partial_scan(size_x, size_y, radius, nsample, x, y, batch_x, batch_y, idx, dist, need, s);
+    return ball_scan_partial(size_x, size_y, radius, nsample, x, y, batch_x, batch_y, idx, dist, need, s);
 }

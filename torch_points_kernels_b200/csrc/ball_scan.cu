@@ -1,0 +1,268 @@
+// Ball query by a scan in index order, one warp per few centres (sm_100a).
+//
+// The rule of the op is "the first nsample candidates within the radius", so a warp that reads 128
+// consecutive points at a time meets its neighbours in the order in which they are returned, and
+// leaves when the list is full: after n * nsample / hits points, 2000 of 16384 where the ball of a
+// centre holds 250.  Against a grid: no build, no candidates to rank, and work for every warp of
+// the GPU whatever the number of clouds (a grid in shared memory is one CTA per cloud and group of
+// layers); the price is the whole cloud for a centre with fewer than nsample neighbours.  So it
+// serves small problems outright, and the centres that a grid leaves over because they are
+// crowded, which are the ones with the shortest scans.
+//
+// Points are read as three 16-byte loads per lane (four points), the next block while this one is
+// tested, distances with the two-wide FP32 instructions, in the arithmetic of the tests:
+// dense   cuda/src/ball_query_gpu.cu:35-36, strict; packed cuda/src/ball_query_gpu.cu:78-82, inclusive.
+// Bound by the issue of instructions where lists stay open, by latency where they fill up.
+#include "scan.cuh"
+
+namespace tpk
+{
+namespace
+{
+
+constexpr int kBsThreads = 256;
+constexpr int kBsBlock = 128;  // points per step of a warp
+
+template <bool PARTIAL, int Q>
+__global__ void __launch_bounds__(kBsThreads)
+    ball_scan_kernel(long long total, int per_warp, long long n, long long m, float radius, int nsample,
+                     const float* __restrict__ y, const float* __restrict__ x, const int64_t* __restrict__ batch_x,
+                     const int64_t* __restrict__ batch_y, int64_t* __restrict__ idx_out, float* __restrict__ dist_out,
+                     const unsigned char* __restrict__ need)
+{
+    const int lane = threadIdx.x & 31;
+    const long long warp = (static_cast<long long>(blockIdx.x) * kBsThreads + threadIdx.x) >> 5;
+    const long long j0 = warp * per_warp;
+    if (j0 >= total) return;
+    const float r2 = __fmul_rn(radius, radius);
+    const uint32_t below = (1u << lane) - 1u;
+    bool mine = lane < per_warp && j0 + lane < total;
+    // `need` (optional): one byte per centre, 0 = already answered by a grid
+    if (mine && need != nullptr) mine = need[j0 + lane] != 0;
+    uint32_t todo = __ballot_sync(kFullMask, mine);
+    while (todo != 0u)
+    {
+        // up to Q centres of one cloud or segment
+        long long row[Q];
+        bool act[Q];
+        long long lo = 0, cnt = n;
+        {
+            int64_t group = 0;
+#pragma unroll
+            for (int q = 0; q < Q; ++q)
+            {
+                act[q] = false;
+                row[q] = row[0];
+                if (todo == 0u) continue;
+                const long long j = j0 + __ffs(todo) - 1;
+                const int64_t g = PARTIAL ? __ldg(batch_y + j) : j / m;
+                if (q == 0) group = g;
+                if (g != group) continue;
+                todo &= todo - 1u;
+                act[q] = true;
+                row[q] = j;
+            }
+            if (PARTIAL)
+            {
+                lo = segment_bound(batch_x, n, group, false);
+                cnt = segment_bound(batch_x, n, group, true) - lo;
+            }
+            else
+                lo = group * n;
+        }
+        const long long base = PARTIAL ? lo : 0;  // dense indices are local to the cloud
+        const float* p = x + lo * 3;
+        float qx[Q], qy[Q], qz[Q];
+        long long first[Q];
+        int found[Q];
+#pragma unroll
+        for (int q = 0; q < Q; ++q)
+        {
+            qx[q] = __ldg(y + row[q] * 3 + 0);
+            qy[q] = __ldg(y + row[q] * 3 + 1);
+            qz[q] = __ldg(y + row[q] * 3 + 2);
+            first[q] = PARTIAL ? -1 : 0;
+            found[q] = act[q] ? 0 : nsample;
+        }
+        auto open = [&]() {
+            bool any = false;
+#pragma unroll
+            for (int q = 0; q < Q; ++q) any |= found[q] < nsample;
+            return any;
+        };
+        // one point per lane: the points before the first 16-byte boundary and behind the last block
+        auto single = [&](long long k0, int count) {
+            const bool in = lane < count;
+            const float* s = p + 3 * (k0 + (in ? lane : 0));
+            const float cx = __ldg(s), cy = __ldg(s + 1), cz = __ldg(s + 2);
+#pragma unroll
+            for (int q = 0; q < Q; ++q)
+            {
+                if (found[q] >= nsample) continue;
+                const float d = PARTIAL ? sumsq_loop(cx - qx[q], cy - qy[q], cz - qz[q]) : sumsq_abc(cx - qx[q], cy - qy[q], cz - qz[q]);
+                const bool hit = in && (PARTIAL ? d <= r2 : d < r2);
+                const uint32_t b = __ballot_sync(kFullMask, hit);
+                if (b == 0u) continue;
+                if (found[q] == 0) first[q] = base + k0 + __ffs(b) - 1;
+                const int at = found[q] + __popc(b & below);
+                if (hit && at < nsample)
+                {
+                    idx_out[row[q] * nsample + at] = base + k0 + lane;
+                    dist_out[row[q] * nsample + at] = d;
+                }
+                found[q] += __popc(b);
+            }
+        };
+        // 16-byte boundaries recur every four points: 12 k = -address (mod 16)
+        const long long head = min(cnt, static_cast<long long>((reinterpret_cast<uintptr_t>(p) >> 2) & 3u));
+        if (head > 0) single(0, static_cast<int>(head));
+        const float4* v = reinterpret_cast<const float4*>(p + 3 * head);
+        const long long blocks = (cnt - head) / kBsBlock;
+        float4 a = {}, b = {}, c = {};
+        if (blocks > 0)
+        {
+            a = __ldg(v + 3 * lane + 0);
+            b = __ldg(v + 3 * lane + 1);
+            c = __ldg(v + 3 * lane + 2);
+        }
+        for (long long t = 0; t < blocks && open(); ++t)
+        {
+            const unsigned long long x01 = pack2(a.x, a.w), x23 = pack2(b.z, c.y);
+            const unsigned long long y01 = pack2(a.y, b.x), y23 = pack2(b.w, c.z);
+            const unsigned long long z01 = pack2(a.z, b.y), z23 = pack2(c.x, c.w);
+            if (t + 1 < blocks)
+            {
+                const float4* next = v + 3 * (kBsBlock / 4) * (t + 1) + 3 * lane;
+                a = __ldg(next + 0);
+                b = __ldg(next + 1);
+                c = __ldg(next + 2);
+            }
+            const long long k0 = head + t * kBsBlock;
+#pragma unroll
+            for (int q = 0; q < Q; ++q)
+            {
+                if (found[q] >= nsample) continue;
+                const unsigned long long nx = pack2(-qx[q], -qx[q]), ny = pack2(-qy[q], -qy[q]), nz = pack2(-qz[q], -qz[q]);
+                const unsigned long long ax = add2(x01, nx), ay = add2(y01, ny), az = add2(z01, nz);
+                const unsigned long long bx = add2(x23, nx), by = add2(y23, ny), bz = add2(z23, nz);
+                const unsigned long long da = PARTIAL ? fma2(az, az, fma2(ay, ay, mul2(ax, ax))) : fma2(az, az, fma2(ax, ax, mul2(ay, ay)));
+                const unsigned long long db = PARTIAL ? fma2(bz, bz, fma2(by, by, mul2(bx, bx))) : fma2(bz, bz, fma2(bx, bx, mul2(by, by)));
+                float d[4];
+                unpack2(da, d[0], d[1]);
+                unpack2(db, d[2], d[3]);
+                bool hit[4];
+#pragma unroll
+                for (int i = 0; i < 4; ++i) hit[i] = PARTIAL ? d[i] <= r2 : d[i] < r2;
+                const uint32_t any = __ballot_sync(kFullMask, hit[0] || hit[1] || hit[2] || hit[3]);
+                if (any == 0u) continue;
+                int at = found[q], all = 0;
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+                {
+                    const uint32_t h = __ballot_sync(kFullMask, hit[i]);
+                    at += __popc(h & below);
+                    all += __popc(h);
+                }
+                if (found[q] == 0)
+                {
+                    const int l = __ffs(any) - 1;
+                    const int i = hit[0] ? 0 : (hit[1] ? 1 : (hit[2] ? 2 : 3));
+                    first[q] = base + k0 + 4 * l + __shfl_sync(kFullMask, i, l);
+                }
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+                    if (hit[i])
+                    {
+                        if (at < nsample)
+                        {
+                            idx_out[row[q] * nsample + at] = base + k0 + 4 * lane + i;
+                            dist_out[row[q] * nsample + at] = d[i];
+                        }
+                        ++at;
+                    }
+                found[q] += all;
+            }
+        }
+        for (long long k = head + blocks * kBsBlock; k < cnt && open(); k += 32)
+            single(k, static_cast<int>(min(32ll, cnt - k)));
+#pragma unroll
+        for (int q = 0; q < Q; ++q)
+        {
+            if (!act[q]) continue;
+            for (int s = min(found[q], nsample) + lane; s < nsample; s += 32)
+            {
+                idx_out[row[q] * nsample + s] = PARTIAL ? -1 : first[q];
+                dist_out[row[q] * nsample + s] = -1.0f;
+            }
+        }
+    }
+}
+
+template <bool PARTIAL>
+int launch_ball_scan(long long total, long long n, long long m, float radius, int nsample, const float* y, const float* x,
+                     const int64_t* batch_x, const int64_t* batch_y, int64_t* idx, float* dist, const unsigned char* need,
+                     cudaStream_t s)
+{
+    // Centres of a warp side by side share its loads, but the first one that stays open keeps the
+    // warp; a single one each while there are too few warps to hide the latency.  4096 centres of
+    // 16384 points, lists that stay open: 64 us with one, 50 with two, 63 with four; lists that fill
+    // up: 31, 35, 43.
+    int q = total >= 16384 ? 4 : (total >= 8192 ? 2 : 1);
+    if (need != nullptr) q = 2;
+    char text[16];
+    if (test_value("ball_warp_scan_q", text, sizeof(text))) q = text[0] == '4' ? 4 : (text[0] == '2' ? 2 : 1);  // test hook
+    long long per_warp = q;
+    if (need != nullptr)
+    {
+        // most bytes are zero: a warp reads the bytes of several centres
+        per_warp = total / (32ll * num_sms());
+        per_warp = per_warp < q ? q : (per_warp > 32 ? 32 : per_warp);
+    }
+    const long long warps = (total + per_warp - 1) / per_warp;
+    const long long blocks = (warps + kBsThreads / 32 - 1) / (kBsThreads / 32);
+    TPK_REQUIRE(blocks < (1ll << 31), "ball_query: too many centres");
+    count_launches(1);
+#define TPK_BALL_SCAN(Q)                                                                                                  \
+    prefer_max_shared(ball_scan_kernel<PARTIAL, Q>),                                                                     \
+        ball_scan_kernel<PARTIAL, Q><<<static_cast<unsigned>(blocks), kBsThreads, 0, s>>>(                               \
+            total, static_cast<int>(per_warp), n, m, radius, nsample, y, x, batch_x, batch_y, idx, dist, need)
+    if (q == 4)
+        TPK_BALL_SCAN(4);
+    else if (q == 2)
+        TPK_BALL_SCAN(2);
+    else
+        TPK_BALL_SCAN(1);
+#undef TPK_BALL_SCAN
+    return check_launch("ball_query scan");
+}
+
+}  // namespace
+
+// Whether the scan is the better way to answer all centres of a dense problem.  Up to here it is
+// where every centre reads its whole cloud, too (points uniform in a ball, 16 neighbours, lists of
+// 32; grid / scan in us): 1 x 1024 points 14.8 / 6.6, 1 x 16384 74 / 64, 16 x 4096 72 / 72,
+// 2 x 16384 76 / 101, but 4 x 16384 76 / 145; where lists fill up (points on surfaces) it is far
+// ahead: 1 x 1024 63 / 6.4, 1 x 16384 549 / 31, 16 x 4096 402 / 40.
+bool ball_scan_wanted(int b, int n, int m)
+{
+    if (test_path("ball_warp_scan")) return true;
+    if (test_path("ball_query_no_warp_scan") || test_path("ball_query_global_grid")) return false;
+    return static_cast<double>(b) * n * m <= 1.2e8;
+}
+
+// need (optional): one byte per centre, the centres with a zero are left as they are.
+int ball_scan_dense(int b, int n, int m, float radius, int nsample, const float* new_xyz, const float* xyz, int64_t* idx,
+                    float* dist, const unsigned char* need, cudaStream_t s)
+{
+    return launch_ball_scan<false>(static_cast<long long>(b) * m, n, m, radius, nsample, new_xyz, xyz, nullptr, nullptr, idx,
+                                   dist, need, s);
+}
+
+int ball_scan_partial(long long size_x, long long size_y, float radius, int nsample, const float* x, const float* y,
+                      const int64_t* batch_x, const int64_t* batch_y, int64_t* idx, float* dist, const unsigned char* need,
+                      cudaStream_t s)
+{
+    return launch_ball_scan<true>(size_y, size_x, 1, radius, nsample, y, x, batch_x, batch_y, idx, dist, need, s);
+}
+
+}  // namespace tpk

@@ -2,6 +2,7 @@
 // distributed-shared-memory primitives of a thread-block cluster.
 #pragma once
 
+#include "packed.cuh"
 #include "tpk_common.cuh"
 
 namespace tpk
@@ -164,36 +165,6 @@ __device__ __forceinline__ uint32_t hilbert3(uint32_t x, uint32_t y, uint32_t z,
     for (uint32_t q = m; q > 1u; q >>= 1)
         if (z & q) t ^= q - 1u;
     return spread3(z ^ t) | (spread3(y ^ t) << 1) | (spread3(x ^ t) << 2);
-}
-
-// packed pairs of floats for the two-wide FP32 instructions of sm_100
-__device__ __forceinline__ unsigned long long pack2(float lo, float hi)
-{
-    unsigned long long r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
-    return r;
-}
-__device__ __forceinline__ void unpack2(unsigned long long v, float& lo, float& hi)
-{
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
-}
-__device__ __forceinline__ unsigned long long add2(unsigned long long a, unsigned long long b)
-{
-    unsigned long long r;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-__device__ __forceinline__ unsigned long long mul2(unsigned long long a, unsigned long long b)
-{
-    unsigned long long r;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-__device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigned long long b, unsigned long long c)
-{
-    unsigned long long r;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-    return r;
 }
 
 }  // namespace tpk

@@ -31,6 +31,7 @@
 
 #include <math_constants.h>
 
+#include "packed.cuh"
 #include "tpk_common.cuh"
 
 namespace tpk
@@ -45,12 +46,6 @@ constexpr float kFilterSlack = 7.62939453125e-06f;  // 2^-17
 constexpr int kScanBatch = TPK_SCAN_BATCH;  // blocks of four candidates per filter branch
 constexpr int kPendCap = 8 * kScanBatch + 8;  // parked pairs per thread between two exact-test batches
 
-__device__ __forceinline__ unsigned long long pack2(float lo, float hi)
-{
-    unsigned long long r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
-    return r;
-}
 __device__ __forceinline__ float lo_f32(unsigned long long v)
 {
     return __uint_as_float(static_cast<uint32_t>(v));
@@ -59,14 +54,6 @@ __device__ __forceinline__ float hi_f32(unsigned long long v)
 {
     return __uint_as_float(static_cast<uint32_t>(v >> 32));
 }
-__device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigned long long b,
-                                                   unsigned long long c)
-{
-    unsigned long long r;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-    return r;
-}
-
 // Filter threshold of a query with squared norm q2 and exact threshold thr.
 __device__ __forceinline__ float filter_threshold(float thr, float q2)
 {
