@@ -250,6 +250,12 @@ bool ball_scan_wanted(int b, int n, int m)
     return static_cast<double>(b) * n * m <= 1.2e8;
 }
 
+// Candidates around a centre from which a grid leaves it to the scan.  A grid spends about two
+// instructions on a candidate, and hits^2 / 8 on the order of its hits; the scan 50 on 128 points,
+// n * nsample / hits of them.  Both are the same at hits^3 = 1.9 n nsample, about 100 of 16384
+// points and lists of 32; 27 cells hold 4.5 times a ball's points (6.5 in space, 2.9 on a surface).
+float ball_scan_crowded(double n, int nsample) { return static_cast<float>(4.5 * cbrt(1.9 * n * nsample)); }
+
 // need (optional): one byte per centre, the centres with a zero are left as they are.
 int ball_scan_dense(int b, int n, int m, float radius, int nsample, const float* new_xyz, const float* xyz, int64_t* idx,
                     float* dist, const unsigned char* need, cudaStream_t s)

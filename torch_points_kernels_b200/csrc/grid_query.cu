@@ -512,7 +512,7 @@ int grid_ball_query_dense(int b, int n, int m, float radius, int nsample, const 
         }
     }
     // above this many candidates in a centre's cell block the early-exit scan is cheaper
-    const float max_cand = 2.0f * sqrtf(6.45f * static_cast<float>(n) * static_cast<float>(nsample));
+    const float max_cand = ball_scan_crowded(n, nsample);
     const long long nq = static_cast<long long>(b) * m;
     const unsigned gq = static_cast<unsigned>((nq + kGridQueryThreads - 1) / kGridQueryThreads);
     count_launches(1), qk<<<gq, kGridQueryThreads, smem, s>>>(b, n, m, radius, nsample, max_cand, cap, new_xyz, info, cells, sorted, idx,

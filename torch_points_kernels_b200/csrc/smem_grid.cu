@@ -982,7 +982,7 @@ int sg_ball_query(int b, int n, int m, float radius, int nsample, const float* n
             return TPK_ERR_CUDA;
         }
     }
-    const float max_cand = 2.0f * sqrtf(6.45f * static_cast<float>(n) * static_cast<float>(nsample));
+    const float max_cand = ball_scan_crowded(n, nsample);
     const long long grid = static_cast<long long>(b) * p.parts;
     TPK_REQUIRE(grid < (1ll << 31), "ball_query_dense: too many clouds");
     count_launches(1), kernel<<<static_cast<unsigned>(grid), kSgThreads, p.smem, s>>>(n, m, p.parts, p.lpp, radius, nsample, max_cand,

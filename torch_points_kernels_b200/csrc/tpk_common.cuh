@@ -56,6 +56,9 @@ struct StatusRegistrar
 int grouping_grad_atomic(int b, int c, int n, int npoint, int nsample, const float* grad_out, long long gbs,
                          const int64_t* idx, float* grad_features, cudaStream_t s);
 
+// ball_scan.cu: candidates around a centre from which a grid leaves it to the scan
+float ball_scan_crowded(double n, int nsample);
+
 constexpr unsigned kFullMask = 0xffffffffu;
 // Dynamic shared memory from which a launcher raises the kernel's limit
 // (cudaFuncAttributeMaxDynamicSharedMemorySize).  Well below the 48 KB a launch may use without
