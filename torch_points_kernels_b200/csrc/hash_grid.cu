@@ -595,8 +595,11 @@ size_t hg_round(size_t v) { return (v + 255) / 256 * 256; }
 uint32_t hg_buckets(long long size_x)
 {
     uint32_t h = 1024;
-    while (h < (1u << 30) && static_cast<long long>(h) * 2 < size_x) h <<= 1;
-    return h;  // a power of two, at least size_x / 2
+    // A query's 27 buckets hold as many strangers as there are points per bucket, times 27: with twice
+    // as many points as buckets most of its candidates were strangers (244345 points, ball query 233 us
+    // against 209, kNN 585 against 568; 114163: 84 and 77, 391 and 384; 7.0 M: the same).
+    while (h < (1u << 30) && static_cast<long long>(h) < size_x) h <<= 1;
+    return h;  // a power of two, at least size_x
 }
 
 }  // namespace
