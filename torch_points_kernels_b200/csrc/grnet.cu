@@ -282,11 +282,18 @@ __global__ void __launch_bounds__(kGrThreads)
     atomicAdd(rows + (pv / per_cloud * cub_scale + vertex) * row + (t - pv * row), __ldg(grad_point_features + t));
 }
 
-// Where the copy pays: two passes over the map against what the rows save.
-bool cubic_by_rows(int n_pts, int nvert, int channels, long long cub_scale)
+// Where the copy pays: two passes over the map against what the rows save.  us, forward / backward,
+// rows and in place, 16 clouds: 2048 points in 8^3 x 128 47 / 55 and 168 / 213, in 16^3 x 64 35 / 39 and
+// 87 / 90, 512 points in 16^3 x 64 18 / 21 and 27 / 29; 4096 points in 32^3 x 32 64 / 71 and 97 / 117,
+// 2048 points 50 / 55 and 53 / 65; but 1400 points in 32^3 x 16 33 / 40 and 19 / 23, and one cloud of
+// 2048 points in 32^3 x 32 10 / 10 and 8 / 10.  So: as many vertices looked up as the map has, or half
+// of them where the map is too large to be found in the L2 cache for the most part.
+bool cubic_by_rows(int b, int n_pts, int nvert, int channels, long long cub_scale, int itemsize)
 {
-    if (test_path("cubic_in_place")) return false;
-    return channels >= 4 && static_cast<long long>(n_pts) * nvert * 3 > cub_scale;
+    if (test_path("cubic_in_place") || channels < 4) return false;
+    const long long looked_up = static_cast<long long>(n_pts) * nvert;
+    const double bytes = static_cast<double>(b) * channels * cub_scale * itemsize;
+    return looked_up >= cub_scale || (2 * looked_up >= cub_scale && bytes >= 48.0e6);
 }
 
 inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
@@ -354,7 +361,7 @@ int64_t rows_scratch(int b, int n_pts, int channels, int scale, int neighborhood
     if (b <= 0 || n_pts <= 0 || channels <= 0 || scale <= 0 || neighborhood_size < 1 || neighborhood_size > 8) return 0;
     const long long cub = static_cast<long long>(scale) * scale * scale;
     const int nvert = 8 * neighborhood_size * neighborhood_size * neighborhood_size;
-    if (cub > INT_MAX || !cubic_by_rows(n_pts, nvert, channels, cub)) return 0;
+    if (cub > INT_MAX || !cubic_by_rows(b, n_pts, nvert, channels, cub, itemsize)) return 0;
     return static_cast<int64_t>(b) * channels * cub * itemsize;
 }
 
