@@ -97,6 +97,7 @@ def region_grow(
     neighbours = ball_query_partial_dense(radius, nsample, local_pos, local_pos, segment, segment)[0]
     seeds = cluster_labels(neighbours)
     seeds, order = torch.sort(seeds, stable=True)  # members ascending inside a cluster
-    counts = torch.unique_consecutive(seeds, return_counts=True)[1].tolist()
-    clusters = torch.split(ind[order], counts)
-    return [c for c in clusters if c.shape[0] >= min_cluster_size]
+    counts = torch.unique_consecutive(seeds, return_counts=True)[1]
+    large = counts >= min_cluster_size
+    members = ind[order[torch.repeat_interleave(large, counts)]]
+    return list(torch.split(members, counts[large].tolist()))
