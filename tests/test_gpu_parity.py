@@ -223,6 +223,20 @@ def test_ball_query_crowded_centres_are_scanned(spread, monkeypatch):
             assert torch.equal(a, b)
 
 
+@pytest.mark.parametrize("k", [1, 2, 7, 31, 32])
+def test_knn_merged_candidates_match_scan(k, monkeypatch):
+    """Steps with a few and with many candidates better than the k-th, equal distances among them."""
+    rng = np.random.default_rng(k)
+    x = np.concatenate([rng.integers(0, 16, (1, 3000, 3)) / 16, rng.random((1, 3000, 3)), 0.5 + 0.01 * rng.random((1, 3000, 3))], 1)
+    x = cu(x.astype(np.float32))
+    q = x[:, ::7].contiguous()
+    data.use_paths(monkeypatch)
+    got = tpk.knn(x, q, k)
+    data.use_paths(monkeypatch, "knn_scan")
+    for a, b in zip(got, tpk.knn(x, q, k)):
+        assert torch.equal(a, b)
+
+
 @pytest.mark.parametrize("family", ["fps_sorted", "fps_sorted,fps_global", "fps_unsorted"])
 def test_fps_coordinates_too_large_for_a_box(family, monkeypatch):
     data.use_paths(monkeypatch, family)
