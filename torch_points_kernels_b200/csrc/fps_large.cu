@@ -18,8 +18,8 @@
 //
 // What bounds it is the latency of a round: two cluster barriers, the dependent loads of chunks from
 // L2, the check of the entries.  Measured, B200, one sample per exchange over the cluster before:
-// 8 clouds of 1048576 -> 65536 252 ms before, 20.2 now; 1048576 -> 16384 30.7 and 6.7;
-// 2 x 200000 -> 5000 8.5 and 2.4; a lattice of 64^3 -> 3000 (ties everywhere) 6.4 and 1.9.
+// 8 clouds of 1048576 -> 65536 252 ms before, 12.5 now; one cloud 7.5 now;
+// 2 x 200000 -> 5000 8.5 and 1.9; a lattice of 64^3 -> 3000 (ties everywhere) 6.4 and 1.6.
 //
 // A sample's minimum is kept where it was: -minimum at its place, which no distance lowers and no
 // test takes for a candidate.  Points that are never candidates hold minus infinity.
@@ -245,7 +245,7 @@ __global__ void __launch_bounds__(kLargeThreads, 1)
     __shared__ unsigned long long s_top;
     __shared__ unsigned long long s_tops[kLargeMaxRanks];
     __shared__ int s_bad;
-    __shared__ int s_tasks, s_next_task;
+    __shared__ int s_tasks, s_next_task, s_listed, s_next_listed;
 
     constexpr int CHUNK = 32 * P;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -291,6 +291,8 @@ __global__ void __launch_bounds__(kLargeThreads, 1)
         s_bad = 0;
         s_tasks = 0;
         s_next_task = 0;
+        s_listed = 0;
+        s_next_listed = 0;
         for (int i = 0; i < 2; ++i) s_note[i] = LargeNote{0, INT_MIN, 0, 0};
     }
     for (int i = tid; i < kLargeBuckets; i += kLargeThreads) hist[i] = 0;
@@ -561,6 +563,8 @@ __global__ void __launch_bounds__(kLargeThreads, 1)
         const int par = round & 1u;
         // ---- 1: samples of the round before, then the active points or chunks
         if (pending > 0) apply(pending);
+        // (the chunks to list go to whichever warp is free, as above: the active ones lie together,
+        // and a warp that listed its own had up to 32 in a row; 17.2 ms for what takes 12.5 now)
         int wmax = INT_MIN;
         for (int g = 0; g < lay.groups; ++g)
         {
@@ -568,89 +572,90 @@ __global__ void __launch_bounds__(kLargeThreads, 1)
             const int at = warp * run + 32 * g + lane;
             const int key = in ? ckey[at] : INT_MIN;
             wmax = max(wmax, key);
-            if (sequential) continue;
-            uint32_t todo = __ballot_sync(kFullMask, key >= tau_key);
-            if (by_chunk && todo != 0u)
-            {
-                int pos = 0;
-                if (lane == 0) pos = atomicAdd(&s_note[par].entries, __popc(todo));
-                pos = __shfl_sync(kFullMask, pos, 0);
-                while (todo != 0u)
-                {
-                    const int c = __ffs(todo) - 1;
-                    todo &= todo - 1u;
-                    if (pos >= kLargeOwnEntries / 2) break;
-                    const long long base = chunk_base(32 * g + c);
-                    const int ck = __shfl_sync(kFullMask, key, c);
-                    unsigned long long best = ~0ull;
-                    int held = 0;
+            const bool active = !sequential && key >= tau_key;
+            const uint32_t b = __ballot_sync(kFullMask, active);
+            if (b == 0u) continue;
+            int pos = 0;
+            if (lane == 0) pos = atomicAdd(&s_listed, __popc(b));
+            pos = __shfl_sync(kFullMask, pos, 0) + __popc(b & ((1u << lane) - 1u));
+            if (active) task_at[pos].x = at;
+        }
+        __syncthreads();
+        const int nlisted = s_listed;
+        while (true)
+        {
+            int t = 0;
+            if (lane == 0) t = atomicAdd(&s_next_listed, 1);
+            t = __shfl_sync(kFullMask, t, 0);
+            if (t >= nlisted) break;
+            const int at = task_at[t].x;
+            const int owner = at / run;
+            const long long base = (static_cast<long long>(owner * nranks + rank) * run + (at - owner * run)) * CHUNK;
+            float md[P];
 #pragma unroll
-                    for (int u = 0; u < P; ++u)
+            for (int u = 0; u < P; ++u)
+            {
+                const long long p = base + u * 32 + lane;
+                md[u] = p < n ? __ldcg(temp + p) : -CUDART_INF_F;
+            }
+            if (by_chunk)
+            {
+                const int ck = ckey[at];
+                unsigned long long best = ~0ull;
+                bool held = false;
+#pragma unroll
+                for (int u = 0; u < P; ++u)
+                    if (__float_as_int(md[u]) == ck)
                     {
-                        const long long p = base + u * 32 + lane;
-                        if (p < n && __float_as_int(__ldcg(temp + p)) == ck)
-                        {
-                            held += 1;
-                            const unsigned long long v = static_cast<unsigned long long>(fps_rank(index_at(static_cast<int>(p)), log2bs)) << 32 |
-                                                         static_cast<unsigned long long>(p);
-                            best = v < best ? v : best;
-                        }
+                        const int p = static_cast<int>(base + u * 32 + lane);
+                        const unsigned long long v = static_cast<unsigned long long>(fps_rank(index_at(p), log2bs)) << 32 |
+                                                     static_cast<unsigned long long>(p);
+                        best = v < best ? v : best;
+                        held = true;
                     }
-                    // the first of the points that hold the chunk's largest minimum
-                    const uint32_t hi = __reduce_min_sync(kFullMask, static_cast<uint32_t>(best >> 32));
-                    const uint32_t who = __ballot_sync(kFullMask, held > 0 && static_cast<uint32_t>(best >> 32) == hi);
-                    if (who != 0u && lane == __ffs(who) - 1)
+                // the first of the points that hold the chunk's largest minimum
+                const uint32_t hi = __reduce_min_sync(kFullMask, static_cast<uint32_t>(best >> 32));
+                const uint32_t who = __ballot_sync(kFullMask, held && static_cast<uint32_t>(best >> 32) == hi);
+                if (who != 0u && lane == __ffs(who) - 1)
+                {
+                    const int pos = atomicAdd(&s_note[par].entries, 1);
+                    if (pos < kLargeOwnEntries / 2)
                     {
-                        const int a = warp * run + 32 * g + c;
-                        own[pos] = make_float4(meta[a], meta[nmeta + a], meta[2 * nmeta + a], __int_as_float(ck));
-                        own[kLargeOwnEntries / 2 + pos] = make_float4(meta[3 * nmeta + a], meta[4 * nmeta + a], meta[5 * nmeta + a], 0.f);
+                        own[pos] = make_float4(meta[at], meta[nmeta + at], meta[2 * nmeta + at], __int_as_float(ck));
+                        own[kLargeOwnEntries / 2 + pos] = make_float4(meta[3 * nmeta + at], meta[4 * nmeta + at], meta[5 * nmeta + at], 0.f);
                         own_pos[pos] = static_cast<int>(best & 0xFFFFFFFFull);
                     }
-                    ++pos;
                 }
+                continue;
             }
-            else
-                while (todo != 0u)
+            uint32_t act[P];
+            int nact = 0;
+#pragma unroll
+            for (int u = 0; u < P; ++u)
+            {
+                const int k = __float_as_int(md[u]);
+                bool a = k >= tau_key;
+                if (a && k == tau_key && tau_rank != kLargeNoRank - 1u)
+                    a = fps_rank(index_at(static_cast<int>(base + u * 32 + lane)), log2bs) <= tau_rank;
+                act[u] = __ballot_sync(kFullMask, a);
+                nact += __popc(act[u]);
+            }
+            if (nact == 0) continue;
+            int pos = 0;
+            if (lane == 0) pos = atomicAdd(&s_note[par].entries, nact);
+            pos = __shfl_sync(kFullMask, pos, 0);
+#pragma unroll
+            for (int u = 0; u < P; ++u)
+            {
+                const int p = pos + __popc(act[u] & ((1u << lane) - 1u));
+                if ((act[u] >> lane & 1u) && p < kLargeOwnEntries)
                 {
-                    const int c = __ffs(todo) - 1;
-                    todo &= todo - 1u;
-                    const long long base = chunk_base(32 * g + c);
-                    float md[P];
-                    uint32_t act[P];
-                    int nact = 0;
-#pragma unroll
-                    for (int u = 0; u < P; ++u)
-                    {
-                        const long long p = base + u * 32 + lane;
-                        md[u] = p < n ? __ldcg(temp + p) : -CUDART_INF_F;
-                    }
-#pragma unroll
-                    for (int u = 0; u < P; ++u)
-                    {
-                        const int k = __float_as_int(md[u]);
-                        bool a = k >= tau_key;
-                        if (a && k == tau_key && tau_rank != kLargeNoRank - 1u)
-                            a = fps_rank(index_at(static_cast<int>(base + u * 32 + lane)), log2bs) <= tau_rank;
-                        act[u] = __ballot_sync(kFullMask, a);
-                        nact += __popc(act[u]);
-                    }
-                    if (nact == 0) continue;
-                    int pos = 0;
-                    if (lane == 0) pos = atomicAdd(&s_note[par].entries, nact);
-                    pos = __shfl_sync(kFullMask, pos, 0);
-#pragma unroll
-                    for (int u = 0; u < P; ++u)
-                    {
-                        const int p = pos + __popc(act[u] & ((1u << lane) - 1u));
-                        if ((act[u] >> lane & 1u) && p < kLargeOwnEntries)
-                        {
-                            const float4 v = __ldg(sorted + base + u * 32 + lane);
-                            own[p] = make_float4(v.x, v.y, v.z, md[u]);
-                            own_pos[p] = static_cast<int>(base + u * 32 + lane);
-                        }
-                        pos += __popc(act[u]);
-                    }
+                    const float4 v = __ldg(sorted + base + u * 32 + lane);
+                    own[p] = make_float4(v.x, v.y, v.z, md[u]);
+                    own_pos[p] = static_cast<int>(base + u * 32 + lane);
                 }
+                pos += __popc(act[u]);
+            }
         }
         wmax = __reduce_max_sync(kFullMask, wmax);
         if (lane == 0) atomicMax(&s_note[par].top, wmax);
@@ -665,7 +670,12 @@ __global__ void __launch_bounds__(kLargeThreads, 1)
         }
         cluster_sync_all();
         if (tid < nranks) s_notes[tid] = *at_rank(&s_note[par], tid);
-        if (tid == 0) s_note[par ^ 1] = LargeNote{0, INT_MIN, 0, 0};  // read by everyone before this barrier
+        if (tid == 0)
+        {
+            s_note[par ^ 1] = LargeNote{0, INT_MIN, 0, 0};  // read by everyone before this barrier
+            s_listed = 0;
+            s_next_listed = 0;
+        }
         __syncthreads();
         int nentries = 0, above = 0, longest = 0, before = 0;
         const int from = warp & (nranks - 1);
