@@ -18,8 +18,8 @@
 //
 // What bounds it is the latency of a round: two cluster barriers, the dependent loads of chunks from
 // L2, the check of the entries.  Measured, B200, one sample per exchange over the cluster before:
-// 8 clouds of 1048576 -> 65536 252 ms before, 12.5 now; one cloud 7.5 now;
-// 2 x 200000 -> 5000 8.5 and 1.9; a lattice of 64^3 -> 3000 (ties everywhere) 6.4 and 1.6.
+// 8 clouds of 1048576 -> 65536 252 ms before, 11.0 now; one cloud 6.7 now;
+// 2 x 200000 -> 5000 8.5 and 1.4; a lattice of 64^3 -> 3000 (ties everywhere) 6.4 and 1.45.
 //
 // A sample's minimum is kept where it was: -minimum at its place, which no distance lowers and no
 // test takes for a candidate.  Points that are never candidates hold minus infinity.
@@ -892,13 +892,16 @@ __global__ void __launch_bounds__(kLargeThreads, 1)
         }
         pending = total;
         taken += total;
-        // more active entries per round mean fewer rounds, but longer ones
-        if (nentries < 512)
+        // more active entries per round mean fewer rounds, but longer ones: 512 to 1024 entries 12.5 ms for
+        // 8 x 1048576 -> 65536 and 2.2 for 200000 -> 8192, 300 to 700 11.4 and 1.8, 160 to 400 11.7 and 1.7
+        // (one cloud of 1048576: 7.5, 7.0, 7.8)
+        if (nentries < 300)
             gap = fminf(fmaxf(gap * 1.25f, 1.0e-3f), 0.5f);
-        else if (nentries > 1024)
-            gap *= nentries > 1536 ? 0.5f : 0.8f;
+        else if (nentries > 700)
+            gap *= nentries > 1200 ? 0.5f : 0.8f;
         if (rank_limit < (kLargeNoRank >> 1) && nentries * 4 < kLargeEntries) rank_limit = rank_limit * 2u + 1u;
-        if (by_chunk && taken > nchunks / 4) by_chunk = false;
+        // (a sample per 8, 16, 32 chunks: 11.4, 11.2, 11.0 ms and 1.79, 1.63, 1.64)
+        if (by_chunk && taken > nchunks / 32) by_chunk = false;
         set_tau();
         __syncthreads();
     }
