@@ -91,6 +91,49 @@ def ref_cuda():
     return points_cuda
 
 
+def _region_grow_on_cpu(monkeypatch):
+    """region_grow with the oracle's neighbour search and traversal behind it."""
+    from torch_points_kernels_b200 import cluster
+
+    def search(radius, nsample, x, y, batch_x, batch_y):
+        assert bool((batch_x[1:] >= batch_x[:-1]).all()), "segments have to be sorted"
+        return tuple(torch.from_numpy(a) for a in orc.ball_query_partial(radius, nsample, x, y, batch_x, batch_y))
+
+    def seeds(neighbours):
+        out = torch.empty(neighbours.shape[0], dtype=torch.int32)
+        for c in orc.grow_proximity(neighbours.numpy(), 1):
+            out[c] = c[0]
+        return out
+
+    monkeypatch.setattr(cluster, "ball_query_partial_dense", search)
+    monkeypatch.setattr(cluster, "cluster_labels", seeds)
+    return cluster.region_grow
+
+
+def _region_grow_by_label(pos, labels, batch, ignore, nsample, radius, min_size):
+    """One search and one traversal per label and sample, as sets in the order of their seeds."""
+    want = []
+    for l in torch.unique(labels).tolist():
+        if l in ignore:
+            continue
+        at = (labels == l).nonzero()[:, 0]
+        inner = torch.unique(batch[at], return_inverse=True)[1]
+        nb = _neighbour_lists(pos[at].numpy(), inner.numpy(), radius, nsample)
+        want += [sorted(at[c].tolist()) for c in orc.grow_proximity(nb, min_size)]
+    return want
+
+
+@pytest.mark.parametrize("ids", [[-1, 0, 1], [-7, -1, 2 ** 62], [-2 ** 63, 0, 2 ** 63 - 1], [0.25, 0.5, 0.75]])
+def test_region_grow_keeps_samples_apart_whatever_their_ids(ids, monkeypatch):
+    g = data.gen(5)
+    n = 600
+    pos = torch.rand(n, 3, generator=g)
+    labels = torch.randint(0, 4, (n,), generator=g)
+    batch = torch.tensor(ids)[torch.sort(torch.randint(0, 3, (n,), generator=g)).values]
+    got = _region_grow_on_cpu(monkeypatch)(pos, labels, batch, ignore_labels=[1], nsample=8, radius=0.15, min_cluster_size=2)
+    assert [c.tolist() for c in got] == _region_grow_by_label(pos, labels, batch, [1], 8, 0.15, 2)
+
+
 def _cu(t):
     return torch.as_tensor(t).to(DEV).contiguous()
 

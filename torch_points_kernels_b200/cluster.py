@@ -53,6 +53,15 @@ def grow_proximity(pos, batch, nsample=16, radius=0.02, min_cluster_size=32):
     return clusters
 
 
+def _segments(rank, sample):
+    """Numbers of the runs of equal (rank, sample), ascending.  The ids are compared, not computed with:
+    any sorted ids of a sample will do, negative and huge ones too."""
+    segment = torch.zeros_like(rank)
+    begins = (rank[1:] != rank[:-1]) | (sample[1:] != sample[:-1])
+    torch.cumsum(begins, 0, out=segment[1:])
+    return segment
+
+
 def region_grow(
     pos, labels, batch, ignore_labels=[], nsample=16, radius=0.02, min_cluster_size=32
 ) -> List[torch.Tensor]:
@@ -91,8 +100,7 @@ def region_grow(
     rank = rank_h.to(pos.device)[label_rank]
     ind = (rank >= 0).nonzero()[:, 0]
     ind = ind[torch.sort(rank[ind], stable=True).indices]
-    sample = batch[ind].long()
-    segment = torch.unique(rank[ind] * (sample.max() + 1) + sample, return_inverse=True)[1]
+    segment = _segments(rank[ind], batch[ind])
     local_pos = pos[ind].float().contiguous()
     neighbours = ball_query_partial_dense(radius, nsample, local_pos, local_pos, segment, segment)[0]
     seeds = cluster_labels(neighbours)
