@@ -134,6 +134,28 @@ def test_region_grow_keeps_samples_apart_whatever_their_ids(ids, monkeypatch):
     assert [c.tolist() for c in got] == _region_grow_by_label(pos, labels, batch, [1], 8, 0.15, 2)
 
 
+@pytest.mark.parametrize("length", [0, 1, 99, 101])
+def test_region_grow_refuses_a_batch_vector_of_another_length(length):
+    """... before anything is looked up with it."""
+    from torch_points_kernels_b200 import cluster
+
+    labels = torch.arange(100) % 3
+    with pytest.raises(IndexError):
+        cluster.region_grow(torch.zeros(100, 3), labels, torch.zeros(length, dtype=torch.int64))
+    with pytest.raises(IndexError):
+        cluster.region_grow(torch.zeros(100, 3), labels, torch.zeros(100, 2, dtype=torch.int64))
+
+
+def test_region_grow_takes_a_column_of_ids(monkeypatch):
+    g = data.gen(6)
+    pos = torch.rand(200, 3, generator=g)
+    labels = torch.randint(0, 2, (200,), generator=g)
+    batch = torch.sort(torch.randint(0, 3, (200,), generator=g)).values
+    grow = _region_grow_on_cpu(monkeypatch)
+    got = grow(pos, labels, batch[:, None], nsample=8, radius=0.2, min_cluster_size=2)
+    assert [c.tolist() for c in got] == _region_grow_by_label(pos, labels, batch, [], 8, 0.2, 2)
+
+
 def _cu(t):
     return torch.as_tensor(t).to(DEV).contiguous()
 

@@ -93,6 +93,9 @@ def region_grow(
     kept = [not (l in ignore_labels) for l in unique_labels.cpu()]
     if not any(kept):
         return []
+    if batch.shape[0] != pos.shape[0] or batch.numel() != pos.shape[0]:
+        raise IndexError("batch of shape %s does not match %d points" % (tuple(batch.shape), pos.shape[0]))
+    batch = batch.reshape(-1)
     # One search and one labelling for all labels: the points ordered by label (original order inside a
     # label), every (label, sample) pair a segment of its own.  Lists, seeds and the order of the clusters
     # are those of a search per label, because the order inside a segment is the same.
