@@ -154,6 +154,9 @@ def test_region_grow_takes_a_column_of_ids(monkeypatch):
     grow = _region_grow_on_cpu(monkeypatch)
     got = grow(pos, labels, batch[:, None], nsample=8, radius=0.2, min_cluster_size=2)
     assert [c.tolist() for c in got] == _region_grow_by_label(pos, labels, batch, [], 8, 0.2, 2)
+    # a cluster that is kept or saved holds its own members only
+    assert all(c.untyped_storage().nbytes() == 8 * c.numel() for c in got)
+    assert grow(pos, labels, batch, nsample=8, radius=0.2, min_cluster_size=201) == []
 
 
 def _cu(t):

@@ -111,4 +111,8 @@ def region_grow(
     counts = torch.unique_consecutive(seeds, return_counts=True)[1]
     large = counts >= min_cluster_size
     members = ind[order[torch.repeat_interleave(large, counts)]]
-    return list(torch.split(members, counts[large].tolist()))
+    sizes = counts[large].tolist()
+    clusters = [members.new_empty(c) for c in sizes]
+    if clusters:
+        torch.split_with_sizes_copy(members, sizes, 0, out=clusters)  # one launch for all
+    return clusters
