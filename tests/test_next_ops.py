@@ -159,6 +159,16 @@ def test_region_grow_takes_a_column_of_ids(monkeypatch):
     assert grow(pos, labels, batch, nsample=8, radius=0.2, min_cluster_size=201) == []
 
 
+def test_region_grow_leaves_out_points_without_a_label(monkeypatch):
+    """A label that equals no label, itself included, selects nothing."""
+    pos, batch = torch.zeros(6, 3), torch.zeros(6, dtype=torch.int64)
+    nan = float("nan")
+    grow = _region_grow_on_cpu(monkeypatch)
+    got = grow(pos, torch.tensor([nan, 2.0, 1.0, nan, 2.0, 1.0]), batch, min_cluster_size=1)
+    assert [c.tolist() for c in got] == [[2, 5], [1, 4]]
+    assert grow(pos, torch.full((6,), nan), batch, min_cluster_size=1) == []
+
+
 def _cu(t):
     return torch.as_tensor(t).to(DEV).contiguous()
 

@@ -90,7 +90,7 @@ def region_grow(
     assert pos.shape[0] == labels.shape[0]
 
     unique_labels, label_rank = torch.unique(labels, return_inverse=True)
-    kept = [not (l in ignore_labels) for l in unique_labels.cpu()]
+    kept = [not (l in ignore_labels) and bool(l == l) for l in unique_labels.cpu()]  # (NaN is no label)
     if not any(kept):
         return []
     if batch.shape[0] != pos.shape[0] or batch.numel() != pos.shape[0]:
