@@ -169,6 +169,18 @@ def test_region_grow_leaves_out_points_without_a_label(monkeypatch):
     assert grow(pos, torch.full((6,), nan), batch, min_cluster_size=1) == []
 
 
+@pytest.mark.parametrize("keep", [torch.ones(2, 4, dtype=torch.bool), torch.ones(1, 5, dtype=torch.bool), torch.ones(10, dtype=torch.bool),
+                                  torch.ones(2, 5), torch.ones(2, 5, dtype=torch.int64),
+                                  torch.ones(2, 5, dtype=torch.bool, device="meta"), [[True] * 5] * 2])
+def test_gridding_refuses_a_mask_the_kernel_cannot_read(keep, monkeypatch):
+    """Another shape, another type, another device: told before anything is launched."""
+    from torch_points_kernels_b200 import gridding
+
+    monkeypatch.setattr(gridding, "_suffix", lambda t, what: "f32")
+    with pytest.raises(RuntimeError, match="keep"):
+        gridding.GriddingFunction.apply(torch.zeros(2, 5, 3), 4, keep)
+
+
 def _cu(t):
     return torch.as_tensor(t).to(DEV).contiguous()
 
@@ -327,6 +339,12 @@ def test_gridding_padding_as_if_it_were_not_there():
         want = torch.zeros(700, 3)
         want[keep] = y.grad[0].cpu() * 8
         np.testing.assert_array_equal(x.grad[b].cpu().numpy(), want.numpy())
+    # a mask that is not contiguous
+    wide = _cu(torch.rand(700, 3, generator=g) < 0.5)
+    masked = gridding.GriddingFunction.apply(x.detach() * 8, 8, wide.t())
+    again = gridding.GriddingFunction.apply(x.detach() * 8, 8, wide.t().contiguous())
+    torch.testing.assert_close(masked, again, rtol=1e-6, atol=1e-6)
+    assert not torch.allclose(masked, grid)
     assert gridding.gridding(_cu(torch.zeros(0, 5, 3)), 4).shape == (1, 512)
     assert _lib.device_status() == 0
 

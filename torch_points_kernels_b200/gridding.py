@@ -23,6 +23,15 @@ class GriddingFunction(torch.autograd.Function):
         sfx = _suffix(ptcloud, "ptcloud")
         ptcloud = ptcloud.contiguous()
         b, n = ptcloud.shape[0], ptcloud.shape[1]
+        if keep is not None:
+            # the kernel reads one byte per point
+            if not torch.is_tensor(keep) or keep.dtype not in (torch.bool, torch.uint8):
+                raise RuntimeError("keep must be a bool tensor")
+            if tuple(keep.shape) != (b, n):
+                raise RuntimeError("keep must be of size (%d, %d), not %s" % (b, n, tuple(keep.shape)))
+            if keep.device != ptcloud.device:
+                raise RuntimeError("keep must be on the device of ptcloud")
+            keep = keep.contiguous()
         length = 2 * int(scale)
         grid = torch.empty((b, length ** 3), dtype=ptcloud.dtype, device=ptcloud.device)
         weights = torch.empty((b, n, 8, 3), dtype=ptcloud.dtype, device=ptcloud.device)
