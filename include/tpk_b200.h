@@ -79,18 +79,18 @@ TPK_API int64_t tpk_kernel_launches(void);
  *
  * scratch: scratch_bytes >= tpk_fps_scratch_bytes(b,n,m) bytes of device memory (16-byte
  * aligned).  Required for clouds of more than 131072 points (sorted copy + running minima);
- * optional below, where it holds a spatially sorted copy that lets most of the cloud skip most
- * rounds (NULL: the kernel without it, same result).  A buffer smaller than
- * tpk_fps_scratch_bytes returns TPK_ERR_SCRATCH and launches nothing.  Content on entry is
- * irrelevant.
+ * 0 below, where everything stays on chip and a buffer is not looked at.  A buffer smaller
+ * than tpk_fps_scratch_bytes returns TPK_ERR_SCRATCH and launches nothing.  Content on entry
+ * is irrelevant.
  */
 TPK_API int tpk_furthest_point_sampling(int b, int n, int m, const float* xyz, void* scratch,
                                 int64_t scratch_bytes, int32_t* idxs, void* stream);
 
 /*
- * The same, followed by a gather of the coordinates of the samples: new_xyz (b,m,3) f32,
- * i.e. xyz[b, idxs[b, j], :] (what callers otherwise do with several tensor operations);
- * NULL skips it.  No counterpart in the reference.
+ * The same with the coordinates of the samples: new_xyz (b,m,3) f32, i.e. xyz[b, idxs[b, j], :]
+ * (what callers otherwise do with several tensor operations); NULL skips it.  Written by the
+ * sampling kernel itself, or by a second one where that takes one sample per exchange.  No
+ * counterpart in the reference.
  */
 TPK_API int tpk_furthest_point_sampling_xyz(int b, int n, int m, const float* xyz, void* scratch,
                                     int64_t scratch_bytes, int32_t* idxs, float* new_xyz,

@@ -58,10 +58,7 @@ def test_fps_refuses_short_scratch_without_gpu():
         rc = fn(2, 200000, 48, fake, fake, need - 1, fake, *extra, None)
         assert rc == 4  # TPK_ERR_SCRATCH
         assert b"scratch of" in l.tpk_last_error()
-    # optional scratch (sorted copy of a cloud that fits on chip) is checked the same way
-    need = l.tpk_fps_scratch_bytes(16, 16384, 4096)
-    assert l.tpk_furthest_point_sampling(16, 16384, 4096, fake, fake, need // 2, fake, None) == 4
-    # and a missing buffer where one is required
+    # a missing buffer where one is required
     assert l.tpk_furthest_point_sampling(2, 200000, 48, fake, None, 0, fake, None) == 4
 
 
@@ -69,11 +66,12 @@ def test_scratch_sizes_are_host_arithmetic(monkeypatch):
     """What the callers must allocate: pure host functions, usable without a GPU."""
     monkeypatch.delenv("TPK_B200_TEST", raising=False)
     l = _lib.lib()
-    # FPS: nothing for small clouds or few samples, the sorted copy (16 B/point) for clouds that stay
-    # on chip, the sorted copy plus the running minima (20 B/point) above 131072 points
+    # FPS: nothing for clouds that stay on chip, the sorted copy plus the running minima (20 B/point)
+    # above 131072 points
     assert l.tpk_fps_scratch_bytes(4, 1024, 256) == 0
     assert l.tpk_fps_scratch_bytes(4, 16384, 64) == 0
-    assert l.tpk_fps_scratch_bytes(16, 16384, 4096) == 16 * 16384 * 16
+    assert l.tpk_fps_scratch_bytes(16, 16384, 4096) == 0
+    assert l.tpk_fps_scratch_bytes(1, 131072, 8192) == 0
     assert l.tpk_fps_scratch_bytes(2, 200000, 48) == 2 * 200000 * 20
     monkeypatch.setenv("TPK_B200_TEST", "fps_unsorted")
     assert l.tpk_fps_scratch_bytes(16, 16384, 4096) == 0
@@ -184,9 +182,9 @@ def test_test_hook_tokens(monkeypatch):
     """TPK_B200_TEST is a comma-separated token list; a token only matches whole names."""
     l = _lib.lib()
     monkeypatch.setenv("TPK_B200_TEST", "fps_unsortedx,xfps_unsorted")
-    assert l.tpk_fps_scratch_bytes(16, 16384, 4096) == 16 * 16384 * 16
+    assert l.tpk_fps_scratch_bytes(2, 200000, 48) == 2 * 200000 * 20
     monkeypatch.setenv("TPK_B200_TEST", "three_nn_scan,fps_unsorted")
-    assert l.tpk_fps_scratch_bytes(16, 16384, 4096) == 0
+    assert l.tpk_fps_scratch_bytes(2, 200000, 48) == 2 * 200000 * 4
     assert l.tpk_three_nn_scratch_bytes(16, 16384, 4096) == 0
     monkeypatch.delenv("TPK_B200_TEST")
     assert l.tpk_three_nn_scratch_bytes(16, 16384, 4096) > 0

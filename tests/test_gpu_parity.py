@@ -100,10 +100,16 @@ def test_fps_tie_break_and_skip_rule(n, monkeypatch):
             np.testing.assert_array_equal(npy(tpk.furthest_point_sample(cu(pts), m)), want)
 
 
-def test_fps_sorted_copy_is_the_default_for_big_on_chip_clouds(monkeypatch):
-    data.use_paths(monkeypatch)
-    assert _lib.lib().tpk_fps_scratch_bytes(4, 16384, 4096) == 4 * 16384 * 16
-    assert _lib.lib().tpk_fps_scratch_bytes(4, 1024, 256) == 0
+@pytest.mark.parametrize("n,m,family,launches", [(16384, 4096, None, 1), (1024, 256, None, 2), (16384, 4096, "fps_unsorted", 2),
+                                                 (1024, 256, "fps_sorted", 1)])
+def test_fps_rounds_are_the_default_for_big_on_chip_clouds(n, m, family, launches, monkeypatch):
+    """The kernel of the rounds writes the coordinates of the samples itself; behind one sample per
+    exchange a second kernel gathers them."""
+    data.use_paths(monkeypatch, family)
+    x = cu(data.unit_ball(1, n, seed=n))
+    before = _lib.kernel_launches()
+    tpk.furthest_point_sample(x, m, return_xyz=True)
+    assert _lib.kernel_launches() - before == launches
 
 
 @pytest.mark.parametrize("kind", ["clustered", "lattice", "planar", "nonfinite", "many_skipped"])

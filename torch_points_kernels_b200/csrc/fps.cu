@@ -739,10 +739,8 @@ extern "C" int64_t tpk_fps_scratch_bytes(int b, int n, int m)
     if (n <= 0 || b <= 0 || m <= 0) return 0;
     switch (tpk::fps_pick_path(n, m, &c))
     {
-    case tpk::kFpsOnchip: return 0;
-    // accepted and not used: the kernel sorts on chip (part of the interface since a kernel took a
-    // sorted copy of clouds of this size from here)
-    case tpk::kFpsRounds: return n >= 4096 && m >= 128 ? static_cast<int64_t>(b) * n * 16 : 0;
+    case tpk::kFpsOnchip:
+    case tpk::kFpsRounds: return 0;
     // large clouds: the running minimum, one float per point, behind the sorted copy if one is used
     case tpk::kFpsLarge: return static_cast<int64_t>(b) * n * 20;
     default: return static_cast<int64_t>(b) * n * 4;
