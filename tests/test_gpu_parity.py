@@ -100,13 +100,17 @@ def test_fps_tie_break_and_skip_rule(n, monkeypatch):
             np.testing.assert_array_equal(npy(tpk.furthest_point_sample(cu(pts), m)), want)
 
 
-@pytest.mark.parametrize("n,m,family,launches", [(16384, 4096, None, 1), (1024, 256, None, 2), (16384, 4096, "fps_unsorted", 2),
-                                                 (1024, 256, "fps_sorted", 1)])
-def test_fps_rounds_are_the_default_for_big_on_chip_clouds(n, m, family, launches, monkeypatch):
+@pytest.mark.parametrize("b,n,m,family,launches", [(1, 16384, 4096, None, 1), (1, 1024, 256, None, 2), (1, 16384, 4096, "fps_unsorted", 2),
+                                                   (1, 1024, 256, "fps_sorted", 1),
+                                                   # few samples: one per exchange, whatever the size
+                                                   (1, 2048, 64, None, 2), (256, 2048, 128, None, 2), (1, 16384, 96, None, 2),
+                                                   (16, 32768, 192, None, 2), (1, 131072, 128, None, 2),
+                                                   (1, 2048, 512, None, 1), (16, 16384, 512, None, 1), (1, 131072, 1024, None, 1)])
+def test_fps_rounds_are_the_default_where_they_are_faster(b, n, m, family, launches, monkeypatch):
     """The kernel of the rounds writes the coordinates of the samples itself; behind one sample per
     exchange a second kernel gathers them."""
     data.use_paths(monkeypatch, family)
-    x = cu(data.unit_ball(1, n, seed=n))
+    x = cu(data.unit_ball(b, n, seed=n))
     before = _lib.kernel_launches()
     tpk.furthest_point_sample(x, m, return_xyz=True)
     assert _lib.kernel_launches() - before == launches

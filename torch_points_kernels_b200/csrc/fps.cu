@@ -31,6 +31,7 @@ TPK_DEFINE_STATUS_WORD()
 
 // fps_rounds.cu
 bool fps_rounds_fits(int n);
+double fps_rounds_us(int b, int n, int m);
 int fps_rounds(int b, int n, int m, int log2bs, const float* xyz, int32_t* idxs, float* new_xyz, cudaStream_t stream);
 
 // fps_large.cu
@@ -707,10 +708,25 @@ int fps_launch_s(const FpsConfig& c, int b, int n, int m, int log2bs, const floa
     return TPK_ERR_UNSUPPORTED;
 }
 
-// Which kernel family a call takes.  One sample per exchange costs 0.26 us a sample on clouds of up
-// to 1024 points, 0.6 us at 16384; the rounds cost a sort and 20 to 60 rounds of 1.7 us and more,
-// whatever the number of samples (256 -> 64: 22 us against 41; 1024 -> 256: 67 against 70;
-// 2048 -> 512: 140 against 115).
+// About how many microseconds m samples take, one per exchange: so much a sample on an idle GPU, more
+// where the clouds share SMs (measured, us a sample: one cloud of 2048 points 0.34, of 16384 0.57, of 131072
+// 1.1; 64 clouds of 16384 0.85, 256 of 2048 0.43, 16 of 32768 0.80, 16 of 65536 1.6).
+double fps_onchip_us(int b, int n, int m, const FpsConfig& c)
+{
+    const double each = n <= 2048 ? 0.38 : (n <= 4096 ? 0.485 : (n <= 8192 ? 0.55 : (n <= 16384 ? 0.59 :
+                        (n <= 32768 ? 0.67 : (n <= 65536 ? 0.78 : 1.05)))));
+    double slower = 0.85 + 0.19 * b * c.nranks * c.nthreads / (128. * kNumSmsB200);
+    if (c.nranks == 16) slower = 0.13 * b;  // seven or so of the largest clusters run at once
+    if (slower < 1.) slower = 1.;
+    if (c.nranks == 8) slower += 0.25 * (b < 16 ? b / 16. : 1.);
+    return 8. + each * slower * m;
+}
+
+// Which kernel family a call takes: one sample per exchange costs the same for every sample, the rounds
+// cost a sort and some rounds whose number grows with the logarithm of the samples.  Measured, us, one per
+// exchange / rounds: one cloud of 2048 points 64 samples 42 / 78, 256 107 / 103, 512 191 / 121; 16384 points
+// 64 57 / 107, 256 166 / 141; 131072 points 64 91 / 266, 512 576 / 436; 16 clouds of 32768 128 125 / 251,
+// 512 432 / 353; 256 of 2048 256 131 / 184, 512 244 / 234.  (512 -> 128 49 / 67, 1024 -> 256 82 / 82.)
 // Test hooks: "fps_global" (large-cloud kernels on any cloud), "fps_unsorted" (one sample per
 // exchange, no sorted copy anywhere), "fps_sorted" (the rounds whatever the size).
 enum FpsPath
@@ -721,13 +737,13 @@ enum FpsPath
     kFpsGlobal   // large clouds, unsorted (4 B/point)
 };
 
-FpsPath fps_pick_path(int n, int m, FpsConfig* c)
+FpsPath fps_pick_path(int b, int n, int m, FpsConfig* c)
 {
     if (test_path("fps_global") || !fps_pick_config(n, m, c))
         return fps_large_fits(n) && !test_path("fps_unsorted") ? kFpsLarge : kFpsGlobal;
-    if (test_path("fps_unsorted")) return kFpsOnchip;
-    const bool rounds = test_path("fps_sorted") || (n > 1100 && m >= 48);
-    return rounds && fps_rounds_fits(n) ? kFpsRounds : kFpsOnchip;
+    if (test_path("fps_unsorted") || !fps_rounds_fits(n)) return kFpsOnchip;
+    if (test_path("fps_sorted")) return kFpsRounds;
+    return n > 1100 && fps_rounds_us(b, n, m) < fps_onchip_us(b, n, m, *c) ? kFpsRounds : kFpsOnchip;
 }
 
 }  // namespace
@@ -737,7 +753,7 @@ extern "C" int64_t tpk_fps_scratch_bytes(int b, int n, int m)
 {
     tpk::FpsConfig c;
     if (n <= 0 || b <= 0 || m <= 0) return 0;
-    switch (tpk::fps_pick_path(n, m, &c))
+    switch (tpk::fps_pick_path(b, n, m, &c))
     {
     case tpk::kFpsOnchip:
     case tpk::kFpsRounds: return 0;
@@ -771,7 +787,7 @@ static int fps_run(int b, int n, int m, const float* xyz, void* scratch, int64_t
         return TPK_ERR_SCRATCH;
     }
     FpsConfig c;
-    const FpsPath path = fps_pick_path(n, m, &c);
+    const FpsPath path = fps_pick_path(b, n, m, &c);
     if (path == kFpsLarge || path == kFpsGlobal)
     {
         if (scratch == nullptr)

@@ -33,6 +33,7 @@
 // one sample per dependent step before: 16384 -> 4096 one cloud 0.97 ms before, 0.29 now; 16 clouds
 // 1.08 and 0.40; 131072 -> 8192 7.3 and 0.94; a lattice of 20^3 (ties everywhere) 17.0 and 2.0.
 #include <climits>
+#include <cmath>
 #include <cstdlib>
 #include <math_constants.h>
 
@@ -998,15 +999,13 @@ int launch_rounds(int b, int n, int m, int log2bs, int bits, const RoundsLayout&
 
 }  // namespace
 
-// Largest cloud the kernel takes: 16 CTAs of 512 threads with 16 points each.
-bool fps_rounds_fits(int n) { return n <= kRoundsMaxRanks * 512 * 16; }
-
-int fps_rounds(int b, int n, int m, int log2bs, const float* xyz, int32_t* idxs, float* new_xyz, cudaStream_t stream)
+// CTAs per cloud, and the cost of the call in the unit below.
+// A round costs about 3300 + (points per CTA) in some unit, 1024 points being as good as fewer, and
+// 148, 72, 32, 15, 7 clusters of 1, 2, 4, 8, 16 such CTAs run at once (measured, 512 threads with
+// 128 registers: one CTA per SM).  16384 -> 4096, us: 8 CTAs 290 up to 15 clouds and 545 for 16,
+// 4 CTAs 400 up to 32 clouds; 4096 -> 1024: 140 with 8 or 4 CTAs, 178 with 2, 228 with 1.
+static int pick_ranks(int b, int n, double* cost_out, int* waves_out)
 {
-    // A round costs about 3300 + (points per CTA) in some unit, 1024 points being as good as fewer, and
-    // 148, 72, 32, 15, 7 clusters of 1, 2, 4, 8, 16 such CTAs run at once (measured, 512 threads with
-    // 128 registers: one CTA per SM).  16384 -> 4096, us: 8 CTAs 290 up to 15 clouds and 545 for 16,
-    // 4 CTAs 400 up to 32 clouds; 4096 -> 1024: 140 with 8 or 4 CTAs, 178 with 2, 228 with 1.
     static const int kAtOnce[5] = {148, 72, 32, 15, 7};
     int nranks = 0;
     double least = 0.;
@@ -1020,8 +1019,33 @@ int fps_rounds(int b, int n, int m, int log2bs, const float* xyz, int32_t* idxs,
         {
             nranks = 1 << l;
             least = cost;
+            *waves_out = waves;
         }
     }
+    *cost_out = least;
+    return nranks;
+}
+
+// Largest cloud the kernel takes: 16 CTAs of 512 threads with 16 points each.
+bool fps_rounds_fits(int n) { return n <= kRoundsMaxRanks * 512 * 16; }
+
+// About how many microseconds the call takes, for the choice of a kernel: points uniform in a ball, where
+// one cloud of 2048 points takes 84, 103, 121 us for 128, 256, 512 samples, of 16384 126, 141, 164, of 131072
+// 317, 370, 436; cheaper by a fifth where clouds run one behind the other or need no exchange (64 of 16384
+// 239, 286, 346; 256 of 2048 147, 184, 234).  On surfaces up to a third more.
+double fps_rounds_us(int b, int n, int m)
+{
+    double cost = 0.;
+    int waves = 1;
+    if (pick_ranks(b, n, &cost, &waves) == 1 || waves > 1) cost *= 0.8;
+    return cost * (0.012 + 0.003 * log2(m > 16 ? m / 16. : 1.));
+}
+
+int fps_rounds(int b, int n, int m, int log2bs, const float* xyz, int32_t* idxs, float* new_xyz, cudaStream_t stream)
+{
+    double cost = 0.;
+    int waves = 1;
+    int nranks = pick_ranks(b, n, &cost, &waves);
     char text[64];
     if (test_value("fps_config", text, sizeof(text)))
     {
