@@ -256,6 +256,46 @@ def test_fps_coordinates_too_large_for_a_box(family, monkeypatch):
     np.testing.assert_array_equal(npy(tpk.furthest_point_sample(cu(x), 90)), orc.fps(x, 90))
 
 
+def fps_us(x, m):
+    """Least time of a few calls, in microseconds."""
+    out = []
+    for _ in range(4):
+        begin, end = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        begin.record()
+        tpk.furthest_point_sample(x, m)
+        end.record()
+        torch.cuda.synchronize()
+        out.append(begin.elapsed_time(end) * 1e3)
+    return min(out[1:])
+
+
+@pytest.mark.parametrize("n,m", [(16384, 4096), (140000, 3000)])
+@pytest.mark.parametrize("kind", ["one", "many", "first", "late"])
+def test_fps_coordinates_that_are_not_finite(n, m, kind, monkeypatch):
+    """Such a point keeps its minimum when it is picked and is picked for ever: no other minimum changes
+    either, so the samples behind it cost nothing (they cost 27 times the whole cloud without it)."""
+    data.use_paths(monkeypatch)
+    x = data.unit_ball(1, n, seed=n).numpy().copy()
+    clean = fps_us(cu(x), m)
+    if kind == "one":
+        x[0, n // 3, 1] = np.nan
+    elif kind == "many":
+        x[0, 5::7] = np.inf
+        x[0, 6::35, 2] = -np.inf
+    elif kind == "first":
+        x[0, 0] = np.nan
+    else:
+        # points out of reach of each other come first: all have the largest minimum
+        x[0, ::2, 0] *= 1e6
+        x[0, 511, 2] = np.nan
+    got, xyz = tpk.furthest_point_sample(cu(x), m, return_xyz=True)
+    np.testing.assert_array_equal(npy(got), orc.fps(x, m))
+    np.testing.assert_array_equal(npy(xyz), np.take_along_axis(x, npy(got).astype(np.int64)[..., None], 1))
+    if kind != "late":
+        assert fps_us(cu(x), m) < 3 * clean
+    assert _lib.device_status() == 0
+
+
 @pytest.mark.parametrize("B,N,m,env", [(3, 1000, 200, None), (2, 16384, 700, None), (2, 16384, 700, "fps_unsorted"),
                                        (1, 150000, 40, None), (1, 150000, 40, "fps_unsorted"), (4, 257, 257, None)])
 def test_fps_returns_sampled_coordinates(B, N, m, env, monkeypatch):

@@ -549,6 +549,7 @@ __global__ void __launch_bounds__(kLargeThreads, 1)
     const int nchunks = static_cast<int>((static_cast<long long>(n) + CHUNK - 1) / CHUNK);
     bool by_chunk = true;
     int top = 0, top_before = INT_MAX, taken = 0, fill = 0;
+    int last = -1;  // one sample per round: the place of the last one
     auto set_tau = [&]() {
         // towards the end not below what the last sample will have: samples beyond m are taken for nothing
         const float part = fminf(static_cast<float>(taken) / static_cast<float>(m), 1.0f);
@@ -715,6 +716,16 @@ __global__ void __launch_bounds__(kLargeThreads, 1)
             else
                 w = find_top(top);
             const int pos = static_cast<int>(w & 0xFFFFFFFFull);
+            if (sequential)
+            {
+                // a sample that comes up again at once has changed no minimum: it is all that follows
+                if (pos == last)
+                {
+                    fill = index_at(pos);
+                    break;
+                }
+                last = pos;
+            }
             taken += 1;
             if (tid == 0)
             {
