@@ -296,6 +296,25 @@ def test_fps_coordinates_that_are_not_finite(n, m, kind, monkeypatch):
     assert _lib.device_status() == 0
 
 
+@pytest.mark.parametrize("kind", ["stray", "origin"])
+def test_fps_large_cloud_ends_with_its_last_sample(kind, monkeypatch):
+    """A distance 65536 times the final spacing: the sampling used to go on until every point was a sample,
+    244 ms where the cloud without the point takes 1."""
+    data.use_paths(monkeypatch)
+    n, m = 140000, 3000
+    x = data.unit_ball(1, n, seed=n).numpy().copy()
+    if kind == "origin":
+        x += np.array([4e5, 5e6, 0.0], np.float32)
+    clean = fps_us(cu(x), m)
+    if kind == "origin":
+        x[0, 0] = 0.0
+    else:
+        x[0, n // 2, 0] = 1e5
+    np.testing.assert_array_equal(npy(tpk.furthest_point_sample(cu(x), m)), orc.fps(x, m))
+    assert fps_us(cu(x), m) < 12 * clean
+    assert _lib.device_status() == 0
+
+
 @pytest.mark.parametrize("B,N,m,env", [(3, 1000, 200, None), (2, 16384, 700, None), (2, 16384, 700, "fps_unsorted"),
                                        (1, 150000, 40, None), (1, 150000, 40, "fps_unsorted"), (4, 257, 257, None)])
 def test_fps_returns_sampled_coordinates(B, N, m, env, monkeypatch):

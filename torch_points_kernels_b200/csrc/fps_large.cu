@@ -45,8 +45,7 @@ constexpr int kLargeEntries = 4096;      // active points (half as many chunks) 
 constexpr int kLargeOwnEntries = 1024;   // of one CTA
 constexpr int kLargePicks = 2048;        // samples of a round
 constexpr int kLargeHits = 128;          // samples applied to a group of chunks at a time
-constexpr int kLargeBuckets = 4096;
-constexpr int kLargeBucketShift = 16;    // while sampling: 128 buckets per octave, 32 octaves
+constexpr int kLargeBuckets = 4096;      // of the final order
 constexpr uint32_t kLargeNoRank = 0xFFFFFFFFu;
 constexpr int kMaxSmemBytes = 227 * 1024;
 
@@ -55,7 +54,7 @@ struct LargeLayout
     int run;        // chunks of a warp
     int groups;     // of up to 32 chunks of a warp
     int cap_picks;  // samples a CTA may take per round
-    int meta, gbox, table, table_pos, own, own_pos, picks, mine_pick, hist;
+    int meta, gbox, table, table_pos, own, own_pos, picks, mine_pick;
     int f_hist, f_base, f_start;
     int bytes;
 };
@@ -268,7 +267,6 @@ __global__ void __launch_bounds__(kLargeThreads, 1)
     int* own_pos = reinterpret_cast<int*>(smem + lay.own_pos);
     float4* picks = reinterpret_cast<float4*>(smem + lay.picks);
     float4* mine_pick = reinterpret_cast<float4*>(smem + lay.mine_pick);
-    int* hist = reinterpret_cast<int*>(smem + lay.hist);
     // while samples are applied, in the place of the table of entries
     uint4* task_mask = reinterpret_cast<uint4*>(smem + lay.table);
     int2* task_at = reinterpret_cast<int2*>(task_mask + nmeta);
@@ -295,7 +293,6 @@ __global__ void __launch_bounds__(kLargeThreads, 1)
         s_next_listed = 0;
         for (int i = 0; i < 2; ++i) s_note[i] = LargeNote{0, INT_MIN, 0, 0};
     }
-    for (int i = tid; i < kLargeBuckets; i += kLargeThreads) hist[i] = 0;
     __syncthreads();
     bool bad = false;
     for (int g = 0; g < lay.groups; ++g)
@@ -526,8 +523,23 @@ __global__ void __launch_bounds__(kLargeThreads, 1)
         cluster_sync_all();  // everyone has read
         return best;
     };
-    int first_top = 0;
-    auto bucket_of = [&](int key) { return max(0, min(kLargeBuckets - 1, (first_top - key) >> kLargeBucketShift)); };
+    // How many samples of this warp's chunks have a minimum above the image `key`.
+    auto count_above = [&](int key) -> int {
+        int count = 0;
+#pragma unroll 4
+        for (int c = 0; c < run; ++c)
+        {
+            const long long base = chunk_base(c);
+#pragma unroll
+            for (int u = 0; u < P; ++u)
+            {
+                const long long p = base + u * 32 + lane;
+                const float md = p < n ? __ldcg(temp + p) : 0.f;
+                count += md < 0.f && md != -CUDART_INF_F && __float_as_int(-md) > key ? 1 : 0;
+            }
+        }
+        return __reduce_add_sync(kFullMask, count);
+    };
 
     // sample 0 is point 0, candidate or not
     if (tid == 0)
@@ -548,7 +560,8 @@ __global__ void __launch_bounds__(kLargeThreads, 1)
     // chunks stand for their points while there are few samples
     const int nchunks = static_cast<int>((static_cast<long long>(n) + CHUNK - 1) / CHUNK);
     bool by_chunk = true;
-    int top = 0, top_before = INT_MAX, taken = 0, fill = 0;
+    int top = 0, first_top = 0, top_before = INT_MAX, taken = 0, fill = 0;
+    int counted = INT_MAX, warp_above = 0;  // samples of this warp above `counted`
     int last = -1;  // one sample per round: the place of the last one
     auto set_tau = [&]() {
         // towards the end not below what the last sample will have: samples beyond m are taken for nothing
@@ -662,12 +675,14 @@ __global__ void __launch_bounds__(kLargeThreads, 1)
         if (lane == 0) atomicMax(&s_note[par].top, wmax);
         if (!sequential && taken >= m - 1)
         {
-            // enough samples: are m - 1 of them above all that is left?
-            const int last = bucket_of(top_before);
-            int above = 0;
-            for (int c = tid; c < last; c += kLargeThreads) above += hist[c];
-            above = __reduce_add_sync(kFullMask, above);
-            if (lane == 0 && above) atomicAdd(&s_note[par].above, above);
+            // Enough samples: are m - 1 of them above all that is left?  Counted from the samples themselves,
+            // once for every largest minimum (later samples are not above it).
+            if (counted != top_before)
+            {
+                counted = top_before;
+                warp_above = count_above(counted);
+            }
+            if (lane == 0 && warp_above) atomicAdd(&s_note[par].above, warp_above);
         }
         cluster_sync_all();
         if (tid < nranks) s_notes[tid] = *at_rank(&s_note[par], tid);
@@ -743,10 +758,7 @@ __global__ void __launch_bounds__(kLargeThreads, 1)
                     }
                 }
                 else if (s_tops[rank] == w)
-                {
                     __stcg(temp + pos, -__int_as_float(top));
-                    atomicAdd(&hist[bucket_of(top)], 1);
-                }
             }
             pending = 1;
         }
@@ -882,7 +894,6 @@ __global__ void __launch_bounds__(kLargeThreads, 1)
                     {
                         mine_pick[p] = t[q];
                         __stcg(temp + tpos[q], -t[q].w);
-                        atomicAdd(&hist[bucket_of(__float_as_int(t[q].w))], 1);
                     }
                 }
         }
@@ -1055,7 +1066,6 @@ LargeLayout large_layout(int n, int nranks, int p)
     };
     lay.meta = take(static_cast<long long>(lay.run) * kLargeWarps * 28);
     lay.gbox = take(static_cast<long long>(lay.groups) * kLargeWarps * 32);
-    lay.hist = take(kLargeBuckets * 4);
     lay.own = take(kLargeOwnEntries * 16);
     lay.own_pos = take(kLargeOwnEntries * 4);
     lay.mine_pick = take(lay.cap_picks * 16);
