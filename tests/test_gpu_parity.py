@@ -315,6 +315,25 @@ def test_fps_large_cloud_ends_with_its_last_sample(kind, monkeypatch):
     assert _lib.device_status() == 0
 
 
+@pytest.mark.parametrize("n,m,stray", [(16384, 4096, True), (2000, 1500, True), (140000, 12000, False), (20000, 9000, False)])
+def test_fps_final_order_over_the_range_of_the_samples(n, m, stray, monkeypatch):
+    """One point far from the others (the order of the samples used to take longer than the sampling), and
+    fewer places than samples, where nothing is left above a minimum of zero."""
+    data.use_paths(monkeypatch, None if stray else "fps_sorted")
+    x = data.unit_ball(1, n if stray else 7001, seed=n).numpy().copy()
+    if stray:
+        clean = fps_us(cu(x), m)
+        x[0, n // 2, 0] = 1e5
+    else:
+        x[0, :40] *= 1e-3 / np.linalg.norm(x[0, :40], axis=1, keepdims=True)  # never candidates
+        x[0, 50:60] = x[0, 40:50] * np.float32(1 + 1e-7)  # a rounding apart
+        x = x[:, np.arange(n) % 7001].copy()
+    np.testing.assert_array_equal(npy(tpk.furthest_point_sample(cu(x), m)), orc.fps(x, m))
+    if stray and n > 4000:
+        assert fps_us(cu(x), m) < 3.3 * clean
+    assert _lib.device_status() == 0
+
+
 @pytest.mark.parametrize("B,N,m,env", [(3, 1000, 200, None), (2, 16384, 700, None), (2, 16384, 700, "fps_unsorted"),
                                        (1, 150000, 40, None), (1, 150000, 40, "fps_unsorted"), (4, 257, 257, None)])
 def test_fps_returns_sampled_coordinates(B, N, m, env, monkeypatch):

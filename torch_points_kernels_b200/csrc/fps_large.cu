@@ -243,7 +243,7 @@ __global__ void __launch_bounds__(kLargeThreads, 1)
     __shared__ int s_scan[32];
     __shared__ unsigned long long s_top;
     __shared__ unsigned long long s_tops[kLargeMaxRanks];
-    __shared__ int s_bad;
+    __shared__ int s_bad, s_low;
     __shared__ int s_tasks, s_next_task, s_listed, s_next_listed;
 
     constexpr int CHUNK = 32 * P;
@@ -287,6 +287,7 @@ __global__ void __launch_bounds__(kLargeThreads, 1)
     if (tid == 0)
     {
         s_bad = 0;
+        s_low = INT_MAX;
         s_tasks = 0;
         s_next_task = 0;
         s_listed = 0;
@@ -935,13 +936,31 @@ __global__ void __launch_bounds__(kLargeThreads, 1)
         int* f_base = reinterpret_cast<int*>(smem + lay.f_base);
         int* f_start = reinterpret_cast<int*>(smem + lay.f_start);
         int* slots = reinterpret_cast<int*>(temp);
+        // Buckets over the images that count: m - 1 samples lie above the largest minimum that is left, or
+        // nothing is left but what coincides with a sample.  (Not over all images below the first one: the
+        // buckets are ordered by comparing all with all.)
+        int low = top;
+        if (top <= 0)
+        {
+            low = INT_MAX;
+            for (int c = 0; c < run; ++c)
+                for (int u = 0; u < P; ++u)
+                {
+                    const long long p = chunk_base(c) + u * 32 + lane;
+                    const float md = p < n ? __ldcg(temp + p) : 0.f;
+                    if (md < 0.f && md != -CUDART_INF_F) low = min(low, __float_as_int(-md));
+                }
+            low = __reduce_min_sync(kFullMask, low);
+            if (lane == 0) atomicMin(&s_low, low);
+        }
         cluster_sync_all();  // the tables have been read everywhere
+        if (top <= 0)
+            for (int r = 0; r < nranks; ++r) low = min(low, *at_rank(&s_low, r));
         for (int c = tid; c < kLargeBuckets; c += kLargeThreads) f_hist[c] = 0;
         __syncthreads();
-        // buckets over the images that samples can have
+        low = min(low, first_top);
         int shift = 0;
-        const int low = max(0, top);
-        while ((max(first_top - low, 0) >> shift) >= kLargeBuckets - 1) ++shift;
+        while (((first_top - low) >> shift) >= kLargeBuckets - 1) ++shift;
         auto bucket = [&](int key) { return max(0, min(kLargeBuckets - 1, (first_top - key) >> shift)); };
         // a warp moves its samples to the front of its run, as (image of the minimum, index)
         int mine = 0;

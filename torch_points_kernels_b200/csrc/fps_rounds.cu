@@ -53,8 +53,7 @@ namespace
 constexpr int kRoundsMaxRanks = 16;
 constexpr int kRoundsThreads = 512;
 constexpr int kRoundsStrongest = 4;  // of a warp's points, compared with its others before they go out
-constexpr int kRoundsBuckets = 4096;     // final order: 32 octaves of the minimum, 128 buckets each
-constexpr int kRoundsBucketShift = 16;   // 2^23 float images per octave / 128
+constexpr int kRoundsBuckets = 4096;     // of the final order
 constexpr uint32_t kNoRank = 0xFFFFFFFFu;
 
 // Offsets into dynamic shared memory.  The sort of the points uses all of it before the rounds
@@ -130,6 +129,7 @@ __global__ void __launch_bounds__(kRoundsThreads, 1)
     __shared__ int s_count[2], s_surv[2], s_npicks[2], s_max[2], s_above[2];  // by parity of the round
     __shared__ __align__(8) uint64_t s_mbar[8];  // notes, entries, sample counts, samples: two of each
     __shared__ uint32_t s_top;
+    __shared__ int s_low;
 
     constexpr int THREADS = kRoundsThreads, NW = THREADS / 32;
     constexpr bool CLUSTERED = NR > 1;
@@ -260,6 +260,7 @@ __global__ void __launch_bounds__(kRoundsThreads, 1)
             asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         }
         s_top = kNoRank;
+        s_low = INT_MAX;
     }
     int* hist = reinterpret_cast<int*>(smem + lay.hist);
     int* base = reinterpret_cast<int*>(smem + lay.base);
@@ -911,10 +912,27 @@ __global__ void __launch_bounds__(kRoundsThreads, 1)
     int2* f_sorted = reinterpret_cast<int2*>(smem + lay.f_sorted);
     // (one sample after the other: they are in place already)
     const int listed = sequential ? 0 : taken;
+    const int mine = nown;
+    // Buckets over the images that count: m - 1 samples lie above the largest minimum that is left, or
+    // nothing is left but what coincides with a sample.  (A fixed number of octaves put nearly all samples
+    // into the last bucket where one point was far from the others, 16384 -> 4096 1236 us instead of 331:
+    // a bucket is ordered by comparing all with all.)
+    int low = top;
+    if (top <= 0)
+    {
+        low = INT_MAX;
+        for (int i = tid; i < mine; i += THREADS) low = min(low, own[i].x);
+        low = __reduce_min_sync(kFullMask, low);
+        if (lane == 0) atomicMin(&s_low, low);
+        sync_all();
+        for (int r = 0; r < nranks; ++r) low = min(low, *at_rank(&s_low, r));
+    }
+    low = min(low, first_top);
+    int shift = 0;
+    while (((first_top - low) >> shift) >= kRoundsBuckets - 1) ++shift;
     for (int c = tid; c < kRoundsBuckets; c += THREADS) f_hist[c] = 0;
     __syncthreads();
-    auto bucket_of = [&](int key) { return max(0, min(kRoundsBuckets - 1, (first_top - key) >> kRoundsBucketShift)); };
-    const int mine = nown;
+    auto bucket_of = [&](int key) { return max(0, min(kRoundsBuckets - 1, (first_top - key) >> shift)); };
     for (int i = tid; i < mine; i += THREADS) atomicAdd(&f_hist[bucket_of(own[i].x)], 1);
     sync_all();
     bin_positions(f_hist, f_base, f_start, kRoundsBuckets);
