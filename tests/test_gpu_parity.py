@@ -334,6 +334,22 @@ def test_fps_final_order_over_the_range_of_the_samples(n, m, stray, monkeypatch)
     assert _lib.device_status() == 0
 
 
+@pytest.mark.parametrize("n,m", [(16384, 4096), (140000, 3000)])
+def test_fps_few_coordinates_too_large_to_square(n, m, monkeypatch):
+    """Finite, but at an infinite distance from the others: samples like any other (a single one made the
+    cloud nine times as expensive as it is without it, one sample per round)."""
+    data.use_paths(monkeypatch)
+    x = data.unit_ball(1, n, seed=n).numpy().copy()
+    clean = fps_us(cu(x), m)
+    x[0, n // 3] = (2e18, 0.0, 1.0)
+    x[0, n // 2] = (-3e38, 3e38, -3e38)
+    x[0, n // 2 + 1] = (3e38, -3e38, 3e38)
+    x[0, n // 5, 2] = -1e19
+    np.testing.assert_array_equal(npy(tpk.furthest_point_sample(cu(x), m)), orc.fps(x, m))
+    assert fps_us(cu(x), m) < 3 * clean
+    assert _lib.device_status() == 0
+
+
 @pytest.mark.parametrize("B,N,m,env", [(3, 1000, 200, None), (2, 16384, 700, None), (2, 16384, 700, "fps_unsorted"),
                                        (1, 150000, 40, None), (1, 150000, 40, "fps_unsorted"), (4, 257, 257, None)])
 def test_fps_returns_sampled_coordinates(B, N, m, env, monkeypatch):

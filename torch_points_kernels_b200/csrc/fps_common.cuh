@@ -2,6 +2,8 @@
 // distributed-shared-memory primitives of a thread-block cluster.
 #pragma once
 
+#include <math_constants.h>
+
 #include "packed.cuh"
 #include "tpk_common.cuh"
 
@@ -108,6 +110,12 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint32_t mbar, uint32_t parity
     }
 }
 
+
+// (false for NaN as well)
+__device__ __forceinline__ bool all_finite(float x, float y, float z)
+{
+    return fabsf(x) <= CUDART_MAX_NORMAL_F && fabsf(y) <= CUDART_MAX_NORMAL_F && fabsf(z) <= CUDART_MAX_NORMAL_F;
+}
 
 __device__ __forceinline__ uint32_t bitrev_low(uint32_t v, int bits)
 {

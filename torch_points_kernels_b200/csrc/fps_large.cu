@@ -278,7 +278,8 @@ __global__ void __launch_bounds__(kLargeThreads, 1)
     auto chunk_base = [&](int c) { return first + static_cast<long long>(c) * CHUNK; };
     auto index_at = [&](int pos) { return __float_as_int(__ldg(&sorted[pos].w)); };
     auto box_dist = [&](const float (&b)[6], float x, float y, float z) {
-        // same expression and rounding as a point's distance: never above that of a point in the box
+        // same expression and rounding as a point's distance: never above that of a point in the box, infinite
+        // where a square is (without NaN: differences of finite coordinates have a sign)
         return sumsq_abc(fmaxf(fmaxf(b[0] - x, x - b[3]), 0.f), fmaxf(fmaxf(b[1] - y, y - b[4]), 0.f),
                          fmaxf(fmaxf(b[2] - z, z - b[5]), 0.f));
     };
@@ -319,17 +320,13 @@ __global__ void __launch_bounds__(kLargeThreads, 1)
                 __stcg(temp + p, first_min);
                 key = max(key, __float_as_int(first_min));
                 if (!in) continue;
-                if (fabsf(v[u].x) < 1.0e18f && fabsf(v[u].y) < 1.0e18f && fabsf(v[u].z) < 1.0e18f)
-                {
-                    lo[0] = fminf(lo[0], v[u].x);
-                    hi[0] = fmaxf(hi[0], v[u].x);
-                    lo[1] = fminf(lo[1], v[u].y);
-                    hi[1] = fmaxf(hi[1], v[u].y);
-                    lo[2] = fminf(lo[2], v[u].z);
-                    hi[2] = fmaxf(hi[2], v[u].z);
-                }
-                else
-                    bad = true;  // not finite, or too large to square
+                lo[0] = fminf(lo[0], v[u].x);
+                hi[0] = fmaxf(hi[0], v[u].x);
+                lo[1] = fminf(lo[1], v[u].y);
+                hi[1] = fmaxf(hi[1], v[u].y);
+                lo[2] = fminf(lo[2], v[u].z);
+                hi[2] = fmaxf(hi[2], v[u].z);
+                bad |= !all_finite(v[u].x, v[u].y, v[u].z);
             }
             const int at = warp * run + 32 * g + c;
 #pragma unroll

@@ -287,6 +287,7 @@ __global__ void __launch_bounds__(kRoundsThreads, 1)
                 px[g] = __ldg(src + 0);
                 py[g] = __ldg(src + 1);
                 pz[g] = __ldg(src + 2);
+                // (a coordinate from 1e18 on can not be squared, and would leave the others one cell)
                 if (fabsf(px[g]) < 1.0e18f && fabsf(py[g]) < 1.0e18f && fabsf(pz[g]) < 1.0e18f)
                 {
                     lo[0] = fminf(lo[0], px[g]);
@@ -296,8 +297,7 @@ __global__ void __launch_bounds__(kRoundsThreads, 1)
                     lo[2] = fminf(lo[2], pz[g]);
                     hi[2] = fmaxf(hi[2], pz[g]);
                 }
-                else
-                    bad = true;  // not finite, or too large to square
+                bad |= !all_finite(px[g], py[g], pz[g]);
             }
         }
 #pragma unroll
@@ -320,7 +320,7 @@ __global__ void __launch_bounds__(kRoundsThreads, 1)
         }
         sync_all();
     }
-    bool sequential = false;
+    bool sequential = false;  // one sample per round, every warp in reach: coordinates that are not finite
     {
         float lo[3] = {CUDART_INF_F, CUDART_INF_F, CUDART_INF_F};
         float ext = 0.f;
@@ -398,7 +398,7 @@ __global__ void __launch_bounds__(kRoundsThreads, 1)
         for (int g = 0; g < PPT; ++g)
         {
             wmax = max(wmax, __float_as_int(md[g]));
-            const bool in = md[g] >= 0.f && fabsf(px[g]) < 1.0e18f && fabsf(py[g]) < 1.0e18f && fabsf(pz[g]) < 1.0e18f;
+            const bool in = md[g] >= 0.f;
             lo[0] = in ? fminf(lo[0], px[g]) : lo[0];
             hi[0] = in ? fmaxf(hi[0], px[g]) : hi[0];
             lo[1] = in ? fminf(lo[1], py[g]) : lo[1];
@@ -451,8 +451,8 @@ __global__ void __launch_bounds__(kRoundsThreads, 1)
             if ((i0 + lane) >> lg_ranks < mine)
             {
                 const float4 s = list[from * cap + ((i0 + lane) >> lg_ranks)];
-                // same expression and rounding as a point's distance: never above that of a point in the box
-                // (which leaves out coordinates of 1e18 and more: then every warp is in reach)
+                // same expression and rounding as a point's distance: never above that of a point in the box, infinite
+                // where a square is (without NaN: differences of finite coordinates have a sign)
                 reach = sequential || sumsq_abc(fmaxf(fmaxf(wlo[0] - s.x, s.x - whi[0]), 0.f), fmaxf(fmaxf(wlo[1] - s.y, s.y - whi[1]), 0.f),
                                   fmaxf(fmaxf(wlo[2] - s.z, s.z - whi[2]), 0.f)) < __int_as_float(wmax);
             }
