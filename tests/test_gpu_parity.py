@@ -350,6 +350,19 @@ def test_fps_few_coordinates_too_large_to_square(n, m, monkeypatch):
     assert _lib.device_status() == 0
 
 
+@pytest.mark.parametrize("b,n", [(1, 200000), (8, 200000), (16, 200000), (40, 140000), (8, 1048576)])
+def test_fps_large_clusters_fill_the_gpu_in_one_go(b, n, monkeypatch):
+    """Clusters that do not all run at once cost the call twice; the largest that do are taken."""
+    data.use_paths(monkeypatch)
+    x = cu(data.unit_ball(1, n, seed=n)).expand(b, -1, -1).contiguous()
+    default = fps_us(x, 256)
+    best = float("inf")
+    for ranks in (2, 4, 8, 16):
+        data.use_paths(monkeypatch, "fps_config=%d" % ranks)
+        best = min(best, fps_us(x, 256))
+    assert default < 1.2 * best
+
+
 @pytest.mark.parametrize("B,N,m,env", [(3, 1000, 200, None), (2, 16384, 700, None), (2, 16384, 700, "fps_unsorted"),
                                        (1, 150000, 40, None), (1, 150000, 40, "fps_unsorted"), (4, 257, 257, None)])
 def test_fps_returns_sampled_coordinates(B, N, m, env, monkeypatch):

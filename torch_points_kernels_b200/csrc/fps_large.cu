@@ -1173,29 +1173,36 @@ int fps_large(int b, int n, int m, int log2bs, const float* xyz, void* scratch, 
     float* temp = reinterpret_cast<float*>(sorted + static_cast<size_t>(b) * n);
     const int rc = sort_points(b, n, xyz, sorted, reinterpret_cast<int*>(temp), stream);
     if (rc != TPK_OK) return rc;
-    // Seven clusters of 16 such CTAs run at once, 15 of eight.
-    int nranks = b <= 7 ? 16 : 8;
-    char text[64];
-    if (test_value("fps_config", text, sizeof(text)))
-    {
-        // test hook "fps_config=nranks:...": another cluster size for the same cloud
-        const int r = atoi(text);
-        if (r >= 1 && r <= kLargeMaxRanks && (r & (r - 1)) == 0) nranks = r;
-    }
     // the smallest chunks of which a warp has at most 32
     auto chunk_of = [&](int ranks) {
         int p = 1;
         while (p < 4 && (static_cast<long long>(n) + 32 * p - 1) / (32 * p) > 32ll * kLargeWarps * ranks) p *= 2;
         return p;
     };
-    int p = chunk_of(nranks);
-    LargeLayout lay = large_layout(n, nranks, p);
-    if (lay.bytes > kMaxSmemBytes - 2048)
+    auto fits = [&](int ranks) { return large_layout(n, ranks, chunk_of(ranks)).bytes <= kMaxSmemBytes - 2048; };
+    // 148, 72, 32, 15, 7 clusters of 1, 2, 4, 8, 16 such CTAs run at once, and a call takes about as long as
+    // 180000 points plus those of a CTA.  256 samples, us, clusters of 2, 4, 8, 16: 7 clouds of 200000 points
+    // 1247, 1006, 886, 775; 8 clouds 1263, 966, 895, 1365; 16 clouds 1353, 1059, 1564, 2005; 40 of 140000
+    // 1223, 1698, 2249, 3742; 8 of 1048576 (8 and 16) 1834, 2374.
+    static const int kAtOnce[5] = {148, 72, 32, 15, 7};
+    int nranks = kLargeMaxRanks;
+    double least = 0.;
+    for (int l = 4; l >= 0; --l)
     {
-        nranks = kLargeMaxRanks;
-        p = chunk_of(nranks);
-        lay = large_layout(n, nranks, p);
+        const double cost = ((b + kAtOnce[l] - 1) / kAtOnce[l]) * (180000. + n / static_cast<double>(1 << l));
+        if (l < 4 && (cost >= least || !fits(1 << l))) continue;
+        nranks = 1 << l;
+        least = cost;
     }
+    char text[64];
+    if (test_value("fps_config", text, sizeof(text)))
+    {
+        // test hook "fps_config=nranks:...": another cluster size for the same cloud
+        const int r = atoi(text);
+        if (r >= 1 && r <= kLargeMaxRanks && (r & (r - 1)) == 0 && fits(r)) nranks = r;
+    }
+    const int p = chunk_of(nranks);
+    const LargeLayout lay = large_layout(n, nranks, p);
     if (p == 1) return launch_large<1>(b, n, m, log2bs, nranks, lay, xyz, sorted, temp, idxs, new_xyz, stream);
     if (p == 2) return launch_large<2>(b, n, m, log2bs, nranks, lay, xyz, sorted, temp, idxs, new_xyz, stream);
     return launch_large<4>(b, n, m, log2bs, nranks, lay, xyz, sorted, temp, idxs, new_xyz, stream);
