@@ -45,7 +45,8 @@ constexpr int kLargeEntries = 4096;      // active points (half as many chunks) 
 constexpr int kLargeOwnEntries = 1024;   // of one CTA
 constexpr int kLargePicks = 2048;        // samples of a round
 constexpr int kLargeHits = 128;          // samples applied to a group of chunks at a time
-constexpr int kLargeBuckets = 4096;      // of the final order
+constexpr int kLargeBuckets = 4096;
+constexpr int kLargeBucketShift = 16;    // while sampling: 128 buckets per octave, 32 octaves
 constexpr uint32_t kLargeNoRank = 0xFFFFFFFFu;
 constexpr int kMaxSmemBytes = 227 * 1024;
 
@@ -54,7 +55,7 @@ struct LargeLayout
     int run;        // chunks of a warp
     int groups;     // of up to 32 chunks of a warp
     int cap_picks;  // samples a CTA may take per round
-    int meta, gbox, table, table_pos, own, own_pos, picks, mine_pick;
+    int meta, gbox, table, table_pos, own, own_pos, picks, mine_pick, hist;
     int f_hist, f_base, f_start;
     int bytes;
 };
@@ -231,6 +232,24 @@ struct LargeNote
     int entries, top, above, picks;
 };
 
+// How many samples of a warp's chunks have a minimum above the image `key`.  (Out of line: rarely called, and
+// not to take registers from the rounds.)
+template <int P>
+__device__ __noinline__ int large_count_above(const float* temp, long long first, int run, int n, int key)
+{
+    const int lane = threadIdx.x & 31;
+    int count = 0;
+    for (int c = 0; c < run; ++c)
+#pragma unroll
+        for (int u = 0; u < P; ++u)
+        {
+            const long long p = first + (static_cast<long long>(c) * P + u) * 32 + lane;
+            const float md = p < n ? __ldcg(temp + p) : 0.f;
+            count += md < 0.f && md != -CUDART_INF_F && __float_as_int(-md) > key ? 1 : 0;
+        }
+    return __reduce_add_sync(kFullMask, count);
+}
+
 template <int P>  // points per lane of a chunk
 __global__ void __launch_bounds__(kLargeThreads, 1)
     fps_large_kernel(int n, int m, int log2bs, int nranks, LargeLayout lay, const float* __restrict__ xyz_all,
@@ -243,7 +262,8 @@ __global__ void __launch_bounds__(kLargeThreads, 1)
     __shared__ int s_scan[32];
     __shared__ unsigned long long s_top;
     __shared__ unsigned long long s_tops[kLargeMaxRanks];
-    __shared__ int s_bad, s_low;
+    __shared__ int s_bad, s_low, s_last[2];  // (the last sample of one per round, by parity of the round)
+    __shared__ int s_counted, s_above[kLargeWarps];  // samples of a warp's chunks above the image s_counted
     __shared__ int s_tasks, s_next_task, s_listed, s_next_listed;
 
     constexpr int CHUNK = 32 * P;
@@ -267,6 +287,7 @@ __global__ void __launch_bounds__(kLargeThreads, 1)
     int* own_pos = reinterpret_cast<int*>(smem + lay.own_pos);
     float4* picks = reinterpret_cast<float4*>(smem + lay.picks);
     float4* mine_pick = reinterpret_cast<float4*>(smem + lay.mine_pick);
+    int* hist = reinterpret_cast<int*>(smem + lay.hist);
     // while samples are applied, in the place of the table of entries
     uint4* task_mask = reinterpret_cast<uint4*>(smem + lay.table);
     int2* task_at = reinterpret_cast<int2*>(task_mask + nmeta);
@@ -289,6 +310,8 @@ __global__ void __launch_bounds__(kLargeThreads, 1)
     {
         s_bad = 0;
         s_low = INT_MAX;
+        s_last[0] = s_last[1] = -1;
+        s_counted = INT_MAX;
         s_tasks = 0;
         s_next_task = 0;
         s_listed = 0;
@@ -297,6 +320,7 @@ __global__ void __launch_bounds__(kLargeThreads, 1)
     }
     __syncthreads();
     bool bad = false;
+    for (int i = tid; i < kLargeBuckets; i += kLargeThreads) hist[i] = 0;
     for (int g = 0; g < lay.groups; ++g)
     {
         const int left = min(32, run - 32 * g);
@@ -521,24 +545,8 @@ __global__ void __launch_bounds__(kLargeThreads, 1)
         cluster_sync_all();  // everyone has read
         return best;
     };
-    // How many samples of this warp's chunks have a minimum above the image `key`.
-    auto count_above = [&](int key) -> int {
-        int count = 0;
-#pragma unroll 4
-        for (int c = 0; c < run; ++c)
-        {
-            const long long base = chunk_base(c);
-#pragma unroll
-            for (int u = 0; u < P; ++u)
-            {
-                const long long p = base + u * 32 + lane;
-                const float md = p < n ? __ldcg(temp + p) : 0.f;
-                count += md < 0.f && md != -CUDART_INF_F && __float_as_int(-md) > key ? 1 : 0;
-            }
-        }
-        return __reduce_add_sync(kFullMask, count);
-    };
-
+    int first_top = 0;
+    auto bucket_of = [&](int key) { return max(0, min(kLargeBuckets - 1, (first_top - key) >> kLargeBucketShift)); };
     // sample 0 is point 0, candidate or not
     if (tid == 0)
     {
@@ -558,9 +566,7 @@ __global__ void __launch_bounds__(kLargeThreads, 1)
     // chunks stand for their points while there are few samples
     const int nchunks = static_cast<int>((static_cast<long long>(n) + CHUNK - 1) / CHUNK);
     bool by_chunk = true;
-    int top = 0, first_top = 0, top_before = INT_MAX, taken = 0, fill = 0;
-    int counted = INT_MAX, warp_above = 0;  // samples of this warp above `counted`
-    int last = -1;  // one sample per round: the place of the last one
+    int top = 0, top_before = INT_MAX, taken = 0, fill = 0;
     auto set_tau = [&]() {
         // towards the end not below what the last sample will have: samples beyond m are taken for nothing
         const float part = fminf(static_cast<float>(taken) / static_cast<float>(m), 1.0f);
@@ -673,14 +679,27 @@ __global__ void __launch_bounds__(kLargeThreads, 1)
         if (lane == 0) atomicMax(&s_note[par].top, wmax);
         if (!sequential && taken >= m - 1)
         {
-            // Enough samples: are m - 1 of them above all that is left?  Counted from the samples themselves,
-            // once for every largest minimum (later samples are not above it).
-            if (counted != top_before)
+            // enough samples: are m - 1 of them above all that is left?
+            const int last = bucket_of(top_before);
+            int above = 0;
+            if (last < kLargeBuckets - 1)
             {
-                counted = top_before;
-                warp_above = count_above(counted);
+                for (int c = tid; c < last; c += kLargeThreads) above += hist[c];
+                above = __reduce_add_sync(kFullMask, above);
             }
-            if (lane == 0 && warp_above) atomicAdd(&s_note[par].above, warp_above);
+            else
+            {
+                // below the histogram, where the first minimum was 65536 times as far as the last: counted from the
+                // samples themselves, once for every largest minimum (later samples are not above it)
+                if (s_counted != top_before)
+                {
+                    above = large_count_above<P>(temp, first, run, n, top_before);
+                    if (lane == 0) s_above[warp] = above;
+                    __syncwarp();
+                }
+                above = s_above[warp];
+            }
+            if (lane == 0 && above) atomicAdd(&s_note[par].above, above);
         }
         cluster_sync_all();
         if (tid < nranks) s_notes[tid] = *at_rank(&s_note[par], tid);
@@ -689,6 +708,7 @@ __global__ void __launch_bounds__(kLargeThreads, 1)
             s_note[par ^ 1] = LargeNote{0, INT_MIN, 0, 0};  // read by everyone before this barrier
             s_listed = 0;
             s_next_listed = 0;
+            if (!sequential && taken >= m - 1) s_counted = top_before;
         }
         __syncthreads();
         int nentries = 0, above = 0, longest = 0, before = 0;
@@ -729,15 +749,11 @@ __global__ void __launch_bounds__(kLargeThreads, 1)
             else
                 w = find_top(top);
             const int pos = static_cast<int>(w & 0xFFFFFFFFull);
-            if (sequential)
+            if (sequential && pos == s_last[par ^ 1])
             {
                 // a sample that comes up again at once has changed no minimum: it is all that follows
-                if (pos == last)
-                {
-                    fill = index_at(pos);
-                    break;
-                }
-                last = pos;
+                fill = index_at(pos);
+                break;
             }
             taken += 1;
             if (tid == 0)
@@ -745,6 +761,7 @@ __global__ void __launch_bounds__(kLargeThreads, 1)
                 const float4 v = __ldg(sorted + pos);
                 picks[0] = v;
                 const int k = __float_as_int(v.w);
+                s_last[par] = pos;
                 if (sequential)
                 {
                     if (rank == 0)
@@ -756,7 +773,10 @@ __global__ void __launch_bounds__(kLargeThreads, 1)
                     }
                 }
                 else if (s_tops[rank] == w)
+                {
                     __stcg(temp + pos, -__int_as_float(top));
+                    atomicAdd(&hist[bucket_of(top)], 1);
+                }
             }
             pending = 1;
         }
@@ -892,6 +912,7 @@ __global__ void __launch_bounds__(kLargeThreads, 1)
                     {
                         mine_pick[p] = t[q];
                         __stcg(temp + tpos[q], -t[q].w);
+                        atomicAdd(&hist[bucket_of(__float_as_int(t[q].w))], 1);
                     }
                 }
         }
@@ -1082,6 +1103,7 @@ LargeLayout large_layout(int n, int nranks, int p)
     };
     lay.meta = take(static_cast<long long>(lay.run) * kLargeWarps * 28);
     lay.gbox = take(static_cast<long long>(lay.groups) * kLargeWarps * 32);
+    lay.hist = take(kLargeBuckets * 4);
     lay.own = take(kLargeOwnEntries * 16);
     lay.own_pos = take(kLargeOwnEntries * 4);
     lay.mine_pick = take(lay.cap_picks * 16);

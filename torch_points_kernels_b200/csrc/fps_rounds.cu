@@ -563,7 +563,6 @@ __global__ void __launch_bounds__(kRoundsThreads, 1)
     int top_before = INT_MAX, first_top = 0, top = 0;
     int taken = 0;  // samples so far, without the first
     int fill = 0;   // index of every sample after the last one that changed a minimum
-    int last = 0;   // one sample per round: the last one
     auto set_tau = [&]() {
         // at least 1: a minimum of zero is a point that coincides with a sample
         // ... and towards the end not below what the last sample will have (its minimum falls at most
@@ -734,12 +733,9 @@ __global__ void __launch_bounds__(kRoundsThreads, 1)
             const int w = find_top(top);
             const int k = s_topidx_of[w];
             // a sample that comes up again at once has changed no minimum: it is all that follows
-            if ((top == 0 && !sequential) || (sequential && k == last))
-            {
-                fill = k;
-                break;
-            }
-            last = k;
+            const bool again = sequential && k == fill;
+            if (again || sequential || top == 0) fill = k;
+            if (again || (top == 0 && !sequential)) break;
             taken += 1;
             if (rank == w && !sequential)
             {
