@@ -299,7 +299,8 @@ def test_fps_coordinates_that_are_not_finite(n, m, kind, monkeypatch):
 @pytest.mark.parametrize("kind", ["stray", "origin"])
 def test_fps_large_cloud_ends_with_its_last_sample(kind, monkeypatch):
     """A distance 65536 times the final spacing: the sampling used to go on until every point was a sample,
-    244 ms where the cloud without the point takes 1."""
+    244 ms where the cloud without the point takes 1; and the cells that order the points are sized by
+    where most of them are."""
     data.use_paths(monkeypatch)
     n, m = 140000, 3000
     x = data.unit_ball(1, n, seed=n).numpy().copy()
@@ -311,7 +312,7 @@ def test_fps_large_cloud_ends_with_its_last_sample(kind, monkeypatch):
     else:
         x[0, n // 2, 0] = 1e5
     np.testing.assert_array_equal(npy(tpk.furthest_point_sample(cu(x), m)), orc.fps(x, m))
-    assert fps_us(cu(x), m) < 12 * clean
+    assert fps_us(cu(x), m) < 3 * clean
     assert _lib.device_status() == 0
 
 

@@ -70,7 +70,13 @@ __device__ __forceinline__ float from_ordered(int o) { return __int_as_float(o >
 // ---------------------------------------------------------------- order of the points
 //
 // Counting sort by cells of a 2^bits-per-axis grid along a Hilbert curve, all clouds at once, the
-// counters (and the box) in the part of the scratch where the running minima will be.
+// counters (and the boxes) in the part of the scratch where the running minima will be.
+//
+// The grid covers the box of all points as far as that is within three times the box of most of them:
+// with one point far away all others shared a cell, and every sample reached every chunk (200000
+// points -> 2000, one point at 1e5: 7.5 ms instead of 1.0).  What lies outside belongs to the cells at
+// the grid's faces.
+constexpr int kLargeBoxInts = 12;  // least and largest coordinates of all points, then of most
 
 struct SortBox
 {
@@ -80,12 +86,15 @@ struct SortBox
 __device__ __forceinline__ SortBox sort_box(const int* box, int bits)
 {
     SortBox s;
-    float ext = 0.f;
+    float ext = 0.f, most = 0.f;
+#pragma unroll
+    for (int a = 0; a < 3; ++a) most = fmaxf(most, from_ordered(box[9 + a]) - from_ordered(box[6 + a]));
+    if (!(most > 0.f)) most = CUDART_INF_F;  // most in one place
 #pragma unroll
     for (int a = 0; a < 3; ++a)
     {
-        s.lo[a] = from_ordered(box[a]);
-        ext = fmaxf(ext, from_ordered(box[3 + a]) - s.lo[a]);
+        s.lo[a] = fmaxf(from_ordered(box[a]), from_ordered(box[6 + a]) - most);
+        ext = fmaxf(ext, fminf(from_ordered(box[3 + a]), from_ordered(box[9 + a]) + most) - s.lo[a]);
     }
     s.qmax = static_cast<float>((1 << bits) - 1);
     s.inv_h = (ext > 0.f && ext < CUDART_INF_F) ? static_cast<float>(1 << bits) * 0.999999f / ext : 0.f;
@@ -103,20 +112,75 @@ __device__ __forceinline__ int sort_cell(const SortBox& s, int bits, float x, fl
 __global__ void __launch_bounds__(256) large_clear_kernel(int n, int cells, int* __restrict__ counters)
 {
     int* cnt = counters + static_cast<size_t>(blockIdx.y) * n;
-    for (int c = blockIdx.x * 256 + threadIdx.x; c < cells + 6; c += gridDim.x * 256)
-        cnt[c] = c < cells ? 0 : (c < cells + 3 ? INT_MAX : INT_MIN);
+    for (int c = blockIdx.x * 256 + threadIdx.x; c < cells + kLargeBoxInts; c += gridDim.x * 256)
+        cnt[c] = c < cells ? 0 : ((c - cells) % 6 < 3 ? INT_MAX : INT_MIN);
+}
+
+// The box of most points, from the boxes of eight groups of 64 points each: the third smallest of their
+// lower and the third largest of their upper faces, so that up to two groups with a point far away do
+// no harm.  All threads of a CTA of 256.
+__device__ void large_box_of_most(int n, const float* __restrict__ xyz, int* __restrict__ box)
+{
+    __shared__ int s_face[6][8];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    int lo[3] = {INT_MAX, INT_MAX, INT_MAX}, hi[3] = {INT_MIN, INT_MIN, INT_MIN};
+#pragma unroll
+    for (int u = 0; u < 2; ++u)
+    {
+        // places that follow no period of the cloud (multiples of the golden ratio)
+        const uint32_t i = static_cast<uint32_t>(u * 256 + tid);
+        const size_t k = static_cast<unsigned long long>(i * 2654435769u) * static_cast<uint32_t>(n) >> 32;
+#pragma unroll
+        for (int a = 0; a < 3; ++a)
+        {
+            const float v = __ldg(xyz + 3 * k + a);
+            if (fabsf(v) < 1.0e18f)
+            {
+                lo[a] = min(lo[a], ordered_image(v));
+                hi[a] = max(hi[a], ordered_image(v));
+            }
+        }
+    }
+#pragma unroll
+    for (int a = 0; a < 3; ++a)
+    {
+        const int l = __reduce_min_sync(kFullMask, lo[a]), h = __reduce_max_sync(kFullMask, hi[a]);
+        if (lane == 0)
+        {
+            s_face[a][warp] = l;
+            s_face[3 + a][warp] = h;
+        }
+    }
+    __syncthreads();
+    if (tid < 48)
+    {
+        // its place among the eight, equal ones by their number
+        const int face = tid >> 3, mine = tid & 7, v = s_face[face][mine];
+        int before = 0;
+        for (int w = 0; w < 8; ++w)
+        {
+            const int o = s_face[face][w];
+            before += (face < 3 ? o < v : o > v) || (o == v && w < mine) ? 1 : 0;
+        }
+        if (before == 2) box[face] = v;
+    }
 }
 
 __global__ void __launch_bounds__(256) large_box_kernel(int n, int cells, const float* __restrict__ xyz_all, int* __restrict__ counters)
 {
     const float* xyz = xyz_all + static_cast<size_t>(blockIdx.y) * n * 3;
     int* box = counters + static_cast<size_t>(blockIdx.y) * n + cells;
+    if (blockIdx.x == gridDim.x - 1)  // the last CTA of a cloud
+    {
+        large_box_of_most(n, xyz, box + 6);
+        return;
+    }
     __shared__ int s_box[6];
     const int tid = threadIdx.x;
     if (tid < 6) s_box[tid] = tid < 3 ? INT_MAX : INT_MIN;
     __syncthreads();
     int lo[3] = {INT_MAX, INT_MAX, INT_MAX}, hi[3] = {INT_MIN, INT_MIN, INT_MIN};
-    for (int k = blockIdx.x * 256 + tid; k < n; k += gridDim.x * 256)
+    for (int k = blockIdx.x * 256 + tid; k < n; k += (gridDim.x - 1) * 256)
 #pragma unroll
         for (int a = 0; a < 3; ++a)
         {
@@ -1159,7 +1223,7 @@ int launch_large(int b, int n, int m, int log2bs, int nranks, const LargeLayout&
 
 int sort_points(int b, int n, const float* xyz, float4* sorted, int* counters, cudaStream_t stream)
 {
-    // about four points per cell and at most 64^3 cells; the counters need 6 words more
+    // about four points per cell and at most 64^3 cells; the counters need kLargeBoxInts words more
     int bits = 2;
     while (bits < 6 && (32ll << (3 * bits)) <= n) ++bits;
     const unsigned blocks = static_cast<unsigned>(n < 256 * 4 ? 1 : (n / (256 * 4) < 592 ? n / (256 * 4) : 592));
@@ -1177,7 +1241,7 @@ int sort_points(int b, int n, const float* xyz, float4* sorted, int* counters, c
         }
         const int cells = 1 << (3 * bits);
         count_launches(1), large_clear_kernel<<<dim3(blocks < 64 ? blocks : 64, nb), 256, 0, stream>>>(n, cells, c);
-        count_launches(1), large_box_kernel<<<grid, 256, 0, stream>>>(n, cells, x, c);
+        count_launches(1), large_box_kernel<<<dim3(blocks + 1, nb), 256, 0, stream>>>(n, cells, x, c);
         count_launches(1), large_cells_kernel<false><<<grid, 256, 0, stream>>>(n, bits, x, c, s);
         count_launches(1), large_scan_kernel<<<nb, 1024, 0, stream>>>(n, cells, c);
         count_launches(1), large_cells_kernel<true><<<grid, 256, 0, stream>>>(n, bits, x, c, s);
