@@ -214,6 +214,53 @@ def test_ball_query_warp_scan_matches_oracle(n, m, ns, r, per_warp, monkeypatch)
     assert _lib.device_status() == 0
 
 
+@pytest.mark.parametrize("share", [0.0, 0.1, 0.45, 0.55, 0.9, 1.0])
+@pytest.mark.parametrize("ns,r", [(70, 0.2), (64, 0.6), (130, 0.3)])
+def test_ball_query_leftovers_in_tiles_or_one_by_one(share, ns, r, monkeypatch):
+    """Centres around a clump, which the grid leaves over, few of them and many: lists that fill up and
+    lists that stay open, against the scans alone."""
+    g = data.gen(ns)
+    B, N, M = 10, 4600, 4133
+    x = data.unit_ball(B, N, seed=ns)
+    x[:, ::3] = 0.04 * x[:, ::3] + 0.1
+    k = int(share * M)
+    y = torch.cat([x[:, ::3].repeat(1, 3, 1)[:, :k] + 0.01, 3 + data.unit_ball(B, M - k, seed=1)], 1)
+    y = y[:, torch.randperm(M, generator=g)].contiguous()
+    y[2, 70:200, 1] = float("nan")
+    got = []
+    for path in (None, "ball_query_scan", "ball_warp_scan"):
+        data.use_paths(monkeypatch, path)
+        got.append(tpk.ball_query(r, ns, cu(x), cu(y), mode="dense"))
+    for other in got[1:]:
+        assert torch.equal(got[0][0], other[0]) and torch.equal(got[0][1], other[1])
+    assert _lib.device_status() == 0
+
+
+@pytest.mark.parametrize("hits,ns", [(130, 128), (200, 256)])
+def test_ball_query_lists_that_stay_open(hits, ns, monkeypatch):
+    """Most centres are left over and their lists take nearly the whole cloud: one by one they took twice
+    the tiled scan."""
+    x = cu(data.unit_ball(16, 16384, seed=hits))
+    y = x[:, ::4].contiguous()
+    radius = (hits / 16384) ** (1 / 3)
+
+    def us():
+        out = []
+        for _ in range(5):
+            begin, end = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            begin.record()
+            tpk.ball_query(radius, ns, x, y, mode="dense")
+            end.record()
+            torch.cuda.synchronize()
+            out.append(begin.elapsed_time(end) * 1e3)
+        return min(out[1:])
+
+    data.use_paths(monkeypatch)
+    default = us()
+    data.use_paths(monkeypatch, "ball_query_scan")
+    assert default < 1.8 * us()
+
+
 @pytest.mark.parametrize("spread", [0.0, 0.02, 1.0])
 def test_ball_query_crowded_centres_are_scanned(spread, monkeypatch):
     """What the grids leave over (more candidates than they take): dense and packed against the scan alone."""

@@ -37,7 +37,7 @@ int sg_ball_query(int b, int n, int m, float radius, int nsample, const float* n
 // ball_scan.cu
 bool ball_scan_wanted(int b, int n, int m);
 int ball_scan_dense(int b, int n, int m, float radius, int nsample, const float* new_xyz, const float* xyz, int64_t* idx,
-                    float* dist, const unsigned char* need, cudaStream_t s);
+                    float* dist, const unsigned char* need, bool unless_most, cudaStream_t s);
 int ball_scan_partial(long long size_x, long long size_y, float radius, int nsample, const float* x, const float* y,
                       const int64_t* batch_x, const int64_t* batch_y, int64_t* idx, float* dist, const unsigned char* need,
                       cudaStream_t s);
@@ -119,8 +119,8 @@ __global__ void __launch_bounds__(THREADS)
 
     if (need != nullptr)
     {
-        // nothing left over for this CTA (the usual case behind the grid kernels): leave
-        // before staging a single tile
+        // behind a grid: all that it left over, or nothing (ball_scan_kernel takes the other case)
+        if (!mostly_left<THREADS>(need, static_cast<long long>(gridDim.x / tiles_per_cloud) * m)) return;
         bool any = false;
 #pragma unroll
         for (int q = 0; q < Q; ++q) any |= op.act[q];
@@ -281,7 +281,7 @@ extern "C" int tpk_ball_query_dense(int b, int n, int m, float radius, int nsamp
     TPK_REQUIRE(new_xyz && idx && dist && (xyz || n == 0), "ball_query_dense: NULL pointer");
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     if (!test_path("ball_query_scan") && ball_scan_wanted(b, n, m))
-        return ball_scan_dense(b, n, m, radius, nsample, new_xyz, xyz, idx, dist, nullptr, s);
+        return ball_scan_dense(b, n, m, radius, nsample, new_xyz, xyz, idx, dist, nullptr, false, s);
     int threads, q;
     pick_shape(static_cast<long long>(b) * m, &threads, &q);
     const int tiles = (m + threads * q - 1) / (threads * q);
@@ -340,7 +340,7 @@ extern "C" int tpk_ball_query_dense_ws(int b, int n, int m, float radius, int ns
     TPK_REQUIRE(new_xyz && xyz && idx && dist, "ball_query_dense: NULL pointer");
     TPK_REQUIRE((reinterpret_cast<uintptr_t>(scratch) & 255u) == 0, "ball_query_dense: scratch must be 256-byte aligned");
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    if (ball_scan_wanted(b, n, m)) return ball_scan_dense(b, n, m, radius, nsample, new_xyz, xyz, idx, dist, nullptr, s);
+    if (ball_scan_wanted(b, n, m)) return ball_scan_dense(b, n, m, radius, nsample, new_xyz, xyz, idx, dist, nullptr, false, s);
     const unsigned char* need = nullptr;
     int rc;
     if (use_smem_grid(b, n, nsample))
@@ -361,16 +361,24 @@ extern "C" int tpk_ball_query_dense_ws(int b, int n, int m, float radius, int ns
         rc = grid_ball_query_dense(b, n, m, radius, nsample, new_xyz, xyz, idx, dist, scratch, &need, s);
     }
     if (rc != TPK_OK) return rc;
-    // centres the grid left over (dense neighbourhoods, degenerate clouds): index-order scan
-    if (need != nullptr) return ball_scan_dense(b, n, m, radius, nsample, new_xyz, xyz, idx, dist, need, s);
     int threads, q;
     pick_shape(static_cast<long long>(b) * m, &threads, &q);
     const int tiles = (m + threads * q - 1) / (threads * q);
     const long long grid = static_cast<long long>(b) * tiles;
     TPK_REQUIRE(grid < (1ll << 31), "ball_query_dense: too many centres");
     const dim3 g(static_cast<unsigned>(grid));
-    TPK_BQ_DISPATCH(ball_query_dense_kernel, n, m, tiles, radius, nsample, new_xyz, xyz, idx, dist, need);
-    return check_launch("ball_query_dense");
+    // Centres the grid left over (dense neighbourhoods, layers that do not fit, degenerate clouds) are scanned
+    // for in index order, one by one, or, where that is most of them and their lists may stay open, by the
+    // tiled scan, which spends a third of the instructions on a pair but reads the whole cloud for a single
+    // centre of a CTA, too.  Which of the two is seen on the device; the other one returns (8 us for both to
+    // find out).  us, one by one and tiled: 16 x 16384 points, 4096 centres, 130 in reach, lists of 128 1300 and
+    // 740, of 64 842 and 704; 32 x 8192, 4096 centres, 200 in reach, lists of 256 1940 and 1160; but with fewer
+    // than two CTAs an SM the tiles wait for their loads (4 x 65536, 8192 centres, 90 in reach, lists of 32 914
+    // and 1280), and short lists fill up (of 16 600 and 910).
+    const bool either = use_smem_grid(b, n, nsample) && nsample >= 64 && grid >= 2 * num_sms();
+    if (need == nullptr || either) TPK_BQ_DISPATCH(ball_query_dense_kernel, n, m, tiles, radius, nsample, new_xyz, xyz, idx, dist, need);
+    if (need == nullptr) return check_launch("ball_query_dense");
+    return ball_scan_dense(b, n, m, radius, nsample, new_xyz, xyz, idx, dist, need, either, s);
 }
 
 static int launch_partial_scan(long long size_x, long long size_y, float radius, int nsample, const float* x,

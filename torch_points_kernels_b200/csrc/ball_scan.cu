@@ -28,11 +28,12 @@ __global__ void __launch_bounds__(kBsThreads)
     ball_scan_kernel(long long total, int per_warp, long long n, long long m, float radius, int nsample,
                      const float* __restrict__ y, const float* __restrict__ x, const int64_t* __restrict__ batch_x,
                      const int64_t* __restrict__ batch_y, int64_t* __restrict__ idx_out, float* __restrict__ dist_out,
-                     const unsigned char* __restrict__ need)
+                     const unsigned char* __restrict__ need, bool unless_most)
 {
     const int lane = threadIdx.x & 31;
     const long long warp = (static_cast<long long>(blockIdx.x) * kBsThreads + threadIdx.x) >> 5;
     const long long j0 = warp * per_warp;
+    if (unless_most && mostly_left<kBsThreads>(need, total)) return;  // the tiled scan has answered them all
     if (j0 >= total) return;
     const float r2 = __fmul_rn(radius, radius);
     const uint32_t below = (1u << lane) - 1u;
@@ -201,7 +202,7 @@ __global__ void __launch_bounds__(kBsThreads)
 template <bool PARTIAL>
 int launch_ball_scan(long long total, long long n, long long m, float radius, int nsample, const float* y, const float* x,
                      const int64_t* batch_x, const int64_t* batch_y, int64_t* idx, float* dist, const unsigned char* need,
-                     cudaStream_t s)
+                     bool unless_most, cudaStream_t s)
 {
     // Centres of a warp side by side share its loads, but the first one that stays open keeps the
     // warp; a single one each while there are too few warps to hide the latency.  4096 centres of
@@ -225,7 +226,7 @@ int launch_ball_scan(long long total, long long n, long long m, float radius, in
 #define TPK_BALL_SCAN(Q)                                                                                                  \
     prefer_max_shared(ball_scan_kernel<PARTIAL, Q>),                                                                     \
         ball_scan_kernel<PARTIAL, Q><<<static_cast<unsigned>(blocks), kBsThreads, 0, s>>>(                               \
-            total, static_cast<int>(per_warp), n, m, radius, nsample, y, x, batch_x, batch_y, idx, dist, need)
+            total, static_cast<int>(per_warp), n, m, radius, nsample, y, x, batch_x, batch_y, idx, dist, need, unless_most)
     if (q == 4)
         TPK_BALL_SCAN(4);
     else if (q == 2)
@@ -257,18 +258,19 @@ bool ball_scan_wanted(int b, int n, int m)
 float ball_scan_crowded(double n, int nsample) { return static_cast<float>(4.5 * cbrt(1.9 * n * nsample)); }
 
 // need (optional): one byte per centre, the centres with a zero are left as they are.
+// unless_most: ... and all of them where mostly_left() says so.
 int ball_scan_dense(int b, int n, int m, float radius, int nsample, const float* new_xyz, const float* xyz, int64_t* idx,
-                    float* dist, const unsigned char* need, cudaStream_t s)
+                    float* dist, const unsigned char* need, bool unless_most, cudaStream_t s)
 {
     return launch_ball_scan<false>(static_cast<long long>(b) * m, n, m, radius, nsample, new_xyz, xyz, nullptr, nullptr, idx,
-                                   dist, need, s);
+                                   dist, need, unless_most, s);
 }
 
 int ball_scan_partial(long long size_x, long long size_y, float radius, int nsample, const float* x, const float* y,
                       const int64_t* batch_x, const int64_t* batch_y, int64_t* idx, float* dist, const unsigned char* need,
                       cudaStream_t s)
 {
-    return launch_ball_scan<true>(size_y, size_x, 1, radius, nsample, y, x, batch_x, batch_y, idx, dist, need, s);
+    return launch_ball_scan<true>(size_y, size_x, 1, radius, nsample, y, x, batch_x, batch_y, idx, dist, need, false, s);
 }
 
 }  // namespace tpk

@@ -231,6 +231,19 @@ __device__ __forceinline__ void scan_candidates(const float* __restrict__ cand, 
     }
 }
 
+// Whether a grid left over most of `total` centres (need: a byte each), by 256 of them at fixed places:
+// the same answer in every CTA and kernel.  All threads of a CTA.
+template <int THREADS>
+__device__ __forceinline__ bool mostly_left(const unsigned char* __restrict__ need, long long total)
+{
+    constexpr int S = 256;
+    int left = 0;
+#pragma unroll
+    for (int i = 0; i < S / THREADS; ++i)
+        left += __syncthreads_count(need[(i * THREADS + static_cast<int>(threadIdx.x)) * total / S] != 0 ? 1 : 0);
+    return 2 * left >= S;
+}
+
 // First position in sorted ids[0..n) whose value is >= v (upper = false) or > v (upper = true).
 __device__ __forceinline__ long long segment_bound(const int64_t* __restrict__ ids, long long n,
                                                    int64_t v, bool upper)
