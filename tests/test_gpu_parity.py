@@ -261,6 +261,53 @@ def test_ball_query_lists_that_stay_open(hits, ns, monkeypatch):
     assert default < 1.8 * us()
 
 
+@pytest.mark.parametrize("n,m,ns,r", [(1, 3, 2, 0.5), (5, 1, 9, 3.0), (127, 33, 8, 0.4), (1025, 70, 32, 0.3), (1027, 9, 3, 0.6),
+                                      (4097, 5, 64, 0.2), (2051, 40, 256, 2.0), (9001, 7, 17, 0.15), (1536, 40, 1, 0.01)])
+@pytest.mark.parametrize("warps", [2, 4, 8])
+def test_ball_query_walk_of_several_warps_matches_oracle(n, m, ns, r, warps, monkeypatch):
+    """Parts without a hit, with some, with more than the list takes; every offset of a cloud from a
+    16-byte boundary; fewer points than parts."""
+    data.use_paths(monkeypatch, "ball_warp_scan", "ball_warp_scan_w=%d" % warps)
+    x = data.unit_ball(4, n, seed=n).numpy().copy()
+    y = data.unit_ball(4, m, seed=n + 1).numpy().copy()
+    x[1, n // 2, 1] = np.nan
+    y[2, 0, 0] = np.inf
+    idx, dist = tpk.ball_query(r, ns, cu(x), cu(y), mode="dense")
+    oi, od = orc.ball_query_dense(r, ns, x, y)
+    np.testing.assert_array_equal(npy(idx), oi)
+    np.testing.assert_array_equal(npy(dist).view(np.int32), od.view(np.int32))
+    assert _lib.device_status() == 0
+
+
+@pytest.mark.parametrize("b,n,m", [(1, 1048576, 100), (1, 1048576, 16), (1, 262144, 450), (1, 65536, 1800), (1, 65536, 100),
+                                   (2, 32768, 64)])
+def test_ball_query_few_centres_of_a_large_cloud(b, n, m, monkeypatch):
+    """The walk of one warp over such a cloud took up to 24 times the grid."""
+    x = data.unit_ball(b, n, seed=m)
+    y = cu(x[:, :: n // m][:, :m].contiguous())
+    x = cu(x)
+
+    def us(radius):
+        out = []
+        for _ in range(6):
+            begin, end = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            begin.record()
+            tpk.ball_query(radius, 32, x, y, mode="dense")
+            end.record()
+            torch.cuda.synchronize()
+            out.append(begin.elapsed_time(end) * 1e3)
+        return min(out[1:])
+
+    for hits in (8, 250):  # lists that stay open, lists that fill up
+        radius = (hits / n) ** (1 / 3)
+        data.use_paths(monkeypatch)
+        got, default = tpk.ball_query(radius, 32, x, y, mode="dense"), us(radius)
+        data.use_paths(monkeypatch, "ball_query_no_warp_scan")
+        want, grid = tpk.ball_query(radius, 32, x, y, mode="dense"), us(radius)
+        assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
+        assert default < 1.4 * grid + 5
+
+
 @pytest.mark.parametrize("spread", [0.0, 0.02, 1.0])
 def test_ball_query_crowded_centres_are_scanned(spread, monkeypatch):
     """What the grids leave over (more candidates than they take): dense and packed against the scan alone."""

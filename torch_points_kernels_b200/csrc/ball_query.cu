@@ -300,6 +300,14 @@ static bool use_smem_grid(int b, int n, int nsample)
     return tpk::sg_ball_query_fits(b, n, nsample) && !tpk::test_path("ball_query_global_grid");
 }
 
+// Whether a warp per centre answers a call that could have a grid.  Not where that is the hashed grid: 1 x 262144
+// points, 450 centres, 8 and 250 in reach, grid 60 and 97 us, one warp a centre 489 and 208; 1 x 1048576, 100 centres,
+// 80 and 120 against 1867 and 709; and eight warps a centre still walk 1024 steps of 0.23 us.
+static bool scan_answers(int b, int n, int m)
+{
+    return n < (1 << 18) && tpk::ball_scan_wanted(b, n, m);
+}
+
 // Clouds the shared-memory grid does not take (2^18 points and more): the hashed grid in
 // global scratch.  The test hook "ball_query_global_grid" selects the older bounding-box grid in
 // global memory instead of either.
@@ -340,7 +348,7 @@ extern "C" int tpk_ball_query_dense_ws(int b, int n, int m, float radius, int ns
     TPK_REQUIRE(new_xyz && xyz && idx && dist, "ball_query_dense: NULL pointer");
     TPK_REQUIRE((reinterpret_cast<uintptr_t>(scratch) & 255u) == 0, "ball_query_dense: scratch must be 256-byte aligned");
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    if (ball_scan_wanted(b, n, m)) return ball_scan_dense(b, n, m, radius, nsample, new_xyz, xyz, idx, dist, nullptr, false, s);
+    if (scan_answers(b, n, m)) return ball_scan_dense(b, n, m, radius, nsample, new_xyz, xyz, idx, dist, nullptr, false, s);
     const unsigned char* need = nullptr;
     int rc;
     if (use_smem_grid(b, n, nsample))

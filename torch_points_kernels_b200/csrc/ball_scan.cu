@@ -9,6 +9,10 @@
 // serves small problems outright, and the centres that a grid leaves over because they are
 // crowded, which are the ones with the shortest scans.
 //
+// A walk over the whole cloud takes 0.23 us per 128 points however idle the GPU is, so where there are
+// few centres, up to eight warps share one: each walks a part of the cloud and keeps up to nsample
+// hits in shared memory, and the lists are joined in the order of the parts.
+//
 // Points are read as three 16-byte loads per lane (four points), the next block while this one is
 // tested, distances with the two-wide FP32 instructions, in the arithmetic of the tests:
 // dense   cuda/src/ball_query_gpu.cu:35-36, strict; packed cuda/src/ball_query_gpu.cu:78-82, inclusive.
@@ -22,19 +26,24 @@ namespace
 
 constexpr int kBsThreads = 256;
 constexpr int kBsBlock = 128;  // points per step of a warp
+constexpr int kBsSplitSamples = 256;  // lists of that length fit shared memory for every warp (16 KB)
 
-template <bool PARTIAL, int Q>
+// W: warps that share a centre (with Q = 1, per_warp = 1 and without `need`).
+template <bool PARTIAL, int Q, int W>
 __global__ void __launch_bounds__(kBsThreads)
     ball_scan_kernel(long long total, int per_warp, long long n, long long m, float radius, int nsample,
                      const float* __restrict__ y, const float* __restrict__ x, const int64_t* __restrict__ batch_x,
                      const int64_t* __restrict__ batch_y, int64_t* __restrict__ idx_out, float* __restrict__ dist_out,
                      const unsigned char* __restrict__ need, bool unless_most)
 {
-    const int lane = threadIdx.x & 31;
-    const long long warp = (static_cast<long long>(blockIdx.x) * kBsThreads + threadIdx.x) >> 5;
+    extern __shared__ int2 s_hits[];  // W > 1: index and distance of the hits, nsample for each warp
+    __shared__ int s_found[kBsThreads / 32];
+    const int lane = threadIdx.x & 31, slot = threadIdx.x >> 5, part = slot % W;
+    const long long warp = ((static_cast<long long>(blockIdx.x) * kBsThreads + threadIdx.x) >> 5) / W;
     const long long j0 = warp * per_warp;
     if (unless_most && mostly_left<kBsThreads>(need, total)) return;  // the tiled scan has answered them all
     if (j0 >= total) return;
+    int2* hits = s_hits + static_cast<size_t>(slot) * nsample;
     const float r2 = __fmul_rn(radius, radius);
     const uint32_t below = (1u << lane) - 1u;
     bool mine = lane < per_warp && j0 + lane < total;
@@ -108,30 +117,37 @@ __global__ void __launch_bounds__(kBsThreads)
                 const int at = found[q] + __popc(b & below);
                 if (hit && at < nsample)
                 {
-                    idx_out[row[q] * nsample + at] = base + k0 + lane;
-                    dist_out[row[q] * nsample + at] = d;
+                    if constexpr (W > 1)
+                        hits[at] = make_int2(static_cast<int>(base + k0 + lane), __float_as_int(d));
+                    else
+                    {
+                        idx_out[row[q] * nsample + at] = base + k0 + lane;
+                        dist_out[row[q] * nsample + at] = d;
+                    }
                 }
                 found[q] += __popc(b);
             }
         };
         // 16-byte boundaries recur every four points: 12 k = -address (mod 16)
         const long long head = min(cnt, static_cast<long long>((reinterpret_cast<uintptr_t>(p) >> 2) & 3u));
-        if (head > 0) single(0, static_cast<int>(head));
+        if (part == 0 && head > 0) single(0, static_cast<int>(head));
         const float4* v = reinterpret_cast<const float4*>(p + 3 * head);
         const long long blocks = (cnt - head) / kBsBlock;
+        const long long t0 = blocks * part / W, t1 = blocks * (part + 1) / W;
         float4 a = {}, b = {}, c = {};
-        if (blocks > 0)
+        if (t0 < t1)
         {
-            a = __ldg(v + 3 * lane + 0);
-            b = __ldg(v + 3 * lane + 1);
-            c = __ldg(v + 3 * lane + 2);
+            const float4* at = v + 3 * (kBsBlock / 4) * t0 + 3 * lane;
+            a = __ldg(at + 0);
+            b = __ldg(at + 1);
+            c = __ldg(at + 2);
         }
-        for (long long t = 0; t < blocks && open(); ++t)
+        for (long long t = t0; t < t1 && open(); ++t)
         {
             const unsigned long long x01 = pack2(a.x, a.w), x23 = pack2(b.z, c.y);
             const unsigned long long y01 = pack2(a.y, b.x), y23 = pack2(b.w, c.z);
             const unsigned long long z01 = pack2(a.z, b.y), z23 = pack2(c.x, c.w);
-            if (t + 1 < blocks)
+            if (t + 1 < t1)
             {
                 const float4* next = v + 3 * (kBsBlock / 4) * (t + 1) + 3 * lane;
                 a = __ldg(next + 0);
@@ -176,33 +192,84 @@ __global__ void __launch_bounds__(kBsThreads)
                     {
                         if (at < nsample)
                         {
-                            idx_out[row[q] * nsample + at] = base + k0 + 4 * lane + i;
-                            dist_out[row[q] * nsample + at] = d[i];
+                            if constexpr (W > 1)
+                                hits[at] = make_int2(static_cast<int>(base + k0 + 4 * lane + i), __float_as_int(d[i]));
+                            else
+                            {
+                                idx_out[row[q] * nsample + at] = base + k0 + 4 * lane + i;
+                                dist_out[row[q] * nsample + at] = d[i];
+                            }
                         }
                         ++at;
                     }
                 found[q] += all;
             }
         }
-        for (long long k = head + blocks * kBsBlock; k < cnt && open(); k += 32)
+        for (long long k = head + blocks * kBsBlock; part == W - 1 && k < cnt && open(); k += 32)
             single(k, static_cast<int>(min(32ll, cnt - k)));
-#pragma unroll
-        for (int q = 0; q < Q; ++q)
+        if constexpr (W > 1)
         {
-            if (!act[q]) continue;
-            for (int s = min(found[q], nsample) + lane; s < nsample; s += 32)
+            // the lists of the W warps, in the order of their parts
+            if (lane == 0) s_found[slot] = min(found[0], nsample);
+            asm volatile("bar.sync %0, %1;" ::"r"(1 + slot / W), "n"(32 * W) : "memory");
+            int before = 0, all = 0;
+            long long head_hit = first[0];
+#pragma unroll
+            for (int w = W - 1; w >= 0; --w)
             {
-                idx_out[row[q] * nsample + s] = PARTIAL ? -1 : first[q];
-                dist_out[row[q] * nsample + s] = -1.0f;
+                const int f = s_found[slot - part + w];
+                before += w < part ? f : 0;
+                all += f;
+                if (f > 0) head_hit = s_hits[static_cast<size_t>(slot - part + w) * nsample].x;
+            }
+            for (int s = lane; s < min(found[0], nsample - before); s += 32)
+            {
+                idx_out[row[0] * nsample + before + s] = hits[s].x;
+                dist_out[row[0] * nsample + before + s] = __int_as_float(hits[s].y);
+            }
+            for (int s = all + 32 * part + lane; s < nsample; s += 32 * W)
+            {
+                idx_out[row[0] * nsample + s] = PARTIAL ? -1 : head_hit;
+                dist_out[row[0] * nsample + s] = -1.0f;
+            }
+            return;
+        }
+        else
+        {
+#pragma unroll
+            for (int q = 0; q < Q; ++q)
+            {
+                if (!act[q]) continue;
+                for (int s = min(found[q], nsample) + lane; s < nsample; s += 32)
+                {
+                    idx_out[row[q] * nsample + s] = PARTIAL ? -1 : first[q];
+                    dist_out[row[q] * nsample + s] = -1.0f;
+                }
             }
         }
     }
 }
 
+template <bool PARTIAL, int Q, int W>
+int launch_ball_scan(long long total, int per_warp, long long n, long long m, float radius, int nsample, const float* y,
+                     const float* x, const int64_t* batch_x, const int64_t* batch_y, int64_t* idx, float* dist,
+                     const unsigned char* need, bool unless_most, cudaStream_t s)
+{
+    const long long warps = (total + per_warp - 1) / per_warp * W;
+    const long long blocks = (warps + kBsThreads / 32 - 1) / (kBsThreads / 32);
+    TPK_REQUIRE(blocks < (1ll << 31), "ball_query: too many centres");
+    const size_t smem = W > 1 ? sizeof(int2) * kBsThreads / 32 * nsample : 0;
+    count_launches(1);
+    prefer_max_shared(ball_scan_kernel<PARTIAL, Q, W>);
+    ball_scan_kernel<PARTIAL, Q, W><<<static_cast<unsigned>(blocks), kBsThreads, smem, s>>>(
+        total, per_warp, n, m, radius, nsample, y, x, batch_x, batch_y, idx, dist, need, unless_most);
+    return check_launch("ball_query scan");
+}
+
 template <bool PARTIAL>
-int launch_ball_scan(long long total, long long n, long long m, float radius, int nsample, const float* y, const float* x,
-                     const int64_t* batch_x, const int64_t* batch_y, int64_t* idx, float* dist, const unsigned char* need,
-                     bool unless_most, cudaStream_t s)
+int pick_ball_scan(long long total, long long n, long long m, float radius, int nsample, const float* y, const float* x,
+                   const int64_t* batch_x, const int64_t* batch_y, int64_t* idx, float* dist, const unsigned char* need,
+                   bool unless_most, cudaStream_t s)
 {
     // Centres of a warp side by side share its loads, but the first one that stays open keeps the
     // warp; a single one each while there are too few warps to hide the latency.  4096 centres of
@@ -210,8 +277,15 @@ int launch_ball_scan(long long total, long long n, long long m, float radius, in
     // up: 31, 35, 43.
     int q = total >= 16384 ? 4 : (total >= 8192 ? 2 : 1);
     if (need != nullptr) q = 2;
+    // Several warps for a centre as long as they all run at once (32 on an SM) and each has 16 steps or
+    // more.
+    int w = 1;
+    if (!PARTIAL && need == nullptr && q == 1 && nsample <= kBsSplitSamples)
+        while (w < 8 && 2 * w * total <= 32ll * num_sms() && n >= 32ll * w * kBsBlock) w *= 2;
     char text[16];
-    if (test_value("ball_warp_scan_q", text, sizeof(text))) q = text[0] == '4' ? 4 : (text[0] == '2' ? 2 : 1);  // test hook
+    if (test_value("ball_warp_scan_q", text, sizeof(text))) q = text[0] == '4' ? 4 : (text[0] == '2' ? 2 : 1), w = 1;  // test hook
+    if (!PARTIAL && need == nullptr && nsample <= kBsSplitSamples && test_value("ball_warp_scan_w", text, sizeof(text)))  // test hook
+        q = 1, w = text[0] == '8' ? 8 : (text[0] == '4' ? 4 : 2);
     long long per_warp = q;
     if (need != nullptr)
     {
@@ -219,31 +293,29 @@ int launch_ball_scan(long long total, long long n, long long m, float radius, in
         per_warp = total / (32ll * num_sms());
         per_warp = per_warp < q ? q : (per_warp > 32 ? 32 : per_warp);
     }
-    const long long warps = (total + per_warp - 1) / per_warp;
-    const long long blocks = (warps + kBsThreads / 32 - 1) / (kBsThreads / 32);
-    TPK_REQUIRE(blocks < (1ll << 31), "ball_query: too many centres");
-    count_launches(1);
-#define TPK_BALL_SCAN(Q)                                                                                                  \
-    prefer_max_shared(ball_scan_kernel<PARTIAL, Q>),                                                                     \
-        ball_scan_kernel<PARTIAL, Q><<<static_cast<unsigned>(blocks), kBsThreads, 0, s>>>(                               \
-            total, static_cast<int>(per_warp), n, m, radius, nsample, y, x, batch_x, batch_y, idx, dist, need, unless_most)
-    if (q == 4)
-        TPK_BALL_SCAN(4);
-    else if (q == 2)
-        TPK_BALL_SCAN(2);
-    else
-        TPK_BALL_SCAN(1);
+#define TPK_BALL_SCAN(Q, W)                                                                                             \
+    launch_ball_scan<PARTIAL, Q, W>(total, static_cast<int>(per_warp), n, m, radius, nsample, y, x, batch_x, batch_y, idx, \
+                                    dist, need, unless_most, s)
+    if constexpr (!PARTIAL)
+    {
+        if (w == 8) return TPK_BALL_SCAN(1, 8);
+        if (w == 4) return TPK_BALL_SCAN(1, 4);
+        if (w == 2) return TPK_BALL_SCAN(1, 2);
+    }
+    if (q == 4) return TPK_BALL_SCAN(4, 1);
+    if (q == 2) return TPK_BALL_SCAN(2, 1);
+    return TPK_BALL_SCAN(1, 1);
 #undef TPK_BALL_SCAN
-    return check_launch("ball_query scan");
 }
 
 }  // namespace
 
-// Whether the scan is the better way to answer all centres of a dense problem.  Up to here it is
-// where every centre reads its whole cloud, too (points uniform in a ball, 16 neighbours, lists of
-// 32; grid / scan in us): 1 x 1024 points 14.8 / 6.6, 1 x 16384 74 / 64, 16 x 4096 72 / 72,
-// 2 x 16384 76 / 101, but 4 x 16384 76 / 145; where lists fill up (points on surfaces) it is far
-// ahead: 1 x 1024 63 / 6.4, 1 x 16384 549 / 31, 16 x 4096 402 / 40.
+// Whether the scan is the better way to answer all centres of a dense problem.  us, grid / scan, lists of
+// 32, 8 to 16 points in reach and 250: 1 x 1024 points 15 / 7 and 63 / 6; 1 x 16384, 4096 centres 92 / 85 and
+// 120 / 46; 1 x 65536, 200 centres (eight warps each) 81 / 44 and 523 / 46; 8 x 131072, 64 centres 1750 / 88 and
+// 881 / 89.  Towards the bound the grid is ahead where few points are in reach, the scan where lists fill up:
+// 1 x 65536, 1800 centres 94 / 133 and 628 / 95; 1 x 32768, 3600 centres 86 / 140 and 673 / 58; 16 x 16384, 440
+// centres 76 / 110 and 290 / 59.
 bool ball_scan_wanted(int b, int n, int m)
 {
     if (test_path("ball_warp_scan")) return true;
@@ -262,7 +334,7 @@ float ball_scan_crowded(double n, int nsample) { return static_cast<float>(4.5 *
 int ball_scan_dense(int b, int n, int m, float radius, int nsample, const float* new_xyz, const float* xyz, int64_t* idx,
                     float* dist, const unsigned char* need, bool unless_most, cudaStream_t s)
 {
-    return launch_ball_scan<false>(static_cast<long long>(b) * m, n, m, radius, nsample, new_xyz, xyz, nullptr, nullptr, idx,
+    return pick_ball_scan<false>(static_cast<long long>(b) * m, n, m, radius, nsample, new_xyz, xyz, nullptr, nullptr, idx,
                                    dist, need, unless_most, s);
 }
 
@@ -270,7 +342,7 @@ int ball_scan_partial(long long size_x, long long size_y, float radius, int nsam
                       const int64_t* batch_x, const int64_t* batch_y, int64_t* idx, float* dist, const unsigned char* need,
                       cudaStream_t s)
 {
-    return launch_ball_scan<true>(size_y, size_x, 1, radius, nsample, y, x, batch_x, batch_y, idx, dist, need, false, s);
+    return pick_ball_scan<true>(size_y, size_x, 1, radius, nsample, y, x, batch_x, batch_y, idx, dist, need, false, s);
 }
 
 }  // namespace tpk
