@@ -80,7 +80,10 @@ def test_scratch_sizes_are_host_arithmetic(monkeypatch):
     assert l.tpk_fps_scratch_bytes(2, 1000, 48) == 2 * 1000 * 20
     assert l.tpk_ball_query_dense_scratch_bytes(16, 16384, 4096, 32) == 0
     monkeypatch.delenv("TPK_B200_TEST")
-    # ball query: one flag per centre with the grid in shared memory, the whole grid for huge clouds
+    # ball query: nothing up to 1.2e8 pairs, which a scan answers, one flag per centre with the grid in shared
+    # memory, the whole grid for huge clouds
+    assert l.tpk_ball_query_dense_scratch_bytes(4, 4096, 1024, 32) == 0
+    assert l.tpk_ball_query_dense_scratch_bytes(1, 65536, 1800, 32) == 0
     assert l.tpk_ball_query_dense_scratch_bytes(2, 256, 64, 32) == 0
     assert l.tpk_ball_query_dense_scratch_bytes(16, 16384, 4096, 32) == 16 * 4096
     assert l.tpk_ball_query_dense_scratch_bytes(2, 300000, 100, 32) > 2 * 300000 * 16

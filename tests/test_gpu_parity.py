@@ -556,10 +556,11 @@ def test_ball_query_dense_grid_path_matches_oracle(case, monkeypatch):
         ns = 1
     if case == "ns100":
         ns, r = 100, 0.2
+    data.use_paths(monkeypatch, "ball_query_no_warp_scan")
     assert _lib.lib().tpk_ball_query_dense_scratch_bytes(B, N, M, ns) > 0
     oi, od = orc.ball_query_dense(r, ns, x, y)
-    # the grid in shared memory (where it fits), the grid in global memory, the plain scan
-    for env in (None, "ball_query_global_grid", "ball_query_scan"):
+    # a warp per centre, the grid in shared memory (where it fits), the grid in global memory, the tiled scan
+    for env in (None, "ball_query_no_warp_scan", "ball_query_global_grid", "ball_query_scan"):
         data.use_paths(monkeypatch, env)
         idx, dist = tpk.ball_query(r, ns, cu(x), cu(y), mode="dense")
         np.testing.assert_array_equal(npy(idx), oi)
@@ -569,7 +570,7 @@ def test_ball_query_dense_grid_path_matches_oracle(case, monkeypatch):
 
 
 @pytest.mark.parametrize("case", ["crowded_layer", "nonfinite_centres", "nonfinite_points", "thin_cells", "many_centres"])
-def test_ball_query_dense_shared_memory_grid_edge_cases(case):
+def test_ball_query_dense_shared_memory_grid_edge_cases(case, monkeypatch):
     """The shared-memory grid hands back what it cannot answer: a layer with more points than
     fit, centres without a cell, clouds without a grid; cells exactly one radius wide; more
     centres than one list pass takes."""
@@ -587,6 +588,7 @@ def test_ball_query_dense_shared_memory_grid_edge_cases(case):
         y[1, 7, 2] = np.inf
     if case == "nonfinite_points":
         x[1, 10, 0] = np.inf
+    data.use_paths(monkeypatch, "ball_query_no_warp_scan")
     assert _lib.lib().tpk_ball_query_dense_scratch_bytes(B, N, M, ns) == (B * M + 255) // 256 * 256
     idx, dist = tpk.ball_query(r, ns, cu(x), cu(y), mode="dense")
     oi, od = orc.ball_query_dense(r, ns, x, y)
@@ -604,7 +606,7 @@ def test_ball_query_dense_huge_clouds_use_the_hashed_grid(kind, monkeypatch):
     need = _lib.lib().tpk_ball_query_dense_scratch_bytes(B, N, M, ns)
     assert need > B * N * 20
     oi, od = orc.ball_query_dense(r, ns, x, y)
-    for env in (None, "ball_query_global_grid", "ball_query_scan"):
+    for env in (None, "ball_query_global_grid", "ball_warp_scan", "ball_query_scan"):
         data.use_paths(monkeypatch, env)
         idx, dist = tpk.ball_query(r, ns, cu(x), cu(y), mode="dense")
         np.testing.assert_array_equal(npy(idx), oi)

@@ -320,7 +320,7 @@ static bool use_hash_grid(int b, int n, int m)
 extern "C" int64_t tpk_ball_query_dense_scratch_bytes(int b, int n, int m, int nsample)
 {
     if (b <= 0 || m <= 0 || nsample <= 0) return 0;
-    if (tpk::test_path("ball_query_scan")) return 0;  // test hook: the index-order scan alone
+    if (tpk::test_path("ball_query_scan") || scan_answers(b, n, m)) return 0;  // (test hook: the index-order scan alone)
     // shared-memory grid: one flag per centre
     if (use_smem_grid(b, n, nsample)) return (static_cast<int64_t>(b) * m + 255) / 256 * 256;
     if (use_hash_grid(b, n, m))
@@ -348,7 +348,6 @@ extern "C" int tpk_ball_query_dense_ws(int b, int n, int m, float radius, int ns
     TPK_REQUIRE(new_xyz && xyz && idx && dist, "ball_query_dense: NULL pointer");
     TPK_REQUIRE((reinterpret_cast<uintptr_t>(scratch) & 255u) == 0, "ball_query_dense: scratch must be 256-byte aligned");
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    if (scan_answers(b, n, m)) return ball_scan_dense(b, n, m, radius, nsample, new_xyz, xyz, idx, dist, nullptr, false, s);
     const unsigned char* need = nullptr;
     int rc;
     if (use_smem_grid(b, n, nsample))
