@@ -91,6 +91,18 @@ def ref_cuda():
     return points_cuda
 
 
+def test_cubic_scratch_only_where_the_copy_pays(monkeypatch):
+    """Few values looked up, or few of the map's: read in place, nothing allocated."""
+    from torch_points_kernels_b200 import _lib
+
+    size = _lib.lib().tpk_cubic_feature_sampling_scratch_bytes
+    monkeypatch.delenv("TPK_B200_TEST", raising=False)
+    assert size(16, 2048, 128, 8, 1, 4) == 4 * 16 * 128 * 8 ** 3
+    assert size(1, 100, 16, 8, 1, 4) == 0
+    assert size(1, 512, 128, 8, 1, 4) == 0
+    assert size(1, 2048, 32, 32, 1, 4) == 0
+
+
 def _region_grow_on_cpu(monkeypatch):
     """region_grow with the oracle's neighbour search and traversal behind it."""
     from torch_points_kernels_b200 import cluster
@@ -364,7 +376,7 @@ def test_cubic_feature_sampling_by_rows_matches_in_place(B, n, c, scale, ns, off
     size = B * n * (2 * ns) ** 3 * c
     gout = _cu(torch.randn(size + offset, generator=g).to(dtype))[offset:].view(B, n, (2 * ns) ** 3, c)  # unaligned rows
     got = []
-    for path in (None, "cubic_in_place"):
+    for path in ("cubic_by_rows", "cubic_in_place"):
         data.use_paths(monkeypatch, path)
         f = cf.clone().requires_grad_(True)
         out = CubicFeatureSamplingFunction.apply(p, f, ns)

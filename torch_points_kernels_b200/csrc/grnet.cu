@@ -287,11 +287,15 @@ __global__ void __launch_bounds__(kGrThreads)
 // 87 / 90, 512 points in 16^3 x 64 18 / 21 and 27 / 29; 4096 points in 32^3 x 32 64 / 71 and 97 / 117,
 // 2048 points 50 / 55 and 53 / 65; but 1400 points in 32^3 x 16 33 / 40 and 19 / 23, and one cloud of
 // 2048 points in 32^3 x 32 10 / 10 and 8 / 10.  So: as many vertices looked up as the map has, or half
-// of them where the map is too large to be found in the L2 cache for the most part.
+// of them where the map is too large to be found in the L2 cache for the most part.  The copy is one more
+// launch in each direction, which is lost below some 1.5 M values looked up (5 us a million in place, 1.5 to 2
+// by rows).
 bool cubic_by_rows(int b, int n_pts, int nvert, int channels, long long cub_scale, int itemsize)
 {
     if (test_path("cubic_in_place") || channels < 4) return false;
+    if (test_path("cubic_by_rows")) return true;
     const long long looked_up = static_cast<long long>(n_pts) * nvert;
+    if (static_cast<double>(looked_up) * b * channels < 1.5e6) return false;
     const double bytes = static_cast<double>(b) * channels * cub_scale * itemsize;
     return looked_up >= cub_scale || (2 * looked_up >= cub_scale && bytes >= 48.0e6);
 }

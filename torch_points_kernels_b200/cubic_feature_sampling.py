@@ -6,10 +6,9 @@ from . import _lib
 from .gridding import _suffix
 
 
-def _rows(b, n, c, scale, neighborhood_size, like):
-    """Scratch for the copy of the map with the channel fastest (empty where the map is read in place)."""
-    size = _lib.lib().tpk_cubic_feature_sampling_scratch_bytes(b, n, c, scale, neighborhood_size, like.element_size())
-    return torch.empty(size, dtype=torch.uint8, device=like.device)
+def _rows(size, like):
+    """Scratch for the copy of the map with the channel fastest (None where the map is read in place)."""
+    return torch.empty(size, dtype=torch.uint8, device=like.device) if size > 0 else None
 
 
 class CubicFeatureSamplingFunction(torch.autograd.Function):
@@ -27,30 +26,31 @@ class CubicFeatureSamplingFunction(torch.autograd.Function):
         nvert = (2 * int(neighborhood_size)) ** 3
         point_features = torch.empty((b, n, nvert, c), dtype=ptcloud.dtype, device=ptcloud.device)
         indexes = torch.empty((b, n, nvert), dtype=torch.int32, device=ptcloud.device)
-        scratch = _rows(b, n, c, scale, int(neighborhood_size), ptcloud)
+        need = _lib.lib().tpk_cubic_feature_sampling_scratch_bytes(b, n, c, scale, int(neighborhood_size), ptcloud.element_size())
+        scratch = _rows(need, ptcloud)
         with torch.cuda.device(ptcloud.device):
             _lib.call("tpk_cubic_feature_sampling_ws_" + sfx, b, n, c, scale, int(neighborhood_size), _lib.ptr(ptcloud),
                       _lib.ptr(cubic_features), _lib.ptr(point_features), _lib.ptr(indexes), _lib.ptr(scratch),
-                      scratch.numel(), _lib.stream_of(ptcloud))
-        ctx.cubic_for_backward = (scale, int(neighborhood_size), c)
+                      need, _lib.stream_of(ptcloud))
+        ctx.cubic_for_backward = (scale, int(neighborhood_size), c, need)
         ctx.save_for_backward(indexes)
         return point_features
 
     @staticmethod
     def backward(ctx, grad_point_features):
         (indexes,) = ctx.saved_tensors
-        scale, neighborhood_size, c = ctx.cubic_for_backward
+        scale, neighborhood_size, c, need = ctx.cubic_for_backward
         grad_point_features = grad_point_features.contiguous()
         sfx = _suffix(grad_point_features, "grad_point_features")
         b, n = indexes.shape[0], indexes.shape[1]
         dt, dev = grad_point_features.dtype, grad_point_features.device
         grad_ptcloud = torch.empty((b, n, 3), dtype=dt, device=dev)
         grad_cubic = torch.empty((b, c, scale, scale, scale), dtype=dt, device=dev)
-        scratch = _rows(b, n, c, scale, neighborhood_size, grad_point_features)
+        scratch = _rows(need, grad_point_features)  # as much as the forward pass needed
         with torch.cuda.device(dev):
             _lib.call("tpk_cubic_feature_sampling_grad_ws_" + sfx, b, n, c, scale, neighborhood_size,
                       _lib.ptr(grad_point_features), _lib.ptr(indexes), _lib.ptr(grad_ptcloud), _lib.ptr(grad_cubic),
-                      _lib.ptr(scratch), scratch.numel(), _lib.stream_of(grad_point_features))
+                      _lib.ptr(scratch), need, _lib.stream_of(grad_point_features))
         return grad_ptcloud, grad_cubic, None
 
 
