@@ -1,10 +1,15 @@
 // Ball query (radius search) for sm_100a: dense (B,N,3) clouds and packed segments.
 //
-// Brute force in candidate-index order, as the reference's rule demands ("the first
-// nsample candidates within the radius"), but query-tiled: a CTA owns THREADS*Q centres
-// and streams the candidates through shared memory (scan.cuh), stopping as soon as all
-// of its centres are full.  Each thread writes the hits of its own centres as it meets
-// them, so index order needs no sorting or compaction pass.
+// The entry points, which pick a search, and the tiled scan.  Dense problems up to 1.2e8 pairs go to a
+// warp per centre (ball_scan.cu), larger ones to a grid in shared memory (smem_grid.cu) or a hashed
+// one (hash_grid.cu, packed problems from 4096 points on as well) and what that leaves over to a scan.
+//
+// The tiled scan serves calls without scratch, packed problems too small for a grid, radii that no grid
+// can have, and what a grid in shared memory leaves over where that is most centres.  Brute force in
+// candidate-index order, as the reference's rule demands ("the first nsample candidates within the
+// radius"), but query-tiled: a CTA owns THREADS*Q centres and streams the candidates through shared
+// memory (scan.cuh), stopping as soon as all of its centres are full.  Each thread writes the hits of its
+// own centres as it meets them, so index order needs no sorting or compaction pass.
 //
 // dense   : cuda/src/ball_query_gpu.cu:9-52   d2 <  r^2, idx padded with the first hit
 //                                             (0 if none), dist padded with -1
@@ -150,7 +155,7 @@ __global__ void __launch_bounds__(THREADS)
                               const float* __restrict__ x, const float* __restrict__ y,
                               const int64_t* __restrict__ batch_x,
                               const int64_t* __restrict__ batch_y, int64_t* __restrict__ idx_out,
-                              float* __restrict__ dist_out, const unsigned char* __restrict__ need)
+                              float* __restrict__ dist_out)
 {
     __shared__ __align__(16) float smem[2 * kScanTileFloats];
     __shared__ long long s_range[2];
@@ -166,8 +171,7 @@ __global__ void __launch_bounds__(THREADS)
     for (int q = 0; q < Q; ++q)
     {
         const long long j = j0 + q * THREADS + threadIdx.x;
-        // `need` (optional): one byte per centre, 0 = already answered by the grid path
-        valid[q] = j < size_y && (need == nullptr || need[j] != 0);
+        valid[q] = j < size_y;
         const long long row = valid[q] ? j : 0;
         seg[q] = valid[q] ? __ldg(batch_y + row) : 0;
         op.cnt[q] = 0;
@@ -179,21 +183,7 @@ __global__ void __launch_bounds__(THREADS)
         op.drow[q] = dist_out + row * nsample;
     }
 
-    // sorted ids: the CTA's first centre still to be answered carries its smallest segment id
-    long long first_valid = 0x7fffffffffffffffll;
-#pragma unroll
-    for (int q = 0; q < Q; ++q)
-        if (valid[q]) first_valid = min(first_valid, j0 + q * THREADS + static_cast<long long>(threadIdx.x));
-    {
-        __shared__ unsigned long long s_first;
-        if (threadIdx.x == 0) s_first = ~0ull;
-        __syncthreads();
-        if (first_valid != 0x7fffffffffffffffll) atomicMin(&s_first, static_cast<unsigned long long>(first_valid));
-        __syncthreads();
-        if (s_first == ~0ull) return;  // nothing left over for this CTA
-        first_valid = static_cast<long long>(s_first);
-    }
-    int64_t cur = __ldg(batch_y + first_valid);
+    int64_t cur = __ldg(batch_y + j0);  // sorted ids: the CTA's first centre has the smallest
     const unsigned long long kNone = ~0ull;
     while (true)
     {
@@ -388,20 +378,6 @@ extern "C" int tpk_ball_query_dense_ws(int b, int n, int m, float radius, int ns
     return ball_scan_dense(b, n, m, radius, nsample, new_xyz, xyz, idx, dist, need, either, s);
 }
 
-static int launch_partial_scan(long long size_x, long long size_y, float radius, int nsample, const float* x,
-                               const float* y, const int64_t* batch_x, const int64_t* batch_y, int64_t* idx,
-                               float* dist, const unsigned char* need, cudaStream_t s)
-{
-    using namespace tpk;
-    int threads, q;
-    pick_shape(size_y, &threads, &q);
-    const long long grid = (size_y + threads * q - 1) / (threads * q);
-    TPK_REQUIRE(grid < (1ll << 31), "ball_query_partial_dense: too many centres");
-    const dim3 g(static_cast<unsigned>(grid));
-    TPK_BQ_DISPATCH(ball_query_partial_kernel, size_x, size_y, radius, nsample, x, y, batch_x, batch_y, idx, dist, need);
-    return check_launch("ball_query_partial_dense");
-}
-
 extern "C" int tpk_ball_query_partial_dense(int64_t size_x, int64_t size_y, float radius,
                                             int nsample, const float* x, const float* y,
                                             const int64_t* batch_x, const int64_t* batch_y,
@@ -413,8 +389,14 @@ extern "C" int tpk_ball_query_partial_dense(int64_t size_x, int64_t size_y, floa
     if (size_y == 0 || nsample == 0) return TPK_OK;
     TPK_REQUIRE(y && batch_y && idx && dist && ((x && batch_x) || size_x == 0),
                 "ball_query_partial_dense: NULL pointer");
-    return launch_partial_scan(size_x, size_y, radius, nsample, x, y, batch_x, batch_y, idx, dist, nullptr,
-                               static_cast<cudaStream_t>(stream));
+    cudaStream_t s = static_cast<cudaStream_t>(stream);
+    int threads, q;
+    pick_shape(size_y, &threads, &q);
+    const long long grid = (size_y + threads * q - 1) / (threads * q);
+    TPK_REQUIRE(grid < (1ll << 31), "ball_query_partial_dense: too many centres");
+    const dim3 g(static_cast<unsigned>(grid));
+    TPK_BQ_DISPATCH(ball_query_partial_kernel, size_x, size_y, radius, nsample, x, y, batch_x, batch_y, idx, dist);
+    return check_launch("ball_query_partial_dense");
 }
 
 // the test hook "ball_query_scan" keeps packed queries on the scan
@@ -451,6 +433,6 @@ extern "C" int tpk_ball_query_partial_dense_ws(int64_t size_x, int64_t size_y, f
     const unsigned char* need = nullptr;
     const int rc = hash_grid_ball_query(size_x, size_y, radius, nsample, x, y, batch_x, batch_y, idx, dist, scratch, &need, s);
     if (rc != TPK_OK) return rc;
-    // queries the grid left over (crowded neighbourhoods, non-finite coordinates): index-order scan
+    // queries the grid left over (crowded neighbourhoods, non-finite coordinates), one by one
     return ball_scan_partial(size_x, size_y, radius, nsample, x, y, batch_x, batch_y, idx, dist, need, s);
 }

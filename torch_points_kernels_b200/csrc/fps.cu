@@ -1,11 +1,13 @@
-// Furthest point sampling for sm_100a.
+// Furthest point sampling for sm_100a: the entry points, the choice of a kernel family, and the kernels
+// that take one sample per exchange.
 //
-// One thread-block cluster per cloud.  Every thread keeps its points' coordinates and
-// running min-distance in registers for the whole call; a round costs one distance
-// update per point, a two-instruction warp arg-max (redux.sync), and one exchange of
-// 20-byte messages between the warps of the cluster through distributed shared
-// memory.  Nothing is re-read from global memory after the initial load and the only
-// global store per round is the selected index.
+// Most clouds go by rounds of independent samples (fps_rounds.cu up to 131072 points, fps_large.cu up to
+// 4 Mi).  One sample per exchange is ahead where there are few samples, and serves small clouds: one
+// thread-block cluster per cloud, every thread keeps its points' coordinates and running min-distance
+// in registers for the whole call; a sample costs one distance update per point, a two-instruction
+// warp arg-max (redux.sync), and one exchange of 20-byte messages between the warps of the cluster
+// through distributed shared memory.  Nothing is re-read from global memory after the initial load and
+// the only global store per sample is the selected index.
 //
 // Behaviour follows cuda/src/sampling_gpu.cu:16-144 of the reference bit for bit:
 // first sample is index 0; squared distance contracted as in tpk::sumsq_abc; points
@@ -492,7 +494,6 @@ __global__ void __launch_bounds__(kFpsBigThreads, 1)
         }
 
         // ---- stage 3: cluster
-        if (nranks > 1)
         {
             if (warp == 0 && lane < nranks)
                 st_async_msg(rem_a[par], rem_z[par], rem_bar[par], static_cast<uint32_t>(msg.key),
@@ -522,13 +523,6 @@ __global__ void __launch_bounds__(kFpsBigThreads, 1)
             msg.x = __shfl_sync(kFullMask, x3, src);
             msg.y = __shfl_sync(kFullMask, y3, src);
             msg.z = __shfl_sync(kFullMask, z3, src);
-        }
-        else if (tid == 0)
-        {
-            // one-CTA cluster: nobody completes the transaction count, do it locally
-            asm volatile("mbarrier.complete_tx.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(mbar + par)),
-                         "r"(static_cast<uint32_t>(nranks * kMsgBytes))
-                         : "memory");
         }
         cx = msg.x;
         cy = msg.y;
@@ -819,9 +813,10 @@ extern "C" int tpk_furthest_point_sampling(int b, int n, int m, const float* xyz
     return fps_run(b, n, m, xyz, scratch, scratch_bytes, idxs, nullptr, &wrote_xyz, stream);
 }
 
-// Coordinates of the samples, new_xyz[b, j, :] = xyz[b, idxs[b, j], :].  A separate pass of a
-// few microseconds: written from inside the sampling kernels the four stores per round sat on
-// the critical path of every round (measured 5 % of the whole call).
+// Coordinates of the samples, new_xyz[b, j, :] = xyz[b, idxs[b, j], :], behind the kernels that take one
+// sample per exchange.  A separate pass of a few microseconds: written from inside those the four
+// stores per sample sat on the critical path of every one (measured 5 % of the whole call).  The
+// kernels that go by rounds write the coordinates themselves, at the end.
 namespace tpk
 {
 namespace
