@@ -70,7 +70,7 @@ def test_random_shapes_agree_across_kernel_families(seed, monkeypatch):
             def f():
                 hook(None); a = tpk.furthest_point_sample(x, m)
                 hook("fps_unsorted"); b = tpk.furthest_point_sample(x, m)
-                hook("fps_sorted,fps_single"); c = tpk.furthest_point_sample(x, m)
+                hook("fps_sorted"); c = tpk.furthest_point_sample(x, m)
                 return bool(torch.equal(a, b) and torch.equal(a, c))
             check(op, (B, N, m), f)
         elif op == "fps_big":

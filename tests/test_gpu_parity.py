@@ -44,9 +44,9 @@ def _guarded(fn):
 
 # ------------------------------------------------------------------------------ FPS
 
-# kernel families of FPS on a cloud that stays on chip: without the spatially sorted copy, with it
-# and one sample per exchange, with it and several samples per exchange (the default)
-FPS_FAMILIES = ["fps_unsorted", "fps_sorted,fps_single", "fps_sorted"]
+# kernel families of FPS on a cloud that stays on chip: one sample per exchange, and rounds of
+# independent samples on points in spatial order
+FPS_FAMILIES = ["fps_unsorted", "fps_sorted"]
 
 
 def test_fps_known_answer(known_answers):
@@ -70,15 +70,25 @@ def test_fps_matches_oracle(B, N, m, family, monkeypatch):
                                  "4,256,4", "8,128,4", "8,64,8", "8,512,1", "16,64,4", "16,512,1",
                                  "16,128,2"])
 def test_fps_every_cluster_shape(cfg, monkeypatch):
-    """Same cloud through every cluster size / block size (cluster x threads x points per thread),
-    with the flat and with the three-stage exchange."""
+    """One sample per exchange: same cloud through every cluster size / block size (cluster x threads x
+    points per thread), with the flat and with the three-stage exchange."""
     x = data.unit_ball(3, 4000, seed=77)
     want = orc.fps(x, 300)
     for tree in (None, "fps_tree"):
-        for family in FPS_FAMILIES:
-            data.use_paths(monkeypatch, "fps_config=" + cfg.replace(",", ":"), tree, family)
-            got = npy(tpk.furthest_point_sample(cu(x), 300))
-            np.testing.assert_array_equal(got, want)
+        data.use_paths(monkeypatch, "fps_config=" + cfg.replace(",", ":"), tree, "fps_unsorted")
+        got = npy(tpk.furthest_point_sample(cu(x), 300))
+        np.testing.assert_array_equal(got, want)
+    assert _lib.device_status() == 0
+
+
+@pytest.mark.parametrize("ranks,n", [(1, 1000), (1, 2049), (1, 4096), (2, 2048), (2, 4001), (2, 8192), (4, 4095), (4, 8192), (4, 16384),
+                                     (8, 8192), (8, 16383), (8, 32768), (16, 32768), (16, 65535), (16, 131072)])
+def test_fps_rounds_every_cluster_size_and_share(ranks, n, monkeypatch):
+    """Rounds: every number of CTAs per cloud with two, four and eight points per lane (sixteen: four,
+    eight and sixteen), up to the largest cloud of each."""
+    data.use_paths(monkeypatch, "fps_sorted", "fps_config=%d" % ranks)
+    x = data.unit_ball(2, n, seed=n)
+    np.testing.assert_array_equal(npy(tpk.furthest_point_sample(cu(x), 300)), orc.fps(x, 300))
     assert _lib.device_status() == 0
 
 
@@ -117,12 +127,11 @@ def test_fps_rounds_are_the_default_where_they_are_faster(b, n, m, family, launc
 
 
 @pytest.mark.parametrize("kind", ["clustered", "lattice", "planar", "nonfinite", "many_skipped"])
-@pytest.mark.parametrize("family", ["fps_sorted", "fps_sorted,fps_single", "fps_sorted,fps_global"])
+@pytest.mark.parametrize("family", ["fps_sorted", "fps_sorted,fps_global"])
 def test_fps_sorted_copy_hard_clouds(kind, family, monkeypatch):
     """Warp and chunk skipping must never change a result: crowded cells, exact ties everywhere,
     a collapsed axis, coordinates that are not finite, and points the skip rule excludes.
-    All kernels that skip: the register-resident ones (several samples per exchange, one sample
-    per exchange) and the one for large clouds."""
+    Both kernels that skip: the register-resident one and the one for large clouds."""
     data.use_paths(monkeypatch, family)
     rng = np.random.default_rng(len(kind))
     B, n, m = 2, 6000, 400
@@ -477,9 +486,9 @@ def test_fps_returns_sampled_coordinates(B, N, m, env, monkeypatch):
 @pytest.mark.parametrize("kind", ["two_blobs", "duplicates", "line", "shell"])
 @pytest.mark.parametrize("cfg", [None, "8:128:4", "2:512:8", "1:128:32", "16:64:4", "1:512:8"])
 def test_fps_several_samples_per_exchange_hard_cases(kind, cfg, monkeypatch):
-    """The batched kernel accepts a candidate only when it is provably the next sample: clouds
-    where the largest minima sit next to each other (two tight blobs, a line), where many points
-    coincide (equal keys everywhere) and a thin shell, through several cluster shapes."""
+    """A round takes a point only when it is provably a sample: clouds where the largest minima sit next
+    to each other (two tight blobs, a line), where many points coincide (equal keys everywhere) and a
+    thin shell, through several cluster sizes."""
     rng = np.random.default_rng(len(kind))
     B, n, m = 3, 3000, 1200
     if kind == "two_blobs":
