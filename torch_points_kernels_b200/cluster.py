@@ -56,7 +56,7 @@ def grow_proximity(pos, batch, nsample=16, radius=0.02, min_cluster_size=32):
 def _segments(rank, sample):
     """Numbers of the runs of equal (rank, sample), ascending.  The ids are compared, not computed with:
     any sorted ids of a sample will do, negative and huge ones too."""
-    segment = torch.zeros_like(rank)
+    segment = torch.zeros(rank.shape, dtype=torch.int64, device=rank.device)
     begins = (rank[1:] != rank[:-1]) | (sample[1:] != sample[:-1])
     torch.cumsum(begins, 0, out=segment[1:])
     return segment
@@ -89,29 +89,29 @@ def region_grow(
     assert pos.dim() == 2
     assert pos.shape[0] == labels.shape[0]
 
-    unique_labels, label_rank = torch.unique(labels, return_inverse=True)
-    kept = [not (l in ignore_labels) and bool(l == l) for l in unique_labels.cpu()]  # (NaN is no label)
+    unique_labels, label_rank, label_counts = torch.unique(labels, return_inverse=True, return_counts=True)
+    unique_labels = unique_labels.cpu()
+    kept = [not (l in ignore_labels) for l in unique_labels]
+    if unique_labels.is_floating_point():
+        kept = [k and l == l for k, l in zip(kept, unique_labels.tolist())]  # (NaN is no label)
     if not any(kept):
         return []
     if batch.shape[0] != pos.shape[0] or batch.numel() != pos.shape[0]:
         raise IndexError("batch of shape %s does not match %d points" % (tuple(batch.shape), pos.shape[0]))
-    batch = batch.reshape(-1)
     # One search and one labelling for all labels: the points ordered by label (original order inside a
     # label), every (label, sample) pair a segment of its own.  Lists, seeds and the order of the clusters
     # are those of a search per label, because the order inside a segment is the same.
-    rank_h = torch.tensor([sum(kept[:i]) if k else -1 for i, k in enumerate(kept)])
-    rank = rank_h.to(pos.device)[label_rank]
-    ind = (rank >= 0).nonzero()[:, 0]
-    ind = ind[torch.sort(rank[ind], stable=True).indices]
-    segment = _segments(rank[ind], batch[ind])
+    rank_h = torch.tensor([sum(kept[:i]) if k else -1 for i, k in enumerate(kept)], dtype=torch.int32)
+    left_out = sum(c for c, k in zip(label_counts.tolist(), kept) if not k)
+    rank, ind = (t[left_out:] for t in torch.sort(rank_h.to(pos.device)[label_rank], stable=True))
+    segment = _segments(rank, batch.reshape(-1)[ind])
     local_pos = pos[ind].float().contiguous()
     neighbours = ball_query_partial_dense(radius, nsample, local_pos, local_pos, segment, segment)[0]
     seeds = cluster_labels(neighbours)
     seeds, order = torch.sort(seeds, stable=True)  # members ascending inside a cluster
     counts = torch.unique_consecutive(seeds, return_counts=True)[1]
-    large = counts >= min_cluster_size
-    members = ind[order[torch.repeat_interleave(large, counts)]]
-    sizes = counts[large].tolist()
+    members = ind[order[torch.repeat_interleave(counts >= min_cluster_size, counts, output_size=order.shape[0])]]
+    sizes = [c for c in counts.tolist() if c >= min_cluster_size]
     clusters = [members.new_empty(c) for c in sizes]
     if clusters:
         torch.split_with_sizes_copy(members, sizes, 0, out=clusters)  # one launch for all
