@@ -130,6 +130,7 @@ __global__ void __launch_bounds__(kRoundsThreads, 1)
     __shared__ __align__(8) uint64_t s_mbar[8];  // notes, entries, sample counts, samples: two of each
     __shared__ uint32_t s_top;
     __shared__ int s_low;
+    __shared__ int s_gone;  // a CTA of the cluster has given up a wait: the next barrier was its last
 
     constexpr int THREADS = kRoundsThreads, NW = THREADS / 32;
     constexpr bool CLUSTERED = NR > 1;
@@ -261,6 +262,7 @@ __global__ void __launch_bounds__(kRoundsThreads, 1)
         }
         s_top = kNoRank;
         s_low = INT_MAX;
+        s_gone = 0;
     }
     int* hist = reinterpret_cast<int*>(smem + lay.hist);
     int* base = reinterpret_cast<int*>(smem + lay.base);
@@ -492,8 +494,8 @@ __global__ void __launch_bounds__(kRoundsThreads, 1)
             wmax = __reduce_max_sync(kFullMask, k);
         }
     };
-    // The point with the largest V, M its minimum: everyone learns it; returns the CTA that holds it.
-    // Its coordinates are in s_top_of, its index in s_topidx_of of that CTA's slot.
+    // The point with the largest V, M its minimum: everyone learns it; returns the CTA that holds it (-1:
+    // another one is gone).  Its coordinates are in s_top_of, its index in s_topidx_of of that CTA's slot.
     auto find_top = [&](int top) -> int {
         bool have = false;
         if (wmax == top)
@@ -526,6 +528,7 @@ __global__ void __launch_bounds__(kRoundsThreads, 1)
         __syncthreads();
         if (tid == 0) s_top = kNoRank;
         sync_all();
+        if (CLUSTERED && s_gone != 0) return -1;
         int w = 0;
         for (int r = 1; r < nranks; ++r)
             if (s_toprank_of[r] < s_toprank_of[w]) w = r;
@@ -731,6 +734,7 @@ __global__ void __launch_bounds__(kRoundsThreads, 1)
         if (alone)
         {
             const int w = find_top(top);
+            if (w < 0) return;
             const int k = s_topidx_of[w];
             // a sample that comes up again at once has changed no minimum: it is all that follows
             const bool again = sequential && k == fill;
@@ -897,8 +901,14 @@ __global__ void __launch_bounds__(kRoundsThreads, 1)
 
     if (failed)
     {
+        // The others may not know yet: they learn of it before the barrier that this CTA takes part in
+        // last, the next one of theirs, and touch its memory no more.
         if (tid == 0) atomicOr(&g_dev_status, kStatusWaitAbandoned);
-        if constexpr (CLUSTERED) cluster_sync_all();
+        if constexpr (CLUSTERED)
+        {
+            if (tid < nranks) *at_rank(&s_gone, tid) = 1;
+            cluster_sync_all();
+        }
         return;
     }
     // ------------------------------------------------ the samples in order
@@ -921,6 +931,7 @@ __global__ void __launch_bounds__(kRoundsThreads, 1)
         low = __reduce_min_sync(kFullMask, low);
         if (lane == 0) atomicMin(&s_low, low);
         sync_all();
+        if (CLUSTERED && s_gone != 0) return;
         for (int r = 0; r < nranks; ++r) low = min(low, *at_rank(&s_low, r));
     }
     low = min(low, first_top);
@@ -931,6 +942,7 @@ __global__ void __launch_bounds__(kRoundsThreads, 1)
     auto bucket_of = [&](int key) { return max(0, min(kRoundsBuckets - 1, (first_top - key) >> shift)); };
     for (int i = tid; i < mine; i += THREADS) atomicAdd(&f_hist[bucket_of(own[i].x)], 1);
     sync_all();
+    if (CLUSTERED && s_gone != 0) return;
     bin_positions(f_hist, f_base, f_start, kRoundsBuckets);
     const int part = max(1, (listed + nranks - 1) / nranks);
     for (int i = tid; i < mine; i += THREADS)
