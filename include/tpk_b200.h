@@ -141,8 +141,9 @@ TPK_API int tpk_ball_query_dense(int b, int n, int m, float radius, int nsample,
  * very dense neighbourhoods, for which the early-exit scan is cheaper, fall through to
  * the scan.  Results are identical to tpk_ball_query_dense bit for bit.
  * scratch: tpk_ball_query_dense_scratch_bytes(b,n,m,nsample) bytes, 256-byte aligned;
- * when that returns 0 (small clouds, nsample > 128) or scratch is NULL the call is
- * tpk_ball_query_dense.  No counterpart in the reference.
+ * when that returns 0 (up to 1.2e8 pairs of clouds below 2^18 points, which the scan
+ * answers, and small clouds) or scratch is NULL the call is tpk_ball_query_dense.  No
+ * counterpart in the reference.
  */
 TPK_API int tpk_ball_query_dense_ws(int b, int n, int m, float radius, int nsample,
                                     const float* new_xyz, const float* xyz, int64_t* idx, float* dist,

@@ -327,6 +327,10 @@ bool ball_scan_wanted(int b, int n, int m)
 // instructions on a candidate, and hits^2 / 8 on the order of its hits; the scan 50 on 128 points,
 // n * nsample / hits of them.  Both are the same at hits^3 = 1.9 n nsample, about 100 of 16384
 // points and lists of 32; 27 cells hold 4.5 times a ball's points (6.5 in space, 2.9 on a surface).
+// Where the lists stay open all the same the whole cloud is read: lists longer than sqrt(1.9 n), for
+// which there is the tiled scan (tpk_ball_query_dense_ws), and centres beside a clump, 4 x 65536 points,
+// 16384 centres, lists of 32, 1.8 radii from clumps 2.2 ms in the grid and 2.5, 1.3 radii 2.4 and 2.5, of
+// 16 2.3 and 1.5, 16 x 16384 points 0.68 and 0.50.
 float ball_scan_crowded(double n, int nsample) { return static_cast<float>(4.5 * cbrt(1.9 * n * nsample)); }
 
 // need (optional): one byte per centre, the centres with a zero are left as they are.
