@@ -22,7 +22,7 @@ class ChamferFunction(torch.autograd.Function):
         idx1 = torch.empty((b, n), dtype=torch.int32, device=xyz1.device)
         idx2 = torch.empty((b, m), dtype=torch.int32, device=xyz1.device)
         name = "tpk_chamfer_dist_f32" if xyz1.dtype == torch.float32 else "tpk_chamfer_dist_f64"
-        with torch.cuda.device(xyz1.device):
+        with _lib.on_device(xyz1):
             need = _lib.lib().tpk_chamfer_dist_scratch_bytes(b, n, m) if xyz1.dtype == torch.float32 else 0
             if need > 0:
                 # large clouds: nearest neighbours on a uniform grid (same results as the all-pairs scan)
@@ -46,7 +46,7 @@ class ChamferFunction(torch.autograd.Function):
         grad_xyz1 = torch.empty_like(xyz1)
         grad_xyz2 = torch.empty_like(xyz2)
         name = "tpk_chamfer_dist_grad_f32" if xyz1.dtype == torch.float32 else "tpk_chamfer_dist_grad_f64"
-        with torch.cuda.device(xyz1.device):
+        with _lib.on_device(xyz1):
             _lib.call(name, b, n, _lib.ptr(xyz1), m, _lib.ptr(xyz2), _lib.ptr(idx1), _lib.ptr(idx2),
                       _lib.ptr(grad_dist1), _lib.ptr(grad_dist2), _lib.ptr(grad_xyz1),
                       _lib.ptr(grad_xyz2), _lib.stream_of(xyz1))

@@ -21,7 +21,7 @@ def cluster_labels(neighbours):
     n, nsample = neighbours.shape
     labels = torch.arange(n, dtype=torch.int32, device=neighbours.device)
     changed = torch.zeros(1, dtype=torch.int32, device=neighbours.device)
-    with torch.cuda.device(neighbours.device):
+    with _lib.on_device(neighbours):
         # chains shorten geometrically; a handful of launches per host check keeps the number of
         # device-to-host reads small
         for _ in range(max(1, n)):

@@ -28,7 +28,7 @@ class CubicFeatureSamplingFunction(torch.autograd.Function):
         indexes = torch.empty((b, n, nvert), dtype=torch.int32, device=ptcloud.device)
         need = _lib.lib().tpk_cubic_feature_sampling_scratch_bytes(b, n, c, scale, int(neighborhood_size), ptcloud.element_size())
         scratch = _rows(need, ptcloud)
-        with torch.cuda.device(ptcloud.device):
+        with _lib.on_device(ptcloud):
             _lib.call("tpk_cubic_feature_sampling_ws_" + sfx, b, n, c, scale, int(neighborhood_size), _lib.ptr(ptcloud),
                       _lib.ptr(cubic_features), _lib.ptr(point_features), _lib.ptr(indexes), _lib.ptr(scratch),
                       need, _lib.stream_of(ptcloud))
@@ -47,7 +47,7 @@ class CubicFeatureSamplingFunction(torch.autograd.Function):
         grad_ptcloud = torch.empty((b, n, 3), dtype=dt, device=dev)
         grad_cubic = torch.empty((b, c, scale, scale, scale), dtype=dt, device=dev)
         scratch = _rows(need, grad_point_features)  # as much as the forward pass needed
-        with torch.cuda.device(dev):
+        with _lib.on_device(grad_point_features):
             _lib.call("tpk_cubic_feature_sampling_grad_ws_" + sfx, b, n, c, scale, neighborhood_size,
                       _lib.ptr(grad_point_features), _lib.ptr(indexes), _lib.ptr(grad_ptcloud), _lib.ptr(grad_cubic),
                       _lib.ptr(scratch), need, _lib.stream_of(grad_point_features))

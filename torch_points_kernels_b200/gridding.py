@@ -36,7 +36,7 @@ class GriddingFunction(torch.autograd.Function):
         grid = torch.empty((b, length ** 3), dtype=ptcloud.dtype, device=ptcloud.device)
         weights = torch.empty((b, n, 8, 3), dtype=ptcloud.dtype, device=ptcloud.device)
         indexes = torch.empty((b, n, 8), dtype=torch.int32, device=ptcloud.device)
-        with torch.cuda.device(ptcloud.device):
+        with _lib.on_device(ptcloud):
             _lib.call("tpk_gridding_keep_" + sfx, b, n, float(-scale), float(scale - 1), float(-scale), float(scale - 1),
                       float(-scale), float(scale - 1), _lib.ptr(ptcloud), _lib.ptr(keep), _lib.ptr(grid),
                       _lib.ptr(weights), _lib.ptr(indexes), _lib.stream_of(ptcloud))
@@ -50,7 +50,7 @@ class GriddingFunction(torch.autograd.Function):
         grad_grid = grad_grid.contiguous()
         b, n = indexes.shape[0], indexes.shape[1]
         grad_ptcloud = torch.empty((b, n, 3), dtype=weights.dtype, device=weights.device)
-        with torch.cuda.device(weights.device):
+        with _lib.on_device(weights):
             _lib.call("tpk_gridding_grad_" + sfx, b, n, grad_grid.shape[1], _lib.ptr(weights), _lib.ptr(indexes),
                       _lib.ptr(grad_grid), _lib.ptr(grad_ptcloud), _lib.stream_of(weights))
         return grad_ptcloud, None, None

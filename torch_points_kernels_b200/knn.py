@@ -38,7 +38,7 @@ def knn(pos_support, pos, k, batch_support=None, batch_pos=None):
             raise RuntimeError("Not enough points in support to find " + str(k) + " neighboors")
         idx = torch.empty((b, m, k), dtype=torch.int64, device=pos.device)
         dist2 = torch.empty((b, m, k), dtype=torch.float32, device=pos.device)
-        with torch.cuda.device(pos.device):
+        with _lib.on_device(pos):
             need = _lib.lib().tpk_knn_dense_scratch_bytes(b, n, m, int(k))
             if need > 0:
                 # large clouds: hashed uniform grid with scratch (same results as the scan)
@@ -64,7 +64,7 @@ def knn(pos_support, pos, k, batch_support=None, batch_pos=None):
     m = pos.shape[0]
     idx = torch.empty((m, k), dtype=torch.int64, device=pos.device)
     dist2 = torch.empty((m, k), dtype=torch.float32, device=pos.device)
-    with torch.cuda.device(pos.device):
+    with _lib.on_device(pos):
         need = _lib.lib().tpk_knn_partial_dense_scratch_bytes(pos_support.shape[0], m, int(k))
         if need > 0:
             scratch = torch.empty((need,), dtype=torch.uint8, device=pos.device)

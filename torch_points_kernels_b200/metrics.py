@@ -53,7 +53,7 @@ def instance_iou(
     proposals_idx = torch.cat([i.to(dev).long() for i in instance_idx]).contiguous() if instance_idx else \
         torch.zeros(0, dtype=torch.long, device=dev)
     out = torch.empty((len(instance_idx), total_gt), dtype=torch.float32, device=dev)
-    with torch.cuda.device(dev):
+    with _lib.on_device(gt_instances):
         _lib.call("tpk_instance_iou", len(instance_idx), total_gt, max_gt, gt_instances.shape[0],
                   _lib.ptr(num_gt_instances), _lib.ptr(proposals_idx), _lib.ptr(proposals_offset),
                   _lib.ptr(gt_instances), _lib.ptr(offset_num_gt), _lib.ptr(batch), _lib.ptr(gt_instance_sizes),

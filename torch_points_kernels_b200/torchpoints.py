@@ -15,6 +15,8 @@ from .knn import knn  # noqa: F401  (re-exported like the reference does)
 
 
 def _f32(t, name):
+    if t.is_cuda and t.dtype is torch.float32 and t.is_contiguous():
+        return t
     _lib.check_contiguous(t, name)
     _lib.check_float(t, name)
     _lib.check_cuda(t, name)
@@ -53,7 +55,7 @@ def furthest_point_sample(xyz, npoint, return_xyz=False):
     out = torch.empty((b, npoint), dtype=torch.int32, device=xyz.device)
     new_xyz = torch.empty((b, npoint, 3), dtype=torch.float32, device=xyz.device) if return_xyz else None
     scratch = None
-    with torch.cuda.device(xyz.device):
+    with _lib.on_device(xyz):
         need = _lib.lib().tpk_fps_scratch_bytes(b, n, npoint)
         if need < 0:
             raise RuntimeError("furthest_point_sample: clouds of %d points are not supported" % n)
@@ -90,7 +92,7 @@ def three_nn(unknown, known):
     m = known.shape[1]
     dist2 = torch.empty((b, n, 3), dtype=torch.float32, device=unknown.device)
     idx = torch.empty((b, n, 3), dtype=torch.int32, device=unknown.device)
-    with torch.cuda.device(unknown.device):
+    with _lib.on_device(unknown):
         need = _lib.lib().tpk_three_nn_scratch_bytes(b, n, m)
         if need > 0:
             # many known points: uniform-grid search with scratch (same results as the scan)
@@ -111,9 +113,18 @@ def three_interpolate_backward(grad_out, idx, weight, m):
     _f32(grad_out, "grad_out")
     B, c, n = grad_out.size()
     grad_features = torch.empty((B, c, m), dtype=torch.float32, device=grad_out.device)
+<<<<<<< ours
     with torch.cuda.device(grad_out.device):
         _lib.call("tpk_three_interpolate_grad", B, c, n, m, _lib.ptr(grad_out), _lib.ptr(idx),
                   _lib.ptr(weight), _lib.ptr(grad_features), _lib.stream_of(grad_out))
+=======
+    with _lib.on_device(grad_out):
+        # scratch for a copy of the gradient with the channel fastest; 0 bytes = sizes of the kernels without it
+        need = _lib.lib().tpk_three_interpolate_grad_cols_scratch_bytes(B, c, n, m)
+        scratch = torch.empty(need, dtype=torch.uint8, device=grad_out.device) if need > 0 else None
+        _lib.call("tpk_three_interpolate_grad_cols", B, c, n, m, _lib.ptr(grad_out), _lib.ptr(idx), _lib.ptr(weight),
+                  _lib.ptr(grad_features), _lib.ptr(scratch), need, _lib.stream_of(grad_out))
+>>>>>>> theirs
     return grad_features
 
 
@@ -133,7 +144,7 @@ class ThreeInterpolate(Function):
         if idx.dtype != torch.int32:
             raise RuntimeError("idx must be an int32 tensor")
         out = torch.empty((B, c, n), dtype=torch.float32, device=features.device)
-        with torch.cuda.device(features.device):
+        with _lib.on_device(features):
             _lib.call("tpk_three_interpolate", B, c, m, n, _lib.ptr(features), _lib.ptr(idx),
                       _lib.ptr(weight), _lib.ptr(out), _lib.stream_of(features))
             if _lib.debug_checks():
@@ -175,10 +186,21 @@ def grouping_backward(grad_out, idx, n):
     _f32(grad_out, "grad_out")
     B, c, npoint, nsample = grad_out.size()
     grad_features = torch.empty((B, c, n), dtype=torch.float32, device=grad_out.device)
+<<<<<<< ours
     with torch.cuda.device(grad_out.device):
         # scratch for the inverted index (positions sorted by target); 0 bytes = shapes the sorted
         # kernels do not cover, which take the atomic kernels
         need = _lib.lib().tpk_grouping_grad_scratch_bytes(B, c, n, npoint, nsample)
+=======
+    with _lib.on_device(grad_out):
+        handle = _lib.lib()
+        # scratch for a copy of the gradient with the channel fastest, or for the inverted index (positions
+        # sorted by target); 0 bytes = sizes where other kernels are ahead
+        need = handle.tpk_grouping_grad_cols_scratch_bytes(B, c, n, npoint, nsample)
+        by_cols = need > 0
+        if not by_cols:
+            need = handle.tpk_grouping_grad_scratch_bytes(B, c, n, npoint, nsample)
+>>>>>>> theirs
         scratch = torch.empty(need, dtype=torch.uint8, device=grad_out.device) if need > 0 else None
         _lib.call("tpk_grouping_grad_ws", B, c, n, npoint, nsample, _lib.ptr(grad_out),
                   _lib.ptr(idx), _lib.ptr(grad_features), _lib.ptr(scratch) if scratch is not None else None,
@@ -200,7 +222,7 @@ class GroupingOperation(Function):
         _, npoint, nsample = idx.size()
         ctx.grouping_for_backward = (idx, n)
         out = torch.empty((B, c, npoint, nsample), dtype=torch.float32, device=features.device)
-        with torch.cuda.device(features.device):
+        with _lib.on_device(features):
             _lib.call("tpk_grouping", B, c, n, npoint, nsample, _lib.ptr(features), _lib.ptr(idx),
                       _lib.ptr(out), _lib.stream_of(features))
             if _lib.debug_checks():
@@ -252,7 +274,7 @@ class SAGroup(Function):
         new_xyz = torch.empty((b, m, 3), dtype=torch.float32, device=xyz.device)
         idx = torch.empty((b, m, nsample), dtype=torch.int64, device=xyz.device)
         out = torch.empty((b, 3 + c, m, nsample), dtype=torch.float32, device=xyz.device)
-        with torch.cuda.device(xyz.device):
+        with _lib.on_device(xyz):
             need = _lib.lib().tpk_sa_group_scratch_bytes(b, n, m, int(nsample))
             scratch = torch.empty((max(need, 1),), dtype=torch.uint8, device=xyz.device)
             _lib.call("tpk_sa_group", b, n, m, c, float(radius), int(nsample), _lib.ptr(xyz), _lib.ptr(features),
@@ -320,7 +342,7 @@ def ball_query_dense(radius, nsample, xyz, new_xyz, batch_xyz=None, batch_new_xy
     n = xyz.shape[1]
     idx = torch.empty((b, m, nsample), dtype=torch.int64, device=new_xyz.device)
     dist = torch.empty((b, m, nsample), dtype=torch.float32, device=new_xyz.device)
-    with torch.cuda.device(new_xyz.device):
+    with _lib.on_device(new_xyz):
         need = _lib.lib().tpk_ball_query_dense_scratch_bytes(b, n, m, int(nsample))
         if need > 0:
             # large clouds: uniform-grid search with scratch (same results as the scan)
@@ -351,7 +373,7 @@ def ball_query_partial_dense(radius, nsample, x, y, batch_x, batch_y, sort=False
     ny = y.shape[0]
     idx = torch.empty((ny, nsample), dtype=torch.int64, device=y.device)
     dist = torch.empty((ny, nsample), dtype=torch.float32, device=y.device)
-    with torch.cuda.device(y.device):
+    with _lib.on_device(y):
         need = _lib.lib().tpk_ball_query_partial_dense_scratch_bytes(x.shape[0], ny, float(radius))
         if need > 0:
             # hashed uniform grid with scratch (same results as the scan of the segments)
