@@ -113,18 +113,9 @@ def three_interpolate_backward(grad_out, idx, weight, m):
     _f32(grad_out, "grad_out")
     B, c, n = grad_out.size()
     grad_features = torch.empty((B, c, m), dtype=torch.float32, device=grad_out.device)
-<<<<<<< ours
-    with torch.cuda.device(grad_out.device):
+    with _lib.on_device(grad_out):
         _lib.call("tpk_three_interpolate_grad", B, c, n, m, _lib.ptr(grad_out), _lib.ptr(idx),
                   _lib.ptr(weight), _lib.ptr(grad_features), _lib.stream_of(grad_out))
-=======
-    with _lib.on_device(grad_out):
-        # scratch for a copy of the gradient with the channel fastest; 0 bytes = sizes of the kernels without it
-        need = _lib.lib().tpk_three_interpolate_grad_cols_scratch_bytes(B, c, n, m)
-        scratch = torch.empty(need, dtype=torch.uint8, device=grad_out.device) if need > 0 else None
-        _lib.call("tpk_three_interpolate_grad_cols", B, c, n, m, _lib.ptr(grad_out), _lib.ptr(idx), _lib.ptr(weight),
-                  _lib.ptr(grad_features), _lib.ptr(scratch), need, _lib.stream_of(grad_out))
->>>>>>> theirs
     return grad_features
 
 
@@ -186,21 +177,10 @@ def grouping_backward(grad_out, idx, n):
     _f32(grad_out, "grad_out")
     B, c, npoint, nsample = grad_out.size()
     grad_features = torch.empty((B, c, n), dtype=torch.float32, device=grad_out.device)
-<<<<<<< ours
-    with torch.cuda.device(grad_out.device):
+    with _lib.on_device(grad_out):
         # scratch for the inverted index (positions sorted by target); 0 bytes = shapes the sorted
         # kernels do not cover, which take the atomic kernels
         need = _lib.lib().tpk_grouping_grad_scratch_bytes(B, c, n, npoint, nsample)
-=======
-    with _lib.on_device(grad_out):
-        handle = _lib.lib()
-        # scratch for a copy of the gradient with the channel fastest, or for the inverted index (positions
-        # sorted by target); 0 bytes = sizes where other kernels are ahead
-        need = handle.tpk_grouping_grad_cols_scratch_bytes(B, c, n, npoint, nsample)
-        by_cols = need > 0
-        if not by_cols:
-            need = handle.tpk_grouping_grad_scratch_bytes(B, c, n, npoint, nsample)
->>>>>>> theirs
         scratch = torch.empty(need, dtype=torch.uint8, device=grad_out.device) if need > 0 else None
         _lib.call("tpk_grouping_grad_ws", B, c, n, npoint, nsample, _lib.ptr(grad_out),
                   _lib.ptr(idx), _lib.ptr(grad_features), _lib.ptr(scratch) if scratch is not None else None,
