@@ -268,6 +268,16 @@ TPK_API int tpk_three_interpolate_grad(int b, int c, int n, int m, const float* 
                                const int32_t* idx, const float* weight, float* grad_points,
                                void* stream);
 
+/*
+ * The same through a copy of the gradient with the channels of a point side by side, in caller
+ * scratch of tpk_three_interpolate_grad_cols_scratch_bytes(b,c,n,m) bytes, 32-byte aligned.
+ * scratch NULL, or 0 bytes asked: tpk_three_interpolate_grad itself.
+ */
+TPK_API int tpk_three_interpolate_grad_cols(int b, int c, int n, int m, const float* grad_out, const int32_t* idx,
+                                            const float* weight, float* grad_points, void* scratch,
+                                            int64_t scratch_bytes, void* stream);
+TPK_API int64_t tpk_three_interpolate_grad_cols_scratch_bytes(int b, int c, int n, int m);
+
 /* ------------------------------------------------------------------ grouping ---- */
 
 /*
@@ -299,6 +309,19 @@ TPK_API int tpk_grouping_grad_ws(int b, int c, int n, int npoint, int nsample, c
                                  const int64_t* idx, float* grad_features, void* scratch, int64_t scratch_bytes,
                                  void* stream);
 TPK_API int64_t tpk_grouping_grad_scratch_bytes(int b, int c, int n, int npoint, int nsample);
+
+/*
+ * The same through a copy of the gradient with the channels of a point side by side, in caller
+ * scratch of tpk_grouping_grad_cols_scratch_bytes(b,c,n,npoint,nsample) bytes, 32-byte aligned.
+ * skip_rows rows of every cloud of grad_out lie ahead of the c that are summed (0 for
+ * grouping_operation, 3 for the gradient of tpk_sa_group); grad_out is
+ * (b, skip_rows + c, npoint, nsample).  scratch NULL, or 0 bytes asked (sizes where the kernels above
+ * are ahead): the atomic kernels.
+ */
+TPK_API int tpk_grouping_grad_cols(int b, int c, int n, int npoint, int nsample, int skip_rows,
+                                   const float* grad_out, const int64_t* idx, float* grad_features, void* scratch,
+                                   int64_t scratch_bytes, void* stream);
+TPK_API int64_t tpk_grouping_grad_cols_scratch_bytes(int b, int c, int n, int npoint, int nsample);
 
 /* ----------------------------------------------------- fused set abstraction ---- */
 

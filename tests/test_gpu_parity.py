@@ -1020,6 +1020,53 @@ def test_grouping_backward_sorted_path(B, C, N, P, S, kind):
     assert _lib.device_status() == 0
 
 
+@pytest.mark.parametrize("B,C,N,P,S,kind", [
+    (1, 1, 1, 1, 1, "random"),        # one channel, one position
+    (2, 3, 50, 11, 3, "random"),      # a tile of channels that is not full, 33 positions
+    (2, 33, 300, 31, 33, "ball"),     # two tiles of channels, neighbourhoods across the sets of 32 positions
+    (1, 40, 70, 16, 32, "one"),       # one target for everything
+    (2, 64, 1000, 65, 16, "bad"),     # indices that address nothing
+    (3, 100, 129, 40, 5, "random"),   # repeated targets within a set
+])
+@pytest.mark.parametrize("skip", [0, 3])
+def test_gradients_by_columns(B, C, N, P, S, kind, skip, monkeypatch):
+    """Grouping and interpolation gradients through the channel-fastest copy against sums in 64 bits.  A sum of
+    t terms in 32 bits, in any order, is off by less than t * 2^-24 times the sum of their magnitudes."""
+    data.use_paths(monkeypatch, "scatter_cols")
+    g = data.gen(17 * N + P + S)
+    idx = torch.randint(0, N, (B, P, S), generator=g)
+    if kind == "ball":
+        idx = torch.where(torch.arange(S) < torch.randint(1, S + 1, (B, P, 1), generator=g), idx, idx[:, :, :1])
+    elif kind == "one":
+        idx[:] = N - 1
+    elif kind == "bad":
+        idx[:, ::7] = N
+        idx[:, 1::7] = -1
+    gout = torch.randn(B, skip + C, P, S, generator=g)
+    _lib.device_status()
+    got = npy(tpk.torchpoints._group_grad(cu(gout), cu(idx), N, C, skip))
+    assert _lib.device_status() == (2 if kind == "bad" else 0)
+    flat = idx.view(B, 1, -1).expand(-1, C, -1)
+    ok = ((flat >= 0) & (flat < N)).double()
+    at = flat.clamp(0, N - 1)
+    v = gout[:, skip:].reshape(B, C, -1).double() * ok
+    want = torch.zeros(B, C, N, dtype=torch.float64).scatter_add_(2, at, v)
+    size = torch.zeros_like(want).scatter_add_(2, at, v.abs())
+    terms = torch.zeros_like(want).scatter_add_(2, at, ok)
+    assert bool(((cu(want) - cu(torch.from_numpy(got)).double()).abs() <= cu(terms * 2.0 ** -24 * size) + 1e-30).all())
+
+    i3 = torch.randint(0, N, (B, P, 3), generator=g).int()
+    w = torch.rand(B, P, 3, generator=g)
+    go = torch.randn(B, C, P, generator=g)
+    got = tpk.torchpoints.three_interpolate_backward(cu(go), cu(i3), cu(w), N).double().cpu()
+    v = (go.double().unsqueeze(-1) * w.double().unsqueeze(1)).reshape(B, C, -1)
+    at = i3.long().view(B, 1, -1).expand(-1, C, -1)
+    want = torch.zeros(B, C, N, dtype=torch.float64).scatter_add_(2, at, v)
+    size = torch.zeros_like(want).scatter_add_(2, at, v.abs())
+    terms = torch.zeros_like(want).scatter_add_(2, at, torch.ones_like(v))
+    assert bool(((want - got).abs() <= (terms + 1) * 2.0 ** -24 * size + 1e-30).all())  # (+ 1: the products)
+
+
 @pytest.mark.parametrize("B,N,M,C,r", [(2, 16384, 4096, 64, 0.1), (3, 4096, 1024, 7, 0.2), (2, 500, 100, 130, 0.4),
                                        (1, 70000, 64, 3, 0.05), (2, 1024, 256, 0, 0.3)])
 def test_fused_sa_group_equals_the_unfused_sequence(B, N, M, C, r):

@@ -41,6 +41,8 @@ _SIGNATURES = {
     "tpk_grouping": [_c_int, _c_int, _c_int, _c_int, _c_int, _ptr, _ptr, _ptr, _ptr],
     "tpk_grouping_grad": [_c_int, _c_int, _c_int, _c_int, _c_int, _ptr, _ptr, _ptr, _ptr],
     "tpk_grouping_grad_ws": [_c_int, _c_int, _c_int, _c_int, _c_int, _ptr, _ptr, _ptr, _ptr, _c_i64, _ptr],
+    "tpk_grouping_grad_cols": [_c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _ptr, _ptr, _ptr, _ptr, _c_i64, _ptr],
+    "tpk_three_interpolate_grad_cols": [_c_int, _c_int, _c_int, _c_int, _ptr, _ptr, _ptr, _ptr, _ptr, _c_i64, _ptr],
     "tpk_sa_group_grad": [_c_int, _c_int, _c_int, _c_int, _c_int, _ptr, _ptr, _ptr, _ptr, _c_i64, _ptr],
     "tpk_chamfer_dist_f32": [_c_int, _c_int, _ptr, _c_int, _ptr, _ptr, _ptr, _ptr, _ptr, _ptr],
     "tpk_chamfer_dist_f64": [_c_int, _c_int, _ptr, _c_int, _ptr, _ptr, _ptr, _ptr, _ptr, _ptr],
@@ -70,7 +72,8 @@ EXPORTS = sorted(list(_SIGNATURES) + ["tpk_version", "tpk_last_error", "tpk_devi
                                        "tpk_three_nn_scratch_bytes", "tpk_chamfer_dist_scratch_bytes",
                                        "tpk_ball_query_partial_dense_scratch_bytes", "tpk_knn_dense_scratch_bytes", "tpk_sa_group_scratch_bytes",
                                        "tpk_knn_partial_dense_scratch_bytes", "tpk_cubic_feature_sampling_scratch_bytes",
-                                       "tpk_grouping_grad_scratch_bytes"])
+                                       "tpk_grouping_grad_scratch_bytes", "tpk_grouping_grad_cols_scratch_bytes",
+                                       "tpk_three_interpolate_grad_cols_scratch_bytes"])
 
 
 def lib():
@@ -110,6 +113,10 @@ def lib():
         handle.tpk_knn_partial_dense_scratch_bytes.restype = _c_i64
         handle.tpk_sa_group_scratch_bytes.argtypes = [_c_int, _c_int, _c_int, _c_int]
         handle.tpk_sa_group_scratch_bytes.restype = _c_i64
+        handle.tpk_grouping_grad_cols_scratch_bytes.argtypes = [_c_int, _c_int, _c_int, _c_int, _c_int]
+        handle.tpk_grouping_grad_cols_scratch_bytes.restype = _c_i64
+        handle.tpk_three_interpolate_grad_cols_scratch_bytes.argtypes = [_c_int, _c_int, _c_int, _c_int]
+        handle.tpk_three_interpolate_grad_cols_scratch_bytes.restype = _c_i64
         handle.tpk_grouping_grad_scratch_bytes.argtypes = [_c_int, _c_int, _c_int, _c_int, _c_int]
         handle.tpk_grouping_grad_scratch_bytes.restype = _c_i64
         handle.tpk_cubic_feature_sampling_scratch_bytes.argtypes = [_c_int] * 6

@@ -1,0 +1,293 @@
+// Gradients of grouping_operation and three_interpolate with the channels of a point side by side
+// (sm_100a).
+//
+//   grouping          : grad_features[b, c, idx[b, p]] += grad_out[b, c, p]
+//   three_interpolate : grad_points[b, c, idx[b, p, k]] += grad_out[b, c, p] * weight[b, p, k], k = 0..2
+//
+// are scatters of long rows, with the same index for all channels.  With a lane per position every
+// lane adds to another place: a shared-memory float atomic is a compare-and-swap loop per lane (13
+// wavefronts per 32 positions), a global one a 32-byte sector per lane.  Here a warp takes 32 positions
+// of up to 32 channels, turns them in shared memory, and adds the channels of a position as one
+// contiguous piece (16-byte vector reductions into a copy of the gradient with the channel fastest, in
+// scratch): eight values per sector.  Positions of a set that repeat an index - a ball query fills the
+// slots that it has no point for with the first one, half of all slots in the usual sizes - are summed
+// in shared memory first.  A tiled transposition writes the result.
+//
+// Bound by the rate of the reductions in L2 and the gradient's bytes: 16 clouds of 16384 points, 64 channels,
+// 4096 x 32 positions (537 MB, 82 us at the copy bandwidth) 212 us, 297 through the inverted index of
+// scatter_sorted.cu; all four levels of the benchmark's step 410 and 582; interpolation 113 and 187.
+//
+// semantics: autograd's scatter-add backward of the gather at torch_points_kernels/torchpoints.py:129-146,
+// and cuda/src/interpolate_gpu.cu:122-152.
+#include "tpk_common.cuh"
+
+namespace tpk
+{
+TPK_DEFINE_STATUS_WORD()
+
+namespace
+{
+
+constexpr int kColsThreads = 256;
+constexpr int kColsWarps = kColsThreads / 32;
+constexpr int kColsMax = 32;    // channels a warp takes at a time
+constexpr int kColsPitch = 33;  // of a channel's 32 positions in shared memory
+constexpr int kColsFold = 3;    // repetitions of an index from which they are summed first
+
+// Channels per point in scratch: whole 32-byte sectors.
+__host__ __device__ inline int cols_pitch(int c) { return (c + 7) & ~7; }
+
+struct ColsWarp
+{
+    float v[kColsMax * kColsPitch];
+    int order[32];  // positions left to add: lane | target << 5
+};
+
+// K = 1: one target per position, int64 (grouping); K = 3: three, int32, with weights (interpolation).
+// Warp w of a cloud and channel tile takes positions [32 w, 32 w + 32).
+template <int K>
+__global__ void __launch_bounds__(kColsThreads)
+    scatter_cols_kernel(int c, int n, long long ps, long long gbs, int tile, int tiles, long long blocks,
+                        const float* __restrict__ grad_out, const void* __restrict__ idx_all, const float* __restrict__ weight,
+                        float* __restrict__ sums)
+{
+    __shared__ ColsWarp s_warp[kColsWarps];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    ColsWarp& s = s_warp[warp];
+    const long long cloud = blockIdx.x / (tiles * blocks);
+    const long long rest = blockIdx.x - cloud * (tiles * blocks);
+    const int c0 = static_cast<int>(rest / blocks) * tile;
+    const int nc = min(tile, c - c0);
+    const long long p0 = ((rest % blocks) * kColsWarps + warp) * 32;
+    if (p0 >= ps) return;
+    const bool in = p0 + lane < ps;
+
+    int id[K];
+    float w[K];
+    bool bad = false, some = false;
+#pragma unroll
+    for (int k = 0; k < K; ++k)
+    {
+        long long t = -1;
+        w[k] = 0.f;
+        if (in)
+        {
+            const size_t o = (static_cast<size_t>(cloud) * ps + p0 + lane) * K + k;
+            t = K == 1 ? __ldg(static_cast<const int64_t*>(idx_all) + o) : __ldg(static_cast<const int32_t*>(idx_all) + o);
+            if (K > 1) w[k] = __ldg(weight + o);
+        }
+        const bool ok = static_cast<unsigned long long>(t) < static_cast<unsigned long long>(n);
+        bad |= in && !ok;
+        some |= ok;
+        id[k] = ok ? static_cast<int>(t) : -1;  // -1: adds nothing
+    }
+    const float* g = grad_out + static_cast<size_t>(cloud) * gbs + static_cast<size_t>(c0) * ps + p0 + (in ? lane : 0);
+    float v[kColsMax];
+#pragma unroll
+    for (int r = 0; r < kColsMax; ++r)
+        if (r < nc) v[r] = __ldcs(g + static_cast<size_t>(r) * ps);
+#pragma unroll
+    for (int r = 0; r < kColsMax; ++r) s.v[r * kColsPitch + lane] = r < nc ? v[r] : 0.f;
+    __syncwarp();
+
+    const int quads = (nc + 3) >> 2;    // 16-byte pieces of a position's channels
+    const int at_once = 32 / quads;     // positions per reduction
+    const int mine = lane / quads, quad = lane - mine * quads;
+    const int pitch = cols_pitch(c);
+    float* out = sums + static_cast<size_t>(cloud) * n * pitch + c0 + 4 * quad;
+    const float* piece = s.v + 4 * quad * kColsPitch;
+    uint32_t left = __ballot_sync(kFullMask, some);
+    if constexpr (K == 1)
+    {
+        // positions with the index of an earlier one of the set: where there are a few they are summed here
+        const uint32_t same = __match_any_sync(kFullMask, id[0]);
+        uint32_t fold = __ballot_sync(kFullMask, some && __ffs(same) - 1 == lane && __popc(same) >= kColsFold);
+        while (fold != 0u)
+        {
+            const int first = __ffs(fold) - 1;
+            fold &= fold - 1u;
+            uint32_t others = __shfl_sync(kFullMask, same, first) & ~(1u << first);
+            left &= ~others;
+            float* row = s.v + lane * kColsPitch;  // lane = channel
+            float a = row[first], b = 0.f;
+            while (others != 0u)
+            {
+                const int p = __ffs(others) - 1;
+                others &= others - 1u;
+                const int q = others != 0u ? __ffs(others) - 1 : -1;
+                others &= others - 1u;  // (zero stays zero)
+                a += row[p];
+                if (q >= 0) b += row[q];
+            }
+            row[first] = a + b;
+        }
+    }
+    if (left >> lane & 1u) s.order[__popc(left & ((1u << lane) - 1u))] = K == 1 ? lane | id[0] << 5 : lane;
+    __syncwarp();
+    const int count = __popc(left);
+    for (int i0 = 0; i0 < count; i0 += at_once)
+    {
+        const int i = i0 + mine;
+        const bool add = mine < at_once && i < count;
+        const int e = s.order[add ? i : 0];
+        const int p = e & 31;
+        const float4 x = make_float4(piece[p], piece[kColsPitch + p], piece[2 * kColsPitch + p], piece[3 * kColsPitch + p]);
+        if constexpr (K == 1)
+        {
+            if (add) atomicAdd(reinterpret_cast<float4*>(out + static_cast<size_t>(e >> 5) * pitch), x);
+        }
+        else
+        {
+#pragma unroll
+            for (int k = 0; k < K; ++k)
+            {
+                const int t = __shfl_sync(kFullMask, id[k], p);
+                const float f = __shfl_sync(kFullMask, w[k], p);
+                if (add && t >= 0)
+                    atomicAdd(reinterpret_cast<float4*>(out + static_cast<size_t>(t) * pitch),
+                              make_float4(__fmul_rn(x.x, f), __fmul_rn(x.y, f), __fmul_rn(x.z, f), __fmul_rn(x.w, f)));
+            }
+        }
+    }
+    if (bad) atomicOr(&g_dev_status, kStatusBadIndex);
+}
+
+// grad[cloud][ch][t] = sums[cloud][t][ch]; a 64 x 32 tile (targets x channels) per CTA.
+__global__ void __launch_bounds__(kColsThreads)
+    cols_to_rows_kernel(int c, int n, int tiles_n, int tiles_c, const float* __restrict__ sums, float* __restrict__ grad)
+{
+    __shared__ float tile[64][33];
+    const int lane = threadIdx.x & 31, line = threadIdx.x >> 5;
+    const long long cloud = blockIdx.x / (static_cast<long long>(tiles_n) * tiles_c);
+    const int rest = static_cast<int>(blockIdx.x - cloud * tiles_n * tiles_c);
+    const int t0 = rest / tiles_c * 64, c0 = rest % tiles_c * 32;
+    const int pitch = cols_pitch(c);
+    const float* src = sums + static_cast<size_t>(cloud) * n * pitch;
+    float* dst = grad + static_cast<size_t>(cloud) * c * n;
+#pragma unroll
+    for (int i = 0; i < 64; i += kColsWarps)
+        if (t0 + line + i < n && c0 + lane < c)
+            tile[line + i][lane] = __ldcs(src + static_cast<size_t>(t0 + line + i) * pitch + c0 + lane);
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < 32; i += kColsWarps)
+        if (c0 + line + i < c)
+#pragma unroll
+            for (int h = 0; h < 64; h += 32)
+                if (t0 + h + lane < n) dst[static_cast<size_t>(c0 + line + i) * n + t0 + h + lane] = tile[h + lane][line + i];
+}
+
+int64_t cols_bytes(int b, int c, int n) { return static_cast<int64_t>(b) * n * cols_pitch(c) * static_cast<int64_t>(sizeof(float)); }
+
+template <int K>
+int scatter_cols(int b, int c, int n, long long ps, long long gbs, const float* grad_out, const void* idx, const float* weight,
+                 float* grad, float* sums, cudaStream_t s, const char* what)
+{
+    cudaError_t err = cudaMemsetAsync(sums, 0, static_cast<size_t>(cols_bytes(b, c, n)), s);
+    if (err != cudaSuccess)
+    {
+        set_error("%s: memset: %s", what, cudaGetErrorString(err));
+        return TPK_ERR_CUDA;
+    }
+    // channel tiles of the same size, in pieces of four
+    const int tiles = (c + kColsMax - 1) / kColsMax;
+    const int tile = ((c + tiles - 1) / tiles + 3) & ~3;
+    const long long blocks = (ps + 32 * kColsWarps - 1) / (32 * kColsWarps);
+    const long long grid = blocks * tiles * b;
+    const int tn = (n + 63) / 64, tc = (c + 31) / 32;
+    const long long grid2 = static_cast<long long>(tn) * tc * b;
+    TPK_REQUIRE(grid < (1ll << 31) && grid2 < (1ll << 31), "%s: grid too large", what);
+    prefer_max_shared(scatter_cols_kernel<K>);
+    count_launches(1), scatter_cols_kernel<K><<<static_cast<unsigned>(grid), kColsThreads, 0, s>>>(
+        c, n, ps, gbs, tile, tiles, blocks, grad_out, idx, weight, sums);
+    prefer_max_shared(cols_to_rows_kernel);
+    count_launches(1), cols_to_rows_kernel<<<static_cast<unsigned>(grid2), kColsThreads, 0, s>>>(c, n, tn, tc, sums, grad);
+    return check_launch(what);
+}
+
+// Sizes the kernels can take: a target next to five bits of position, grids that fit a launch.  (test hooks: the
+// other families)
+bool cols_fit(int b, int c, int n, long long ps)
+{
+    if (b <= 0 || c <= 0 || n <= 0 || ps <= 0 || n >= (1 << 26)) return false;
+    const double warps = static_cast<double>(b) * (ps / 32 + kColsWarps) * (c / kColsMax + 1);
+    const double tiles = static_cast<double>(b) * (n / 64 + 1) * (c / 32 + 1);
+    return warps < 1.0e9 && tiles < 1.0e9 && !test_path("scatter_atomic") && !test_path("scatter_global") && !test_path("scatter_sorted");
+}
+
+// Where three launches (zeros, sums, transposition; 8 us at least) pay.  us, rows of atomics or inverted index
+// and columns: 16 clouds of 16384 points, 64 channels, 4096 x 32 positions 297 and 212, 4096 points x 128 channels
+// 165 and 109, 256 x 512 46 and 32; one cloud 59 and 19; 8 x 32768 x 96, 8192 x 64 positions 1199 and 586; but 16 x
+// 256 x 64, 64 x 32 positions 9.2 and 10.2, 4 x 2048 x 180, 512 x 16 16.3 and 18.1.  The rows cost the positions times
+// the rows that an SM has; neighbourhoods of a size that is no power of two, whose padding the rows do not
+// sum first, up to several times that (8 x 64 x 192, 16 x 48 positions 31 and 8.4; 3 x 625 x 140, 156 x 24
+// 7.4 and 10.5, with little padding).
+bool cols_pay_grouping(int b, int c, long long ps, int nsample)
+{
+    if (test_path("scatter_cols")) return true;
+    const long long rows = static_cast<long long>(b) * c, rows_sm = (rows + num_sms() - 1) / num_sms();
+    const double per = (nsample & (nsample - 1)) == 0 ? 0.33e-3 : 1.2e-3;
+    const double by_rows = 4.5 + per * static_cast<double>(ps) * static_cast<double>(rows_sm);
+    return 8.2 + 1.5e-6 * static_cast<double>(rows) * static_cast<double>(ps) < by_rows;
+}
+
+// us, rows of atomics and columns: 16 clouds of 16384 points from 4096, 64 channels 86 and 50; one cloud 42 and
+// 10; 1 x 600 from 150 points, 96 channels 16 and 9.4; 16 x 512 x 16 14 and 8.3; 16 x 256 x 64 9.3 and 9.7,
+// 16 x 256 x 512 14.0 and 13.7.
+bool cols_pay_interp(int n) { return n >= 384 || test_path("scatter_cols"); }
+
+}  // namespace
+}  // namespace tpk
+
+extern "C" int64_t tpk_grouping_grad_cols_scratch_bytes(int b, int c, int n, int npoint, int nsample)
+{
+    if (npoint <= 0 || nsample <= 0) return 0;
+    const long long ps = static_cast<long long>(npoint) * nsample;
+    return tpk::cols_fit(b, c, n, ps) && tpk::cols_pay_grouping(b, c, ps, nsample) ? tpk::cols_bytes(b, c, n) : 0;
+}
+
+extern "C" int tpk_grouping_grad_cols(int b, int c, int n, int npoint, int nsample, int skip_rows, const float* grad_out,
+                                      const int64_t* idx, float* grad_features, void* scratch, int64_t scratch_bytes,
+                                      void* stream)
+{
+    using namespace tpk;
+    TPK_REQUIRE(b >= 0 && c >= 0 && n >= 0 && npoint >= 0 && nsample >= 0 && skip_rows >= 0, "grouping_grad: negative size");
+    const int64_t want = tpk_grouping_grad_cols_scratch_bytes(b, c, n, npoint, nsample);
+    const long long ps = static_cast<long long>(npoint) * nsample, gbs = (static_cast<long long>(skip_rows) + c) * ps;
+    const float* g = grad_out ? grad_out + skip_rows * ps : nullptr;
+    cudaStream_t s = static_cast<cudaStream_t>(stream);
+    if (scratch == nullptr || want == 0) return grouping_grad_atomic(b, c, n, npoint, nsample, g, gbs, idx, grad_features, s);
+    if (scratch_bytes < want)
+    {
+        set_error("grouping_grad: scratch of %lld bytes given, %lld needed", static_cast<long long>(scratch_bytes),
+                  static_cast<long long>(want));
+        return TPK_ERR_SCRATCH;
+    }
+    TPK_REQUIRE(grad_out && idx && grad_features, "grouping_grad: NULL pointer");
+    TPK_REQUIRE((reinterpret_cast<uintptr_t>(scratch) & 31u) == 0, "grouping_grad: scratch must be 32-byte aligned");
+    return scatter_cols<1>(b, c, n, ps, gbs, g, idx, nullptr, grad_features, static_cast<float*>(scratch), s, "grouping_grad");
+}
+
+extern "C" int64_t tpk_three_interpolate_grad_cols_scratch_bytes(int b, int c, int n, int m)
+{
+    return tpk::cols_fit(b, c, m, n) && tpk::cols_pay_interp(n) ? tpk::cols_bytes(b, c, m) : 0;
+}
+
+extern "C" int tpk_three_interpolate_grad_cols(int b, int c, int n, int m, const float* grad_out, const int32_t* idx,
+                                               const float* weight, float* grad_points, void* scratch, int64_t scratch_bytes,
+                                               void* stream)
+{
+    using namespace tpk;
+    const int64_t want = tpk_three_interpolate_grad_cols_scratch_bytes(b, c, n, m);
+    if (scratch == nullptr || want == 0) return tpk_three_interpolate_grad(b, c, n, m, grad_out, idx, weight, grad_points, stream);
+    if (scratch_bytes < want)
+    {
+        set_error("three_interpolate_grad: scratch of %lld bytes given, %lld needed", static_cast<long long>(scratch_bytes),
+                  static_cast<long long>(want));
+        return TPK_ERR_SCRATCH;
+    }
+    TPK_REQUIRE(grad_out && idx && weight && grad_points, "three_interpolate_grad: NULL pointer");
+    TPK_REQUIRE((reinterpret_cast<uintptr_t>(scratch) & 31u) == 0, "three_interpolate_grad: scratch must be 32-byte aligned");
+    return scatter_cols<3>(b, c, m, n, static_cast<long long>(c) * n, grad_out, idx, weight, grad_points,
+                           static_cast<float*>(scratch), static_cast<cudaStream_t>(stream), "three_interpolate_grad");
+}

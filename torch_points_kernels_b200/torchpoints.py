@@ -114,8 +114,11 @@ def three_interpolate_backward(grad_out, idx, weight, m):
     B, c, n = grad_out.size()
     grad_features = torch.empty((B, c, m), dtype=torch.float32, device=grad_out.device)
     with _lib.on_device(grad_out):
-        _lib.call("tpk_three_interpolate_grad", B, c, n, m, _lib.ptr(grad_out), _lib.ptr(idx),
-                  _lib.ptr(weight), _lib.ptr(grad_features), _lib.stream_of(grad_out))
+        # scratch for a copy of the gradient with the channel fastest; 0 bytes = sizes of the kernels without it
+        need = _lib.lib().tpk_three_interpolate_grad_cols_scratch_bytes(B, c, n, m)
+        scratch = torch.empty(need, dtype=torch.uint8, device=grad_out.device) if need > 0 else None
+        _lib.call("tpk_three_interpolate_grad_cols", B, c, n, m, _lib.ptr(grad_out), _lib.ptr(idx), _lib.ptr(weight),
+                  _lib.ptr(grad_features), _lib.ptr(scratch), need, _lib.stream_of(grad_out))
     return grad_features
 
 
@@ -176,15 +179,27 @@ def grouping_backward(grad_out, idx, n):
     grad_out = grad_out.contiguous()
     _f32(grad_out, "grad_out")
     B, c, npoint, nsample = grad_out.size()
+    return _group_grad(grad_out, idx, n, c, 0)
+
+
+def _group_grad(grad_out, idx, n, c, skip_rows):
+    """Rows skip_rows .. skip_rows + c of the gradient, summed by neighbour."""
+    B, _, npoint, nsample = grad_out.size()
     grad_features = torch.empty((B, c, n), dtype=torch.float32, device=grad_out.device)
     with _lib.on_device(grad_out):
-        # scratch for the inverted index (positions sorted by target); 0 bytes = shapes the sorted
-        # kernels do not cover, which take the atomic kernels
-        need = _lib.lib().tpk_grouping_grad_scratch_bytes(B, c, n, npoint, nsample)
+        handle = _lib.lib()
+        # scratch for a copy of the gradient with the channel fastest, or for the inverted index (positions
+        # sorted by target); 0 bytes = sizes where other kernels are ahead
+        need = handle.tpk_grouping_grad_cols_scratch_bytes(B, c, n, npoint, nsample)
+        by_cols = need > 0
+        if not by_cols:
+            need = handle.tpk_grouping_grad_scratch_bytes(B, c, n, npoint, nsample)
         scratch = torch.empty(need, dtype=torch.uint8, device=grad_out.device) if need > 0 else None
-        _lib.call("tpk_grouping_grad_ws", B, c, n, npoint, nsample, _lib.ptr(grad_out),
-                  _lib.ptr(idx), _lib.ptr(grad_features), _lib.ptr(scratch) if scratch is not None else None,
-                  need, _lib.stream_of(grad_out))
+        args = (_lib.ptr(grad_out), _lib.ptr(idx), _lib.ptr(grad_features), _lib.ptr(scratch), need, _lib.stream_of(grad_out))
+        if by_cols:
+            _lib.call("tpk_grouping_grad_cols", B, c, n, npoint, nsample, skip_rows, *args)
+        else:
+            _lib.call("tpk_sa_group_grad" if skip_rows else "tpk_grouping_grad_ws", B, c, n, npoint, nsample, *args)
     return grad_features
 
 
@@ -271,16 +286,10 @@ class SAGroup(Function):
         if c > 0:
             # the feature rows of the gradient; the coordinates get none (indices and centres are
             # selections, and PointNet++ does not train through the point positions)
-            # read in place (tpk_sa_group_grad takes the whole (B, 3+c, npoint, nsample) gradient)
+            # read in place (the kernels take the whole (B, 3+c, npoint, nsample) gradient)
             grad_out = grad_out.contiguous()
             _f32(grad_out, "grad_out")
-            B, _, npoint, nsample = grad_out.size()
-            grad_features = torch.empty((B, c, n), dtype=torch.float32, device=grad_out.device)
-            with torch.cuda.device(grad_out.device):
-                need = _lib.lib().tpk_grouping_grad_scratch_bytes(B, c, n, npoint, nsample)
-                scratch = torch.empty(need, dtype=torch.uint8, device=grad_out.device) if need > 0 else None
-                _lib.call("tpk_sa_group_grad", B, c, n, npoint, nsample, _lib.ptr(grad_out), _lib.ptr(idx),
-                          _lib.ptr(grad_features), _lib.ptr(scratch), need, _lib.stream_of(grad_out))
+            grad_features = _group_grad(grad_out, idx, n, c, 3)
         return None, grad_features, None, None, None
 
 
