@@ -1020,6 +1020,58 @@ def test_grouping_backward_sorted_path(B, C, N, P, S, kind):
     assert _lib.device_status() == 0
 
 
+@pytest.mark.parametrize("case", ["ids", "thin", "one_place", "tiny_segments"])
+@pytest.mark.parametrize("k", [1, 20, 40])
+def test_packed_searches_on_ranges_of_blocks(case, k, monkeypatch):
+    """Packed ball query and kNN on the hashed grid against the scans, bit for bit: ids without a range of
+    their own (too large, or with gaps), places so thin that whole blocks or the scan answer, all points of a segment
+    in one place, segments that end inside the points of a block."""
+    g = data.gen(len(case) + k)
+    r, ns = 0.05, 37
+    if case == "ids":
+        sizes, ids = [3000, 1500, 900, 40], [3, 700000, 700001, 1 << 40]
+    elif case == "tiny_segments":
+        sizes = [1 + 7 * (i % 19) for i in range(120)]
+        ids = list(range(0, 360, 3))
+    else:
+        sizes, ids = [5000, 2500], [0, 1]
+    x = torch.rand(sum(sizes), 3, generator=g)
+    if case == "thin":
+        x[: 4700] = 0.5 + 0.004 * (x[: 4700] - 0.5)  # nearly all of the first segment in a small cube, the rest far apart
+        x[4990:5000] *= 300.0
+    if case == "one_place":
+        x[5000:] = 0.25
+    batch = torch.repeat_interleave(torch.tensor(ids), torch.tensor(sizes))
+    at = torch.arange(0, x.shape[0], 3)
+    y, by = (x[at] + 0.01 * torch.randn(len(at), 3, generator=g)).contiguous(), batch[at]
+    assert _lib.lib().tpk_knn_partial_dense_scratch_bytes(x.shape[0], y.shape[0], k) > 0
+    got = []
+    for path in ((), ("ball_query_scan", "knn_scan")):
+        data.use_paths(monkeypatch, *path)
+        got.append(tpk.ball_query(r, ns, cu(x), cu(y), mode="partial_dense", batch_x=cu(batch), batch_y=cu(by)) +
+                   tpk.knn(cu(x), cu(y), k, cu(batch), cu(by)))
+    for a, b in zip(*got):
+        assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("ns", [1, 32, 200, 400])
+def test_dense_ball_query_of_a_large_cloud_in_parts(ns, monkeypatch):
+    """Clouds of 2^18 points are binned in three parts; centres whose list is full after the first, the second
+    and the last part, or not at all, against the scan."""
+    g = data.gen(ns)
+    n, m = (1 << 18) + 77, 600
+    x = torch.rand(2, n, 3, generator=g)
+    x[:, ::2] = 0.5 + 0.02 * torch.randn(2, (n + 1) // 2, 3, generator=g)   # thousands of points in reach
+    x[:, 1::64] = 0.2 + 0.01 * torch.randn(2, len(range(1, n, 64)), 3, generator=g)
+    y = torch.cat([x[:, :400], torch.rand(2, m - 400, 3, generator=g)], 1).contiguous()
+    got = []
+    for path in ((), ("ball_query_scan",)):
+        data.use_paths(monkeypatch, *path)
+        got.append(tpk.ball_query(0.015, ns, cu(x), cu(y), mode="dense"))
+    for a, b in zip(*got):
+        assert torch.equal(a, b)
+
+
 @pytest.mark.parametrize("B,C,N,P,S,kind", [
     (1, 1, 1, 1, 1, "random"),        # one channel, one position
     (2, 3, 50, 11, 3, "random"),      # a tile of channels that is not full, 33 positions

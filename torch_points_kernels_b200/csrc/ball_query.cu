@@ -28,7 +28,7 @@ int grid_ball_query_dense(int b, int n, int m, float radius, int nsample, const 
                           const unsigned char** need_scan_out, cudaStream_t s);
 // hash_grid.cu
 bool hash_grid_fits(long long size_x, long long size_y);
-size_t hash_grid_scratch_bytes(long long size_x, long long size_y);
+size_t hash_grid_scratch_bytes(long long size_x, long long size_y, long long clouds);
 int hash_grid_ball_query(long long size_x, long long size_y, float radius, int nsample, const float* x, const float* y,
                          const int64_t* batch_x, const int64_t* batch_y, int64_t* idx, float* dist, void* scratch,
                          const unsigned char** need_out, cudaStream_t s);
@@ -314,7 +314,7 @@ extern "C" int64_t tpk_ball_query_dense_scratch_bytes(int b, int n, int m, int n
     // shared-memory grid: one flag per centre
     if (use_smem_grid(b, n, nsample)) return (static_cast<int64_t>(b) * m + 255) / 256 * 256;
     if (use_hash_grid(b, n, m))
-        return static_cast<int64_t>(tpk::hash_grid_scratch_bytes(static_cast<long long>(b) * n, static_cast<long long>(b) * m));
+        return static_cast<int64_t>(tpk::hash_grid_scratch_bytes(static_cast<long long>(b) * n, static_cast<long long>(b) * m, b));
     // the grid in global memory needs clouds worth binning and a hit list that fits shared memory
     if (n < 8192 || nsample > 128) return 0;
     return static_cast<int64_t>(tpk::grid_scratch_bytes(b, n, m));
@@ -409,7 +409,7 @@ static bool partial_wants_grid(int64_t size_x, int64_t size_y, float radius)
 extern "C" int64_t tpk_ball_query_partial_dense_scratch_bytes(int64_t size_x, int64_t size_y, float radius)
 {
     if (!partial_wants_grid(size_x, size_y, radius)) return 0;
-    return static_cast<int64_t>(tpk::hash_grid_scratch_bytes(size_x, size_y));
+    return static_cast<int64_t>(tpk::hash_grid_scratch_bytes(size_x, size_y, 0));
 }
 
 extern "C" int tpk_ball_query_partial_dense_ws(int64_t size_x, int64_t size_y, float radius, int nsample,

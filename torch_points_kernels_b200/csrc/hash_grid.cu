@@ -1,19 +1,28 @@
-// Ball query on a hashed uniform grid (sm_100a): the packed (partial_dense) layout, and dense
-// clouds too large for the grids in shared memory.
+// Ball query and k nearest neighbours on a hashed uniform grid (sm_100a): the packed (partial_dense)
+// layout, and dense clouds too large for the grids in shared memory.
 //
-// The packed layout holds many scenes of different sizes, each with its own extent, so
-// there is no common bounding box to lay a grid over.  Points are instead binned by the
-// hash of (segment id, cell coordinates) with cells one radius wide: a bucket holds the
-// points of one cell, plus, rarely, those of other cells that hash to the same bucket;
-// the exact test (same segment, squared distance <= r^2 in the reference's arithmetic,
-// cuda/src/ball_query_gpu.cu:54-95) rejects the strangers.  A query looks at the 27
-// buckets of the cells around it, one warp per query, 32 candidates at a time; a hit's
-// output position is its rank by point index among the hits, so the first `nsample`
-// neighbours in index order come out without a sort.  Queries the grid cannot answer
-// (non-finite coordinates, too many candidates or hits) are flagged and left to the scan.
+// The packed layout holds many scenes of different sizes, each with its own extent, so there is no
+// common bounding box to lay a grid over.  Every segment (scene, or dense cloud) has a range of counters
+// of its own, about two per point, in blocks of 8 x 4 x 4 cells; the block of a cell is picked by a hash
+// of its coordinates among the blocks of the segment.  So the counters of the three cells of a row around
+// a query are neighbours, as are their points: a query reads nine or eighteen short runs instead of 27
+// random ones, and the queries of a scene find its points and counters, 24 bytes per point, in the L2
+// cache.  With all cells of all scenes hashed over one range of as many counters as points, 7.0 M points in 64
+// scenes, 703 k queries: binning 350 us, ball query 1246, kNN 1784 and up to 1600 for the queries that it left
+// over; now 245, 444 and 1037, and none left over.  (One counter per point: 474 and 1279.)
+// A block may hold cells of several places; the exact tests reject the strangers (same segment, squared
+// distance within r^2 in the reference's arithmetic, cuda/src/ball_query_gpu.cu:54-95).
 //
-// Pipeline on the caller's stream: zero counters, count, prefix sum (three launches),
-// fill, query.
+// Ball query: cells one radius wide, a warp per query, 32 candidates at a time.  The result is the nsample
+// lowest indices among the hits: those are kept in a buffer, which is cut to the lowest ones when it fills
+// up, and a hit's output position is its rank by index.  Dense clouds are binned in three parts, the first
+// 64th of the points, the rest of the first eighth, and the rest: a centre whose list is full after a part
+// needs nothing of the parts behind it, so that a crowded centre reads a 64th of its candidates (8 x 1048576
+// points, 65536 centres: 2900 us and 820 for the crowded ones that were left to the scan, 1334 and 6 now).
+// Queries the grid cannot answer (non-finite coordinates, too many candidates) are flagged and left to the scan.
+//
+// Pipeline on the caller's stream: zero counters, bounds of the segments, [cell widths], count, places of
+// the blocks, fill, query.
 #include <climits>
 #include <math_constants.h>
 
@@ -26,8 +35,36 @@ namespace
 
 constexpr int kHgThreads = 256;
 constexpr int kHgWarps = kHgThreads / 32;
-constexpr int kHgHitCap = 512;        // hits per query the buffer takes
 constexpr int kHgCoordLimit = 1 << 20;
+constexpr int kHgBlock = 128;       // counters of a block: 8 x 4 x 4 cells, x fastest
+constexpr int kHgBlockPoints = 6;   // a block per 2^6 points of a segment
+constexpr int kHgHitCap = 512;      // hits per query the buffer takes at most
+constexpr int kHgCut = 96;          // room for hits beyond nsample from which the buffer is cut
+
+struct HgHead
+{
+    int cursor;  // sorted points placed so far
+    int mixed;   // segment ids without a range of their own, or not in order: hits compare the ids
+    int pad[62];
+};
+
+struct HgSeg
+{
+    int start, end;  // its points in x
+    float inv_h, h;  // kNN: cell width
+};
+
+// How points are binned, the same for all kernels of a call.
+struct HgSpace
+{
+    uint32_t size_x;
+    uint32_t per_cloud;  // dense layout: points per cloud
+    uint32_t blocks;
+    uint32_t cap;        // segments with a range of their own (packed), or clouds (dense)
+    float inv_h;         // ball query: reciprocal cell width
+    const HgSeg* segs;
+    const HgHead* head;
+};
 
 __device__ __forceinline__ int hg_cell(float v, float inv_h)
 {
@@ -35,131 +72,187 @@ __device__ __forceinline__ int hg_cell(float v, float inv_h)
     return static_cast<int>(fminf(fmaxf(t, -static_cast<float>(kHgCoordLimit)), static_cast<float>(kHgCoordLimit)));
 }
 
-__device__ __forceinline__ uint32_t hg_bucket(long long seg, int cx, int cy, int cz, uint32_t mask)
-{
-    uint32_t h = static_cast<uint32_t>(seg) * 0x9E3779B1u;
-    h ^= static_cast<uint32_t>(cx) * 0x85EBCA77u;
-    h = (h << 13) | (h >> 19);
-    h ^= static_cast<uint32_t>(cy) * 0xC2B2AE3Du;
-    h = (h << 13) | (h >> 19);
-    h ^= static_cast<uint32_t>(cz) * 0x27D4EB2Fu;
-    h ^= h >> 15;
-    h *= 0x2C1B3C6Du;
-    h ^= h >> 12;
-    return h & mask;
-}
-
 __device__ __forceinline__ bool hg_finite(float x, float y, float z)
 {
     return fabsf(x) < 1.0e18f && fabsf(y) < 1.0e18f && fabsf(z) < 1.0e18f;
 }
 
-// FILL == false: count points per bucket (counter of bucket c at counts[c + 1]);
-// FILL == true: the prefix sum left the first slot of bucket c in counts[c + 1]; handing
-// slots out advances it to the bucket's end, which is the beginning of bucket c + 1.
-// Points with non-finite coordinates are not binned (no ball contains them).
-// inv_h_dev (optional): the reciprocal cell width in device memory, where an earlier kernel of the
-// same call computed it (kNN, which has no radius to size the cells by).
-template <bool FILL>
+// The blocks of a segment: first and number.  Ranges of segments in order do not meet; whatever the
+// values are, the blocks lie inside the space.
+struct HgRange
+{
+    uint32_t first, count, salt;
+};
+
+__device__ __forceinline__ HgRange hg_range(uint32_t start, uint32_t end, uint32_t id)
+{
+    const uint32_t a = start >> kHgBlockPoints, b = max(start, end) >> kHgBlockPoints;
+    return HgRange{a + id, b - a + 1u, 0u};
+}
+
+// Dense clouds in three parts (PARTS == 3): [0, n / 64), [n / 64, n / 8), [n / 8, n) of every cloud.
+template <int PARTS>
+__device__ __forceinline__ HgRange hg_cloud_range(const HgSpace& sp, uint32_t cloud, int part)
+{
+    const uint32_t n = sp.per_cloud, base = cloud * n;
+    if (PARTS == 1) return hg_range(base, base + n, cloud);
+    const uint32_t lo = part == 0 ? 0u : (part == 1 ? n >> 6 : n >> 3), hi = part == 0 ? n >> 6 : (part == 1 ? n >> 3 : n);
+    return hg_range(base + lo, base + hi, cloud * PARTS + part);
+}
+
+// Packed: ids without a range of their own share the whole space.  No blocks: a segment without points.
+__device__ __forceinline__ HgRange hg_seg_range(const HgSpace& sp, long long seg, const HgSeg& e)
+{
+    if (static_cast<unsigned long long>(seg) < sp.cap)
+    {
+        HgRange r = hg_range(e.start, e.end, static_cast<uint32_t>(seg));
+        if (e.end == 0) r.count = 0u;
+        return r;
+    }
+    return HgRange{0u, sp.blocks, static_cast<uint32_t>(seg) * 0x9E3779B1u};
+}
+
+__device__ __forceinline__ HgSeg hg_seg(const HgSpace& sp, long long seg)
+{
+    const uint32_t i = static_cast<unsigned long long>(seg) < sp.cap ? static_cast<uint32_t>(seg) : sp.cap;
+    const int4 v = __ldg(reinterpret_cast<const int4*>(sp.segs) + i);
+    return HgSeg{v.x, v.y, __int_as_float(v.z), __int_as_float(v.w)};
+}
+
+// Block of the cells (8 bx .., 4 by .., 4 bz ..) of a segment.
+__device__ __forceinline__ uint32_t hg_block(const HgRange& r, int bx, int by, int bz)
+{
+    uint32_t h = static_cast<uint32_t>(bx) * 0x8DA6B343u ^ static_cast<uint32_t>(by) * 0xD8163841u ^
+                 static_cast<uint32_t>(bz) * 0xCB1AB31Fu ^ r.salt;
+    h ^= h >> 15;
+    h *= 0x2C1B3C6Du;
+    h ^= h >> 12;
+    h *= 0x297A2D39u;
+    return r.first + __umulhi(h, r.count);
+}
+__device__ __forceinline__ size_t hg_counter(uint32_t block, int x, int y, int z)
+{
+    return static_cast<size_t>(block) * kHgBlock + static_cast<uint32_t>((z & 3) << 5 | (y & 3) << 3 | (x & 7));
+}
+
+// Where the points of every segment begin and end (packed); four ids per thread.
 __global__ void __launch_bounds__(kHgThreads)
-    hg_bin_kernel(long long size_x, long long per_cloud, float inv_h, const float* __restrict__ inv_h_dev, uint32_t mask,
-                  const float* __restrict__ x, const int64_t* __restrict__ batch_x, int* __restrict__ counts,
-                  float4* __restrict__ sorted, int* __restrict__ sorted_seg)
+    hg_bounds_kernel(uint32_t size_x, uint32_t cap, const int64_t* __restrict__ batch_x, HgHead* head, HgSeg* segs)
 {
-    const long long k = static_cast<long long>(blockIdx.x) * kHgThreads + threadIdx.x;
-    if (k >= size_x) return;
-    if (inv_h_dev != nullptr) inv_h = __ldg(inv_h_dev);
-    const float px = __ldg(x + 3 * k + 0), py = __ldg(x + 3 * k + 1), pz = __ldg(x + 3 * k + 2);
+    const uint32_t k0 = (blockIdx.x * kHgThreads + threadIdx.x) * 4;
+    bool odd = false;
+    if (k0 < size_x)
+    {
+        long long id[6];  // one before, four, one behind
+#pragma unroll
+        for (int i = 0; i < 6; ++i)
+        {
+            const uint32_t k = k0 + i;  // place of id[i] + 1
+            id[i] = k > 0 && k <= size_x ? __ldg(batch_x + (k - 1)) : -1;
+        }
+#pragma unroll
+        for (int i = 1; i < 5; ++i)
+        {
+            const uint32_t k = k0 + i - 1;
+            if (k >= size_x) break;
+            const long long seg = id[i];
+            const bool own = static_cast<unsigned long long>(seg) < cap;
+            odd |= !own || seg < id[i - 1];
+            if (own && (k == 0 || id[i - 1] != seg)) segs[seg].start = static_cast<int>(k);
+            if (own && (k + 1 == size_x || id[i + 1] != seg)) segs[seg].end = static_cast<int>(k + 1);
+        }
+    }
+    if (__any_sync(kFullMask, odd) && (threadIdx.x & 31) == 0) head->mixed = 1;
+}
+
+// FILL == false: counts the points of every cell.  FILL == true: hg_place_kernel left the end of a cell's
+// points in its counter; handing the places out from there leaves their beginning.
+// Points with non-finite coordinates are not binned (no ball contains them).
+template <bool DENSE, int PARTS, bool WIDTHS, bool FILL>
+__global__ void __launch_bounds__(kHgThreads)
+    hg_bin_kernel(HgSpace sp, const float* __restrict__ x, const int64_t* __restrict__ batch_x, int* __restrict__ counts,
+                  float4* __restrict__ sorted)
+{
+    const uint32_t k = blockIdx.x * kHgThreads + threadIdx.x;
+    if (k >= sp.size_x) return;
+    const float px = __ldg(x + 3 * static_cast<size_t>(k) + 0), py = __ldg(x + 3 * static_cast<size_t>(k) + 1),
+                pz = __ldg(x + 3 * static_cast<size_t>(k) + 2);
     if (!hg_finite(px, py, pz)) return;
-    // packed layout: the segment id of the point; dense layout (batch_x == NULL): its cloud
-    const long long seg = batch_x ? __ldg(batch_x + k) : k / per_cloud;
-    const uint32_t bkt = hg_bucket(seg, hg_cell(px, inv_h), hg_cell(py, inv_h), hg_cell(pz, inv_h), mask);
-    const int pos = atomicAdd(counts + bkt + 1, 1);
-    if (FILL)
+    HgRange r;
+    float inv_h = sp.inv_h;
+    if constexpr (DENSE)
     {
-        sorted[pos] = make_float4(px, py, pz, __int_as_float(static_cast<int>(k)));
-        sorted_seg[pos] = static_cast<int>(seg);
+        const uint32_t cloud = k / sp.per_cloud, local = k - cloud * sp.per_cloud;
+        r = hg_cloud_range<PARTS>(sp, cloud, local < sp.per_cloud >> 6 ? 0 : (local < sp.per_cloud >> 3 ? 1 : 2));
+        if (WIDTHS) inv_h = __ldg(&sp.segs[cloud].inv_h);
     }
+    else
+    {
+        const long long seg = __ldg(batch_x + k);
+        const HgSeg e = hg_seg(sp, seg);
+        r = hg_seg_range(sp, seg, e);
+        if (WIDTHS) inv_h = e.inv_h;
+    }
+    const int cx = hg_cell(px, inv_h), cy = hg_cell(py, inv_h), cz = hg_cell(pz, inv_h);
+    int* c = counts + hg_counter(hg_block(r, cx >> 3, cy >> 2, cz >> 2), cx, cy, cz);
+    if constexpr (FILL)
+        sorted[atomicSub(c, 1) - 1] = make_float4(px, py, pz, __int_as_float(static_cast<int>(k)));
+    else
+        atomicAdd(c, 1);
 }
 
-// Exclusive prefix sum over data[0..n), three launches: per-block scan + block totals,
-// scan of the totals (one block), add.
-__global__ void __launch_bounds__(1024) hg_scan_blocks_kernel(int* __restrict__ data, long long n, int* __restrict__ totals)
+// Places for the points of every block: counts[i] becomes the end of cell i, ends[block] that of its last
+// cell.  Which block comes first does not matter, so a CTA (32 blocks) takes its place from a cursor instead
+// of a prefix sum over all of them.
+__global__ void __launch_bounds__(kHgThreads) hg_place_kernel(uint32_t blocks, HgHead* head, int* __restrict__ counts, int* __restrict__ ends)
 {
-    __shared__ int s_warp[32];
+    constexpr int B = 4;  // blocks of a warp
+    __shared__ int s_warp[kHgWarps];
+    __shared__ int s_base;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const long long i = static_cast<long long>(blockIdx.x) * 1024 + threadIdx.x;
-    const int v = i < n ? data[i] : 0;
-    int incl = v;
+    const uint32_t b0 = (blockIdx.x * kHgWarps + warp) * B;
+    int4 v[B];
+    int incl[B], total[B], sum = 0;
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1)
+    for (int j = 0; j < B; ++j)
+        v[j] = b0 + j < blocks ? reinterpret_cast<const int4*>(counts)[static_cast<size_t>(b0 + j) * 32 + lane] : make_int4(0, 0, 0, 0);
+#pragma unroll
+    for (int j = 0; j < B; ++j)
     {
-        const int t = __shfl_up_sync(kFullMask, incl, o);
-        if (lane >= o) incl += t;
-    }
-    if (lane == 31) s_warp[warp] = incl;
-    __syncthreads();
-    if (warp == 0)
-    {
-        int w = s_warp[lane];
+        incl[j] = v[j].x + v[j].y + v[j].z + v[j].w;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1)
         {
-            const int t = __shfl_up_sync(kFullMask, w, o);
-            if (lane >= o) w += t;
+            const int t = __shfl_up_sync(kFullMask, incl[j], o);
+            if (lane >= o) incl[j] += t;
         }
-        s_warp[lane] = w;
+        total[j] = __shfl_sync(kFullMask, incl[j], 31);
+        sum += total[j];
     }
+    if (lane == 0) s_warp[warp] = sum;
     __syncthreads();
-    const int before = (warp ? s_warp[warp - 1] : 0) + incl - v;
-    if (i < n) data[i] = before;
-    if (threadIdx.x == 1023) totals[blockIdx.x] = before + v;
-}
-
-__global__ void __launch_bounds__(1024) hg_scan_totals_kernel(int* __restrict__ totals, int nblocks)
-{
-    __shared__ int s_warp[32];
-    __shared__ int s_carry;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    if (threadIdx.x == 0) s_carry = 0;
-    __syncthreads();
-    for (int base = 0; base < nblocks; base += 1024)
+    if (threadIdx.x == 0)
     {
-        const int i = base + threadIdx.x;
-        const int v = i < nblocks ? totals[i] : 0;
-        int incl = v;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1)
+        int all = 0;
+        for (int w = 0; w < kHgWarps; ++w)
         {
-            const int t = __shfl_up_sync(kFullMask, incl, o);
-            if (lane >= o) incl += t;
+            const int t = s_warp[w];
+            s_warp[w] = all;
+            all += t;
         }
-        if (lane == 31) s_warp[warp] = incl;
-        __syncthreads();
-        if (warp == 0)
-        {
-            int w = s_warp[lane];
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1)
-            {
-                const int t = __shfl_up_sync(kFullMask, w, o);
-                if (lane >= o) w += t;
-            }
-            s_warp[lane] = w;
-        }
-        __syncthreads();
-        const int before = s_carry + (warp ? s_warp[warp - 1] : 0) + incl - v;
-        if (i < nblocks) totals[i] = before;
-        __syncthreads();
-        if (threadIdx.x == 1023) s_carry = before + v;
-        __syncthreads();
+        s_base = all ? atomicAdd(&head->cursor, all) : 0;
     }
-}
-
-__global__ void __launch_bounds__(1024) hg_scan_add_kernel(int* __restrict__ data, long long n, const int* __restrict__ totals)
-{
-    const long long i = static_cast<long long>(blockIdx.x) * 1024 + threadIdx.x;
-    if (i < n) data[i] += totals[blockIdx.x];
+    __syncthreads();
+    int base = s_base + s_warp[warp];
+#pragma unroll
+    for (int j = 0; j < B; ++j)
+    {
+        if (total[j] == 0) continue;  // counters of an empty block stay zero: runs from 0 to 0
+        const int w = base + incl[j], z = w - v[j].w, y = z - v[j].z, x = y - v[j].y;
+        reinterpret_cast<int4*>(counts)[static_cast<size_t>(b0 + j) * 32 + lane] = make_int4(x, y, z, w);
+        base += total[j];
+        if (lane == 0) ends[b0 + j] = base;
+    }
 }
 
 // The run that candidate v lies in: the number of lanes whose inclusive prefix `incl` of the run
@@ -174,170 +267,247 @@ __device__ __forceinline__ int hg_run_of(int incl, int v)
     return r;
 }
 
-struct HgWarpScratch
+__device__ __forceinline__ int hg_inclusive(int v, int lane)
 {
-    uint32_t hit_idx[kHgHitCap];  // original index of the hit
-    int hit_pos[kHgHitCap];       // its slot in the sorted copy
-    int run_shift[32];            // slot of candidate v of run r = run_shift[r] + v
-    int first;                    // dense layout: index of the first hit, repeated in unused slots
-};
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1)
+    {
+        const int t = __shfl_up_sync(kFullMask, v, o);
+        if (lane >= o) v += t;
+    }
+    return v;
+}
+
+// Points of the cells [xa, xb] of a row: beginning in the sorted copy, and number.  xa and xb lie in one block.
+__device__ __forceinline__ int2 hg_run(const HgRange& r, const int* __restrict__ counts, const int* __restrict__ ends, int xa, int xb,
+                                       int y, int z)
+{
+    const uint32_t block = hg_block(r, xa >> 3, y >> 2, z >> 2);
+    const size_t i0 = hg_counter(block, xa, y, z), i1 = hg_counter(block, xb, y, z);
+    const int beg = __ldg(counts + i0);
+    const int end = (i1 & (kHgBlock - 1)) == kHgBlock - 1 ? __ldg(ends + block) : __ldg(counts + i1 + 1);
+    return make_int2(beg, end - beg);
+}
+
+// Cuts a list of hits to little more than the `keep` lowest indices (all below `limit`); returns their number,
+// `limit` becomes a bound of theirs.
+__device__ __forceinline__ int hg_cut(uint32_t* idx, float* dist, int nh, int keep, uint32_t& limit, int lane)
+{
+    uint32_t lo = 0, hi = limit;  // fewer than keep below lo, at least as many below hi
+    int below = nh;
+    while (hi - lo > 1u && below > keep + 16)
+    {
+        const uint32_t mid = lo + ((hi - lo) >> 1);
+        int c = 0;
+        for (int h0 = 0; h0 < nh; h0 += 32) c += __popc(__ballot_sync(kFullMask, h0 + lane < nh && idx[h0 + lane] < mid));
+        if (c >= keep)
+        {
+            hi = mid;
+            below = c;
+        }
+        else
+            lo = mid;
+    }
+    limit = hi;
+    int kept = 0;
+    for (int h0 = 0; h0 < nh; h0 += 32)
+    {
+        const bool in = h0 + lane < nh;
+        const uint32_t i = in ? idx[h0 + lane] : 0xFFFFFFFFu;
+        const float d = in ? dist[h0 + lane] : 0.f;
+        const bool stay = in && i < hi;
+        const uint32_t b = __ballot_sync(kFullMask, stay);
+        __syncwarp();
+        if (stay)
+        {
+            const int to = kept + __popc(b & ((1u << lane) - 1u));
+            idx[to] = i;
+            dist[to] = d;
+        }
+        kept += __popc(b);
+    }
+    __syncwarp();
+    return kept;
+}
+
+__host__ __device__ inline int hg_hits(int nsample)
+{
+    // room for two cuts' worth of hits beyond nsample; above that, more hits than fit are left to the scan
+    return nsample + 2 * kHgCut <= kHgHitCap ? nsample + 2 * kHgCut : kHgHitCap;
+}
 
 // DENSE: (b, n, 3) clouds and (b, m, 3) centres instead of packed segments: the segment of a
 // query is its cloud, the test is the dense kernel's (strict, ball_query_gpu.cu:35-36),
 // indices are local to the cloud and unused slots repeat the first hit.
-template <bool DENSE>
+template <bool DENSE, int PARTS>
 __global__ void __launch_bounds__(kHgThreads)
-    hg_query_kernel(long long size_y, long long per_cloud_x, long long per_cloud_y, float radius, int nsample, int max_candidates,
-                    float inv_h, uint32_t mask,
-                    const float* __restrict__ y, const int64_t* __restrict__ batch_y, const int* __restrict__ counts,
-                    const float4* __restrict__ sorted, const int* __restrict__ sorted_seg,
+    hg_query_kernel(HgSpace sp, uint32_t size_y, uint32_t per_cloud_y, float radius, int nsample, int max_candidates,
+                    const float* __restrict__ y, const int64_t* __restrict__ batch_x, const int64_t* __restrict__ batch_y,
+                    const int* __restrict__ counts, const int* __restrict__ ends, const float4* __restrict__ sorted,
                     int64_t* __restrict__ idx_out, float* __restrict__ dist_out, unsigned char* __restrict__ need)
 {
-    __shared__ HgWarpScratch s_scr[kHgWarps];
+    extern __shared__ uint32_t s_hits[];
+    __shared__ int s_shift[kHgWarps][32];  // slot of candidate v of run r = shift[r] + v
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    HgWarpScratch& ws = s_scr[warp];
-    const float r2 = __fmul_rn(radius, radius);
-    const long long nwarps_total = static_cast<long long>(gridDim.x) * kHgWarps;
-    for (long long j = static_cast<long long>(blockIdx.x) * kHgWarps + warp; j < size_y; j += nwarps_total)
+    const int cap = hg_hits(nsample);
+    uint32_t* hit_idx = s_hits + static_cast<size_t>(warp) * 2 * cap;
+    float* hit_dist = reinterpret_cast<float*>(hit_idx + cap);
+    int* shift = s_shift[warp];
+    const bool cuts = nsample + kHgCut <= cap - 32;
+    const float r2 = __fmul_rn(radius, radius), inv_h = sp.inv_h;
+    const bool mixed = !DENSE && __ldg(&sp.head->mixed) != 0;
+    // lane l < 18: part l & 1 (of at most two blocks) of row l >> 1 of the 3 x 3 rows of cells
+    const int row_y = (lane >> 1) % 3, row_z = (lane >> 1) / 3, second = lane & 1;
+    const uint32_t nwarps_total = gridDim.x * kHgWarps;
+    for (uint32_t j = blockIdx.x * kHgWarps + warp; j < size_y; j += nwarps_total)
     {
         // the query is the same in all lanes: everything up to the candidate loop is warp-uniform
-        const float qx = __ldg(y + 3 * j + 0), qy = __ldg(y + 3 * j + 1), qz = __ldg(y + 3 * j + 2);
-        if (!hg_finite(qx, qy, qz))
-        {
-            if (lane == 0) need[j] = 1;
-            continue;
-        }
+        const float* yp = y + 3 * static_cast<size_t>(j);
+        const float qx = __ldg(yp + 0), qy = __ldg(yp + 1), qz = __ldg(yp + 2);
         const long long seg = DENSE ? j / per_cloud_y : __ldg(batch_y + j);
-        // the ball, enlarged by the rounding of the exact test and of q +- r, must stay inside the
-        // three cells per axis around the query's cell; it does unless q sits on a cell face
+        // the cells of the ball, enlarged by the rounding of the exact test and of q +- r: three per axis,
+        // unless q sits on a cell face
         const float pad = radius * 1.00001f + 1.0e-30f;
-        const int cx = hg_cell(qx, inv_h), cy = hg_cell(qy, inv_h), cz = hg_cell(qz, inv_h);
         const float ex = pad + fabsf(qx) * 2.0e-7f, ey = pad + fabsf(qy) * 2.0e-7f, ez = pad + fabsf(qz) * 2.0e-7f;
-        const bool inside = hg_cell(qx - ex, inv_h) >= cx - 1 && hg_cell(qx + ex, inv_h) <= cx + 1 &&
-                            hg_cell(qy - ey, inv_h) >= cy - 1 && hg_cell(qy + ey, inv_h) <= cy + 1 &&
-                            hg_cell(qz - ez, inv_h) >= cz - 1 && hg_cell(qz + ez, inv_h) <= cz + 1 &&
-                            abs(cx) < kHgCoordLimit - 1 && abs(cy) < kHgCoordLimit - 1 && abs(cz) < kHgCoordLimit - 1;
-        if (!inside)
+        const int x0 = hg_cell(qx - ex, inv_h), x1 = hg_cell(qx + ex, inv_h);
+        const int y0 = hg_cell(qy - ey, inv_h), y1 = hg_cell(qy + ey, inv_h);
+        const int z0 = hg_cell(qz - ez, inv_h), z1 = hg_cell(qz + ez, inv_h);
+        const int out = kHgCoordLimit - 1;
+        if (!hg_finite(qx, qy, qz) || x1 - x0 > 2 || y1 - y0 > 2 || z1 - z0 > 2 || min(x0, min(y0, z0)) <= -out ||
+            max(x1, max(y1, z1)) >= out)
         {
             if (lane == 0) need[j] = 1;
             continue;
         }
-        // lane l < 27: bucket of neighbour cell l; a bucket reached through two cells counts once
-        uint32_t bkt = 0xFFFFFFFFu - static_cast<uint32_t>(lane);  // distinct dummies for lanes 27..31
-        if (lane < 27) bkt = hg_bucket(seg, cx + lane % 3 - 1, cy + (lane / 3) % 3 - 1, cz + lane / 9 - 1, mask);
-        const uint32_t same = __match_any_sync(kFullMask, bkt);
-        int beg = 0, len = 0;
-        if (lane < 27 && (same & ((1u << lane) - 1u)) == 0u)
-        {
-            beg = __ldg(counts + bkt);
-            len = __ldg(counts + bkt + 1) - beg;
-        }
-        int incl = len;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1)
-        {
-            const int v = __shfl_up_sync(kFullMask, incl, o);
-            if (lane >= o) incl += v;
-        }
-        const int total = __shfl_sync(kFullMask, incl, 31);
-        if (total > max_candidates)  // crowded: the scan, which stops at the nsample-th hit, is cheaper
-        {
-            if (lane == 0) need[j] = 1;
-            continue;
-        }
-        __syncwarp();  // the previous query's reads of the scratch are done
-        ws.run_shift[lane] = beg - (incl - len);
-        __syncwarp();
         int nh = 0;
-        for (int v0 = 0; v0 < total; v0 += 32)
+        uint32_t limit = 0x80000000u;  // indices below this are wanted
+        bool answered = true;
+#pragma unroll
+        for (int part = 0; part < PARTS; ++part)
         {
-            const int v = v0 + lane;
-            const bool valid = v < total;
-            const int r = hg_run_of(incl, v);
-            const int p = valid ? ws.run_shift[r] + v : 0;
-            const float4 c = __ldg(sorted + p);
-            const int cseg = __ldg(sorted_seg + p);
-            // the packed kernel's arithmetic (ball_query_gpu.cu:78-82) and its inclusive test, or the dense one's
-            const float d = DENSE ? sumsq_abc(qx - c.x, qy - c.y, qz - c.z) : sumsq_loop(qx - c.x, qy - c.y, qz - c.z);
-            const bool hit = valid && cseg == static_cast<int>(seg) && (DENSE ? d < r2 : d <= r2);
-            const uint32_t bal = __ballot_sync(kFullMask, hit);
-            if (hit)
+            HgRange range;
+            if constexpr (DENSE)
+                range = hg_cloud_range<PARTS>(sp, static_cast<uint32_t>(seg), part);
+            else
+                range = hg_seg_range(sp, seg, hg_seg(sp, seg));
+            int beg = 0, len = 0;
+            const int cy = y0 + row_y, cz = z0 + row_z;
+            const int xa = second ? x1 & ~7 : x0, xb = second ? x1 : min(x1, x0 | 7);
+            if (lane < 18 && cy <= y1 && cz <= z1 && !(second && (x0 >> 3) == (x1 >> 3)) && range.count != 0u)
             {
+                const int2 run = hg_run(range, counts, ends, xa, xb, cy, cz);
+                beg = run.x;
+                len = run.y;
+            }
+            const int incl = hg_inclusive(len, lane);
+            const int total = __shfl_sync(kFullMask, incl, 31);
+            if (total > max_candidates)  // crowded: the scan, which stops at the nsample-th hit, is cheaper
+            {
+                answered = false;
+                break;
+            }
+            __syncwarp();  // earlier reads of the scratch are done
+            shift[lane] = beg - (incl - len);
+            __syncwarp();
+            for (int v0 = 0; v0 < total; v0 += 32)
+            {
+                const int v = v0 + lane;
+                const bool valid = v < total;
+                const int run = hg_run_of(incl, v);
+                const float4 c = __ldg(sorted + (valid ? shift[run] + v : 0));
+                // the packed kernel's arithmetic (ball_query_gpu.cu:78-82) and its inclusive test, or the dense one's
+                const float d = DENSE ? sumsq_abc(qx - c.x, qy - c.y, qz - c.z) : sumsq_loop(qx - c.x, qy - c.y, qz - c.z);
+                const uint32_t ci = static_cast<uint32_t>(__float_as_int(c.w));
+                bool hit = valid && (DENSE ? d < r2 : d <= r2) && ci < limit;
+                if (mixed && hit) hit = __ldg(batch_x + ci) == seg;
+                const uint32_t bal = __ballot_sync(kFullMask, hit);
                 const int pos = nh + __popc(bal & ((1u << lane) - 1u));
-                if (pos < kHgHitCap)
+                if (hit && pos < cap)
                 {
-                    ws.hit_idx[pos] = static_cast<uint32_t>(__float_as_int(c.w));
-                    ws.hit_pos[pos] = p;
+                    hit_idx[pos] = ci;
+                    hit_dist[pos] = d;
+                }
+                nh += __popc(bal);
+                if (nh > cap - 32 && cuts)
+                {
+                    __syncwarp();
+                    nh = hg_cut(hit_idx, hit_dist, nh, nsample, limit, lane);
                 }
             }
-            nh += __popc(bal);
+            if (nh > cap)
+            {
+                answered = false;
+                break;
+            }
+            if (PARTS > 1 && nh >= nsample) break;
         }
-        if (nh > kHgHitCap)
+        if (!answered)
         {
             if (lane == 0) need[j] = 1;
             continue;
         }
         __syncwarp();
-        int64_t* orow = idx_out + j * nsample;
-        float* drow = dist_out + j * nsample;
-        const long long base = DENSE ? seg * per_cloud_x : 0;  // dense indices are local to the cloud
-        __syncwarp();
+        if (nh > max(64, nsample + 16)) nh = hg_cut(hit_idx, hit_dist, nh, nsample, limit, lane);
+        int64_t* orow = idx_out + static_cast<size_t>(j) * nsample;
+        float* drow = dist_out + static_cast<size_t>(j) * nsample;
+        const long long base = DENSE ? seg * sp.per_cloud : 0;  // dense indices are local to the cloud
+        int64_t fill = DENSE ? 0 : -1;
         for (int h0 = 0; h0 < nh; h0 += 32)
         {
             const int h = h0 + lane;
-            if (h < nh)
+            const uint32_t e = h < nh ? hit_idx[h] : 0xFFFFFFFFu;
+            int rank = 0;
+            for (int k = 0; k < nh; ++k) rank += hit_idx[k] < e ? 1 : 0;
+            if (h < nh && rank < nsample)
             {
-                const uint32_t e = ws.hit_idx[h];
-                int rank = 0;
-                for (int k = 0; k < nh; ++k) rank += ws.hit_idx[k] < e ? 1 : 0;
-                if (rank < nsample)
-                {
-                    const float4 c = __ldg(sorted + ws.hit_pos[h]);
-                    orow[rank] = static_cast<int64_t>(e) - base;
-                    drow[rank] = DENSE ? sumsq_abc(qx - c.x, qy - c.y, qz - c.z) : sumsq_loop(qx - c.x, qy - c.y, qz - c.z);
-                    if (rank == 0) ws.first = static_cast<int>(static_cast<long long>(e) - base);
-                }
+                orow[rank] = static_cast<int64_t>(e) - base;
+                drow[rank] = hit_dist[h];
+            }
+            if (DENSE)
+            {
+                const uint32_t lowest = __ballot_sync(kFullMask, h < nh && rank == 0);
+                if (lowest != 0u) fill = static_cast<int64_t>(__shfl_sync(kFullMask, e, __ffs(lowest) - 1)) - base;
             }
         }
-        __syncwarp();
-        const int64_t fill = DENSE ? (nh ? static_cast<int64_t>(ws.first) : 0) : -1;
         for (int s = min(nh, nsample) + lane; s < nsample; s += 32)
         {
             orow[s] = fill;
             drow[s] = -1.0f;
         }
-        if (lane == 0) need[j] = 0;
+        __syncwarp();  // the lists are free for the next query
     }
 }
 
-
 // ------------------------------------------------------------------ k nearest neighbours
 //
-// kNN on the same hashed grid.  There is no radius to size the cells by, so the call first
-// measures the bounding box of all support points and picks a cell width that puts about
-// max(k, 8) / 4 points into a cell of an average segment (hg_knn_params_kernel; the width
-// stays in device memory, no host round trip).  A query (one warp) then examines the 27
-// cells around its own cell, keeps the k best candidates in (distance, index) order in
+// On the same grid, with a cell width of every segment's own, about the distance to the k-th neighbour
+// (hg_width_kernel measures it; the widths stay in device memory, no host round trip).  A query (one warp)
+// examines the 27 cells around its own, keeps the k best candidates in (distance, index) order in
 // registers (slot s of the list in lane s & 31), and is done when the k-th best distance is
 // no larger than the distance to the nearest face of the block it has searched; otherwise
-// it searches the next shell of cells (up to kHgKnnMaxRing shells), and what is still open
-// after that (sparse regions, segments with fewer than k points, coordinates that are not
-// finite) is flagged for the scan kernel.  A candidate is taken only from the bucket of its
-// own cell, so a bucket that two cells of the search hash to never yields a point twice.
+// it searches the next shell of cells, and after four shells whole blocks, shell by shell, which
+// serves the thin places of a cloud (without: 1.1 to 1.6 ms of scans for some hundred points of 64 scenes;
+// with one shell of cells before, kNN of all 64 45 % slower).  What is still open then (segments with fewer
+// than k points, coordinates that are not finite) is flagged for the scan kernel.  A candidate is taken only
+// where its own cell lies in the run, so a block that two places of the search hash to never yields a point twice.
 // Distances use the arithmetic of the reference's kd-tree metric (sumsq_unfused).
 // candidates of a step from which they are sorted and merged (about 170 instructions, whatever their
 // number) instead of inserted one by one (25 each).  The kernel is bound by the issue of
 // instructions: with this and hg_run_of 7.0 M points in 64 scenes, k = 16, 3.10 -> 2.07 ms a call,
 // 244345 points, k = 8, 568 -> 395 us, 114163, k = 32, 385 -> 250, 22627, k = 8, 100 -> 84.
 constexpr int kHgKnnMergeFrom = 7;
-constexpr int kHgKnnMaxRing = 3;  // shells beyond the first 3 x 3 x 3 block
+constexpr int kHgKnnRings = 4;       // shells of cells, the first 3 x 3 x 3 among them (rows of up to nine cells: two blocks)
+constexpr int kHgKnnBlockRings = 8;  // shells of blocks after that
 
-struct HgKnnParams
-{
-    float inv_h, h;
-    int box[6];  // ordered-int images of min x, y, z and max x, y, z
-    int pad[8];
-};
+// The cell width of a segment, from up to 2048 of its points: around 32 of them the others within R and
+// R / 2 are counted, R the radius that would hold eight of a uniform cloud in the box.  The two counts give
+// the dimension of the cloud (2 for surfaces), and with it the radius that holds k of all points; the width
+// is their geometric mean.  From the volume of the box alone a scan of rooms, which is surfaces, had 200
+// candidates around a query, and scenes with fewer points than the average a second shell or the scan.
+// (0.85 and 1.2 times that width: kNN of 64 scenes 14 and 6 % slower, of 20 small ones 12 and 10 %.)
+constexpr int kHgWidthThreads = 512;
+constexpr int kHgWidthPoints = 2048;
+constexpr int kHgWidthQueries = 32;  // two per warp
 
 __device__ __forceinline__ int hg_ordered(float v)
 {
@@ -346,93 +516,130 @@ __device__ __forceinline__ int hg_ordered(float v)
 }
 __device__ __forceinline__ float hg_unordered(int o) { return __int_as_float(o >= 0 ? o : o ^ 0x7FFFFFFF); }
 
-__global__ void hg_knn_init_kernel(HgKnnParams* prm)
+__global__ void __launch_bounds__(kHgWidthThreads)
+    hg_width_kernel(HgSpace sp, int k, const float* __restrict__ x, const int64_t* __restrict__ batch_x, HgSeg* segs)
 {
-    if (threadIdx.x < 3) prm->box[threadIdx.x] = INT_MAX;
-    if (threadIdx.x >= 3 && threadIdx.x < 6) prm->box[threadIdx.x] = INT_MIN;
-}
-
-__global__ void __launch_bounds__(kHgThreads)
-    hg_knn_bbox_kernel(long long size_x, const float* __restrict__ x, HgKnnParams* prm)
-{
-    __shared__ float s_lo[3][kHgWarps], s_hi[3][kHgWarps];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    float lo[3] = {CUDART_INF_F, CUDART_INF_F, CUDART_INF_F};
-    float hi[3] = {-CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F};
-    for (long long k = static_cast<long long>(blockIdx.x) * kHgThreads + threadIdx.x; k < size_x;
-         k += static_cast<long long>(gridDim.x) * kHgThreads)
+    __shared__ float4 s_p[kHgWidthPoints];
+    __shared__ int s_box[6];
+    __shared__ int s_near[2][kHgWidthQueries];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    // segments to look at; the last entry is that of all ids without a range of their own
+    long long count = sp.cap;
+    bool mixed = false;
+    if (batch_x != nullptr)
     {
-        const float p[3] = {__ldg(x + 3 * k + 0), __ldg(x + 3 * k + 1), __ldg(x + 3 * k + 2)};
-        if (!hg_finite(p[0], p[1], p[2])) continue;
+        mixed = __ldg(&sp.head->mixed) != 0;
+        if (!mixed) count = min(count, static_cast<long long>(__ldg(batch_x + sp.size_x - 1)) + 1);
+    }
+    for (long long s = blockIdx.x; s < count + (mixed ? 1 : 0); s += gridDim.x)
+    {
+        uint32_t start = 0, end = sp.size_x;
+        if (batch_x == nullptr)
+        {
+            start = static_cast<uint32_t>(s) * sp.per_cloud;
+            end = start + sp.per_cloud;
+        }
+        else if (s < count)
+        {
+            start = segs[s].start;
+            end = segs[s].end;
+        }
+        if (end <= start) continue;
+        const uint32_t len = end - start, taken = min(len, static_cast<uint32_t>(kHgWidthPoints));
+        __syncthreads();  // the last segment's values have been read
+        if (tid < 6) s_box[tid] = tid < 3 ? INT_MAX : INT_MIN;
+        __syncthreads();
+        int lo[3] = {INT_MAX, INT_MAX, INT_MAX}, hi[3] = {INT_MIN, INT_MIN, INT_MIN};
+#pragma unroll
+        for (int u = 0; u < kHgWidthPoints / kHgWidthThreads; ++u)
+        {
+            const uint32_t i = u * kHgWidthThreads + tid;
+            const bool in = i < taken;
+            const size_t at = start + static_cast<uint32_t>(static_cast<unsigned long long>(in ? i : 0) * len / taken);
+            const float v[3] = {__ldg(x + 3 * at), __ldg(x + 3 * at + 1), __ldg(x + 3 * at + 2)};
+            const bool use = in && hg_finite(v[0], v[1], v[2]);
+#pragma unroll
+            for (int a = 0; a < 3; ++a)
+            {
+                if (use) lo[a] = min(lo[a], hg_ordered(v[a]));
+                if (use) hi[a] = max(hi[a], hg_ordered(v[a]));
+            }
+            s_p[i] = use ? make_float4(v[0], v[1], v[2], 0.f) : make_float4(CUDART_INF_F, CUDART_INF_F, CUDART_INF_F, 0.f);
+        }
 #pragma unroll
         for (int a = 0; a < 3; ++a)
         {
-            lo[a] = fminf(lo[a], p[a]);
-            hi[a] = fmaxf(hi[a], p[a]);
+            const int l = __reduce_min_sync(kFullMask, lo[a]), h = __reduce_max_sync(kFullMask, hi[a]);
+            if (lane == 0)
+            {
+                atomicMin(&s_box[a], l);
+                atomicMax(&s_box[3 + a], h);
+            }
         }
-    }
+        __syncthreads();
+        float ext[3], longest = 0.f, volume = 1.f;
 #pragma unroll
-    for (int a = 0; a < 3; ++a)
-    {
+        for (int a = 0; a < 3; ++a)
+        {
+            ext[a] = s_box[a] <= s_box[3 + a] ? hg_unordered(s_box[3 + a]) - hg_unordered(s_box[a]) : 0.f;
+            longest = fmaxf(longest, ext[a]);
+        }
+        if (!(longest > 0.f) || !(longest < 1.0e18f)) longest = 1.0f;
 #pragma unroll
-        for (int o = 16; o >= 1; o >>= 1)
+        for (int a = 0; a < 3; ++a) volume *= fmaxf(ext[a], longest * 1.0e-3f);  // flat clouds still have a volume
+        const float radius = cbrtf(volume * (8.0f / 4.18879f) / static_cast<float>(taken)), r2 = radius * radius;
         {
-            lo[a] = fminf(lo[a], __shfl_xor_sync(kFullMask, lo[a], o));
-            hi[a] = fmaxf(hi[a], __shfl_xor_sync(kFullMask, hi[a], o));
+            // queries: points spread over the sample
+            const int q = warp * 2;
+            const float4 a = s_p[static_cast<uint32_t>(q) * taken / kHgWidthQueries], b = s_p[static_cast<uint32_t>(q + 1) * taken / kHgWidthQueries];
+            int wide_a = 0, close_a = 0, wide_b = 0, close_b = 0;
+#pragma unroll 4
+            for (int i = lane; i < static_cast<int>(taken); i += 32)
+            {
+                // (infinite coordinates give distances that are infinite or not a number: none is counted)
+                const float4 c = s_p[i];
+                const float da = sumsq_abc(c.x - a.x, c.y - a.y, c.z - a.z), db = sumsq_abc(c.x - b.x, c.y - b.y, c.z - b.z);
+                wide_a += da < r2 ? 1 : 0;
+                close_a += da < 0.25f * r2 ? 1 : 0;
+                wide_b += db < r2 ? 1 : 0;
+                close_b += db < 0.25f * r2 ? 1 : 0;
+            }
+            wide_a = __reduce_add_sync(kFullMask, wide_a);
+            close_a = __reduce_add_sync(kFullMask, close_a);
+            wide_b = __reduce_add_sync(kFullMask, wide_b);
+            close_b = __reduce_add_sync(kFullMask, close_b);
+            if (lane == 0)
+            {
+                s_near[0][q] = wide_a;
+                s_near[1][q] = close_a;
+                s_near[0][q + 1] = wide_b;
+                s_near[1][q + 1] = close_b;
+            }
         }
-        if (lane == 0)
+        __syncthreads();
+        if (warp == 0)
         {
-            s_lo[a][warp] = lo[a];
-            s_hi[a][warp] = hi[a];
-        }
-    }
-    __syncthreads();
-    if (threadIdx.x < 3)
-    {
-        float l = s_lo[threadIdx.x][0], h = s_hi[threadIdx.x][0];
-        for (int w = 1; w < kHgWarps; ++w)
-        {
-            l = fminf(l, s_lo[threadIdx.x][w]);
-            h = fmaxf(h, s_hi[threadIdx.x][w]);
-        }
-        if (l <= h)
-        {
-            atomicMin(&prm->box[threadIdx.x], hg_ordered(l));
-            atomicMax(&prm->box[3 + threadIdx.x], hg_ordered(h));
+            const int wide = s_near[0][lane], close = s_near[1][lane];  // (0: no point of the sample)
+            const int all_wide = __reduce_add_sync(kFullMask, max(wide - 1, 0)), all_close = __reduce_add_sync(kFullMask, max(close - 1, 0));
+            const float dim = all_close >= 8 ? fminf(fmaxf(log2f(static_cast<float>(all_wide) / static_cast<float>(all_close)), 1.2f), 3.0f) : 3.0f;
+            // log of the radius that holds k points around this one
+            const float held = fmaxf(static_cast<float>(wide - 1), 0.5f) * static_cast<float>(len) / static_cast<float>(taken);
+            float log_r = wide > 0 ? log2f(static_cast<float>(k) / held) / dim : 0.f;
+            const int used = __popc(__ballot_sync(kFullMask, wide > 0));
+#pragma unroll
+            for (int o = 16; o >= 1; o >>= 1) log_r += __shfl_xor_sync(kFullMask, log_r, o);
+            const float by_volume = cbrtf(volume * static_cast<float>(k > 8 ? k : 8) * 0.25f / static_cast<float>(len));
+            float h = used > 0 ? radius * exp2f(log_r / static_cast<float>(used)) : by_volume;
+            h = fminf(fmaxf(h, 0.05f * by_volume), 1.5f * by_volume);
+            h = fminf(fmaxf(h, longest * 1.0e-5f), longest);
+            if (lane == 0)
+            {
+                segs[s].h = h;
+                segs[s].inv_h = 1.0f / h;
+            }
         }
     }
 }
-
-// Cell width from the mean density of a segment inside the common bounding box (segments of
-// a packed batch usually share their coordinate range; where they do not, cells come out
-// wider than needed, which costs candidates, not correctness).
-__global__ void hg_knn_params_kernel(long long size_x, long long nclouds, int k, const int64_t* __restrict__ batch_x,
-                                     HgKnnParams* prm)
-{
-    if (threadIdx.x != 0) return;
-    float ext[3], longest = 0.f;
-    for (int a = 0; a < 3; ++a)
-    {
-        ext[a] = prm->box[a] <= prm->box[3 + a] ? hg_unordered(prm->box[3 + a]) - hg_unordered(prm->box[a]) : 0.f;
-        longest = fmaxf(longest, ext[a]);
-    }
-    if (!(longest > 0.f) || !(longest < 1.0e18f)) longest = 1.0f;
-    float volume = 1.f;
-    for (int a = 0; a < 3; ++a) volume *= fmaxf(ext[a], longest * 1.0e-3f);  // flat clouds still have a volume
-    const long long nseg = batch_x ? __ldg(batch_x + size_x - 1) + 1 : nclouds;
-    const float per_seg = static_cast<float>(size_x) / static_cast<float>(nseg > 0 ? nseg : 1);
-    const float per_cell = static_cast<float>(k > 8 ? k : 8) * 0.25f;
-    float h = cbrtf(volume * per_cell / fmaxf(per_seg, 1.f));
-    h = fminf(fmaxf(h, longest * 1.0e-5f), longest);
-    prm->h = h;
-    prm->inv_h = 1.0f / h;
-}
-
-struct HgKnnWarpScratch
-{
-    int run_shift[32];  // slot of candidate v of run r = run_shift[r] + v
-    int run_cell[32];   // the run's cell, packed relative to the query's cell
-};
 
 // Sorted list of the best candidates, slot s in lane s & 31 (d0/i0: slots 0..31, d1/i1: 32..63).
 // Inserts (nd, ni), the same in all lanes, dropping the last slot.
@@ -513,123 +720,179 @@ __device__ __forceinline__ void hg_knn_merge(float d, int i, int lane, float& d0
     i0 = static_cast<int>(static_cast<uint32_t>(key));
 }
 
+// (five CTAs an SM: 64 registers without the bound, 1.5 to 7 % slower)
 template <bool DENSE, bool K32>
-__global__ void __launch_bounds__(kHgThreads)
-    hg_knn_kernel(long long size_q, long long per_cloud_s, long long per_cloud_q, int k, const HgKnnParams* __restrict__ prm,
-                  uint32_t mask, const float* __restrict__ query, const int64_t* __restrict__ batch_q,
-                  const int* __restrict__ counts, const float4* __restrict__ sorted, const int* __restrict__ sorted_seg,
-                  int64_t* __restrict__ idx_out, float* __restrict__ dist_out, unsigned char* __restrict__ need)
+__global__ void __launch_bounds__(kHgThreads, 5)
+    hg_knn_kernel(HgSpace sp, uint32_t size_q, uint32_t per_cloud_q, int k, const float* __restrict__ query,
+                  const int64_t* __restrict__ batch_s, const int64_t* __restrict__ batch_q, const int* __restrict__ counts,
+                  const int* __restrict__ ends, const float4* __restrict__ sorted, int64_t* __restrict__ idx_out,
+                  float* __restrict__ dist_out, unsigned char* __restrict__ need)
 {
-    __shared__ HgKnnWarpScratch s_scr[kHgWarps];
+    __shared__ int2 s_run[kHgWarps][32];  // slot of candidate v of run r = x + v; y: its place, see `examine`
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    HgKnnWarpScratch& ws = s_scr[warp];
-    const float inv_h = __ldg(&prm->inv_h), h = __ldg(&prm->h);
-    const long long nwarps_total = static_cast<long long>(gridDim.x) * kHgWarps;
-    for (long long j = static_cast<long long>(blockIdx.x) * kHgWarps + warp; j < size_q; j += nwarps_total)
+    int2* runs = s_run[warp];
+    const bool mixed = !DENSE && __ldg(&sp.head->mixed) != 0;
+    const uint32_t nwarps_total = gridDim.x * kHgWarps;
+    for (uint32_t j = blockIdx.x * kHgWarps + warp; j < size_q; j += nwarps_total)
     {
         // the query is the same in all lanes: everything outside the candidate loop is warp-uniform
-        const float qx = __ldg(query + 3 * j + 0), qy = __ldg(query + 3 * j + 1), qz = __ldg(query + 3 * j + 2);
+        const float* qp = query + 3 * static_cast<size_t>(j);
+        const float qx = __ldg(qp + 0), qy = __ldg(qp + 1), qz = __ldg(qp + 2);
+        const long long seg = DENSE ? j / per_cloud_q : __ldg(batch_q + j);
+        const HgSeg e = hg_seg(sp, seg);
+        const HgRange range = DENSE ? hg_cloud_range<1>(sp, static_cast<uint32_t>(seg), 0) : hg_seg_range(sp, seg, e);
+        const float inv_h = e.inv_h, h = e.h;
         const int cx = hg_cell(qx, inv_h), cy = hg_cell(qy, inv_h), cz = hg_cell(qz, inv_h);
-        if (!hg_finite(qx, qy, qz) || abs(cx) >= kHgCoordLimit - 8 || abs(cy) >= kHgCoordLimit - 8 ||
-            abs(cz) >= kHgCoordLimit - 8)
+        const int far = kHgCoordLimit - 128;  // beyond all that the shells of blocks reach
+        if (!hg_finite(qx, qy, qz) || abs(cx) >= far || abs(cy) >= far || abs(cz) >= far ||
+            (!DENSE && !mixed && e.end - e.start < k))
         {
             if (lane == 0) need[j] = 1;
             continue;
         }
-        const long long seg = DENSE ? j / per_cloud_q : __ldg(batch_q + j);
+        const float slack = (fabsf(qx) + fabsf(qy) + fabsf(qz) + h) * 2.0e-6f;  // of the coordinates of cell faces
         float d0 = CUDART_INF_F, d1 = CUDART_INF_F;  // empty slots: (+inf, INT_MAX)
         int i0 = INT_MAX, i1 = INT_MAX;
         float kd = CUDART_INF_F;  // the k-th best so far
         int ki = INT_MAX;
-        bool done = false;
-        for (int ring = 0; ring <= kHgKnnMaxRing && !done; ++ring)
-        {
-            // ring 0: the 3 x 3 x 3 block; ring r >= 1: the shell of cells at Chebyshev distance r + 1
-            const int rad = ring + 1, side = 2 * rad + 1;
-            const int ncell = side * side * side;
-            for (int t0 = 0; t0 < ncell; t0 += 32)
+        // The runs of all lanes: a candidate counts where its own cell, in units of 2^sx, 2^sy, 2^sy cells,
+        // lies `oy`, `oz` and `ox` to `ox + span` from the query's, and in its own segment.
+        auto examine = [&](int2 run, int ox, int oy, int oz, int span, int sx, int sy) {
+            const int incl = hg_inclusive(run.y, lane);
+            const int total = __shfl_sync(kFullMask, incl, 31);
+            if (total == 0) return;
+            __syncwarp();  // earlier reads of the scratch are done
+            runs[lane] = make_int2(run.x - (incl - run.y), (oy + 16) | (oz + 16) << 6 | (ox + 16) << 12 | span << 18);
+            __syncwarp();
+            for (int v0 = 0; v0 < total; v0 += 32)
             {
-                int t = t0 + lane;
-                if (ring == 0) t = lane == 0 ? 13 : (lane <= 13 ? lane - 1 : lane);  // the query's own cell first
-                const int ox = t % side - rad, oy = (t / side) % side - rad, oz = t / (side * side) - rad;
-                const bool shell = t < ncell && (ring == 0 || max(max(abs(ox), abs(oy)), abs(oz)) == rad);
-                int beg = 0, len = 0;
-                if (shell)
+                const int v = v0 + lane;
+                const bool valid = v < total;
+                const int2 r = runs[hg_run_of(incl, v)];
+                const float4 c = __ldg(sorted + (valid ? r.x + v : 0));
+                const float d = sumsq_unfused(qx - c.x, qy - c.y, qz - c.z);
+                const int ci = __float_as_int(c.w);
+                bool want = valid && d < CUDART_INF_F && (d < kd || (d == kd && ci < ki));
+                if (want)
                 {
-                    const uint32_t bkt = hg_bucket(seg, cx + ox, cy + oy, cz + oz, mask);
-                    beg = __ldg(counts + bkt);
-                    len = __ldg(counts + bkt + 1) - beg;
+                    want = (hg_cell(c.y, inv_h) >> sy) == (cy >> sy) + (r.y & 63) - 16 &&
+                           (hg_cell(c.z, inv_h) >> sy) == (cz >> sy) + ((r.y >> 6) & 63) - 16 &&
+                           static_cast<uint32_t>((hg_cell(c.x, inv_h) >> sx) - ((cx >> sx) + ((r.y >> 12) & 63) - 16)) <=
+                               static_cast<uint32_t>(r.y >> 18);
+                    if (mixed && want) want = __ldg(batch_s + ci) == seg;
                 }
-                int incl = len;
-#pragma unroll
-                for (int o = 1; o < 32; o <<= 1)
+                uint32_t bal = __ballot_sync(kFullMask, want);
+                if (K32 && __popc(bal) >= kHgKnnMergeFrom)
                 {
-                    const int v = __shfl_up_sync(kFullMask, incl, o);
-                    if (lane >= o) incl += v;
+                    hg_knn_merge(want ? d : CUDART_INF_F, want ? ci : INT_MAX, lane, d0, i0);
+                    kd = __shfl_sync(kFullMask, d0, k - 1);
+                    ki = __shfl_sync(kFullMask, i0, k - 1);
+                    continue;
                 }
-                const int total = __shfl_sync(kFullMask, incl, 31);
-                if (total == 0) continue;
-                __syncwarp();  // earlier reads of the scratch are done
-                ws.run_shift[lane] = beg - (incl - len);
-                ws.run_cell[lane] = ((ox + 8) << 8) | ((oy + 8) << 4) | (oz + 8);
-                __syncwarp();
-                for (int v0 = 0; v0 < total; v0 += 32)
+                while (bal != 0u)
                 {
-                    const int v = v0 + lane;
-                    const bool valid = v < total;
-                    const int r = hg_run_of(incl, v);
-                    const int p = valid ? ws.run_shift[r] + v : 0;
-                    const float4 c = __ldg(sorted + p);
-                    const float d = sumsq_unfused(qx - c.x, qy - c.y, qz - c.z);
-                    const int ci = __float_as_int(c.w);
-                    bool want = valid && d < CUDART_INF_F && (d < kd || (d == kd && ci < ki));
-                    if (want)
+                    const int src = __ffs(bal) - 1;
+                    bal &= bal - 1u;
+                    const float nd = __shfl_sync(kFullMask, d, src);
+                    const int ni = __shfl_sync(kFullMask, ci, src);
+                    if (nd < kd || (nd == kd && ni < ki))
                     {
-                        // a candidate counts in the bucket of its own cell and segment only
-                        const int rc = ws.run_cell[r];
-                        want = __ldg(sorted_seg + p) == static_cast<int>(seg) &&
-                               hg_cell(c.x, inv_h) == cx + ((rc >> 8) & 15) - 8 &&
-                               hg_cell(c.y, inv_h) == cy + ((rc >> 4) & 15) - 8 && hg_cell(c.z, inv_h) == cz + (rc & 15) - 8;
-                    }
-                    uint32_t bal = __ballot_sync(kFullMask, want);
-                    if (K32 && __popc(bal) >= kHgKnnMergeFrom)
-                    {
-                        hg_knn_merge(want ? d : CUDART_INF_F, want ? ci : INT_MAX, lane, d0, i0);
-                        kd = __shfl_sync(kFullMask, d0, k - 1);
-                        ki = __shfl_sync(kFullMask, i0, k - 1);
-                        continue;
-                    }
-                    while (bal != 0u)
-                    {
-                        const int src = __ffs(bal) - 1;
-                        bal &= bal - 1u;
-                        const float nd = __shfl_sync(kFullMask, d, src);
-                        const int ni = __shfl_sync(kFullMask, ci, src);
-                        if (nd < kd || (nd == kd && ni < ki))
-                        {
-                            hg_knn_insert<K32>(nd, ni, lane, d0, i0, d1, i1);
-                            const int ks = k - 1;
-                            kd = __shfl_sync(kFullMask, (K32 || ks < 32) ? d0 : d1, ks & 31);
-                            ki = __shfl_sync(kFullMask, (K32 || ks < 32) ? i0 : i1, ks & 31);
-                        }
+                        hg_knn_insert<K32>(nd, ni, lane, d0, i0, d1, i1);
+                        const int ks = k - 1;
+                        kd = __shfl_sync(kFullMask, (K32 || ks < 32) ? d0 : d1, ks & 31);
+                        ki = __shfl_sync(kFullMask, (K32 || ks < 32) ? i0 : i1, ks & 31);
                     }
                 }
             }
-            // every point closer than the nearest face of the searched block has been seen
-            const float fx = fminf(qx - static_cast<float>(cx - rad) * h, static_cast<float>(cx + rad + 1) * h - qx);
-            const float fy = fminf(qy - static_cast<float>(cy - rad) * h, static_cast<float>(cy + rad + 1) * h - qy);
-            const float fz = fminf(qz - static_cast<float>(cz - rad) * h, static_cast<float>(cz + rad + 1) * h - qz);
-            const float reach = fminf(fminf(fx, fy), fz) * 0.9999f - (fabsf(qx) + fabsf(qy) + fabsf(qz) + h) * 2.0e-6f;
+        };
+        // what lies between the query and the cells [c, c + 1) of an axis, in units of w: no more than that far away
+        auto gap = [&](int c, float q, float w) {
+            const float below = static_cast<float>(c) * w - q, above = q - static_cast<float>(c + 1) * w;
+            return fmaxf(fmaxf(below, above) * 0.9999f - slack, 0.f);
+        };
+        // all points closer than this have been seen once the cells [c - rad, c + rad] of every axis have
+        auto reach_of = [&](int c, float q, float w, int rad) {
+            return fminf(q - static_cast<float>(c - rad) * w, static_cast<float>(c + rad + 1) * w - q) * 0.9999f - slack;
+        };
+        bool done = false;
+        for (int rad = 1; rad <= kHgKnnRings && !done; ++rad)
+        {
+            // rad 1: the 3 x 3 x 3 block; above: the shell of cells at Chebyshev distance rad.  A row of cells
+            // along x is two runs, one in each of at most two blocks; of an inner row of a shell only the two
+            // end cells are looked at.
+            const int side = 2 * rad + 1, tasks = 2 * side * side;
+            for (int t0 = 0; t0 < tasks; t0 += 32)
+            {
+                const int t = t0 + lane, second = t & 1;
+                int row = t >> 1;
+                if (rad == 1) row = row == 0 ? 4 : (row <= 4 ? row - 1 : row);  // the query's own row first
+                const int oz = row / side - rad, oy = row - (oz + rad) * side - rad;
+                int xa = cx - rad, xb = cx + rad;
+                bool any = t < tasks && range.count != 0u;
+                if (rad == 1 || max(abs(oy), abs(oz)) == rad)
+                {
+                    any &= !second || (xa >> 3) != (xb >> 3);
+                    if (second)
+                        xa = xb & ~7;
+                    else
+                        xb = min(xb, xa | 7);
+                }
+                else if (second)
+                    xa = xb;
+                else
+                    xb = xa;
+                int2 run = make_int2(0, 0);
+                if (any)
+                {
+                    // a row no nearer than the k-th best has nothing to offer
+                    const float gy = gap(cy + oy, qy, h), gz = gap(cz + oz, qz, h);
+                    if (gy * gy + gz * gz <= kd) run = hg_run(range, counts, ends, xa, xb, cy + oy, cz + oz);
+                }
+                examine(run, xa - cx, oy, oz, xb - xa, 0, 0);
+            }
+            const float reach = fminf(fminf(reach_of(cx, qx, h, rad), reach_of(cy, qy, h, rad)), reach_of(cz, qz, h, rad));
             done = reach > 0.f && kd <= reach * reach;
+        }
+        if (!done)
+        {
+            // A thin place: whole blocks of 8 x 4 x 4 cells, from the beginning (their points are one run each),
+            // but for what is farther than the k-th best so far.
+            const float bound = kd;
+            d0 = d1 = kd = CUDART_INF_F;
+            i0 = i1 = ki = INT_MAX;
+            const int bx = cx >> 3, by = cy >> 2, bz = cz >> 2;
+            for (int rad = 1; rad <= kHgKnnBlockRings && !done; ++rad)
+            {
+                const int side = 2 * rad + 1, tasks = side * side * side;
+                for (int t0 = 0; t0 < tasks; t0 += 32)
+                {
+                    const int t = t0 + lane;
+                    const int oz = t / (side * side) - rad, oy = (t / side) % side - rad, ox = t % side - rad;
+                    int2 run = make_int2(0, 0);
+                    if (t < tasks && range.count != 0u && (rad == 1 || max(max(abs(ox), abs(oy)), abs(oz)) == rad))
+                    {
+                        const float gx = gap(bx + ox, qx, 8.0f * h), gy = gap(by + oy, qy, 4.0f * h), gz = gap(bz + oz, qz, 4.0f * h);
+                        if (gx * gx + gy * gy + gz * gz <= fminf(bound, kd))
+                        {
+                            const uint32_t block = hg_block(range, bx + ox, by + oy, bz + oz);
+                            run.x = __ldg(counts + static_cast<size_t>(block) * kHgBlock);
+                            run.y = __ldg(ends + block) - run.x;
+                        }
+                    }
+                    examine(run, ox, oy, oz, 0, 3, 2);
+                }
+                const float reach = fminf(fminf(reach_of(bx, qx, 8.0f * h, rad), reach_of(by, qy, 4.0f * h, rad)), reach_of(bz, qz, 4.0f * h, rad));
+                done = reach > 0.f && kd <= reach * reach;
+            }
         }
         if (!done)
         {
             if (lane == 0) need[j] = 1;
             continue;
         }
-        const long long base = DENSE ? seg * per_cloud_s : 0;  // dense indices are local to the cloud
-        int64_t* orow = idx_out + j * k;
-        float* drow = dist_out + j * k;
+        const long long base = DENSE ? seg * sp.per_cloud : 0;  // dense indices are local to the cloud
+        int64_t* orow = idx_out + static_cast<size_t>(j) * k;
+        float* drow = dist_out + static_cast<size_t>(j) * k;
         if (lane < k)
         {
             orow[lane] = static_cast<int64_t>(i0) - base;
@@ -640,108 +903,127 @@ __global__ void __launch_bounds__(kHgThreads)
             orow[lane + 32] = static_cast<int64_t>(i1) - base;
             drow[lane + 32] = d1;
         }
-        if (lane == 0) need[j] = 0;
     }
 }
 
+// ------------------------------------------------------------------------------- host side
+
 size_t hg_round(size_t v) { return (v + 255) / 256 * 256; }
 
-uint32_t hg_buckets(long long size_x)
+// Segments with a range of their own: enough for the ids of any batch of scenes, few enough not to cost
+// counters (a block each).  Others share the whole space.
+uint32_t hg_cap(long long size_x)
 {
-    uint32_t h = 1024;
-    // A query's 27 buckets hold as many strangers as there are points per bucket, times 27: with twice
-    // as many points as buckets most of its candidates were strangers (244345 points, ball query 233 us
-    // against 209, kNN 585 against 568; 114163: 84 and 77, 391 and 384; 7.0 M: the same).
-    while (h < (1u << 30) && static_cast<long long>(h) < size_x) h <<= 1;
-    return h;  // a power of two, at least size_x
+    const long long c = size_x / 64;
+    return static_cast<uint32_t>(c < 256 ? 256 : (c > 65536 ? 65536 : c));
+}
+
+struct HgPlan
+{
+    HgSpace sp;
+    HgHead* head;
+    HgSeg* segs;
+    int *counts, *ends;
+    float4* sorted;
+    unsigned char* need;
+    size_t zeroed, bytes;
+};
+
+// Layout of the scratch: what is zeroed first (head, segments, counters, block ends, flags), then the sorted
+// points.  clouds: 0 for the packed layout; parts: of a dense cloud.
+HgPlan hg_plan(long long size_x, long long size_y, long long clouds, int parts, void* scratch)
+{
+    HgPlan p = {};
+    p.sp.size_x = static_cast<uint32_t>(size_x);
+    p.sp.per_cloud = clouds > 0 ? static_cast<uint32_t>(size_x / clouds) : 0u;
+    p.sp.cap = clouds > 0 ? static_cast<uint32_t>(clouds) : hg_cap(size_x);
+    p.sp.blocks = static_cast<uint32_t>((size_x >> kHgBlockPoints) + static_cast<long long>(p.sp.cap) * parts + 1);
+    unsigned char* at = static_cast<unsigned char*>(scratch);
+    size_t used = 0;
+    auto take = [&](size_t bytes) {
+        unsigned char* q = at + used;
+        used += hg_round(bytes);
+        return q;
+    };
+    p.head = reinterpret_cast<HgHead*>(take(sizeof(HgHead)));
+    p.segs = reinterpret_cast<HgSeg*>(take((static_cast<size_t>(p.sp.cap) + 1) * sizeof(HgSeg)));
+    p.counts = reinterpret_cast<int*>(take(static_cast<size_t>(p.sp.blocks) * kHgBlock * sizeof(int)));
+    p.ends = reinterpret_cast<int*>(take(static_cast<size_t>(p.sp.blocks) * sizeof(int)));
+    p.need = take(static_cast<size_t>(size_y));
+    p.zeroed = used;
+    p.sorted = reinterpret_cast<float4*>(take(static_cast<size_t>(size_x) * sizeof(float4)));
+    p.bytes = used;
+    p.sp.segs = p.segs;
+    p.sp.head = p.head;
+    return p;
+}
+
+constexpr int kHgParts = 3;  // of a dense cloud in a ball query
+
+// Everything up to the sorted copy.  WIDTHS: kNN, which measures its cell widths.
+template <bool DENSE, int PARTS, bool WIDTHS>
+int hg_build(const HgPlan& p, int k, const float* x, const int64_t* batch_x, cudaStream_t s, const char* what)
+{
+    cudaError_t err = cudaMemsetAsync(p.head, 0, p.zeroed, s);
+    if (err != cudaSuccess)
+    {
+        set_error("%s: memset: %s", what, cudaGetErrorString(err));
+        return TPK_ERR_CUDA;
+    }
+    const unsigned gp = (p.sp.size_x + kHgThreads - 1) / kHgThreads;
+    if (!DENSE) count_launches(1), hg_bounds_kernel<<<(gp + 3) / 4, kHgThreads, 0, s>>>(p.sp.size_x, p.sp.cap, batch_x, p.head, p.segs);
+    if (WIDTHS)
+    {
+        const unsigned g = p.sp.cap < 4u * num_sms() ? p.sp.cap : 4u * num_sms();
+        count_launches(1), hg_width_kernel<<<g, kHgWidthThreads, 0, s>>>(p.sp, k, x, batch_x, p.segs);
+    }
+    count_launches(1), hg_bin_kernel<DENSE, PARTS, WIDTHS, false><<<gp, kHgThreads, 0, s>>>(p.sp, x, batch_x, p.counts, p.sorted);
+    const unsigned gb = (p.sp.blocks + 4 * kHgWarps - 1) / (4 * kHgWarps);
+    count_launches(1), hg_place_kernel<<<gb, kHgThreads, 0, s>>>(p.sp.blocks, p.head, p.counts, p.ends);
+    count_launches(1), hg_bin_kernel<DENSE, PARTS, WIDTHS, true><<<gp, kHgThreads, 0, s>>>(p.sp, x, batch_x, p.counts, p.sorted);
+    return check_launch(what);
+}
+
+unsigned hg_query_grid(long long size_q)
+{
+    const long long g = (size_q + kHgWarps - 1) / kHgWarps, cap = 32ll * num_sms();
+    return static_cast<unsigned>(g < cap ? g : cap);
 }
 
 }  // namespace
 
-// Whether the hashed grid serves a packed problem (indices must fit 31 bits, one int per segment id).
+// Whether the hashed grid serves a problem (indices must fit 31 bits).
 bool hash_grid_fits(long long size_x, long long size_y)
 {
-    return size_x >= 4096 && size_x < (1ll << 31) && size_y > 0;
+    return size_x >= 4096 && size_x < (1ll << 31) && size_y > 0 && size_y < (1ll << 31);
 }
 
-size_t hash_grid_scratch_bytes(long long size_x, long long size_y)
+// clouds: 0 for the packed layout
+size_t hash_grid_scratch_bytes(long long size_x, long long size_y, long long clouds)
 {
-    const size_t h = hg_buckets(size_x);
-    return hg_round((h + 1) * sizeof(int)) + hg_round(((h + 1 + 1023) / 1024) * sizeof(int)) +
-           hg_round(static_cast<size_t>(size_x) * sizeof(float4)) + hg_round(static_cast<size_t>(size_x) * sizeof(int)) +
-           hg_round(static_cast<size_t>(size_y));
+    return hg_plan(size_x, size_y, clouds, clouds > 0 ? kHgParts : 1, nullptr).bytes;
 }
 
 // Answers the queries the grid is good for; *need_out: one byte per query, 1 = left to the scan.
-// Packed layout: batch_x / batch_y give the segments.  Dense layout (both NULL): size_x = b * n,
-// size_y = b * m, per_cloud_x = n, per_cloud_y = m.
-static int hash_grid_run(long long size_x, long long size_y, long long per_cloud_x, long long per_cloud_y, float radius,
-                         int nsample, const float* x, const float* y, const int64_t* batch_x, const int64_t* batch_y,
-                         int64_t* idx, float* dist, void* scratch, const unsigned char** need_out, cudaStream_t s)
-{
-    const uint32_t h = hg_buckets(size_x);
-    const uint32_t mask = h - 1u;
-    const long long ncount = static_cast<long long>(h) + 1;
-    const int nblocks = static_cast<int>((ncount + 1023) / 1024);
-    unsigned char* p = static_cast<unsigned char*>(scratch);
-    int* counts = reinterpret_cast<int*>(p);
-    p += hg_round((static_cast<size_t>(h) + 1) * sizeof(int));
-    int* totals = reinterpret_cast<int*>(p);
-    p += hg_round(static_cast<size_t>(nblocks) * sizeof(int));
-    float4* sorted = reinterpret_cast<float4*>(p);
-    p += hg_round(static_cast<size_t>(size_x) * sizeof(float4));
-    int* sorted_seg = reinterpret_cast<int*>(p);
-    p += hg_round(static_cast<size_t>(size_x) * sizeof(int));
-    unsigned char* need = p;
-
-    // cells a shade wider than the radius: the ball never reaches past the neighbouring cells
-    const float inv_h = 1.0f / (radius * 1.0001f);
-    cudaError_t err = cudaMemsetAsync(counts, 0, (static_cast<size_t>(h) + 1) * sizeof(int), s);
-    if (err != cudaSuccess)
-    {
-        set_error("ball_query hash grid: memset: %s", cudaGetErrorString(err));
-        return TPK_ERR_CUDA;
-    }
-    const unsigned gp = static_cast<unsigned>((size_x + kHgThreads - 1) / kHgThreads);
-    count_launches(1), hg_bin_kernel<false><<<gp, kHgThreads, 0, s>>>(size_x, per_cloud_x, inv_h, nullptr, mask, x, batch_x, counts, sorted, sorted_seg);
-    count_launches(1), hg_scan_blocks_kernel<<<nblocks, 1024, 0, s>>>(counts, ncount, totals);
-    count_launches(1), hg_scan_totals_kernel<<<1, 1024, 0, s>>>(totals, nblocks);
-    count_launches(1), hg_scan_add_kernel<<<nblocks, 1024, 0, s>>>(counts, ncount, totals);
-    count_launches(1), hg_bin_kernel<true><<<gp, kHgThreads, 0, s>>>(size_x, per_cloud_x, inv_h, nullptr, mask, x, batch_x, counts, sorted, sorted_seg);
-    // Above this many candidates around a query the scan, which stops at the nsample-th hit, is cheaper.
-    // Not earlier: in clouds of this size a scan reads the points from L2.  8 x 1048576 points: 3.7 ms;
-    // from 1800 candidates on, the bound of the grids in shared memory, 8.0 (packed segments have no
-    // common size to derive it from).
-    int max_cand = 16384;
-    if (batch_y == nullptr)
-    {
-        const double v = 2.0 * sqrt(6.45 * static_cast<double>(per_cloud_x) * nsample);
-        max_cand = v < 4096.0 ? 4096 : (v > 1.0e6 ? 1000000 : static_cast<int>(v));
-    }
-    long long gq = (size_y + kHgWarps - 1) / kHgWarps;
-    const long long cap = 32ll * num_sms();
-    if (gq > cap) gq = cap;
-    if (batch_y == nullptr)
-    {
-        prefer_max_shared(hg_query_kernel<true>);
-        count_launches(1), hg_query_kernel<true><<<static_cast<unsigned>(gq), kHgThreads, 0, s>>>(
-            size_y, per_cloud_x, per_cloud_y, radius, nsample, max_cand, inv_h, mask, y, batch_y, counts, sorted, sorted_seg, idx, dist, need);
-    }
-    else
-    {
-        prefer_max_shared(hg_query_kernel<false>);
-        count_launches(1), hg_query_kernel<false><<<static_cast<unsigned>(gq), kHgThreads, 0, s>>>(
-            size_y, per_cloud_x, per_cloud_y, radius, nsample, max_cand, inv_h, mask, y, batch_y, counts, sorted, sorted_seg, idx, dist, need);
-    }
-    *need_out = need;
-    return check_launch("ball_query hash grid");
-}
-
+// Packed layout: batch_x / batch_y give the segments.
 int hash_grid_ball_query(long long size_x, long long size_y, float radius, int nsample, const float* x, const float* y,
                          const int64_t* batch_x, const int64_t* batch_y, int64_t* idx, float* dist, void* scratch,
                          const unsigned char** need_out, cudaStream_t s)
 {
-    return hash_grid_run(size_x, size_y, 1, 1, radius, nsample, x, y, batch_x, batch_y, idx, dist, scratch, need_out, s);
+    HgPlan p = hg_plan(size_x, size_y, 0, 1, scratch);
+    // cells a shade wider than the radius: the ball never reaches past the neighbouring cells
+    p.sp.inv_h = 1.0f / (radius * 1.0001f);
+    const int rc = hg_build<false, 1, false>(p, 0, x, batch_x, s, "ball_query hash grid");
+    if (rc != TPK_OK) return rc;
+    // above this many candidates around a query the scan, which stops at the nsample-th hit, is cheaper
+    const int max_cand = 16384;
+    auto kernel = hg_query_kernel<false, 1>;
+    prefer_max_shared(kernel);
+    const size_t smem = static_cast<size_t>(kHgWarps) * 8 * hg_hits(nsample);
+    count_launches(1), kernel<<<hg_query_grid(size_y), kHgThreads, smem, s>>>(
+        p.sp, static_cast<uint32_t>(size_y), 1u, radius, nsample, max_cand, y, batch_x, batch_y, p.counts, p.ends, p.sorted, idx, dist, p.need);
+    *need_out = p.need;
+    return check_launch("ball_query hash grid");
 }
 
 // Dense clouds (b, n, 3) / centres (b, m, 3) on the hashed grid (for clouds too large for the
@@ -749,14 +1031,29 @@ int hash_grid_ball_query(long long size_x, long long size_y, float radius, int n
 int hash_grid_ball_query_dense(int b, int n, int m, float radius, int nsample, const float* new_xyz, const float* xyz,
                                int64_t* idx, float* dist, void* scratch, const unsigned char** need_out, cudaStream_t s)
 {
-    return hash_grid_run(static_cast<long long>(b) * n, static_cast<long long>(b) * m, n, m, radius, nsample, xyz, new_xyz,
-                         nullptr, nullptr, idx, dist, scratch, need_out, s);
+    const long long size_x = static_cast<long long>(b) * n, size_y = static_cast<long long>(b) * m;
+    HgPlan p = hg_plan(size_x, size_y, b, kHgParts, scratch);
+    p.sp.inv_h = 1.0f / (radius * 1.0001f);
+    const int rc = hg_build<true, kHgParts, false>(p, 0, xyz, nullptr, s, "ball_query hash grid");
+    if (rc != TPK_OK) return rc;
+    // Above this many candidates in a part of the cloud the scan is cheaper.  Not earlier: in clouds of this
+    // size a scan reads the points from L2.
+    const double v = 2.0 * sqrt(6.45 * static_cast<double>(n) * nsample);
+    const int max_cand = v < 4096.0 ? 4096 : (v > 1.0e6 ? 1000000 : static_cast<int>(v));
+    auto kernel = hg_query_kernel<true, kHgParts>;
+    prefer_max_shared(kernel);
+    const size_t smem = static_cast<size_t>(kHgWarps) * 8 * hg_hits(nsample);
+    count_launches(1), kernel<<<hg_query_grid(size_y), kHgThreads, smem, s>>>(
+        p.sp, static_cast<uint32_t>(size_y), static_cast<uint32_t>(m), radius, nsample, max_cand, new_xyz, nullptr, nullptr, p.counts,
+        p.ends, p.sorted, idx, dist, p.need);
+    *need_out = p.need;
+    return check_launch("ball_query hash grid");
 }
 
-// ---- kNN on the hashed grid: scratch = parameters, then the ball query's layout
-size_t hash_grid_knn_scratch_bytes(long long size_s, long long size_q)
+// clouds: 0 for the packed layout
+size_t hash_grid_knn_scratch_bytes(long long size_s, long long size_q, long long clouds)
 {
-    return 256 + hash_grid_scratch_bytes(size_s, size_q);
+    return hg_plan(size_s, size_q, clouds, 1, nullptr).bytes;
 }
 
 // Answers the queries the grid is good for; *need_out: one byte per query, 1 = left to the scan.
@@ -766,52 +1063,18 @@ int hash_grid_knn(long long size_s, long long size_q, long long per_cloud_s, lon
                   const float* support, const float* query, const int64_t* batch_s, const int64_t* batch_q, int64_t* idx,
                   float* dist2, void* scratch, const unsigned char** need_out, cudaStream_t s)
 {
-    const uint32_t h = hg_buckets(size_s);
-    const uint32_t mask = h - 1u;
-    const long long ncount = static_cast<long long>(h) + 1;
-    const int nblocks = static_cast<int>((ncount + 1023) / 1024);
-    unsigned char* p = static_cast<unsigned char*>(scratch);
-    HgKnnParams* prm = reinterpret_cast<HgKnnParams*>(p);
-    p += 256;
-    int* counts = reinterpret_cast<int*>(p);
-    p += hg_round((static_cast<size_t>(h) + 1) * sizeof(int));
-    int* totals = reinterpret_cast<int*>(p);
-    p += hg_round(static_cast<size_t>(nblocks) * sizeof(int));
-    float4* sorted = reinterpret_cast<float4*>(p);
-    p += hg_round(static_cast<size_t>(size_s) * sizeof(float4));
-    int* sorted_seg = reinterpret_cast<int*>(p);
-    p += hg_round(static_cast<size_t>(size_s) * sizeof(int));
-    unsigned char* need = p;
-
-    cudaError_t err = cudaMemsetAsync(counts, 0, (static_cast<size_t>(h) + 1) * sizeof(int), s);
-    if (err != cudaSuccess)
-    {
-        set_error("knn hash grid: memset: %s", cudaGetErrorString(err));
-        return TPK_ERR_CUDA;
-    }
-    const unsigned gp = static_cast<unsigned>((size_s + kHgThreads - 1) / kHgThreads);
-    long long gb = (size_s + 8ll * kHgThreads - 1) / (8ll * kHgThreads);
-    if (gb > 8ll * num_sms()) gb = 8ll * num_sms();
-    const long long nclouds = per_cloud_s > 0 ? size_s / per_cloud_s : 1;
-    count_launches(3);
-    hg_knn_init_kernel<<<1, 32, 0, s>>>(prm);
-    hg_knn_bbox_kernel<<<static_cast<unsigned>(gb), kHgThreads, 0, s>>>(size_s, support, prm);
-    hg_knn_params_kernel<<<1, 32, 0, s>>>(size_s, nclouds, k, batch_s, prm);
-    count_launches(1), hg_bin_kernel<false><<<gp, kHgThreads, 0, s>>>(size_s, per_cloud_s, 0.f, &prm->inv_h, mask, support, batch_s, counts, sorted, sorted_seg);
-    count_launches(1), hg_scan_blocks_kernel<<<nblocks, 1024, 0, s>>>(counts, ncount, totals);
-    count_launches(1), hg_scan_totals_kernel<<<1, 1024, 0, s>>>(totals, nblocks);
-    count_launches(1), hg_scan_add_kernel<<<nblocks, 1024, 0, s>>>(counts, ncount, totals);
-    count_launches(1), hg_bin_kernel<true><<<gp, kHgThreads, 0, s>>>(size_s, per_cloud_s, 0.f, &prm->inv_h, mask, support, batch_s, counts, sorted, sorted_seg);
-    long long gq = (size_q + kHgWarps - 1) / kHgWarps;
-    const long long cap = 32ll * num_sms();
-    if (gq > cap) gq = cap;
-    const unsigned g = static_cast<unsigned>(gq);
+    const bool dense = batch_q == nullptr;
+    const HgPlan p = hg_plan(size_s, size_q, dense ? size_s / per_cloud_s : 0, 1, scratch);
+    const int rc = dense ? hg_build<true, 1, true>(p, k, support, nullptr, s, "knn hash grid")
+                         : hg_build<false, 1, true>(p, k, support, batch_s, s, "knn hash grid");
+    if (rc != TPK_OK) return rc;
+    const unsigned g = hg_query_grid(size_q);
     count_launches(1);
 #define TPK_HG_KNN(DENSE, K32)                                                                                          \
     prefer_max_shared(hg_knn_kernel<DENSE, K32>),                                                                       \
-        hg_knn_kernel<DENSE, K32><<<g, kHgThreads, 0, s>>>(size_q, per_cloud_s, per_cloud_q, k, prm, mask, query, batch_q, \
-                                                           counts, sorted, sorted_seg, idx, dist2, need)
-    if (batch_q == nullptr)
+        hg_knn_kernel<DENSE, K32><<<g, kHgThreads, 0, s>>>(p.sp, static_cast<uint32_t>(size_q), static_cast<uint32_t>(per_cloud_q), \
+                                                           k, query, batch_s, batch_q, p.counts, p.ends, p.sorted, idx, dist2, p.need)
+    if (dense)
     {
         if (k <= 32)
             TPK_HG_KNN(true, true);
@@ -826,7 +1089,7 @@ int hash_grid_knn(long long size_s, long long size_q, long long per_cloud_s, lon
             TPK_HG_KNN(false, false);
     }
 #undef TPK_HG_KNN
-    *need_out = need;
+    *need_out = p.need;
     return check_launch("knn hash grid");
 }
 

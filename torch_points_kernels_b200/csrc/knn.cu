@@ -470,7 +470,7 @@ namespace tpk
 {
 // hash_grid.cu
 bool hash_grid_fits(long long size_x, long long size_y);
-size_t hash_grid_knn_scratch_bytes(long long size_s, long long size_q);
+size_t hash_grid_knn_scratch_bytes(long long size_s, long long size_q, long long clouds);
 int hash_grid_knn(long long size_s, long long size_q, long long per_cloud_s, long long per_cloud_q, int k,
                   const float* support, const float* query, const int64_t* batch_s, const int64_t* batch_q, int64_t* idx,
                   float* dist2, void* scratch, const unsigned char** need_out, cudaStream_t s);
@@ -517,7 +517,7 @@ static bool knn_dense_wants_grid(int b, int n, int m)
 extern "C" int64_t tpk_knn_dense_scratch_bytes(int b, int n, int m, int k)
 {
     if (b <= 0 || n <= 0 || m <= 0 || k <= 0 || !knn_dense_wants_grid(b, n, m)) return 0;
-    return static_cast<int64_t>(tpk::hash_grid_knn_scratch_bytes(static_cast<long long>(b) * n, static_cast<long long>(b) * m));
+    return static_cast<int64_t>(tpk::hash_grid_knn_scratch_bytes(static_cast<long long>(b) * n, static_cast<long long>(b) * m, b));
 }
 
 extern "C" int tpk_knn_dense_ws(int b, int n, int m, int k, const float* support, const float* query, int64_t* idx,
@@ -583,7 +583,7 @@ static bool knn_partial_wants_grid(int64_t size_s, int64_t size_q)
 extern "C" int64_t tpk_knn_partial_dense_scratch_bytes(int64_t size_s, int64_t size_q, int k)
 {
     if (k <= 0 || !knn_partial_wants_grid(size_s, size_q)) return 0;
-    return static_cast<int64_t>(tpk::hash_grid_knn_scratch_bytes(size_s, size_q));
+    return static_cast<int64_t>(tpk::hash_grid_knn_scratch_bytes(size_s, size_q, 0));
 }
 
 extern "C" int tpk_knn_partial_dense_ws(int64_t size_s, int64_t size_q, int k, const float* support,
