@@ -201,6 +201,9 @@ TPK_API int tpk_three_nn(int b, int n, int m, const float* unknown, const float*
 TPK_API int tpk_three_nn_ws(int b, int n, int m, const float* unknown, const float* known, float* dist2,
                             int32_t* idx, void* scratch, int64_t scratch_bytes, void* stream);
 TPK_API int64_t tpk_three_nn_scratch_bytes(int b, int n, int m);
+/* With this much scratch (0: sizes where the kernels above are ahead) tpk_three_nn_ws sorts both clouds by cells of
+ * a grid first and searches the sorted copies; the results are the same. */
+TPK_API int64_t tpk_three_nn_sorted_scratch_bytes(int b, int n, int m);
 
 /*
  * k nearest support points per query.  support (b,n,3), query (b,m,3) ->
@@ -381,6 +384,9 @@ TPK_API int tpk_chamfer_dist_f32_ws(int b, int n, const float* xyz1, int m, cons
                                     float* dist2, int32_t* idx1, int32_t* idx2, void* scratch,
                                     int64_t scratch_bytes, void* stream);
 TPK_API int64_t tpk_chamfer_dist_scratch_bytes(int b, int n, int m);
+/* With this much scratch (0: sizes where the kernels above are ahead) tpk_chamfer_dist_f32_ws sorts both clouds by
+ * cells of a grid first and searches the sorted copies; the results are the same. */
+TPK_API int64_t tpk_chamfer_dist_sorted_scratch_bytes(int b, int n, int m);
 
 /*
  * Gradient of both directions w.r.t. both clouds; grad_xyz1 (b,n,3) and grad_xyz2

@@ -1020,6 +1020,51 @@ def test_grouping_backward_sorted_path(B, C, N, P, S, kind):
     assert _lib.device_status() == 0
 
 
+@pytest.mark.parametrize("kind", ["ball", "surface", "plane", "one_place", "padded", "far_point", "nonfinite", "huge"])
+@pytest.mark.parametrize("b,n,m", [(1, 1, 1), (2, 5, 2), (1, 33, 700), (3, 1000, 1500), (20, 2100, 300), (40, 600, 1025),
+                                   (2, 9001, 4097), (1, 20000, 16385)])
+def test_nearest_neighbours_on_sorted_copies(b, n, m, kind, monkeypatch):
+    """Chamfer and three_nn on the grids of sorted points against the scans, bit for bit: one to eight CTAs a cloud,
+    one to four lanes a query, and clouds whose queries are left over, few of them (a warp each) and many (tiles)."""
+    g = data.gen(n + m)
+    x, y = torch.randn(b, n, 3, generator=g), torch.randn(b, m, 3, generator=g)
+    if kind == "surface":
+        x, y = x / x.norm(dim=2, keepdim=True), y / y.norm(dim=2, keepdim=True) + 0.01 * torch.randn(b, m, 3, generator=g)
+    elif kind == "plane":
+        x[..., 2], y[..., 2] = 0.5, 0.5
+    elif kind == "one_place":
+        y[:] = y[:, :1]
+    elif kind == "padded":
+        x[:, n // 2:], y[:, m // 3:] = 0.0, 0.0
+    elif kind == "far_point":
+        y[:, m // 2] *= 1e4
+        x[:, n // 3] = 1e6
+    elif kind == "nonfinite":
+        y[:, m // 2, 1], y[:, m // 3, 0] = float("nan"), float("inf")
+        x[:, n // 2, 2], x[:, n // 3, 0] = float("nan"), float("-inf")
+    elif kind == "huge":
+        x, y = x * 3e18, y * 3e18
+        y[:, 0] = 3e38
+    got = []
+    for path in (("nn_sorted",), ("chamfer_scan", "three_nn_scan")):
+        data.use_paths(monkeypatch, *path)
+        one = cd.ChamferFunction.apply(cu(x), cu(y))
+        idx = one[0].new_zeros(0)
+        got.append(list(one) + (list(tpk.three_nn(cu(x), cu(y))) if n >= 3 else [idx]))
+        i1, i2 = (torch.empty((b, k), dtype=torch.int32, device="cuda") for k in (n, m))
+        d1, d2 = torch.empty((b, n), device="cuda"), torch.empty((b, m), device="cuda")
+        handle = _lib.lib()
+        need = handle.tpk_chamfer_dist_sorted_scratch_bytes(b, n, m)
+        assert (need > 0) == (path[0] == "nn_sorted")
+        scratch = torch.empty(max(need, 1), dtype=torch.uint8, device="cuda")
+        a, c = cu(x), cu(y)
+        _lib.call("tpk_chamfer_dist_f32_ws", b, n, _lib.ptr(a), m, _lib.ptr(c), _lib.ptr(d1), _lib.ptr(d2), _lib.ptr(i1),
+                  _lib.ptr(i2), _lib.ptr(scratch) if need else None, need, _lib.stream_of(a))
+        got[-1] += [i1, i2]
+    for a, c in zip(*got):
+        assert torch.equal(a, c)
+
+
 @pytest.mark.parametrize("case", ["ids", "thin", "one_place", "tiny_segments"])
 @pytest.mark.parametrize("k", [1, 20, 40])
 def test_packed_searches_on_ranges_of_blocks(case, k, monkeypatch):

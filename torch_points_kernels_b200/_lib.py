@@ -73,7 +73,8 @@ EXPORTS = sorted(list(_SIGNATURES) + ["tpk_version", "tpk_last_error", "tpk_devi
                                        "tpk_ball_query_partial_dense_scratch_bytes", "tpk_knn_dense_scratch_bytes", "tpk_sa_group_scratch_bytes",
                                        "tpk_knn_partial_dense_scratch_bytes", "tpk_cubic_feature_sampling_scratch_bytes",
                                        "tpk_grouping_grad_scratch_bytes", "tpk_grouping_grad_cols_scratch_bytes",
-                                       "tpk_three_interpolate_grad_cols_scratch_bytes"])
+                                       "tpk_three_interpolate_grad_cols_scratch_bytes",
+                                       "tpk_three_nn_sorted_scratch_bytes", "tpk_chamfer_dist_sorted_scratch_bytes"])
 
 
 def lib():
@@ -105,6 +106,9 @@ def lib():
         handle.tpk_ball_query_partial_dense_scratch_bytes.restype = _c_i64
         handle.tpk_chamfer_dist_scratch_bytes.argtypes = [_c_int, _c_int, _c_int]
         handle.tpk_chamfer_dist_scratch_bytes.restype = _c_i64
+        for name in ("tpk_three_nn_sorted_scratch_bytes", "tpk_chamfer_dist_sorted_scratch_bytes"):
+            getattr(handle, name).argtypes = [_c_int, _c_int, _c_int]
+            getattr(handle, name).restype = _c_i64
         handle.tpk_three_nn_scratch_bytes.argtypes = [_c_int, _c_int, _c_int]
         handle.tpk_three_nn_scratch_bytes.restype = _c_i64
         handle.tpk_knn_dense_scratch_bytes.argtypes = [_c_int, _c_int, _c_int, _c_int]

@@ -23,7 +23,11 @@ class ChamferFunction(torch.autograd.Function):
         idx2 = torch.empty((b, m), dtype=torch.int32, device=xyz1.device)
         name = "tpk_chamfer_dist_f32" if xyz1.dtype == torch.float32 else "tpk_chamfer_dist_f64"
         with _lib.on_device(xyz1):
-            need = _lib.lib().tpk_chamfer_dist_scratch_bytes(b, n, m) if xyz1.dtype == torch.float32 else 0
+            need = 0
+            if xyz1.dtype == torch.float32:
+                # grids over sorted copies, or else one flag per point for the grids without
+                handle = _lib.lib()
+                need = handle.tpk_chamfer_dist_sorted_scratch_bytes(b, n, m) or handle.tpk_chamfer_dist_scratch_bytes(b, n, m)
             if need > 0:
                 # large clouds: nearest neighbours on a uniform grid (same results as the all-pairs scan)
                 scratch = torch.empty((need,), dtype=torch.uint8, device=xyz1.device)

@@ -29,35 +29,13 @@ int sg_nn(int k, int b, int n, int m, const float* unknown, const float* known, 
 bool sg_nn_slab_fits(int b, int n, int m);
 int sg_nn_slab(int k, int b, int n, int m, const float* unknown, const float* known, float* dist2, int32_t* idx,
                unsigned char* need, cudaStream_t s);
+// nn_grid.cu
+size_t nn_grid_scratch_bytes(int b, int n, int m, bool both);
+int nn_grid_both(int b, int n, int m, const float* xyz1, const float* xyz2, float* dist1, int32_t* idx1, float* dist2, int32_t* idx2,
+                 void* scratch, cudaStream_t s);
 
 namespace
 {
-
-template <int Q>
-struct ArgMinOp
-{
-    float qx[Q], qy[Q], qz[Q];
-    float best[Q];
-    int besti[Q];
-    bool act[Q];
-
-    __device__ __forceinline__ float threshold(int q) const { return act[q] ? best[q] : -CUDART_INF_F; }
-    __device__ __forceinline__ bool finished() const
-    {
-        bool done = true;
-#pragma unroll
-        for (int q = 0; q < Q; ++q) done &= !act[q];
-        return done;
-    }
-    __device__ __forceinline__ bool exact(int q, long long k, float cx, float cy, float cz)
-    {
-        const float d = sumsq_abc(cx - qx[q], cy - qy[q], cz - qz[q]);
-        if (!act[q] || !(d < best[q])) return false;
-        best[q] = d;
-        besti[q] = static_cast<int>(k);
-        return true;
-    }
-};
 
 template <int THREADS, int Q>
 __global__ void __launch_bounds__(THREADS)
@@ -315,11 +293,25 @@ static int chamfer_dir_grid(int b, int queries, const float* q, int known, const
     return tpk::grid_nn(1, b, queries, known, q, c, dist, idx, scratch, need, s);
 }
 
+extern "C" int64_t tpk_chamfer_dist_sorted_scratch_bytes(int b, int n, int m)
+{
+    if (tpk::test_path("chamfer_scan") || tpk::test_path("nn_global_grid") || tpk::test_path("nn_unsorted")) return 0;
+    return static_cast<int64_t>(tpk::nn_grid_scratch_bytes(b, n, m, true));
+}
+
 extern "C" int tpk_chamfer_dist_f32_ws(int b, int n, const float* xyz1, int m, const float* xyz2,
                                        float* dist1, float* dist2, int32_t* idx1, int32_t* idx2,
                                        void* scratch, int64_t scratch_bytes, void* stream)
 {
     using namespace tpk;
+    // scratch for the sorted copies: both directions on grids over them
+    const int64_t sorted = tpk_chamfer_dist_sorted_scratch_bytes(b, n, m);
+    if (sorted > 0 && scratch != nullptr && scratch_bytes >= sorted)
+    {
+        TPK_REQUIRE(xyz1 && xyz2 && dist1 && dist2 && idx1 && idx2, "chamfer_dist: NULL pointer");
+        TPK_REQUIRE((reinterpret_cast<uintptr_t>(scratch) & 255u) == 0, "chamfer_dist: scratch must be 256-byte aligned");
+        return nn_grid_both(b, n, m, xyz1, xyz2, dist1, idx1, dist2, idx2, scratch, static_cast<cudaStream_t>(stream));
+    }
     const int64_t want = tpk_chamfer_dist_scratch_bytes(b, n, m);
     if (want == 0 || scratch == nullptr)
         return tpk_chamfer_dist_f32(b, n, xyz1, m, xyz2, dist1, dist2, idx1, idx2, stream);

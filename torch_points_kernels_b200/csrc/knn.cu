@@ -19,46 +19,6 @@ namespace tpk
 namespace
 {
 
-template <int Q>
-struct ThreeNnOp
-{
-    float qx[Q], qy[Q], qz[Q];
-    float b1[Q], b2[Q], b3[Q];
-    int i1[Q], i2[Q], i3[Q];
-    bool act[Q];
-
-    __device__ __forceinline__ float threshold(int q) const { return act[q] ? b3[q] : -CUDART_INF_F; }
-    __device__ __forceinline__ bool finished() const
-    {
-        bool done = true;
-#pragma unroll
-        for (int q = 0; q < Q; ++q) done &= !act[q];
-        return done;
-    }
-    __device__ __forceinline__ bool exact(int q, long long k, float cx, float cy, float cz)
-    {
-        const float v = sumsq_abc(qx[q] - cx, qy[q] - cy, qz[q] - cz);
-        if (!act[q] || !(v < b3[q])) return false;
-        const int kk = static_cast<int>(k);
-        if (v < b1[q])
-        {
-            b3[q] = b2[q]; i3[q] = i2[q];
-            b2[q] = b1[q]; i2[q] = i1[q];
-            b1[q] = v;     i1[q] = kk;
-        }
-        else if (v < b2[q])
-        {
-            b3[q] = b2[q]; i3[q] = i2[q];
-            b2[q] = v;     i2[q] = kk;
-        }
-        else
-        {
-            b3[q] = v; i3[q] = kk;
-        }
-        return true;
-    }
-};
-
 template <int THREADS, int Q>
 __global__ void __launch_bounds__(THREADS)
     three_nn_kernel(int n, int m, int tiles_per_cloud, const float* __restrict__ unknown,
@@ -404,11 +364,33 @@ extern "C" int64_t tpk_three_nn_scratch_bytes(int b, int n, int m)
     return static_cast<int64_t>(tpk::grid_three_nn_scratch_bytes(b, n, m));
 }
 
+namespace tpk
+{
+// nn_grid.cu
+size_t nn_grid_scratch_bytes(int b, int n, int m, bool both);
+int nn_grid_three(int b, int n, int m, const float* unknown, const float* known, float* dist2, int32_t* idx, void* scratch,
+                  cudaStream_t s);
+}  // namespace tpk
+
+extern "C" int64_t tpk_three_nn_sorted_scratch_bytes(int b, int n, int m)
+{
+    if (tpk::test_path("three_nn_scan") || tpk::test_path("three_nn_global_grid") || tpk::test_path("nn_unsorted")) return 0;
+    return static_cast<int64_t>(tpk::nn_grid_scratch_bytes(b, n, m, false));
+}
+
 extern "C" int tpk_three_nn_ws(int b, int n, int m, const float* unknown, const float* known,
                                float* dist2, int32_t* idx, void* scratch, int64_t scratch_bytes,
                                void* stream)
 {
     using namespace tpk;
+    // scratch for the sorted copies: the grids over them
+    const int64_t sorted = tpk_three_nn_sorted_scratch_bytes(b, n, m);
+    if (sorted > 0 && scratch != nullptr && scratch_bytes >= sorted)
+    {
+        TPK_REQUIRE(unknown && known && dist2 && idx, "three_nn: NULL pointer");
+        TPK_REQUIRE((reinterpret_cast<uintptr_t>(scratch) & 255u) == 0, "three_nn: scratch must be 256-byte aligned");
+        return nn_grid_three(b, n, m, unknown, known, dist2, idx, scratch, static_cast<cudaStream_t>(stream));
+    }
     const int64_t want = tpk_three_nn_scratch_bytes(b, n, m);
     if (want == 0 || scratch == nullptr) return tpk_three_nn(b, n, m, unknown, known, dist2, idx, stream);
     if (scratch_bytes < want)

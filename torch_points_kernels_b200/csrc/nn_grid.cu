@@ -1,0 +1,840 @@
+// Nearest neighbours (three_nn: the three nearest; Chamfer: the nearest) on a uniform grid of sorted points
+// (sm_100a).
+//
+//   nn_sort_kernel  : a cluster per cloud sorts its points by cells of a grid over it (counting sort, counters in
+//                     shared memory) and leaves the sorted copy, the first slot of every cell and the grid's
+//                     geometry in scratch;
+//   nn_query_kernel : G lanes per query.  The 2 x 2 x 2 cells whose common corner is nearest first, four runs of
+//                     the sorted copy that the G lanes share out, then whatever cells the ball of the K-th
+//                     best distance touches besides.
+//   nn_scan_kernel  : the queries that were left over, mostly none: those with too many candidates or too few
+//
+// The queries come from the sorted copy of their own cloud, so that the lanes of a warp look at the same
+// cells, which lie in L1.  The grids of smem_grid.cu need no scratch, but every CTA of a cloud bins all its
+// points again (66 of 120 k cycles of a CTA for 16384 points), and a thread walks 27 cells and rings of more
+// with some 150 candidates; here the eight cells whose common corner is nearest hold 40, and the rest are looked
+// at as far as the best distance reaches.  The sort is bound by the stores of one SM and the latency of its
+// passes (chamfer of 32 x 16384 points: 30 us for the 64 clouds), the search by the issue of instructions (62).
+//
+// The cells are sized by the population that a point meets in its own cell: clouds are surfaces more often than
+// not, and cells sized by the volume then hold several times as many points.
+//
+// Results are those of the scans bit for bit: the reference's arithmetic (cuda/src/interpolate_gpu.cu:12-60,
+// cuda/src/chamfer_dist_gpu.cu:8-155), candidates ordered by (distance, index), index 0 where there is none.
+// Points that are not finite are in no cell: no distance to them is smaller than another.
+#include <climits>
+#include <type_traits>
+#include <math_constants.h>
+
+#include <cooperative_groups.h>
+
+#include "scan.cuh"
+
+namespace cg = cooperative_groups;
+
+namespace tpk
+{
+namespace
+{
+
+constexpr int kNnSortThreads = 1024;  // at most
+constexpr int kNnMaxCells = 40960;   // 160 KB of counters
+constexpr int kNnQueryThreads = 128;
+constexpr int kNnMaxPoints = 65536;  // per cloud
+constexpr int kNnBudget = 768;       // candidates, and
+constexpr int kNnMaxRows = 144;      // rows of cells that a query looks at before it is left to the scan
+
+struct NnGrid
+{
+    float minx, miny, minz, inv_h, h;
+    int dx, dy, dz;
+    int left;  // number of queries of this cloud left to the scan
+};
+
+// One side of a call: clouds of n points, their sorted copies, cells and grids.
+struct NnSide
+{
+    const float* xyz;
+    float4* sorted;   // n per cloud; the first `count` are points
+    int* cells;       // cap + 1 per cloud
+    NnGrid* grids;
+    int n, cap;
+    int* places;      // n per cloud: the cell of every point, -1: none; then the queries left to the scan
+    float per_cell;   // points that a cell should hold on average
+    bool searched;    // (else only the order of the points matters)
+};
+
+__device__ __forceinline__ bool nn_finite(float x, float y, float z)
+{
+    return fabsf(x) < CUDART_INF_F && fabsf(y) < CUDART_INF_F && fabsf(z) < CUDART_INF_F;
+}
+
+// The cell of a coordinate, monotone in v: the same function bins points and bounds a query's range of cells.
+// (Rounded by adding 1.5 * 2^23: floorf and the conversion go to a unit with a quarter of the lanes, which
+// was most of a pass over the points.  A point at a face may go to either side.)
+__device__ __forceinline__ int nn_cell(float v, float mn, float inv_h, int d)
+{
+    const float t = fminf(fmaxf(__fmaf_rn(__fsub_rn(v, mn), inv_h, -0.5f), 0.f), static_cast<float>(d - 1));
+    return __float_as_int(__fadd_rn(t, 12582912.0f)) - 0x4B400000;
+}
+
+__device__ __forceinline__ int nn_ordered(float v)
+{
+    const int b = __float_as_int(v);
+    return b >= 0 ? b : b ^ 0x7FFFFFFF;
+}
+__device__ __forceinline__ float nn_unordered(int o) { return __int_as_float(o >= 0 ? o : o ^ 0x7FFFFFFF); }
+
+// Calls f(k, x, y, z) for this thread's share of the points [begin, n), eight of them in flight.
+template <class F>
+__device__ __forceinline__ void nn_for_points(const float* __restrict__ xyz, int begin, int n, F&& f)
+{
+    constexpr int U = 8;
+    const int threads = blockDim.x;
+    for (int k0 = begin + threadIdx.x; k0 < n; k0 += U * threads)
+    {
+        float v[U][3];
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+        {
+            const int k = k0 + u * threads;
+#pragma unroll
+            for (int a = 0; a < 3; ++a) v[u][a] = k < n ? __ldg(xyz + 3 * static_cast<size_t>(k) + a) : 0.f;
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+            if (k0 + u * threads < n) f(k0 + u * threads, v[u][0], v[u][1], v[u][2]);
+    }
+}
+
+// atomicAdd(p, 1), once for all lanes where they meet at one counter (padded clouds)
+__device__ __forceinline__ int nn_add(int* p)
+{
+    const uint32_t active = __activemask();
+    const int lead = __ffs(active) - 1, lane = threadIdx.x & 31;
+    const unsigned long long mine = reinterpret_cast<unsigned long long>(p);
+    if (__all_sync(active, mine == __shfl_sync(active, mine, lead)))
+    {
+        int at = 0;
+        if (lane == lead) at = atomicAdd(p, __popc(active));
+        return __shfl_sync(active, at, lead) + __popc(active & ((1u << lane) - 1u));
+    }
+    return atomicAdd(p, 1);
+}
+
+// Cells of width h over the box, wider ones where they would be more than `cap`.
+__device__ __forceinline__ void nn_dims(NnGrid& g, const float (&ext)[3], float h, int cap)
+{
+    while (true)
+    {
+        const float inv = 1.0f / h;
+        const float nx = floorf(ext[0] * inv) + 1.f, ny = floorf(ext[1] * inv) + 1.f, nz = floorf(ext[2] * inv) + 1.f;
+        if (nx * ny * nz <= static_cast<float>(cap) && inv < CUDART_INF_F)
+        {
+            g.dx = static_cast<int>(nx);
+            g.dy = static_cast<int>(ny);
+            g.dz = static_cast<int>(nz);
+            g.h = h;
+            g.inv_h = inv;
+            return;
+        }
+        h *= 1.1f;
+    }
+}
+
+// A cluster of `ranks` CTAs per cloud, the clouds of side a, then those of side b.  A rank finds the cells of its
+// share of the points and leaves them in scratch, then counts and places those of its share of the cells, for
+// which it reads all of these numbers.  (With atomics on the counters of the other ranks eight of them were no
+// faster than one: a remote one takes an SM ten cycles.  One CTA alone spends 27 of its 57 k cycles for 16384
+// points on storing the sorted copy, 32 sectors a warp.)
+__global__ void __launch_bounds__(kNnSortThreads) nn_sort_kernel(NnSide a, NnSide b, int clouds, int ranks)
+{
+    extern __shared__ int s_cells[];
+    __shared__ int s_box[7], s_all[7], s_warp[32], s_rest, s_total;  // box: also the number of points
+    __shared__ float s_square;
+    const int rank = ranks > 1 ? static_cast<int>(cg::this_cluster().block_rank()) : 0;
+    const int job = blockIdx.x / ranks;
+    const bool second = job >= clouds;
+    const NnSide side = second ? b : a;
+    const int cloud = job - (second ? clouds : 0);
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, threads = blockDim.x, n = side.n;
+    const float* xyz = side.xyz + static_cast<size_t>(cloud) * n * 3;
+    float4* sorted = side.sorted + static_cast<size_t>(cloud) * n;
+    int* cells = side.cells + static_cast<size_t>(cloud) * (side.cap + 1);
+    int* places = side.places + static_cast<size_t>(cloud) * n;
+    const int k0 = static_cast<int>(static_cast<long long>(n) * rank / ranks), k1 = static_cast<int>(static_cast<long long>(n) * (rank + 1) / ranks);
+    auto sync = [&]() {
+        if (ranks > 1)
+            cg::this_cluster().sync();  // (what was written to global memory is visible to the other ranks, too)
+        else
+            __syncthreads();
+    };
+    auto at_rank = [&](auto* p, int r) { return ranks > 1 ? cg::this_cluster().map_shared_rank(p, static_cast<unsigned>(r)) : p; };
+
+    // ---- box
+    if (tid < 7) s_all[tid] = s_box[tid] = tid == 6 ? 0 : (tid < 3 ? INT_MAX : INT_MIN);
+    if (tid == 0) s_square = 0.f;
+    __syncthreads();
+    int lo[3] = {INT_MAX, INT_MAX, INT_MAX}, hi[3] = {INT_MIN, INT_MIN, INT_MIN}, used = 0;
+    nn_for_points(xyz, k0, k1, [&](int, float x, float y, float z) {
+        if (!nn_finite(x, y, z)) return;
+        const int o[3] = {nn_ordered(x), nn_ordered(y), nn_ordered(z)};
+        ++used;
+#pragma unroll
+        for (int i = 0; i < 3; ++i)
+        {
+            lo[i] = min(lo[i], o[i]);
+            hi[i] = max(hi[i], o[i]);
+        }
+    });
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+    {
+        const int l = __reduce_min_sync(kFullMask, lo[i]), h = __reduce_max_sync(kFullMask, hi[i]);
+        if (lane == 0)
+        {
+            atomicMin(&s_box[i], l);
+            atomicMax(&s_box[3 + i], h);
+        }
+    }
+    used = __reduce_add_sync(kFullMask, used);
+    if (lane == 0) atomicAdd(&s_box[6], used);
+    sync();
+    if (tid < 7 * ranks)
+    {
+        const int i = tid % 7, v = at_rank(s_box, tid / 7)[i];
+        if (i == 6)
+            atomicAdd(&s_all[6], v);
+        else if (i < 3)
+            atomicMin(&s_all[i], v);
+        else
+            atomicMax(&s_all[i], v);
+    }
+    __syncthreads();
+    const int points = s_all[6];
+    int box[6];
+#pragma unroll
+    for (int i = 0; i < 6; ++i) box[i] = s_all[i];
+    NnGrid g;
+    float ext[3], longest = 0.f, volume = 1.f;
+    g.minx = points ? nn_unordered(box[0]) : 0.f;
+    g.miny = points ? nn_unordered(box[1]) : 0.f;
+    g.left = 0;
+    g.minz = points ? nn_unordered(box[2]) : 0.f;
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+    {
+        ext[i] = points ? fminf(nn_unordered(box[3 + i]) - nn_unordered(box[i]), 1.0e37f) : 0.f;
+        longest = fmaxf(longest, ext[i]);
+    }
+    if (!(longest > 1.0e-30f)) longest = 1.0f;  // one place (or a box too small to divide): one cell
+#pragma unroll
+    for (int i = 0; i < 3; ++i) volume *= fmaxf(ext[i] / longest, 1.0e-2f);
+    nn_dims(g, ext, longest * cbrtf(volume * side.per_cell / static_cast<float>(max(points, 1))), side.cap);
+
+    // ---- points per cell, once more with smaller cells where they turn out to be crowded
+    int ncell, first, own;  // first: of this rank's own cells
+    const int4* places4 = reinterpret_cast<const int4*>(places);
+    const bool four = (reinterpret_cast<uintptr_t>(places) & 15u) == 0;
+    // calls f(k, place) for all points, four or sixteen of them in flight
+    auto for_places = [&](auto&& f) {
+        const int n4 = four ? n >> 2 : 0;
+        for (int i0 = tid; i0 < n4; i0 += 4 * threads)
+        {
+            int4 v[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+                v[u] = i0 + u * threads < n4 ? __ldcg(places4 + i0 + u * threads) : make_int4(-2, -2, -2, -2);
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+            {
+                const int k = 4 * (i0 + u * threads);
+                f(k, v[u].x);
+                f(k + 1, v[u].y);
+                f(k + 2, v[u].z);
+                f(k + 3, v[u].w);
+            }
+        }
+        for (int k = 4 * n4 + tid; k < n; k += threads) f(k, __ldcg(places + k));
+    };
+    for (int attempt = 0;; ++attempt)
+    {
+        ncell = g.dx * g.dy * g.dz;
+        const int share = (ncell + ranks - 1) / ranks;
+        first = min(rank * share, ncell);
+        own = min(share, ncell - first);
+        for (int c = tid; c < own; c += threads) s_cells[c] = 0;
+        nn_for_points(xyz, k0, k1, [&](int k, float x, float y, float z) {
+            const int c = (nn_cell(z, g.minz, g.inv_h, g.dz) * g.dy + nn_cell(y, g.miny, g.inv_h, g.dy)) * g.dx + nn_cell(x, g.minx, g.inv_h, g.dx);
+            __stcg(places + k, nn_finite(x, y, z) ? c : -1);
+        });
+        sync();
+        for_places([&](int, int c) {
+            if (static_cast<unsigned>(c - first) < static_cast<unsigned>(own)) (void)nn_add(&s_cells[c - first]);
+        });
+        __syncthreads();
+        if (attempt == 1 || !side.searched) break;
+        float square = 0.f;
+        for (int c = tid; c < own; c += threads) square += static_cast<float>(s_cells[c]) * static_cast<float>(s_cells[c]);
+#pragma unroll
+        for (int o = 16; o >= 1; o >>= 1) square += __shfl_xor_sync(kFullMask, square, o);
+        if (lane == 0 && square > 0.f) atomicAdd(&s_square, square);
+        sync();
+        // (every rank adds the sums in the same order: all decide alike)
+        square = 0.f;
+        for (int r = 0; r < ranks; ++r) square += *at_rank(&s_square, r);
+        // a point meets 1 + per_cell others where they are spread evenly over the box, twice that in a ball
+        const float met = square / static_cast<float>(max(points, 1)), want = 1.0f + side.per_cell;
+        if (!(met > 2.5f * want) || ncell >= side.cap / 2) break;
+        nn_dims(g, ext, g.h * fmaxf(sqrtf(want / met), 0.25f), side.cap);
+    }
+
+    // ---- first slots: every thread a run of this rank's cells
+    const int per = ((own + threads - 1) / threads) | 1;  // (odd: the threads start in different banks)
+    const int c0 = min(tid * per, own), c1 = min(c0 + per, own);
+    int sum = 0;
+    for (int c = c0; c < c1; ++c) sum += s_cells[c];
+    int incl = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1)
+    {
+        const int t = __shfl_up_sync(kFullMask, incl, o);
+        if (lane >= o) incl += t;
+    }
+    if (lane == 31) s_warp[warp] = incl;
+    __syncthreads();
+    if (warp == 0)
+    {
+        int w = lane < threads / 32 ? s_warp[lane] : 0;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1)
+        {
+            const int t = __shfl_up_sync(kFullMask, w, o);
+            if (lane >= o) w += t;
+        }
+        s_warp[lane] = w;
+        if (lane == 31) s_total = w;
+    }
+    if (tid == 0) s_rest = points;  // where points that are in no cell go: behind the others
+    sync();
+    int at = (warp ? s_warp[warp - 1] : 0) + incl - sum;
+    for (int r = 0; r < rank; ++r) at += *at_rank(&s_total, r);
+    for (int c = c0; c < c1; ++c)
+    {
+        const int v = s_cells[c];
+        s_cells[c] = at;
+        at += v;
+    }
+    __syncthreads();
+    for (int c = tid; c < own; c += threads) cells[first + c] = s_cells[c];
+    if (rank == 0 && tid == 0)
+    {
+        cells[ncell] = points;
+        side.grids[cloud] = g;
+    }
+    __syncthreads();
+
+    // ---- sorted copy
+    for_places([&](int k, int c) {
+        int* slot = static_cast<unsigned>(c - first) < static_cast<unsigned>(own) ? &s_cells[c - first] : (c == -1 && rank == 0 ? &s_rest : nullptr);
+        if (slot != nullptr)
+        {
+            const float* p = xyz + 3 * static_cast<size_t>(k);
+            sorted[nn_add(slot)] = make_float4(__ldg(p), __ldg(p + 1), __ldg(p + 2), __int_as_float(k));
+        }
+    });
+    sync();  // shared memory stays until every rank is done with it
+}
+
+// The K nearest so far, by (distance, index).
+template <int K>
+struct NnBest
+{
+    float d[K];
+    int i[K];
+
+    __device__ __forceinline__ void clear()
+    {
+#pragma unroll
+        for (int k = 0; k < K; ++k)
+        {
+            d[k] = CUDART_INF_F;
+            i[k] = INT_MAX;
+        }
+    }
+    __device__ __forceinline__ void take(float nd, int ni)
+    {
+#pragma unroll
+        for (int k = 0; k < K; ++k)
+        {
+            const bool less = nd < d[k] || (nd == d[k] && ni < i[k]);
+            const float od = d[k];
+            const int oi = i[k];
+            d[k] = less ? nd : od;
+            i[k] = less ? ni : oi;
+            nd = less ? od : nd;
+            ni = less ? oi : ni;
+        }
+    }
+};
+
+// G lanes per query; grid: blocks per cloud x (clouds of a against b, then of b against a where `both`).
+template <int K, int G>
+__global__ void __launch_bounds__(kNnQueryThreads)
+    nn_query_kernel(NnSide a, NnSide b, int clouds, int blocks_a, int blocks_b, float* __restrict__ dist_a, int32_t* __restrict__ idx_a,
+                    float* __restrict__ dist_b, int32_t* __restrict__ idx_b)
+{
+    long long block = blockIdx.x;
+    const bool second = block >= static_cast<long long>(clouds) * blocks_a;
+    if (second) block -= static_cast<long long>(clouds) * blocks_a;
+    const int blocks = second ? blocks_b : blocks_a;
+    const int cloud = static_cast<int>(block / blocks), part = static_cast<int>(block - static_cast<long long>(cloud) * blocks);
+    const NnSide& from = second ? b : a;
+    const NnSide& to = second ? a : b;
+    const int g = threadIdx.x & (G - 1);
+    const int qi = part * (kNnQueryThreads / G) + threadIdx.x / G;
+    const bool in = qi < from.n;
+    const NnGrid grid = to.grids[cloud];
+    const float4* sorted = to.sorted + static_cast<size_t>(cloud) * to.n;
+    const int* cells = to.cells + static_cast<size_t>(cloud) * (to.cap + 1);
+    const float4 q = __ldg(from.sorted + static_cast<size_t>(cloud) * from.n + (in ? qi : 0));
+    bool search = in && nn_finite(q.x, q.y, q.z), crowded = false;
+
+    NnBest<K> best;
+    best.clear();
+    float limit = CUDART_INF_F;  // what a candidate must not exceed: the K-th best of all lanes so far
+    auto scan = [&](int beg, int end) {
+        constexpr int U = G == 1 ? 4 : 2;
+        for (int p = beg + g; p < end; p += U * G)
+        {
+            // (what is read behind the run lies in the scratch and is not looked at)
+            float4 c[U];
+            float d[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u) c[u] = __ldg(sorted + p + u * G);
+#pragma unroll
+            for (int u = 0; u < U; ++u) d[u] = sumsq_abc(q.x - c[u].x, q.y - c[u].y, q.z - c[u].z);
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+            {
+                if constexpr (K == 1)
+                {
+                    // (nearly always some lane of a warp has a better one: no branch)
+                    const int i = __float_as_int(c[u].w);
+                    const bool less = p + u * G < end && (d[u] < best.d[0] || (d[u] == best.d[0] && i < best.i[0]));
+                    best.d[0] = less ? d[u] : best.d[0];
+                    best.i[0] = less ? i : best.i[0];
+                }
+                else if (d[u] <= fminf(limit, best.d[K - 1]) && p + u * G < end)
+                    best.take(d[u], __float_as_int(c[u].w));
+            }
+        }
+    };
+    // joins the lists of the G lanes; `limit` becomes the K-th best
+    auto join = [&]() {
+        if constexpr (G > 1)
+        {
+#pragma unroll
+            for (int o = G / 2; o >= 1; o >>= 1)
+            {
+                NnBest<K> other;
+#pragma unroll
+                for (int k = 0; k < K; ++k)
+                {
+                    other.d[k] = __shfl_xor_sync(kFullMask, best.d[k], o);
+                    other.i[k] = __shfl_xor_sync(kFullMask, best.i[k], o);
+                }
+#pragma unroll
+                for (int k = 0; k < K; ++k) best.take(other.d[k], other.i[k]);
+            }
+        }
+        limit = best.d[K - 1];
+    };
+    const int cx = nn_cell(q.x, grid.minx, grid.inv_h, grid.dx), cy = nn_cell(q.y, grid.miny, grid.inv_h, grid.dy),
+              cz = nn_cell(q.z, grid.minz, grid.inv_h, grid.dz);
+    // The cells seen so far: first the 2 x 2 x 2 whose common corner is nearest.
+    auto lower = [](float v, float mn, float h, int c) { return c - (v - (mn + static_cast<float>(c) * h) < 0.5f * h ? 1 : 0); };
+    int sx0 = lower(q.x, grid.minx, grid.h, cx), sy0 = lower(q.y, grid.miny, grid.h, cy), sz0 = lower(q.z, grid.minz, grid.h, cz);
+    int sx1 = min(sx0 + 1, grid.dx - 1), sy1 = min(sy0 + 1, grid.dy - 1), sz1 = min(sz0 + 1, grid.dz - 1);
+    sx0 = max(sx0, 0);
+    sy0 = max(sy0, 0);
+    sz0 = max(sz0, 0);
+    int budget = max(kNnBudget, to.n >> 4);  // candidates
+    {
+        int beg[4], end[4];
+#pragma unroll
+        for (int r = 0; r < 4; ++r)
+        {
+            const int y = sy0 + (r & 1), z = sz0 + (r >> 1);
+            const bool valid = search && y <= sy1 && z <= sz1;
+            const int* c = cells + (valid ? (z * grid.dy + y) * grid.dx : 0);
+            beg[r] = __ldg(c + sx0);
+            end[r] = valid ? __ldg(c + sx1 + 1) : 0;
+        }
+        // (a scan of the whole cloud takes a seventh of the instructions for a candidate)
+        int total = 0;
+#pragma unroll
+        for (int r = 0; r < 4; ++r) total += max(end[r] - beg[r], 0);
+        crowded = total > budget;
+        search = search && !crowded;
+        budget -= total;
+#pragma unroll
+        for (int r = 0; r < 4; ++r)
+            if (search) scan(beg[r], end[r]);
+    }
+    join();
+    // Further cells: the ones of [x0, x1] x [y0, y1] x [z0, z1] that have not been seen, rows no farther than the limit.
+    const float slack = (fabsf(q.x) + fabsf(q.y) + fabsf(q.z) + fabsf(grid.minx) + fabsf(grid.miny) + fabsf(grid.minz)) * 4.0e-7f + 1.0e-3f * grid.h;
+    auto widen = [&](int x0, int x1, int y0, int y1, int z0, int z1) {
+        auto run = [&](const int* c, int xa, int xb) {
+            const int beg = __ldg(c + xa), end = __ldg(c + xb + 1);
+            budget -= end - beg;
+            if (budget >= 0) scan(beg, end);
+        };
+        if ((y1 - y0 + 1) * (z1 - z0 + 1) > kNnMaxRows) budget = -1;
+        for (int z = z0; z <= z1 && budget >= 0; ++z)
+        {
+            const float bz = grid.minz + static_cast<float>(z) * grid.h;
+            const float gz = fmaxf(fmaxf(bz - q.z, q.z - (bz + grid.h)) - slack, 0.f);
+            for (int y = y0; y <= y1; ++y)
+            {
+                const float by = grid.miny + static_cast<float>(y) * grid.h;
+                const float gy = fmaxf(fmaxf(by - q.y, q.y - (by + grid.h)) - slack, 0.f);
+                if (__fmul_rn(gz, gz) + __fmul_rn(gy, gy) > fminf(limit, best.d[K - 1]) * 1.0001f) continue;
+                const int* c = cells + (z * grid.dy + y) * grid.dx;
+                if (z < sz0 || z > sz1 || y < sy0 || y > sy1)
+                    run(c, x0, x1);
+                else
+                {
+                    if (x0 < sx0) run(c, x0, sx0 - 1);
+                    if (x1 > sx1) run(c, sx1 + 1, x1);
+                }
+            }
+        }
+        sx0 = min(sx0, x0);
+        sx1 = max(sx1, x1);
+        sy0 = min(sy0, y0);
+        sy1 = max(sy1, y1);
+        sz0 = min(sz0, z0);
+        sz1 = max(sz1, z1);
+    };
+    // (the lanes of a query prune rows by their own lists, and meet different numbers of candidates)
+    auto agree = [&]() {
+        const uint32_t lanes = (G == 32 ? kFullMask : (1u << G) - 1u) << (threadIdx.x & 31 & ~(G - 1));
+        const uint32_t over = __ballot_sync(kFullMask, search && budget < 0);
+        crowded = crowded || (over & lanes) != 0u;
+        search = search && !crowded;
+    };
+    // one cell more on every side, up to three times, where there are not K candidates yet
+    for (int more = 0;; ++more)
+    {
+        const bool open = search && limit == CUDART_INF_F &&
+                          (sx0 > 0 || sy0 > 0 || sz0 > 0 || sx1 < grid.dx - 1 || sy1 < grid.dy - 1 || sz1 < grid.dz - 1);
+        if (__any_sync(kFullMask, open) == 0) break;
+        if (more == 3)
+        {
+            if (open) crowded = true;  // (a lonely query: rather the scan as well)
+            search = search && !crowded;
+            break;
+        }
+        if (g > 0) best.clear();  // (joined again below: the first lane has them)
+        if (open)
+            widen(max(sx0 - 1, 0), min(sx1 + 1, grid.dx - 1), max(sy0 - 1, 0), min(sy1 + 1, grid.dy - 1), max(sz0 - 1, 0),
+                  min(sz1 + 1, grid.dz - 1));
+        join();
+        agree();
+    }
+    // the other cells that the ball of the K-th best distance touches
+    {
+        const float reach = sqrtf(limit) * 1.0001f + slack;
+        const int x0 = nn_cell(q.x - reach, grid.minx, grid.inv_h, grid.dx), x1 = nn_cell(q.x + reach, grid.minx, grid.inv_h, grid.dx);
+        const int y0 = nn_cell(q.y - reach, grid.miny, grid.inv_h, grid.dy), y1 = nn_cell(q.y + reach, grid.miny, grid.inv_h, grid.dy);
+        const int z0 = nn_cell(q.z - reach, grid.minz, grid.inv_h, grid.dz), z1 = nn_cell(q.z + reach, grid.minz, grid.inv_h, grid.dz);
+        const bool open = search && limit < CUDART_INF_F && (x0 < sx0 || x1 > sx1 || y0 < sy0 || y1 > sy1 || z0 < sz0 || z1 > sz1);
+        if (__any_sync(kFullMask, open))
+        {
+            if (g > 0) best.clear();
+            if (open) widen(x0, x1, y0, y1, z0, z1);
+            join();
+            agree();
+        }
+    }
+    if (!in) return;
+    if (crowded)
+    {
+        // (listed where the cells of the points were, which are no longer needed)
+        if (g == 0) from.places[static_cast<size_t>(cloud) * from.n + nn_add(&from.grids[cloud].left)] = qi;
+        return;
+    }
+    const size_t o = (static_cast<size_t>(cloud) * from.n + __float_as_int(q.w)) * K;
+    float* dist = second ? dist_b : dist_a;
+    int32_t* idx = second ? idx_b : idx_a;
+#pragma unroll
+    for (int k = 0; k < K; ++k)
+        if (g == k % G)
+        {
+            dist[o + k] = best.d[k];
+            idx[o + k] = best.d[k] < CUDART_INF_F ? best.i[k] : 0;
+        }
+}
+
+// The queries that were left over, against all points of the other cloud: a warp each where that is at most ten for
+// a warp (as many instructions as ten queries cost it), else in tiles of the scan (scan.cuh).  `parts` CTAs per cloud; those of clouds
+// without any return.
+template <int K>
+__global__ void __launch_bounds__(kNnQueryThreads)
+    nn_scan_kernel(NnSide a, NnSide b, int clouds, int parts, float* __restrict__ dist_a, int32_t* __restrict__ idx_a,
+                   float* __restrict__ dist_b, int32_t* __restrict__ idx_b)
+{
+    constexpr int THREADS = kNnQueryThreads, Q = 2;
+    __shared__ __align__(16) float smem[2 * kScanTileFloats];
+    const int side = blockIdx.x / parts, part = blockIdx.x - side * parts;
+    const bool second = side >= clouds;
+    const int cloud = second ? side - clouds : side;
+    const NnSide& from = second ? b : a;
+    const NnSide& to = second ? a : b;
+    const int count = from.grids[cloud].left;
+    if (count == 0) return;
+    const float* known = to.xyz + static_cast<size_t>(cloud) * to.n * 3;
+    const int* list = from.places + static_cast<size_t>(cloud) * from.n;
+    const float4* sorted = from.sorted + static_cast<size_t>(cloud) * from.n;
+    float* dist = (second ? dist_b : dist_a) + static_cast<size_t>(cloud) * from.n * K;
+    int32_t* idx = (second ? idx_b : idx_a) + static_cast<size_t>(cloud) * from.n * K;
+    const int lane = threadIdx.x & 31, warps = parts * (THREADS / 32);
+    if (count <= 10 * warps)
+    {
+        for (int w = part * (THREADS / 32) + (threadIdx.x >> 5); w < count; w += warps)
+        {
+            const float4 q = __ldg(sorted + __ldg(list + w));
+            NnBest<K> best;
+            best.clear();
+            for (int k0 = lane; k0 < to.n; k0 += 4 * 32)
+            {
+                float c[4][3];
+#pragma unroll
+                for (int u = 0; u < 4; ++u)
+#pragma unroll
+                    for (int i = 0; i < 3; ++i) c[u][i] = __ldg(known + 3 * static_cast<size_t>(min(k0 + 32 * u, to.n - 1)) + i);
+#pragma unroll
+                for (int u = 0; u < 4; ++u)
+                {
+                    const float d = sumsq_abc(q.x - c[u][0], q.y - c[u][1], q.z - c[u][2]);
+                    if (k0 + 32 * u < to.n && d <= best.d[K - 1]) best.take(d, k0 + 32 * u);
+                }
+            }
+#pragma unroll
+            for (int o = 16; o >= 1; o >>= 1)
+            {
+                NnBest<K> other;
+#pragma unroll
+                for (int k = 0; k < K; ++k)
+                {
+                    other.d[k] = __shfl_xor_sync(kFullMask, best.d[k], o);
+                    other.i[k] = __shfl_xor_sync(kFullMask, best.i[k], o);
+                }
+#pragma unroll
+                for (int k = 0; k < K; ++k) best.take(other.d[k], other.i[k]);
+            }
+            const size_t o = static_cast<size_t>(__float_as_int(q.w)) * K;
+#pragma unroll
+            for (int k = 0; k < K; ++k)
+                if (lane == k)
+                {
+                    dist[o + k] = best.d[k];
+                    idx[o + k] = best.d[k] < CUDART_INF_F ? best.i[k] : 0;
+                }
+        }
+        return;
+    }
+    for (int base = part * THREADS * Q; base < count; base += parts * THREADS * Q)
+    {
+        using Op = typename std::conditional<K == 1, ArgMinOp<Q>, ThreeNnOp<Q>>::type;
+        Op op;
+        int j[Q];
+#pragma unroll
+        for (int q = 0; q < Q; ++q)
+        {
+            const int at = base + q * THREADS + threadIdx.x;
+            op.act[q] = at < count;
+            const float4 p = __ldg(sorted + __ldg(list + min(at, count - 1)));
+            j[q] = __float_as_int(p.w);
+            op.qx[q] = op.act[q] ? p.x : 0.f;
+            op.qy[q] = op.act[q] ? p.y : 0.f;
+            op.qz[q] = op.act[q] ? p.z : 0.f;
+            if constexpr (K == 1)
+            {
+                op.best[q] = CUDART_INF_F;
+                op.besti[q] = 0;
+            }
+            else
+            {
+                op.b1[q] = op.b2[q] = op.b3[q] = CUDART_INF_F;
+                op.i1[q] = op.i2[q] = op.i3[q] = 0;
+            }
+        }
+        scan_candidates<THREADS, Q>(known, to.n, smem, op.qx, op.qy, op.qz, op);
+#pragma unroll
+        for (int q = 0; q < Q; ++q)
+        {
+            if (!op.act[q]) continue;
+            const size_t o = static_cast<size_t>(j[q]) * K;
+            if constexpr (K == 1)
+            {
+                dist[o] = op.best[q];
+                idx[o] = op.besti[q];
+            }
+            else
+            {
+                dist[o + 0] = op.b1[q];
+                dist[o + 1] = op.b2[q];
+                dist[o + 2] = op.b3[q];
+                idx[o + 0] = op.i1[q];
+                idx[o + 1] = op.i2[q];
+                idx[o + 2] = op.i3[q];
+            }
+        }
+        __syncthreads();
+    }
+}
+
+// Cells that a side may have: smaller cells than those of one point each only help surfaces.
+int nn_cap(int n)
+{
+    const long long c = 4ll * n;
+    return static_cast<int>(c < 512 ? 512 : (c > kNnMaxCells ? kNnMaxCells : c));
+}
+
+size_t nn_round(size_t v) { return (v + 255) / 256 * 256; }
+
+size_t nn_side_bytes(int b, int n)
+{
+    return nn_round(static_cast<size_t>(b) * n * sizeof(float4)) + nn_round(static_cast<size_t>(b) * (nn_cap(n) + 1) * sizeof(int)) +
+           nn_round(static_cast<size_t>(b) * n * sizeof(int)) + nn_round(static_cast<size_t>(b) * sizeof(NnGrid));
+}
+
+NnSide nn_side(int b, int n, const float* xyz, float per_cell, bool searched, unsigned char*& at)
+{
+    NnSide s;
+    s.searched = searched;
+    s.xyz = xyz;
+    s.n = n;
+    s.cap = nn_cap(n);
+    s.per_cell = per_cell;
+    s.sorted = reinterpret_cast<float4*>(at);
+    at += nn_round(static_cast<size_t>(b) * n * sizeof(float4));
+    s.cells = reinterpret_cast<int*>(at);
+    at += nn_round(static_cast<size_t>(b) * (s.cap + 1) * sizeof(int));
+    s.places = reinterpret_cast<int*>(at);
+    at += nn_round(static_cast<size_t>(b) * n * sizeof(int));
+    s.grids = reinterpret_cast<NnGrid*>(at);
+    at += nn_round(static_cast<size_t>(b) * sizeof(NnGrid));
+    return s;
+}
+
+template <int K, int G>
+int nn_launch_query(const NnSide& a, const NnSide& b, int clouds, bool both, float* dist_a, int32_t* idx_a, float* dist_b, int32_t* idx_b,
+                    cudaStream_t s)
+{
+    const int per = kNnQueryThreads / G;
+    const int blocks_a = (a.n + per - 1) / per, blocks_b = both ? (b.n + per - 1) / per : 1;
+    const long long grid = static_cast<long long>(clouds) * (blocks_a + (both ? blocks_b : 0));
+    TPK_REQUIRE(grid < (1ll << 31), "nearest neighbours: too many clouds");
+    // (no prefer_max_shared: without shared memory of its own the kernel lives from L1)
+    count_launches(1), nn_query_kernel<K, G><<<static_cast<unsigned>(grid), kNnQueryThreads, 0, s>>>(a, b, clouds, blocks_a, blocks_b, dist_a,
+                                                                                                 idx_a, dist_b, idx_b);
+    // what is left over, mostly nothing
+    const int sides = both ? 2 * clouds : clouds, longest = both && b.n > a.n ? b.n : a.n;
+    int parts = (4 * num_sms() + sides - 1) / sides;
+    if (parts > (longest + 3) / 4) parts = (longest + 3) / 4;  // (a warp per query)
+    prefer_max_shared(nn_scan_kernel<K>);
+    count_launches(1), nn_scan_kernel<K><<<static_cast<unsigned>(sides) * parts, kNnQueryThreads, 0, s>>>(a, b, clouds, parts, dist_a, idx_a,
+                                                                                                       dist_b, idx_b);
+    return check_launch("nearest neighbours");
+}
+
+template <int K>
+int nn_run(int clouds, int n, int m, const float* xyz1, const float* xyz2, bool both, float* dist1, int32_t* idx1, float* dist2, int32_t* idx2,
+           void* scratch, cudaStream_t s)
+{
+    unsigned char* at = static_cast<unsigned char*>(scratch);
+    // Points per cell.  us, 0.5, 1, 2, 4, 8: three nearest of 16 x 16384 points in 4096 83, 75, 72, 69, 75, 3 x 10007 in
+    // 2501 45, 37, 32, 30, 31; nearest on spheres, 32 x 16384 both ways 91, 95, 96, 96, 115.  Where only the
+    // order of the points matters, four.
+    const float per_cell = K == 1 ? 0.5f : 4.0f;
+    const NnSide a = nn_side(clouds, n, xyz1, both ? per_cell : 4.0f, both, at), b = nn_side(clouds, m, xyz2, per_cell, true, at);
+    // CTAs per cloud: as many as run at once (74, 33, 15 clusters of 2, 4, 8), of at least 1024 points each
+    const int jobs = 2 * clouds, points = n > m ? n : m;
+    int ranks = jobs <= 15 ? 8 : (jobs <= 33 ? 4 : (jobs <= 74 ? 2 : 1));
+    while (ranks > 1 && points < 1024 * ranks) ranks >>= 1;
+    const int threads = points > 4096 || jobs <= 2 * num_sms() ? kNnSortThreads : (points > 1024 ? 512 : 256);
+    int most = a.cap > b.cap ? a.cap : b.cap;
+    most = (most + ranks - 1) / ranks;
+    const int smem = most * static_cast<int>(sizeof(int));
+    prefer_max_shared(nn_sort_kernel);
+    cudaError_t err = cudaFuncSetAttribute(nn_sort_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (err == cudaSuccess)
+    {
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(static_cast<unsigned>(jobs) * ranks, 1, 1);
+        cfg.blockDim = dim3(threads, 1, 1);
+        cfg.dynamicSmemBytes = smem;
+        cfg.stream = s;
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = ranks;
+        attr[0].val.clusterDim.y = 1;
+        attr[0].val.clusterDim.z = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        count_launches(1);
+        err = cudaLaunchKernelEx(&cfg, nn_sort_kernel, a, b, clouds, ranks);
+    }
+    if (err != cudaSuccess)
+    {
+        set_error("nearest neighbours: launch of the sort: %s", cudaGetErrorString(err));
+        return TPK_ERR_CUDA;
+    }
+    const long long queries = static_cast<long long>(clouds) * (n + (both ? m : 0));
+    // lanes per query: as many as it takes to have a few warps per scheduler (16 x 4096 queries 1, 2, 4 lanes 22.7, 17.6,
+    // 20.7 us, 3 x 2501 18.3, 13.3, 10.3, 16 x 16384 46, 51, 64)
+    const int g = queries >= 131072 ? 1 : (queries >= 65536 ? 2 : 4);
+    switch (g)
+    {
+    case 1: return nn_launch_query<K, 1>(a, b, clouds, both, dist1, idx1, dist2, idx2, s);
+    case 2: return nn_launch_query<K, 2>(a, b, clouds, both, dist1, idx1, dist2, idx2, s);
+    default: return nn_launch_query<K, 4>(a, b, clouds, both, dist1, idx1, dist2, idx2, s);
+    }
+}
+
+}  // namespace
+
+// Scratch for both clouds of a call, 0 where the sizes are not for these kernels.  both: the nearest in either
+// direction (Chamfer), else the three nearest.
+//
+// us, grids of smem_grid.cu and these.  Chamfer, forward: 32 x 16384 points 349 and 97, 64 x 2048 67 and 39,
+// 1 x 16384 99 and 33, 1 x 256 44 and 19, 64 x 256 on surfaces 47 and 57, 256 x 256 65 and 92 (a CTA to sort a cloud is too
+// much there).  Three nearest: 2 x 65536 in 65536 1007 and 93, 8 x 16384 in 16384 298 and 64, but 16 x 4096 in 1024 32
+// and 38, and where the clouds above are padded with one point 2281 and 3975 (4 x 16384 in 4096 745 and 1046):
+// they come from 8192 known points on, where the other grid has to be cut into layers.
+size_t nn_grid_scratch_bytes(int b, int n, int m, bool both)
+{
+    if (b < 1 || b > (1 << 26) || n < 1 || m < 1 || n > kNnMaxPoints || m > kNnMaxPoints) return 0;
+    if (!test_path("nn_sorted"))
+    {
+        if (both ? b > 32 && n < 512 && m < 512 : m <= 8192) return 0;
+    }
+    return nn_side_bytes(b, n) + nn_side_bytes(b, m);
+}
+
+int nn_grid_three(int b, int n, int m, const float* unknown, const float* known, float* dist2, int32_t* idx, void* scratch, cudaStream_t s)
+{
+    return nn_run<3>(b, n, m, unknown, known, false, dist2, idx, nullptr, nullptr, scratch, s);
+}
+
+int nn_grid_both(int b, int n, int m, const float* xyz1, const float* xyz2, float* dist1, int32_t* idx1, float* dist2, int32_t* idx2,
+                 void* scratch, cudaStream_t s)
+{
+    return nn_run<1>(b, n, m, xyz1, xyz2, true, dist1, idx1, dist2, idx2, scratch, s);
+}
+
+}  // namespace tpk

@@ -261,4 +261,71 @@ __device__ __forceinline__ long long segment_bound(const int64_t* __restrict__ i
     return lo;
 }
 
+// What the scans for the three nearest candidates and for the nearest one keep, by the reference's strict '<'.
+template <int Q>
+struct ThreeNnOp
+{
+    float qx[Q], qy[Q], qz[Q];
+    float b1[Q], b2[Q], b3[Q];
+    int i1[Q], i2[Q], i3[Q];
+    bool act[Q];
+
+    __device__ __forceinline__ float threshold(int q) const { return act[q] ? b3[q] : -CUDART_INF_F; }
+    __device__ __forceinline__ bool finished() const
+    {
+        bool done = true;
+#pragma unroll
+        for (int q = 0; q < Q; ++q) done &= !act[q];
+        return done;
+    }
+    __device__ __forceinline__ bool exact(int q, long long k, float cx, float cy, float cz)
+    {
+        const float v = sumsq_abc(qx[q] - cx, qy[q] - cy, qz[q] - cz);
+        if (!act[q] || !(v < b3[q])) return false;
+        const int kk = static_cast<int>(k);
+        if (v < b1[q])
+        {
+            b3[q] = b2[q]; i3[q] = i2[q];
+            b2[q] = b1[q]; i2[q] = i1[q];
+            b1[q] = v;     i1[q] = kk;
+        }
+        else if (v < b2[q])
+        {
+            b3[q] = b2[q]; i3[q] = i2[q];
+            b2[q] = v;     i2[q] = kk;
+        }
+        else
+        {
+            b3[q] = v; i3[q] = kk;
+        }
+        return true;
+    }
+};
+
+template <int Q>
+struct ArgMinOp
+{
+    float qx[Q], qy[Q], qz[Q];
+    float best[Q];
+    int besti[Q];
+    bool act[Q];
+
+    __device__ __forceinline__ float threshold(int q) const { return act[q] ? best[q] : -CUDART_INF_F; }
+    __device__ __forceinline__ bool finished() const
+    {
+        bool done = true;
+#pragma unroll
+        for (int q = 0; q < Q; ++q) done &= !act[q];
+        return done;
+    }
+    __device__ __forceinline__ bool exact(int q, long long k, float cx, float cy, float cz)
+    {
+        const float d = sumsq_abc(cx - qx[q], cy - qy[q], cz - qz[q]);
+        if (!act[q] || !(d < best[q])) return false;
+        best[q] = d;
+        besti[q] = static_cast<int>(k);
+        return true;
+    }
+};
+
 }  // namespace tpk

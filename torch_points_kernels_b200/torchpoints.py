@@ -93,7 +93,9 @@ def three_nn(unknown, known):
     dist2 = torch.empty((b, n, 3), dtype=torch.float32, device=unknown.device)
     idx = torch.empty((b, n, 3), dtype=torch.int32, device=unknown.device)
     with _lib.on_device(unknown):
-        need = _lib.lib().tpk_three_nn_scratch_bytes(b, n, m)
+        handle = _lib.lib()
+        # grids over sorted copies, or else one flag per point for the grids without
+        need = handle.tpk_three_nn_sorted_scratch_bytes(b, n, m) or handle.tpk_three_nn_scratch_bytes(b, n, m)
         if need > 0:
             # many known points: uniform-grid search with scratch (same results as the scan)
             scratch = torch.empty((need,), dtype=torch.uint8, device=unknown.device)
