@@ -187,6 +187,15 @@ def test_fps_scratch_kernel_tie_break_and_skip_rule(n, sorted_copy, monkeypatch)
     np.testing.assert_array_equal(npy(tpk.furthest_point_sample(cu(x), mm)), orc.fps(x, mm))
 
 
+@pytest.mark.parametrize("ranks", [3, 5, 6, 7, 9, 10, 13])
+@pytest.mark.parametrize("n,m", [(1500, 400), (50001, 3000)])
+def test_fps_large_rounds_every_cluster_size(n, m, ranks, monkeypatch):
+    """Clusters whose size is no power of two: warps share out the lists of the CTAs unevenly."""
+    data.use_paths(monkeypatch, "fps_global", "fps_config=%d" % ranks)
+    x = data.gaussian_mixture(2, n, seed=n + ranks).numpy()
+    np.testing.assert_array_equal(npy(tpk.furthest_point_sample(cu(x), m)), orc.fps(x, m))
+
+
 @pytest.mark.parametrize("n,m,ranks", [(1500, 1500, 8), (33000, 9000, 16), (33000, 3000, 1), (70001, 2000, 1),
                                        (140000, 700, 1), (140000, 5000, 2)])
 @pytest.mark.parametrize("kind", ["mixture", "lattice"])

@@ -18,7 +18,7 @@
 //
 // What bounds it is the latency of a round: two cluster barriers, the dependent loads of chunks from
 // L2, the check of the entries.  Measured, B200, one sample per exchange over the cluster before:
-// 8 clouds of 1048576 -> 65536 252 ms before, 11.0 now; one cloud 6.7 now;
+// 8 clouds of 1048576 -> 65536 252 ms before, 10.3 now;
 // 2 x 200000 -> 5000 8.5 and 1.4; a lattice of 64^3 -> 3000 (ties everywhere) 6.4 and 1.45.
 //
 // A sample's minimum is kept where it was: -minimum at its place, which no distance lowers and no
@@ -44,6 +44,7 @@ constexpr int kLargeMaxRanks = 16;
 constexpr int kLargeEntries = 4096;      // active points (half as many chunks) of a round
 constexpr int kLargeOwnEntries = 1024;   // of one CTA
 constexpr int kLargePicks = 2048;        // samples of a round
+constexpr int kLargeGroups = 2;          // groups of chunks of a warp, at most
 constexpr int kLargeHits = 128;          // samples applied to a group of chunks at a time
 constexpr int kLargeBuckets = 4096;
 constexpr int kLargeBucketShift = 16;    // while sampling: 128 buckets per octave, 32 octaves
@@ -53,7 +54,8 @@ constexpr int kMaxSmemBytes = 227 * 1024;
 struct LargeLayout
 {
     int run;        // chunks of a warp
-    int groups;     // of up to 32 chunks of a warp
+    int unit_bits;  // a unit of 2^unit_bits chunks in a row, 16 or 32, is a group of a warp
+    int groups;     // units of a warp
     int cap_picks;  // samples a CTA may take per round
     int meta, gbox, table, table_pos, own, own_pos, picks, mine_pick, hist;
     int f_hist, f_base, f_start;
@@ -296,10 +298,21 @@ struct LargeNote
     int entries, top, above, picks;
 };
 
+// The first point of chunk c of a warp.  The units of chunks go round the CTAs of the cluster, then round their warps:
+// a round lasts as long as its busiest CTA, and the samples of a round lie together.  With 32 chunks in a row for every warp
+// a CTA waited 27 of 90 k cycles of a round for the others; units of 8 halve that but cost as much in
+// groups to look at.  us, units of 8, 16, 32: 8 x 1048576 -> 65536 11035, 10924, 12200, 4 x 500000 -> 20000 3910,
+// 3601, 3859, 12 x 200000 -> 5000 1910, 1832, 1874.
+__device__ __forceinline__ int large_chunk(int warp, int c, int rank, int nranks, int unit_bits, int points)
+{
+    const int unit = ((c >> unit_bits) * kLargeWarps + warp) * nranks + rank;
+    return ((unit << unit_bits) + (c & ((1 << unit_bits) - 1))) * points;
+}
+
 // How many samples of a warp's chunks have a minimum above the image `key`.  (Out of line: rarely called, and
 // not to take registers from the rounds.)
 template <int P>
-__device__ __noinline__ int large_count_above(const float* temp, long long first, int run, int n, int key)
+__device__ __noinline__ int large_count_above(const float* temp, int warp, int rank, int nranks, int unit_bits, int run, int n, int key)
 {
     const int lane = threadIdx.x & 31;
     int count = 0;
@@ -307,7 +320,7 @@ __device__ __noinline__ int large_count_above(const float* temp, long long first
 #pragma unroll
         for (int u = 0; u < P; ++u)
         {
-            const long long p = first + (static_cast<long long>(c) * P + u) * 32 + lane;
+            const int p = large_chunk(warp, c, rank, nranks, unit_bits, 32 * P) + u * 32 + lane;
             const float md = p < n ? __ldcg(temp + p) : 0.f;
             count += md < 0.f && md != -CUDART_INF_F && __float_as_int(-md) > key ? 1 : 0;
         }
@@ -358,9 +371,9 @@ __global__ void __launch_bounds__(kLargeThreads, 1)
     uint16_t* hits = reinterpret_cast<uint16_t*>(task_at + nmeta);
 
     auto at_rank = [&](auto* p, int r) { return cg::this_cluster().map_shared_rank(p, static_cast<unsigned>(r)); };
-    // Neighbouring runs belong to different CTAs: a round lasts as long as its busiest CTA.
-    const long long first = static_cast<long long>(warp * nranks + rank) * run * CHUNK;
-    auto chunk_base = [&](int c) { return first + static_cast<long long>(c) * CHUNK; };
+    const int unit = 1 << lay.unit_bits, sets = (run + 31) / 32;  // sets: of up to 32 chunks of a warp
+    auto chunk_at = [&](int owner, int c) { return large_chunk(owner, c, rank, nranks, lay.unit_bits, CHUNK); };
+    auto chunk_base = [&](int c) { return chunk_at(warp, c); };
     auto index_at = [&](int pos) { return __float_as_int(__ldg(&sorted[pos].w)); };
     auto box_dist = [&](const float (&b)[6], float x, float y, float z) {
         // same expression and rounding as a point's distance: never above that of a point in the box, infinite
@@ -377,7 +390,7 @@ __global__ void __launch_bounds__(kLargeThreads, 1)
         s_last[0] = s_last[1] = -1;
         s_counted = INT_MAX;
         s_tasks = 0;
-        s_next_task = 0;
+        s_next_task = kLargeWarps;  // (the first task of a warp is its own number)
         s_listed = 0;
         s_next_listed = 0;
         for (int i = 0; i < 2; ++i) s_note[i] = LargeNote{0, INT_MIN, 0, 0};
@@ -387,11 +400,10 @@ __global__ void __launch_bounds__(kLargeThreads, 1)
     for (int i = tid; i < kLargeBuckets; i += kLargeThreads) hist[i] = 0;
     for (int g = 0; g < lay.groups; ++g)
     {
-        const int left = min(32, run - 32 * g);
         float glo[3] = {CUDART_INF_F, CUDART_INF_F, CUDART_INF_F}, ghi[3] = {-CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F};
-        for (int c = 0; c < left; ++c)
+        for (int c = 0; c < unit; ++c)
         {
-            const long long base = chunk_base(32 * g + c);
+            const int base = chunk_base(g * unit + c);
             float lo[3] = {CUDART_INF_F, CUDART_INF_F, CUDART_INF_F}, hi[3] = {-CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F};
             int key = INT_MIN;
             float4 v[P];
@@ -401,7 +413,7 @@ __global__ void __launch_bounds__(kLargeThreads, 1)
 #pragma unroll
             for (int u = 0; u < P; ++u)
             {
-                const long long p = base + u * 32 + lane;
+                const int p = base + u * 32 + lane;
                 if (p >= n) continue;
                 const bool in = !(static_cast<double>(sumsq_abc(v[u].x, v[u].y, v[u].z)) <= 1e-3);
                 const float first_min = in ? 1e10f : -CUDART_INF_F;
@@ -416,7 +428,7 @@ __global__ void __launch_bounds__(kLargeThreads, 1)
                 hi[2] = fmaxf(hi[2], v[u].z);
                 bad |= !all_finite(v[u].x, v[u].y, v[u].z);
             }
-            const int at = warp * run + 32 * g + c;
+            const int at = warp * run + g * unit + c;
 #pragma unroll
             for (int a = 0; a < 3; ++a)
             {
@@ -444,22 +456,33 @@ __global__ void __launch_bounds__(kLargeThreads, 1)
     bool sequential = false;  // one sample per round, every chunk in reach: coordinates that are not finite
     for (int r = 0; r < nranks; ++r) sequential |= *at_rank(&s_bad, r) != 0;
 
-    // Lowers the minima of a chunk by the samples hits[bit] of a mask of 128; returns its key.
-    auto lower_chunk = [&](long long base, const uint16_t* hits, uint4 mask) -> int {
+    // Lowers the minima of a chunk by the samples hits[bit] of a mask of 128; returns its key.  (Most chunks are reached
+    // by one sample, and what they cost is the instructions around that: no 64-bit addresses, no bounds
+    // where the chunk is full.)
+    auto lower_chunk = [&](int base, const uint16_t* hits, uint4 mask) -> int {
+        const bool full = base + CHUNK <= n;
+        const float4* at = sorted + base + lane;
+        float* min_at = temp + base + lane;
         float4 v[P];
         float d0[P], md[P];
-#pragma unroll
-        for (int u = 0; u < P; ++u)
+        if (full)
         {
-            const long long p = base + u * 32 + lane;
-            d0[u] = -CUDART_INF_F;
-            v[u] = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (p < n)
+#pragma unroll
+            for (int u = 0; u < P; ++u)
             {
-                v[u] = __ldg(sorted + p);
-                d0[u] = __ldcg(temp + p);
+                v[u] = __ldg(at + u * 32);
+                md[u] = d0[u] = __ldcg(min_at + u * 32);
             }
-            md[u] = d0[u];
+        }
+        else
+        {
+#pragma unroll
+            for (int u = 0; u < P; ++u)
+            {
+                const bool in = base + u * 32 + lane < n;
+                v[u] = in ? __ldg(at + u * 32) : make_float4(0.f, 0.f, 0.f, 0.f);
+                md[u] = d0[u] = in ? __ldcg(min_at + u * 32) : -CUDART_INF_F;
+            }
         }
 #pragma unroll
         for (int w = 0; w < 4; ++w)
@@ -477,8 +500,8 @@ __global__ void __launch_bounds__(kLargeThreads, 1)
 #pragma unroll
         for (int u = 0; u < P; ++u)
         {
-            const long long p = base + u * 32 + lane;
-            if (p < n && md[u] != d0[u]) __stcg(temp + p, md[u]);
+            // (minus infinity behind the end of the cloud: never lower)
+            if (md[u] != d0[u]) __stcg(min_at + u * 32, md[u]);
             key = max(key, __float_as_int(md[u]));
         }
         return __reduce_max_sync(kFullMask, key);
@@ -492,53 +515,80 @@ __global__ void __launch_bounds__(kLargeThreads, 1)
         for (bool first_pass = true;; first_pass = false)
         {
             bool more = false;
-            for (int g = 0; g < lay.groups; ++g)
+            // which samples reach which group of this warp, all groups side by side
+            float whole[kLargeGroups][6];
+            int gkey[kLargeGroups], from[kLargeGroups], nhits[kLargeGroups], start = count;
+#pragma unroll
+            for (int g = 0; g < kLargeGroups; ++g)
             {
+                const bool in = g < lay.groups;
+                const int slot = warp * lay.groups + (in ? g : 0);
+                const float* gb = gbox + slot * 8;
+#pragma unroll
+                for (int a = 0; a < 6; ++a) whole[g][a] = gb[a];
+                gkey[g] = __reduce_max_sync(kFullMask, in ? ckey[warp * run + g * unit + (lane & (unit - 1))] : INT_MIN);
+                from[g] = !in || gkey[g] <= 0 ? count : (first_pass ? 0 : *reinterpret_cast<const int*>(gb + 6));
+                nhits[g] = 0;
+                start = min(start, from[g]);
+            }
+            for (int i0 = start; i0 < count; i0 += 32)
+            {
+                const float4 s = picks[min(i0 + lane, count - 1)];
+                const bool in = i0 + lane < count;
+#pragma unroll
+                for (int g = 0; g < kLargeGroups; ++g)
+                {
+                    const bool reach = in && (sequential || box_dist(whole[g], s.x, s.y, s.z) < __int_as_float(gkey[g]));
+                    const uint32_t b = __ballot_sync(kFullMask, reach);
+                    if (b == 0u || from[g] > i0 || nhits[g] < 0) continue;
+                    if (nhits[g] + __popc(b) > kLargeHits)
+                    {
+                        // the rest in another pass: from here on
+                        from[g] = i0;
+                        nhits[g] = ~nhits[g];
+                        continue;
+                    }
+                    if (reach) hits[(warp * lay.groups + g) * kLargeHits + nhits[g] + __popc(b & ((1u << lane) - 1u))] = static_cast<uint16_t>(i0 + lane);
+                    nhits[g] += __popc(b);
+                }
+            }
+#pragma unroll
+            for (int g = 0; g < kLargeGroups; ++g)
+            {
+                if (g >= lay.groups) continue;
                 const int slot = warp * lay.groups + g;
                 int* progress = reinterpret_cast<int*>(gbox + slot * 8 + 6);
-                int i0 = 0;
-                if (!first_pass) i0 = *progress;
-                if (i0 >= count) continue;
-                const bool in = 32 * g + lane < run;
-                const int at = warp * run + 32 * g + lane;
-                const int key = in ? ckey[at] : INT_MIN;
-                const int gkey = __reduce_max_sync(kFullMask, key);
-                uint16_t* list = hits + slot * kLargeHits;
-                int nh = 0;
-                if (gkey <= 0) i0 = count;
-                for (; i0 < count; i0 += 32)
-                {
-                    bool reach = false;
-                    if (i0 + lane < count)
-                    {
-                        const float4 s = picks[i0 + lane];
-                        const float* gb = gbox + slot * 8;
-                        const float b[6] = {gb[0], gb[1], gb[2], gb[3], gb[4], gb[5]};
-                        reach = sequential || box_dist(b, s.x, s.y, s.z) < __int_as_float(gkey);
-                    }
-                    const uint32_t b = __ballot_sync(kFullMask, reach);
-                    if (b == 0u) continue;
-                    if (nh + __popc(b) > kLargeHits) break;
-                    if (reach) list[nh + __popc(b & ((1u << lane) - 1u))] = static_cast<uint16_t>(i0 + lane);
-                    nh += __popc(b);
-                }
+                const int i0 = nhits[g] < 0 ? from[g] : count, nh = nhits[g] < 0 ? ~nhits[g] : nhits[g];
+                const uint16_t* list = hits + slot * kLargeHits;
+                // lane: chunk lane & (unit - 1) of the group, and one of the 32 / unit samples of a step
+                const int at = warp * run + g * unit + (lane & (unit - 1));
+                const int key = ckey[at];
                 __syncwarp();
                 if (lane == 0) *progress = i0;
                 more |= i0 < count;
                 if (nh == 0) continue;
                 float box[6];
 #pragma unroll
-                for (int a = 0; a < 6; ++a) box[a] = in ? meta[a * nmeta + at] : 0.f;
+                for (int a = 0; a < 6; ++a) box[a] = meta[a * nmeta + at];
+                const int step = 32 >> lay.unit_bits, sub = lane >> lay.unit_bits, me = lane & (unit - 1);
                 uint32_t mask[4] = {0, 0, 0, 0};
-                if (key > 0)
 #pragma unroll
-                    for (int w = 0; w < 4; ++w)
-                        for (int h = 32 * w; h < min(nh, 32 * w + 32); ++h)
+                for (int w = 0; w < 4; ++w)
+                    for (int h = 32 * w; h < min(nh, 32 * w + 32); h += step)
+                    {
+                        bool reach = false;
+                        if (h + sub < nh && key > 0)
                         {
-                            const float4 s = picks[list[h]];
-                            if (sequential || box_dist(box, s.x, s.y, s.z) < __int_as_float(key)) mask[w] |= 1u << (h & 31);
+                            const float4 s = picks[list[h + sub]];
+                            reach = sequential || box_dist(box, s.x, s.y, s.z) < __int_as_float(key);
                         }
-                const bool any = (mask[0] | mask[1] | mask[2] | mask[3]) != 0u;
+                        // bit sub * unit + chunk: the samples of this lane's chunk together
+                        const uint32_t b = __ballot_sync(kFullMask, reach) >> me;
+                        uint32_t mine = b & 1u;
+                        if (step > 1) mine |= (b >> unit & 1u) << 1;
+                        mask[w] |= mine << (h & 31);
+                    }
+                const bool any = sub == 0 && (mask[0] | mask[1] | mask[2] | mask[3]) != 0u;
                 const uint32_t b = __ballot_sync(kFullMask, any);
                 int pos = 0;
                 if (lane == 0 && b != 0u) pos = atomicAdd(&s_tasks, __popc(b));
@@ -546,28 +596,25 @@ __global__ void __launch_bounds__(kLargeThreads, 1)
                 if (any)
                 {
                     task_mask[pos] = make_uint4(mask[0], mask[1], mask[2], mask[3]);
-                    task_at[pos] = make_int2(at, slot);
+                    task_at[pos] = make_int2(chunk_base(g * unit + me), at << 8 | slot);  // (slots: 128 at most)
                 }
             }
             __syncthreads();
             const int ntasks = s_tasks;
-            while (true)
+            int t = warp;
+            while (t < ntasks)
             {
-                int t = 0;
+                const int2 task = task_at[t];
+                const int key = lower_chunk(task.x, hits + (task.y & 255) * kLargeHits, task_mask[t]);
+                if (lane == 0) ckey[task.y >> 8] = key;
                 if (lane == 0) t = atomicAdd(&s_next_task, 1);
                 t = __shfl_sync(kFullMask, t, 0);
-                if (t >= ntasks) break;
-                const int2 task = task_at[t];
-                const int owner = task.x / run;
-                const long long base = (static_cast<long long>(owner * nranks + rank) * run + (task.x - owner * run)) * CHUNK;
-                const int key = lower_chunk(base, hits + task.y * kLargeHits, task_mask[t]);
-                if (lane == 0) ckey[task.x] = key;
             }
             more = __syncthreads_or(more ? 1 : 0) != 0;
             if (tid == 0)
             {
                 s_tasks = 0;
-                s_next_task = 0;
+                s_next_task = kLargeWarps;
             }
             if (!more) break;
             __syncthreads();
@@ -578,7 +625,7 @@ __global__ void __launch_bounds__(kLargeThreads, 1)
     auto find_top = [&](int top) -> unsigned long long {
         if (tid == 0) s_top = ~0ull;
         __syncthreads();
-        for (int g = 0; g < lay.groups; ++g)
+        for (int g = 0; g < sets; ++g)
         {
             const bool in = 32 * g + lane < run;
             const int key = in ? ckey[warp * run + 32 * g + lane] : INT_MIN;
@@ -588,10 +635,10 @@ __global__ void __launch_bounds__(kLargeThreads, 1)
             {
                 const int c = __ffs(todo) - 1;
                 todo &= todo - 1u;
-                const long long base = chunk_base(32 * g + c);
+                const int base = chunk_base(32 * g + c);
                 for (int u = 0; u < P; ++u)
                 {
-                    const long long p = base + u * 32 + lane;
+                    const int p = base + u * 32 + lane;
                     if (p >= n) continue;
                     const int k = __float_as_int(__ldcg(temp + p));
                     const bool zero_like = k == 0 || (k < 0 && k != __float_as_int(-CUDART_INF_F));
@@ -648,7 +695,7 @@ __global__ void __launch_bounds__(kLargeThreads, 1)
         // (the chunks to list go to whichever warp is free, as above: the active ones lie together,
         // and a warp that listed its own had up to 32 in a row; 17.2 ms for what takes 12.5 now)
         int wmax = INT_MIN;
-        for (int g = 0; g < lay.groups; ++g)
+        for (int g = 0; g < sets; ++g)
         {
             const bool in = 32 * g + lane < run;
             const int at = warp * run + 32 * g + lane;
@@ -660,7 +707,7 @@ __global__ void __launch_bounds__(kLargeThreads, 1)
             int pos = 0;
             if (lane == 0) pos = atomicAdd(&s_listed, __popc(b));
             pos = __shfl_sync(kFullMask, pos, 0) + __popc(b & ((1u << lane) - 1u));
-            if (active) task_at[pos].x = at;
+            if (active) task_at[pos] = make_int2(chunk_base(32 * g + lane), at);
         }
         __syncthreads();
         const int nlisted = s_listed;
@@ -670,14 +717,12 @@ __global__ void __launch_bounds__(kLargeThreads, 1)
             if (lane == 0) t = atomicAdd(&s_next_listed, 1);
             t = __shfl_sync(kFullMask, t, 0);
             if (t >= nlisted) break;
-            const int at = task_at[t].x;
-            const int owner = at / run;
-            const long long base = (static_cast<long long>(owner * nranks + rank) * run + (at - owner * run)) * CHUNK;
+            const int base = task_at[t].x, at = task_at[t].y;
             float md[P];
 #pragma unroll
             for (int u = 0; u < P; ++u)
             {
-                const long long p = base + u * 32 + lane;
+                const int p = base + u * 32 + lane;
                 md[u] = p < n ? __ldcg(temp + p) : -CUDART_INF_F;
             }
             if (by_chunk)
@@ -757,7 +802,7 @@ __global__ void __launch_bounds__(kLargeThreads, 1)
                 // samples themselves, once for every largest minimum (later samples are not above it)
                 if (s_counted != top_before)
                 {
-                    above = large_count_above<P>(temp, first, run, n, top_before);
+                    above = large_count_above<P>(temp, warp, rank, nranks, lay.unit_bits, run, n, top_before);
                     if (lane == 0) s_above[warp] = above;
                     __syncwarp();
                 }
@@ -776,7 +821,8 @@ __global__ void __launch_bounds__(kLargeThreads, 1)
         }
         __syncthreads();
         int nentries = 0, above = 0, longest = 0, before = 0;
-        const int from = warp & (nranks - 1);
+        const int from = warp % nranks;  // the CTA whose lists this warp copies, with the other warps that do
+        const int copy_at = (warp / nranks) * 32 + lane, copy_step = (kLargeWarps - 1 - from) / nranks * 32 + 32;
         top = INT_MIN;
         for (int r = 0; r < nranks; ++r)
         {
@@ -869,10 +915,10 @@ __global__ void __launch_bounds__(kLargeThreads, 1)
         overflow_before = false;
         {
             // the lists of all CTAs: warps share out a CTA's list
-            const int count = s_notes[from].entries, step = kLargeThreads / nranks;
+            const int count = s_notes[from].entries;
             const float4* src = at_rank(own, from);
             const int* src_pos = at_rank(own_pos, from);
-            for (int i = (warp / nranks) * 32 + lane; i < count; i += step)
+            for (int i = copy_at; i < count; i += copy_step)
             {
                 table[before + i] = src[i];
                 if (by_chunk) table[kLargeEntries / 2 + before + i] = src[kLargeOwnEntries / 2 + i];
@@ -991,9 +1037,9 @@ __global__ void __launch_bounds__(kLargeThreads, 1)
             total += s_notes[r].picks;
         }
         {
-            const int count = s_notes[from].picks, step = kLargeThreads / nranks;
+            const int count = s_notes[from].picks;
             const float4* src = at_rank(mine_pick, from);
-            for (int i = (warp / nranks) * 32 + lane; i < count; i += step) picks[before + i] = src[i];
+            for (int i = copy_at; i < count; i += copy_step) picks[before + i] = src[i];
         }
         pending = total;
         taken += total;
@@ -1028,7 +1074,7 @@ __global__ void __launch_bounds__(kLargeThreads, 1)
             for (int c = 0; c < run; ++c)
                 for (int u = 0; u < P; ++u)
                 {
-                    const long long p = chunk_base(c) + u * 32 + lane;
+                    const int p = chunk_base(c) + u * 32 + lane;
                     const float md = p < n ? __ldcg(temp + p) : 0.f;
                     if (md < 0.f && md != -CUDART_INF_F) low = min(low, __float_as_int(-md));
                 }
@@ -1044,18 +1090,19 @@ __global__ void __launch_bounds__(kLargeThreads, 1)
         int shift = 0;
         while (((first_top - low) >> shift) >= kLargeBuckets - 1) ++shift;
         auto bucket = [&](int key) { return max(0, min(kLargeBuckets - 1, (first_top - key) >> shift)); };
-        // a warp moves its samples to the front of its run, as (image of the minimum, index)
+        // a warp moves its samples to the front of its chunks, as (image of the minimum, index)
+        auto place = [&](int i) { return chunk_base(i / CHUNK) + i % CHUNK; };
         int mine = 0;
         for (int c = 0; c < run; ++c)
         {
-            const long long base = chunk_base(c);
+            const int base = chunk_base(c);
             if (base >= n) break;
             int key[P], idx[P];
             bool is[P];
 #pragma unroll
             for (int u = 0; u < P; ++u)
             {
-                const long long p = base + u * 32 + lane;
+                const int p = base + u * 32 + lane;
                 const float md = p < n ? __ldcg(temp + p) : 0.f;
                 is[u] = md < 0.f && md != -CUDART_INF_F;
                 key[u] = __float_as_int(-md);
@@ -1068,7 +1115,7 @@ __global__ void __launch_bounds__(kLargeThreads, 1)
                 const uint32_t b = __ballot_sync(kFullMask, is[u]);
                 if (is[u])
                 {
-                    __stcg(reinterpret_cast<int2*>(sorted + first + mine + __popc(b & ((1u << lane) - 1u))), make_int2(key[u], idx[u]));
+                    __stcg(reinterpret_cast<int2*>(sorted + place(mine + __popc(b & ((1u << lane) - 1u)))), make_int2(key[u], idx[u]));
                     atomicAdd(&f_hist[bucket(key[u])], 1);
                 }
                 mine += __popc(b);
@@ -1115,9 +1162,10 @@ __global__ void __launch_bounds__(kLargeThreads, 1)
         }
         for (int i = lane; i < mine; i += 32)
         {
-            const int2 e = __ldcg(reinterpret_cast<const int2*>(sorted + first + i));
+            const int at = place(i);
+            const int2 e = __ldcg(reinterpret_cast<const int2*>(sorted + at));
             const int b = bucket(e.x);
-            __stcg(slots + f_start[b] + atomicAdd(&f_base[b], 1), static_cast<int>(first) + i);
+            __stcg(slots + f_start[b] + atomicAdd(&f_base[b], 1), static_cast<int>(at));
         }
         cluster_sync_all();
         for (int i = rank * kLargeThreads + tid; i < taken; i += nranks * kLargeThreads)
@@ -1156,8 +1204,10 @@ LargeLayout large_layout(int n, int nranks, int p)
     LargeLayout lay = {};
     const long long nchunks = (static_cast<long long>(n) + 32 * p - 1) / (32 * p);
     const int warps = nranks * kLargeWarps;
-    lay.run = static_cast<int>((nchunks + warps - 1) / warps);
-    lay.groups = (lay.run + 31) / 32;
+    lay.unit_bits = nchunks <= 32ll * warps ? 4 : 5;
+    const long long units = (nchunks + (1 << lay.unit_bits) - 1) >> lay.unit_bits;
+    lay.groups = static_cast<int>((units + warps - 1) / warps);
+    lay.run = lay.groups << lay.unit_bits;
     lay.cap_picks = kLargePicks / nranks < 512 ? kLargePicks / nranks : 512;
     long long at = 0;
     auto take = [&](long long bytes) {
@@ -1265,19 +1315,23 @@ int fps_large(int b, int n, int m, int log2bs, const float* xyz, void* scratch, 
         while (p < 4 && (static_cast<long long>(n) + 32 * p - 1) / (32 * p) > 32ll * kLargeWarps * ranks) p *= 2;
         return p;
     };
-    auto fits = [&](int ranks) { return large_layout(n, ranks, chunk_of(ranks)).bytes <= kMaxSmemBytes - 2048; };
-    // 148, 72, 32, 15, 7 clusters of 1, 2, 4, 8, 16 such CTAs run at once, and a call takes about as long as
-    // 180000 points plus those of a CTA.  256 samples, us, clusters of 2, 4, 8, 16: 7 clouds of 200000 points
+    auto fits = [&](int ranks) {
+        const LargeLayout l = large_layout(n, ranks, chunk_of(ranks));
+        return l.groups <= kLargeGroups && l.bytes <= kMaxSmemBytes - 2048;
+    };
+    // How many clusters of 1, 2, .. 16 such CTAs run at once (seven of the eight groups of SMs have 16 and more,
+    // one ten), and a call takes about as long as 180000 points plus those of a CTA.  256 samples, us, clusters of 2, 4, 8, 16: 7 clouds of 200000 points
     // 1247, 1006, 886, 775; 8 clouds 1263, 966, 895, 1365; 16 clouds 1353, 1059, 1564, 2005; 40 of 140000
     // 1223, 1698, 2249, 3742; 8 of 1048576 (8 and 16) 1834, 2374.
-    static const int kAtOnce[5] = {148, 72, 32, 15, 7};
+    // Clusters that are no power of two: 12 x 200000 -> 5000 1960 us with 8 CTAs, 1830 with 9; 20 x 200000 2400 with 4, 2090 with 6.
+    static const int kAtOnce[kLargeMaxRanks] = {148, 74, 45, 33, 26, 22, 15, 15, 15, 11, 7, 7, 7, 7, 7, 7};
     int nranks = kLargeMaxRanks;
     double least = 0.;
-    for (int l = 4; l >= 0; --l)
+    for (int r = kLargeMaxRanks; r >= 1; --r)
     {
-        const double cost = ((b + kAtOnce[l] - 1) / kAtOnce[l]) * (180000. + n / static_cast<double>(1 << l));
-        if (l < 4 && (cost >= least || !fits(1 << l))) continue;
-        nranks = 1 << l;
+        const double cost = ((b + kAtOnce[r - 1] - 1) / kAtOnce[r - 1]) * (180000. + n / static_cast<double>(r));
+        if (r < kLargeMaxRanks && (cost >= least || !fits(r))) continue;
+        nranks = r;
         least = cost;
     }
     char text[64];
@@ -1285,7 +1339,7 @@ int fps_large(int b, int n, int m, int log2bs, const float* xyz, void* scratch, 
     {
         // test hook "fps_config=nranks:...": another cluster size for the same cloud
         const int r = atoi(text);
-        if (r >= 1 && r <= kLargeMaxRanks && (r & (r - 1)) == 0 && fits(r)) nranks = r;
+        if (r >= 1 && r <= kLargeMaxRanks && fits(r)) nranks = r;
     }
     const int p = chunk_of(nranks);
     const LargeLayout lay = large_layout(n, nranks, p);
