@@ -29,12 +29,12 @@ constexpr int kBsBlock = 128;  // points per step of a warp
 constexpr int kBsSplitSamples = 256;  // lists of that length fit shared memory for every warp (16 KB)
 
 // W: warps that share a centre (with Q = 1, per_warp = 1 and without `need`).
-template <bool PARTIAL, int Q, int W>
-__global__ void __launch_bounds__(kBsThreads)
-    ball_scan_kernel(long long total, int per_warp, long long n, long long m, float radius, int nsample,
-                     const float* __restrict__ y, const float* __restrict__ x, const int64_t* __restrict__ batch_x,
-                     const int64_t* __restrict__ batch_y, int64_t* __restrict__ idx_out, float* __restrict__ dist_out,
-                     const unsigned char* __restrict__ need, bool unless_most)
+// D: blocks of points on their way.
+template <bool PARTIAL, int Q, int W, int D>
+__device__ __forceinline__ void
+    ball_scan(long long total, int per_warp, long long n, long long m, float radius, int nsample, const float* __restrict__ y,
+              const float* __restrict__ x, const int64_t* __restrict__ batch_x, const int64_t* __restrict__ batch_y,
+              int64_t* __restrict__ idx_out, float* __restrict__ dist_out, const unsigned char* __restrict__ need, bool unless_most)
 {
     extern __shared__ int2 s_hits[];  // W > 1: index and distance of the hits, nsample for each warp
     __shared__ int s_found[kBsThreads / 32];
@@ -134,26 +134,26 @@ __global__ void __launch_bounds__(kBsThreads)
         const float4* v = reinterpret_cast<const float4*>(p + 3 * head);
         const long long blocks = (cnt - head) / kBsBlock;
         const long long t0 = blocks * part / W, t1 = blocks * (part + 1) / W;
-        float4 a = {}, b = {}, c = {};
-        if (t0 < t1)
+        float4 a[D] = {}, b[D] = {}, c[D] = {};
+        auto fetch = [&](int u, long long t) {
+            const float4* at = v + 3 * (kBsBlock / 4) * t + 3 * lane;
+            a[u] = __ldg(at + 0);
+            b[u] = __ldg(at + 1);
+            c[u] = __ldg(at + 2);
+        };
+#pragma unroll
+        for (int u = 0; u < D; ++u)
+            if (t0 + u < t1) fetch(u, t0 + u);
+        for (long long tb = t0; tb < t1 && open(); tb += D)
+#pragma unroll
+        for (int u = 0; u < D; ++u)
         {
-            const float4* at = v + 3 * (kBsBlock / 4) * t0 + 3 * lane;
-            a = __ldg(at + 0);
-            b = __ldg(at + 1);
-            c = __ldg(at + 2);
-        }
-        for (long long t = t0; t < t1 && open(); ++t)
-        {
-            const unsigned long long x01 = pack2(a.x, a.w), x23 = pack2(b.z, c.y);
-            const unsigned long long y01 = pack2(a.y, b.x), y23 = pack2(b.w, c.z);
-            const unsigned long long z01 = pack2(a.z, b.y), z23 = pack2(c.x, c.w);
-            if (t + 1 < t1)
-            {
-                const float4* next = v + 3 * (kBsBlock / 4) * (t + 1) + 3 * lane;
-                a = __ldg(next + 0);
-                b = __ldg(next + 1);
-                c = __ldg(next + 2);
-            }
+            const long long t = tb + u;
+            if (u > 0 && t >= t1) break;
+            const unsigned long long x01 = pack2(a[u].x, a[u].w), x23 = pack2(b[u].z, c[u].y);
+            const unsigned long long y01 = pack2(a[u].y, b[u].x), y23 = pack2(b[u].w, c[u].z);
+            const unsigned long long z01 = pack2(a[u].z, b[u].y), z23 = pack2(c[u].x, c[u].w);
+            if (t + D < t1) fetch(u, t + D);
             const long long k0 = head + t * kBsBlock;
 #pragma unroll
             for (int q = 0; q < Q; ++q)
@@ -251,6 +251,30 @@ __global__ void __launch_bounds__(kBsThreads)
 }
 
 template <bool PARTIAL, int Q, int W>
+__global__ void __launch_bounds__(kBsThreads)
+    ball_scan_kernel(long long total, int per_warp, long long n, long long m, float radius, int nsample,
+                     const float* __restrict__ y, const float* __restrict__ x, const int64_t* __restrict__ batch_x,
+                     const int64_t* __restrict__ batch_y, int64_t* __restrict__ idx_out, float* __restrict__ dist_out,
+                     const unsigned char* __restrict__ need, bool unless_most)
+{
+    ball_scan<PARTIAL, Q, W, 1>(total, per_warp, n, m, radius, nsample, y, x, batch_x, batch_y, idx_out, dist_out, need, unless_most);
+}
+
+// Two or four warps to a centre, long walks: they are too few for an SM to hide the latency with one block on its way
+// (1 x 65536 points, 1800 centres, 8 and 250 in reach 106 and 56 us with one, 99 and 50 with two, in 64
+// registers, so that all run at once; but 1 x 4096, 1024 centres 8.2 and 9.8, and eight warps, 8 x 131072, 64
+// centres, 64 and 67).
+template <int W>
+__global__ void __launch_bounds__(kBsThreads, 4)
+    ball_scan_shared_kernel(long long total, int per_warp, long long n, long long m, float radius, int nsample,
+                            const float* __restrict__ y, const float* __restrict__ x, const int64_t* __restrict__ batch_x,
+                            const int64_t* __restrict__ batch_y, int64_t* __restrict__ idx_out, float* __restrict__ dist_out,
+                            const unsigned char* __restrict__ need, bool unless_most)
+{
+    ball_scan<false, 1, W, 2>(total, per_warp, n, m, radius, nsample, y, x, batch_x, batch_y, idx_out, dist_out, need, unless_most);
+}
+
+template <bool PARTIAL, int Q, int W>
 int launch_ball_scan(long long total, int per_warp, long long n, long long m, float radius, int nsample, const float* y,
                      const float* x, const int64_t* batch_x, const int64_t* batch_y, int64_t* idx, float* dist,
                      const unsigned char* need, bool unless_most, cudaStream_t s)
@@ -260,8 +284,11 @@ int launch_ball_scan(long long total, int per_warp, long long n, long long m, fl
     TPK_REQUIRE(blocks < (1ll << 31), "ball_query: too many centres");
     const size_t smem = W > 1 ? sizeof(int2) * kBsThreads / 32 * nsample : 0;
     count_launches(1);
-    prefer_max_shared(ball_scan_kernel<PARTIAL, Q, W>);
-    ball_scan_kernel<PARTIAL, Q, W><<<static_cast<unsigned>(blocks), kBsThreads, smem, s>>>(
+    auto kernel = ball_scan_kernel<PARTIAL, Q, W>;
+    if constexpr (!PARTIAL && (W == 2 || W == 4))
+        if (n >= 32768) kernel = ball_scan_shared_kernel<W>;
+    prefer_max_shared(kernel);
+    kernel<<<static_cast<unsigned>(blocks), kBsThreads, smem, s>>>(
         total, per_warp, n, m, radius, nsample, y, x, batch_x, batch_y, idx, dist, need, unless_most);
     return check_launch("ball_query scan");
 }
