@@ -230,54 +230,51 @@ __global__ void __launch_bounds__(256)
     }
 }
 
-// Counters to first positions; one CTA per cloud.  cells: 8^bits, at least 64.
+// Counters to first positions, 8192 cells to a CTA.  cells: 8^bits, at least 64.  First (SUMS) what a CTA's cells hold,
+// in the words behind the box; then every CTA adds up those before it.  (One CTA per cloud took 187 us for 64^3
+// cells, 8 clouds; both together take 19.5.)
+constexpr int kLargeScanCells = 8192;
+
+template <bool SUMS>
 __global__ void __launch_bounds__(1024) large_scan_kernel(int n, int cells, int* __restrict__ counters)
 {
-    int* cnt = counters + static_cast<size_t>(blockIdx.x) * n;
-    __shared__ int s_warp[33];
+    int* cnt = counters + static_cast<size_t>(blockIdx.y) * n;
+    int* sums = cnt + cells + kLargeBoxInts;
+    __shared__ int s_warp[32];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    constexpr int V = 8;
-    int before = 0;
-    for (int c0 = 0; c0 < cells; c0 += 1024 * V)
+    constexpr int V = kLargeScanCells / 1024;
+    const int c = blockIdx.x * kLargeScanCells + tid * V;
+    int v[V], sum = 0;
+#pragma unroll
+    for (int i = 0; i < V; ++i)
     {
-        const int c = c0 + tid * V;
-        int v[V], sum = 0;
+        v[i] = c + i < cells ? cnt[c + i] : 0;
+        sum += v[i];
+    }
+    int incl = sum;
 #pragma unroll
-        for (int i = 0; i < V; ++i)
-        {
-            v[i] = c + i < cells ? cnt[c + i] : 0;
-            sum += v[i];
-        }
-        int incl = sum;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1)
-        {
-            const int t = __shfl_up_sync(kFullMask, incl, o);
-            if (lane >= o) incl += t;
-        }
-        if (lane == 31) s_warp[warp] = incl;
-        __syncthreads();
-        if (warp == 0)
-        {
-            int w = s_warp[lane];
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1)
-            {
-                const int t = __shfl_up_sync(kFullMask, w, o);
-                if (lane >= o) w += t;
-            }
-            s_warp[lane] = w;
-        }
-        __syncthreads();
-        int run = before + (warp ? s_warp[warp - 1] : 0) + incl - sum;
+    for (int o = 1; o < 32; o <<= 1)
+    {
+        const int t = __shfl_up_sync(kFullMask, incl, o);
+        if (lane >= o) incl += t;
+    }
+    if (lane == 31) s_warp[warp] = incl;
+    __syncthreads();
+    int run = incl - sum;
+    for (int w = 0; w < warp; ++w) run += s_warp[w];
+    if constexpr (SUMS)
+    {
+        if (tid == 1023) sums[blockIdx.x] = run + sum;
+    }
+    else
+    {
+        for (unsigned k = 0; k < blockIdx.x; ++k) run += sums[k];
 #pragma unroll
         for (int i = 0; i < V; ++i)
         {
             if (c + i < cells) cnt[c + i] = run;
             run += v[i];
         }
-        before += s_warp[31];
-        __syncthreads();
     }
 }
 
@@ -1273,7 +1270,8 @@ int launch_large(int b, int n, int m, int log2bs, int nranks, const LargeLayout&
 
 int sort_points(int b, int n, const float* xyz, float4* sorted, int* counters, cudaStream_t stream)
 {
-    // about four points per cell and at most 64^3 cells; the counters need kLargeBoxInts words more
+    // about four points per cell and at most 64^3 cells; the counters need kLargeBoxInts words more, and one for
+    // every 8192 cells
     int bits = 2;
     while (bits < 6 && (32ll << (3 * bits)) <= n) ++bits;
     const unsigned blocks = static_cast<unsigned>(n < 256 * 4 ? 1 : (n / (256 * 4) < 592 ? n / (256 * 4) : 592));
@@ -1293,7 +1291,9 @@ int sort_points(int b, int n, const float* xyz, float4* sorted, int* counters, c
         count_launches(1), large_clear_kernel<<<dim3(blocks < 64 ? blocks : 64, nb), 256, 0, stream>>>(n, cells, c);
         count_launches(1), large_box_kernel<<<dim3(blocks + 1, nb), 256, 0, stream>>>(n, cells, x, c);
         count_launches(1), large_cells_kernel<false><<<grid, 256, 0, stream>>>(n, bits, x, c, s);
-        count_launches(1), large_scan_kernel<<<nb, 1024, 0, stream>>>(n, cells, c);
+        const unsigned parts = static_cast<unsigned>((cells + kLargeScanCells - 1) / kLargeScanCells);
+        if (parts > 1) count_launches(1), large_scan_kernel<true><<<dim3(parts, nb), 1024, 0, stream>>>(n, cells, c);
+        count_launches(1), large_scan_kernel<false><<<dim3(parts, nb), 1024, 0, stream>>>(n, cells, c);
         count_launches(1), large_cells_kernel<true><<<grid, 256, 0, stream>>>(n, bits, x, c, s);
     }
     return check_launch("fps sort");
