@@ -14,8 +14,8 @@
 // in shared memory first.  A tiled transposition writes the result.
 //
 // Bound by the rate of the reductions in L2 and the gradient's bytes: 16 clouds of 16384 points, 64 channels,
-// 4096 x 32 positions (537 MB, 82 us at the copy bandwidth) 212 us, 297 through the inverted index of
-// scatter_sorted.cu; all four levels of the benchmark's step 410 and 582; interpolation 113 and 187.
+// 4096 x 32 positions (537 MB, 82 us at the copy bandwidth) 204 us, 297 through the inverted index of
+// scatter_sorted.cu; all four levels of the benchmark's step 395 and 582; interpolation 112 and 187.
 //
 // semantics: autograd's scatter-add backward of the gather at torch_points_kernels/torchpoints.py:129-146,
 // and cuda/src/interpolate_gpu.cu:122-152.
@@ -47,18 +47,19 @@ struct ColsWarp
 // Warp w of a cloud and channel tile takes positions [32 w, 32 w + 32).
 template <int K>
 __global__ void __launch_bounds__(kColsThreads)
-    scatter_cols_kernel(int c, int n, long long ps, long long gbs, int tile, int tiles, long long blocks,
+    scatter_cols_kernel(int c, int n, long long ps, long long gbs, int tile, unsigned tiles, unsigned blocks,
                         const float* __restrict__ grad_out, const void* __restrict__ idx_all, const float* __restrict__ weight,
                         float* __restrict__ sums)
 {
     __shared__ ColsWarp s_warp[kColsWarps];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     ColsWarp& s = s_warp[warp];
-    const long long cloud = blockIdx.x / (tiles * blocks);
-    const long long rest = blockIdx.x - cloud * (tiles * blocks);
-    const int c0 = static_cast<int>(rest / blocks) * tile;
-    const int nc = min(tile, c - c0);
-    const long long p0 = ((rest % blocks) * kColsWarps + warp) * 32;
+    // (in 32 bits: by 64-bit divisions 16 x 64 x 16384, 4096 x 32 positions took 212 us against 204, and 8 x 96 x 32768
+    // 586 against 561)
+    const unsigned row = blockIdx.x / blocks, cloud = row / tiles;
+    const int c0 = static_cast<int>(row - cloud * tiles) * tile;
+    const int nc = min(tile, c - c0), nc4 = (nc + 3) & ~3;
+    const long long p0 = (static_cast<long long>(blockIdx.x - row * blocks) * kColsWarps + warp) * 32;
     if (p0 >= ps) return;
     const bool in = p0 + lane < ps;
 
@@ -87,10 +88,11 @@ __global__ void __launch_bounds__(kColsThreads)
     for (int r = 0; r < kColsMax; ++r)
         if (r < nc) v[r] = __ldcs(g + static_cast<size_t>(r) * ps);
 #pragma unroll
-    for (int r = 0; r < kColsMax; ++r) s.v[r * kColsPitch + lane] = r < nc ? v[r] : 0.f;
+    for (int r = 0; r < kColsMax; ++r)
+        if (r < nc4) s.v[r * kColsPitch + lane] = r < nc ? v[r] : 0.f;
     __syncwarp();
 
-    const int quads = (nc + 3) >> 2;    // 16-byte pieces of a position's channels
+    const int quads = nc4 >> 2;         // 16-byte pieces of a position's channels
     const int at_once = 32 / quads;     // positions per reduction
     const int mine = lane / quads, quad = lane - mine * quads;
     const int pitch = cols_pitch(c);
@@ -158,9 +160,8 @@ __global__ void __launch_bounds__(kColsThreads)
 {
     __shared__ float tile[64][33];
     const int lane = threadIdx.x & 31, line = threadIdx.x >> 5;
-    const long long cloud = blockIdx.x / (static_cast<long long>(tiles_n) * tiles_c);
-    const int rest = static_cast<int>(blockIdx.x - cloud * tiles_n * tiles_c);
-    const int t0 = rest / tiles_c * 64, c0 = rest % tiles_c * 32;
+    const unsigned row = blockIdx.x / static_cast<unsigned>(tiles_c), cloud = row / static_cast<unsigned>(tiles_n);
+    const int t0 = static_cast<int>(row - cloud * tiles_n) * 64, c0 = static_cast<int>(blockIdx.x - row * tiles_c) * 32;
     const int pitch = cols_pitch(c);
     const float* src = sums + static_cast<size_t>(cloud) * n * pitch;
     float* dst = grad + static_cast<size_t>(cloud) * c * n;
@@ -199,7 +200,7 @@ int scatter_cols(int b, int c, int n, long long ps, long long gbs, const float* 
     TPK_REQUIRE(grid < (1ll << 31) && grid2 < (1ll << 31), "%s: grid too large", what);
     prefer_max_shared(scatter_cols_kernel<K>);
     count_launches(1), scatter_cols_kernel<K><<<static_cast<unsigned>(grid), kColsThreads, 0, s>>>(
-        c, n, ps, gbs, tile, tiles, blocks, grad_out, idx, weight, sums);
+        c, n, ps, gbs, tile, static_cast<unsigned>(tiles), static_cast<unsigned>(blocks), grad_out, idx, weight, sums);
     prefer_max_shared(cols_to_rows_kernel);
     count_launches(1), cols_to_rows_kernel<<<static_cast<unsigned>(grid2), kColsThreads, 0, s>>>(c, n, tn, tc, sums, grad);
     return check_launch(what);
@@ -216,8 +217,8 @@ bool cols_fit(int b, int c, int n, long long ps)
 }
 
 // Where three launches (zeros, sums, transposition; 8 us at least) pay.  us, rows of atomics or inverted index
-// and columns: 16 clouds of 16384 points, 64 channels, 4096 x 32 positions 297 and 212, 4096 points x 128 channels
-// 165 and 109, 256 x 512 46 and 32; one cloud 59 and 19; 8 x 32768 x 96, 8192 x 64 positions 1199 and 586; but 16 x
+// and columns: 16 clouds of 16384 points, 64 channels, 4096 x 32 positions 297 and 204, 4096 points x 128 channels
+// 165 and 104, 256 x 512 46 and 31; one cloud 59 and 19; 8 x 32768 x 96, 8192 x 64 positions 1199 and 561; but 16 x
 // 256 x 64, 64 x 32 positions 9.2 and 10.2, 4 x 2048 x 180, 512 x 16 16.3 and 18.1.  The rows cost the positions times
 // the rows that an SM has; neighbourhoods of a size that is no power of two, whose padding the rows do not
 // sum first, up to several times that (8 x 64 x 192, 16 x 48 positions 31 and 8.4; 3 x 625 x 140, 156 x 24
@@ -231,8 +232,8 @@ bool cols_pay_grouping(int b, int c, long long ps, int nsample)
     return 8.2 + 1.5e-6 * static_cast<double>(rows) * static_cast<double>(ps) < by_rows;
 }
 
-// us, rows of atomics and columns: 16 clouds of 16384 points from 4096, 64 channels 86 and 50; one cloud 42 and
-// 10; 1 x 600 from 150 points, 96 channels 16 and 9.4; 16 x 512 x 16 14 and 8.3; 16 x 256 x 64 9.3 and 9.7,
+// us, rows of atomics and columns: 16 clouds of 16384 points from 4096, 64 channels 86 and 49; one cloud 42 and
+// 9; 1 x 600 from 150 points, 96 channels 16 and 9.4; 16 x 512 x 16 14 and 8.3; 16 x 256 x 64 9.3 and 9.7,
 // 16 x 256 x 512 14.0 and 13.7.
 bool cols_pay_interp(int n) { return n >= 384 || test_path("scatter_cols"); }
 
