@@ -293,6 +293,14 @@ TPK_API int tpk_grouping(int b, int c, int n, int npoint, int nsample, const flo
                  const int64_t* idx, float* out, void* stream);
 
 /*
+ * The same by a 16-bit copy of the indices, which is made in `scratch` (16-byte aligned) and read once for every two
+ * rows of features.  tpk_grouping_scratch_bytes: 0 where the call above is the faster one (this one then is the same).
+ */
+TPK_API int tpk_grouping_ws(int b, int c, int n, int npoint, int nsample, const float* features, const int64_t* idx,
+                            float* out, void* scratch, int64_t scratch_bytes, void* stream);
+TPK_API int64_t tpk_grouping_scratch_bytes(int b, int c, int n, int npoint, int nsample);
+
+/*
  * grad_features[b,c,idx[b,p,s]] += grad_out[b,c,p,s]; grad_features (b,c,n) is fully
  * written.  Stands in for autograd's scatter-add backward of the gather at
  * torch_points_kernels/torchpoints.py:145.

@@ -1173,6 +1173,50 @@ def test_gradients_by_columns(B, C, N, P, S, kind, skip, monkeypatch):
     assert bool(((want - got).abs() <= (terms + 1) * 2.0 ** -24 * size + 1e-30).all())  # (+ 1: the products)
 
 
+@pytest.mark.parametrize("B,C,N,P,S", [
+    (2, 17, 1023, 8192, 32),     # one point short of the 16-bit copy
+    (2, 17, 1024, 8192, 32),     # four rows a CTA, the last alone
+    (3, 16, 1025, 7001, 28),     # two rows; a part that is not full
+    (1, 64, 14336, 4681, 28), (1, 65, 14337, 4681, 28),    # the largest rows of which two CTAs fit an SM, and the next
+    (2, 16, 25600, 2731, 96), (2, 19, 25601, 2731, 96),    # two rows of 1024 threads, one
+    (2, 16, 51200, 2731, 96), (1, 16, 51201, 5462, 96),    # the longest rows that fit, and the next
+])
+def test_grouping_by_short_indices(B, C, N, P, S):
+    """Forward grouping of many values against an indexed gather, bit for bit, with indices at both ends of the
+    rows and some that address nothing (zeros, and the status word)."""
+    g = data.gen(N + P)
+    idx = torch.randint(0, N, (B, P, S), generator=g)
+    idx[:, 0, 0], idx[:, -1, -1] = 0, N - 1
+    features = torch.randn(B, C, N, generator=g)
+    want = torch.gather(cu(features), 2, cu(idx).view(B, 1, -1).expand(-1, C, -1)).view(B, C, P, S)
+    _lib.device_status()
+    assert torch.equal(tpk.grouping_operation(cu(features), cu(idx)), want)
+    assert _lib.device_status() == 0
+    idx[:, ::5, 3] = N
+    idx[:, 1::5, 3] = -1
+    idx[:, 2::5, 3] = 65535 + N
+    want[:, :, ::5, 3], want[:, :, 1::5, 3], want[:, :, 2::5, 3] = 0, 0, 0
+    assert torch.equal(tpk.grouping_operation(cu(features), cu(idx)), want)
+    assert _lib.device_status() == 2
+
+
+@pytest.mark.parametrize("B,C,M,N", [
+    (1, 9, 300, 1024), (1, 33, 50, 1025), (2, 7, 1000, 4100),   # four rows; without shared rows, few channels a CTA
+    (2, 64, 3590, 32768), (2, 65, 3572, 32768),                 # eight rows: of 512 threads, of 256
+    (3, 70, 12800, 20004), (16, 33, 12801, 16388),              # the longest rows that fit, and the next
+])
+def test_interpolation_by_rows_and_parts(B, C, M, N):
+    """Forward interpolation in every split of its positions against the same sum of three products."""
+    g = data.gen(M + N)
+    p, w = torch.randn(B, C, M, generator=g), torch.rand(B, N, 3, generator=g)
+    idx = torch.randint(0, M, (B, N, 3), generator=g).int()
+    k = [torch.gather(cu(p), 2, cu(idx)[:, :, t].long().unsqueeze(1).expand(-1, C, -1)) * cu(w)[:, :, t].unsqueeze(1)
+         for t in range(3)]
+    # (each side rounds its two sums: 2 * 2^-24 of the magnitudes, and as much again)
+    got, size = tpk.three_interpolate(cu(p), cu(idx), cu(w)), k[0].abs() + k[1].abs() + k[2].abs()
+    assert bool(((got - (k[0] + k[1] + k[2])).abs() <= 2.0 ** -22 * size).all())
+
+
 @pytest.mark.parametrize("B,N,M,C,r", [(2, 16384, 4096, 64, 0.1), (3, 4096, 1024, 7, 0.2), (2, 500, 100, 130, 0.4),
                                        (1, 70000, 64, 3, 0.05), (2, 1024, 256, 0, 0.3)])
 def test_fused_sa_group_equals_the_unfused_sequence(B, N, M, C, r):

@@ -39,6 +39,7 @@ _SIGNATURES = {
     "tpk_three_interpolate": [_c_int, _c_int, _c_int, _c_int, _ptr, _ptr, _ptr, _ptr, _ptr],
     "tpk_three_interpolate_grad": [_c_int, _c_int, _c_int, _c_int, _ptr, _ptr, _ptr, _ptr, _ptr],
     "tpk_grouping": [_c_int, _c_int, _c_int, _c_int, _c_int, _ptr, _ptr, _ptr, _ptr],
+    "tpk_grouping_ws": [_c_int, _c_int, _c_int, _c_int, _c_int, _ptr, _ptr, _ptr, _ptr, _c_i64, _ptr],
     "tpk_grouping_grad": [_c_int, _c_int, _c_int, _c_int, _c_int, _ptr, _ptr, _ptr, _ptr],
     "tpk_grouping_grad_ws": [_c_int, _c_int, _c_int, _c_int, _c_int, _ptr, _ptr, _ptr, _ptr, _c_i64, _ptr],
     "tpk_grouping_grad_cols": [_c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _ptr, _ptr, _ptr, _ptr, _c_i64, _ptr],
@@ -72,7 +73,8 @@ EXPORTS = sorted(list(_SIGNATURES) + ["tpk_version", "tpk_last_error", "tpk_devi
                                        "tpk_three_nn_scratch_bytes", "tpk_chamfer_dist_scratch_bytes",
                                        "tpk_ball_query_partial_dense_scratch_bytes", "tpk_knn_dense_scratch_bytes", "tpk_sa_group_scratch_bytes",
                                        "tpk_knn_partial_dense_scratch_bytes", "tpk_cubic_feature_sampling_scratch_bytes",
-                                       "tpk_grouping_grad_scratch_bytes", "tpk_grouping_grad_cols_scratch_bytes",
+                                       "tpk_grouping_scratch_bytes", "tpk_grouping_grad_scratch_bytes",
+                                       "tpk_grouping_grad_cols_scratch_bytes",
                                        "tpk_three_interpolate_grad_cols_scratch_bytes",
                                        "tpk_three_nn_sorted_scratch_bytes", "tpk_chamfer_dist_sorted_scratch_bytes"])
 
@@ -117,6 +119,8 @@ def lib():
         handle.tpk_knn_partial_dense_scratch_bytes.restype = _c_i64
         handle.tpk_sa_group_scratch_bytes.argtypes = [_c_int, _c_int, _c_int, _c_int]
         handle.tpk_sa_group_scratch_bytes.restype = _c_i64
+        handle.tpk_grouping_scratch_bytes.argtypes = [_c_int, _c_int, _c_int, _c_int, _c_int]
+        handle.tpk_grouping_scratch_bytes.restype = _c_i64
         handle.tpk_grouping_grad_cols_scratch_bytes.argtypes = [_c_int, _c_int, _c_int, _c_int, _c_int]
         handle.tpk_grouping_grad_cols_scratch_bytes.restype = _c_i64
         handle.tpk_three_interpolate_grad_cols_scratch_bytes.argtypes = [_c_int, _c_int, _c_int, _c_int]

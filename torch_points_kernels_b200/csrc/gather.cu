@@ -29,6 +29,7 @@ constexpr int kGatherThreads = 256;
 constexpr int kScatterThreads = 512;
 constexpr int kChanChunk = 16;
 constexpr size_t kRowSmemBudget = 200 * 1024;
+constexpr size_t kRowSmemPerSm = 228 * 1024;
 
 // p1*w1 + p2*w2 + p3*w3 as nvcc contracts the reference expression (interpolate_gpu.cu:105)
 __device__ __forceinline__ float interp3(float p1, float w1, float p2, float w2, float p3, float w3)
@@ -57,14 +58,14 @@ __device__ __forceinline__ float ldg_or_zero(const float* row, int i) { return i
 
 // ------------------------------------------------------------------ grouping forward
 
-template <bool VEC>
+template <bool VEC, int CHAN>
 __global__ void __launch_bounds__(kGatherThreads)
     grouping_fwd_kernel(int c, int n, long long ps, int out_c, int out_off, const float* __restrict__ features,
                         const int64_t* __restrict__ idx, float* __restrict__ out)
 {
     const int bi = blockIdx.z;
-    const int c0 = blockIdx.y * kChanChunk;
-    const int c1 = min(c, c0 + kChanChunk);
+    const int c0 = blockIdx.y * CHAN;
+    const int c1 = min(c, c0 + CHAN);
     const long long pos = (static_cast<long long>(blockIdx.x) * kGatherThreads + threadIdx.x) * 4;
     if (pos >= ps) return;
     const int64_t* ip = idx + static_cast<size_t>(bi) * ps + pos;
@@ -151,6 +152,32 @@ __device__ __forceinline__ bool wait_bulk_copy(uint32_t mbar)
 // indices loaded once (two 16-byte loads), ROWS x 4 shared-memory gathers, ROWS 16-byte
 // streaming stores.  Gathering from shared memory instead of L1/L2 removes the
 // sector-per-lane traffic that bounds the direct-gather kernel.
+// Channels that a CTA of the kernels without shared rows loops over: kChanChunk, a quarter where the positions alone
+// give less than two CTAs an SM (interpolation, 3 x 35 x 10007: 13.4 us -> 10.7; 3 x 70 x 2501: 10.1 -> 6.7).
+inline int channels_per_cta(long long ctas, int c)
+{
+    return ctas * ((c + kChanChunk - 1) / kChanChunk) < 2ll * num_sms() ? kChanChunk / 4 : kChanChunk;
+}
+
+// Positions that a CTA of the row-resident kernels takes, a multiple of the 4 x `threads` that one sweep covers: the
+// split into up to 64 parts whose whole waves take the least time, where rows are staged in the time of `stage`
+// positions.  (Interpolation, 1 x 128 x 4096 of 1024: 11.2 us by parts of 4096 and more, 5.1 by this; 3 x 35 x 10008
+// 13.3, 7.5; grouping, 8 x 192 x 8192 -> 2048 x 64: 214, 168.)
+inline long long split_positions(long long groups, long long ps, int threads, long long stage, size_t smem)
+{
+    int per_sm = static_cast<int>(kRowSmemPerSm / (smem + 2048));
+    per_sm = per_sm > 2048 / threads ? 2048 / threads : (per_sm < 1 ? 1 : per_sm);
+    const long long slots = static_cast<long long>(per_sm) * num_sms(), sweep = 4ll * threads;
+    long long best = -1, chunk = 0;
+    for (long long t = 1; t == 1 || (t <= 64 && t * sweep < ps + sweep); ++t)
+    {
+        const long long len = ((ps + t - 1) / t + sweep - 1) / sweep * sweep;
+        const long long cost = (groups * ((ps + len - 1) / len) + slots - 1) / slots * (len + stage);
+        if (best < 0 || cost < best) best = cost, chunk = len;
+    }
+    return chunk;
+}
+
 // Four consecutive indices of a position run: int64 as the callers pass them, or the 16-bit
 // copy the fused set-abstraction op makes (0xFFFF = out of range).
 constexpr uint16_t kBadIdx16 = 0xFFFFu;
@@ -172,8 +199,8 @@ __device__ __forceinline__ void load_four(const uint16_t* p, int, bool&, int& i0
     i3 = a.w == kBadIdx16 ? -1 : a.w;
 }
 
-template <int ROWS, class IdxT>
-__global__ void __launch_bounds__(kScatterThreads)
+template <int ROWS, class IdxT, int THREADS>
+__global__ void __launch_bounds__(THREADS)
     grouping_fwd_rows_kernel(int c, int n, long long ps, long long chunk, int use_tma, int out_c, int out_off,
                              const float* __restrict__ features, const IdxT* __restrict__ idx,
                              float* __restrict__ out)
@@ -214,7 +241,7 @@ __global__ void __launch_bounds__(kScatterThreads)
     }
     if (!use_tma)
     {
-        for (int i = threadIdx.x; i < nrows * n; i += kScatterThreads) rows[i] = __ldg(src + i);
+        for (int i = threadIdx.x; i < nrows * n; i += THREADS) rows[i] = __ldg(src + i);
         __syncthreads();
     }
 
@@ -223,7 +250,7 @@ __global__ void __launch_bounds__(kScatterThreads)
     const IdxT* ib = idx + static_cast<size_t>(bi) * ps;
     float* ob = out + (static_cast<size_t>(bi) * out_c + out_off + c0) * ps;
     bool bad = false;
-    for (long long p = p0 + static_cast<long long>(threadIdx.x) * 4; p < p1; p += kScatterThreads * 4)
+    for (long long p = p0 + static_cast<long long>(threadIdx.x) * 4; p < p1; p += THREADS * 4)
     {
         int i0, i1, i2, i3;
         load_four(ib + p, n, bad, i0, i1, i2, i3);
@@ -242,11 +269,11 @@ __global__ void __launch_bounds__(kScatterThreads)
     report_bad(bad);
 }
 
-template <int ROWS, class IdxT>
+template <int ROWS, class IdxT, int THREADS>
 int launch_grouping_fwd_rows(int b, int c, int n, long long ps, int out_c, int out_off, const float* features,
                              const IdxT* idx, float* out, cudaStream_t s)
 {
-    auto kernel = grouping_fwd_rows_kernel<ROWS, IdxT>;
+    auto kernel = grouping_fwd_rows_kernel<ROWS, IdxT, THREADS>;
     prefer_max_shared(kernel);
     const size_t smem = static_cast<size_t>(ROWS) * n * sizeof(float);
     if (smem > kDynSmemOptIn)
@@ -260,33 +287,26 @@ int launch_grouping_fwd_rows(int b, int c, int n, long long ps, int out_c, int o
         }
     }
     const long long groups = static_cast<long long>(b) * ((c + ROWS - 1) / ROWS);
-    // split the positions so that every SM gets a few CTAs, in multiples of the 2048
-    // positions one sweep of the CTA covers
-    long long nchunks = (4ll * num_sms() + groups - 1) / groups;
-    const long long max_chunks = (ps + 8191) / 8192;
-    if (nchunks > max_chunks) nchunks = max_chunks;
-    if (nchunks < 1) nchunks = 1;
-    long long chunk = (ps + nchunks - 1) / nchunks;
-    chunk = (chunk + 2047) / 2048 * 2048;
-    nchunks = (ps + chunk - 1) / chunk;
+    const long long chunk = split_positions(groups, ps, THREADS, n / 2, smem);
+    const long long nchunks = (ps + chunk - 1) / chunk;
     TPK_REQUIRE(groups <= 65535 && nchunks < (1ll << 31), "grouping: grid too large");
     const int use_tma = (n % 4 == 0) && ((reinterpret_cast<uintptr_t>(features) & 15u) == 0);
     const dim3 g(static_cast<unsigned>(nchunks), static_cast<unsigned>(groups));
-    count_launches(1), kernel<<<g, kScatterThreads, smem, s>>>(c, n, ps, chunk, use_tma, out_c, out_off, features, idx, out);
+    count_launches(1), kernel<<<g, THREADS, smem, s>>>(c, n, ps, chunk, use_tma, out_c, out_off, features, idx, out);
     return check_launch("grouping");
 }
 
 // ---------------------------------------------------------- three_interpolate forward
 
-template <bool VEC>
+template <bool VEC, int CHAN>
 __global__ void __launch_bounds__(kGatherThreads)
     interp_fwd_kernel(int c, int m, int n, const float* __restrict__ points,
                       const int32_t* __restrict__ idx, const float* __restrict__ weight,
                       float* __restrict__ out)
 {
     const int bi = blockIdx.z;
-    const int c0 = blockIdx.y * kChanChunk;
-    const int c1 = min(c, c0 + kChanChunk);
+    const int c0 = blockIdx.y * CHAN;
+    const int c1 = min(c, c0 + CHAN);
     const int j0 = (blockIdx.x * kGatherThreads + threadIdx.x) * 4;
     if (j0 >= n) return;
     bool bad = false;
@@ -332,8 +352,8 @@ __global__ void __launch_bounds__(kGatherThreads)
 // with TMA bulk copies, then every thread produces four consecutive outputs per row
 // from 12 shared-memory gathers; the 12 indices and weights of its four points are
 // loaded once (six 16-byte loads) for all rows.
-template <int ROWS>
-__global__ void __launch_bounds__(kGatherThreads)
+template <int ROWS, int THREADS>
+__global__ void __launch_bounds__(THREADS)
     interp_fwd_rows_kernel(int c, int m, int n, int chunk, int use_tma,
                            const float* __restrict__ points, const int32_t* __restrict__ idx,
                            const float* __restrict__ weight, float* __restrict__ out)
@@ -370,14 +390,14 @@ __global__ void __launch_bounds__(kGatherThreads)
     }
     if (!use_tma)
     {
-        for (int i = threadIdx.x; i < nrows * m; i += kGatherThreads) rows[i] = __ldg(src + i);
+        for (int i = threadIdx.x; i < nrows * m; i += THREADS) rows[i] = __ldg(src + i);
         __syncthreads();
     }
 
     const int j_begin = blockIdx.x * chunk;
     const int j_end = min(n, j_begin + chunk);
     bool bad = false;
-    for (int j0 = j_begin + threadIdx.x * 4; j0 < j_end; j0 += kGatherThreads * 4)
+    for (int j0 = j_begin + threadIdx.x * 4; j0 < j_end; j0 += THREADS * 4)
     {
         const size_t o = (static_cast<size_t>(bi) * n + j0) * 3;  // multiple of 12: 16-byte aligned
         int id[12];
@@ -410,11 +430,11 @@ __global__ void __launch_bounds__(kGatherThreads)
     report_bad(bad);
 }
 
-template <int ROWS>
+template <int ROWS, int THREADS>
 int launch_interp_fwd_rows(int b, int c, int m, int n, const float* points, const int32_t* idx,
                            const float* weight, float* out, cudaStream_t s)
 {
-    auto kernel = interp_fwd_rows_kernel<ROWS>;
+    auto kernel = interp_fwd_rows_kernel<ROWS, THREADS>;
     prefer_max_shared(kernel);
     const size_t smem = static_cast<size_t>(ROWS) * m * sizeof(float);
     if (smem > kDynSmemOptIn)
@@ -428,18 +448,13 @@ int launch_interp_fwd_rows(int b, int c, int m, int n, const float* points, cons
         }
     }
     const long long groups = static_cast<long long>(b) * ((c + ROWS - 1) / ROWS);
-    long long nchunks = (4ll * num_sms() + groups - 1) / groups;
-    const long long max_chunks = (n + 4095) / 4096;
-    if (nchunks > max_chunks) nchunks = max_chunks;
-    if (nchunks < 1) nchunks = 1;
-    int chunk = static_cast<int>((n + nchunks - 1) / nchunks);
-    chunk = (chunk + 1023) / 1024 * 1024;
-    nchunks = (n + chunk - 1) / chunk;
+    const int chunk = static_cast<int>(split_positions(groups, n, THREADS, m / 2, smem));
+    const long long nchunks = (n + static_cast<long long>(chunk) - 1) / chunk;
     TPK_REQUIRE(groups <= 65535, "three_interpolate: grid too large");
     const int use_tma = (m % 4 == 0) && ((reinterpret_cast<uintptr_t>(points) & 15u) == 0) &&
                         static_cast<size_t>(ROWS) * m * 4 < (1u << 20);
     const dim3 g(static_cast<unsigned>(nchunks), static_cast<unsigned>(groups));
-    count_launches(1), kernel<<<g, kGatherThreads, smem, s>>>(c, m, n, chunk, use_tma, points, idx, weight, out);
+    count_launches(1), kernel<<<g, THREADS, smem, s>>>(c, m, n, chunk, use_tma, points, idx, weight, out);
     return check_launch("three_interpolate");
 }
 
@@ -882,15 +897,22 @@ int grouping_forward(int b, int c, int n, long long ps, int out_c, int out_off, 
     if (ps % 4 == 0 && aligned16(idx) && aligned16(out) && row_bytes <= kRowSmemBudget && ps >= 4096 &&
         static_cast<long long>(b) * c <= 65535 && !test_path("gather_direct"))
     {
-        // rows per CTA: as many as fit the shared memory of one SM, at most 4 (the indices
-        // of a position are loaded once for all rows of the CTA)
-        int rows = static_cast<int>(kRowSmemBudget / row_bytes);
-        if (rows < 1) rows = 1;
-        if (rows > 4) rows = 4;
+        // Rows per CTA: 16-bit indices are read so cheaply that two rows share them, four of up to 1024 points; 64-bit
+        // ones are shared by as many rows as fit, at most 4.  Where two CTAs do not fit an SM, one of 1024 threads.
+        // us at 16 x 64 x 16384 -> 4096 x 32, three rows of 512 threads and 64 bits 161; 16 bits: 143, one / two rows of
+        // 1024 threads 120 / 112 (HBM: 95).  16 x 128 x 4096 -> 1024 x 32: 61; 16 bits, four rows 56, two 53.
+        // 16 x 256 x 1024 -> 256 x 32: two rows 29, four 25.  8 x 96 x 32768 -> 8192 x 64: 512 threads 785, 16 bits 645,
+        // 1024 threads 424 (there gathers from shared memory, three or four banks deep, bound it: HBM 267).
+        int rows = idx16 && n > 1024 ? 2 : 4;
+        while (rows > 1 && rows * row_bytes > kRowSmemBudget) --rows;
         if (rows > c) rows = c;
+        const bool two = 2 * (rows * row_bytes + 2048) <= kRowSmemPerSm;
+#define TPK_GFT(R, T)                                                                                                  \
+    return idx16 ? launch_grouping_fwd_rows<R, uint16_t, T>(b, c, n, ps, out_c, out_off, features, idx16, out, s)      \
+                 : launch_grouping_fwd_rows<R, int64_t, T>(b, c, n, ps, out_c, out_off, features, idx, out, s)
 #define TPK_GF(R)                                                                                                      \
-    return idx16 ? launch_grouping_fwd_rows<R, uint16_t>(b, c, n, ps, out_c, out_off, features, idx16, out, s)         \
-                 : launch_grouping_fwd_rows<R, int64_t>(b, c, n, ps, out_c, out_off, features, idx, out, s)
+    if (two) TPK_GFT(R, 512);                                                                                          \
+    TPK_GFT(R, 1024)
         switch (rows)
         {
         case 1: TPK_GF(1);
@@ -898,16 +920,18 @@ int grouping_forward(int b, int c, int n, long long ps, int out_c, int out_off, 
         case 3: TPK_GF(3);
         default: TPK_GF(4);
         }
+#undef TPK_GFT
 #undef TPK_GF
     }
     const long long gx = (ps + kGatherThreads * 4 - 1) / (kGatherThreads * 4);
-    const int gy = (c + kChanChunk - 1) / kChanChunk;
+    const int chan = channels_per_cta(gx * b, c), gy = (c + chan - 1) / chan;
     TPK_REQUIRE(gx < (1ll << 31) && gy <= 65535 && b <= 65535, "grouping: grid too large");
     const dim3 g(static_cast<unsigned>(gx), gy, b);
+    const auto launch = [&](auto kernel) { count_launches(1), kernel<<<g, kGatherThreads, 0, s>>>(c, n, ps, out_c, out_off, features, idx, out); };
     if (ps % 4 == 0 && aligned16(idx) && aligned16(out))
-        count_launches(1), grouping_fwd_kernel<true><<<g, kGatherThreads, 0, s>>>(c, n, ps, out_c, out_off, features, idx, out);
+        launch(chan == kChanChunk ? grouping_fwd_kernel<true, kChanChunk> : grouping_fwd_kernel<true, kChanChunk / 4>);
     else
-        count_launches(1), grouping_fwd_kernel<false><<<g, kGatherThreads, 0, s>>>(c, n, ps, out_c, out_off, features, idx, out);
+        launch(chan == kChanChunk ? grouping_fwd_kernel<false, kChanChunk> : grouping_fwd_kernel<false, kChanChunk / 4>);
     return check_launch("grouping");
 }
 
@@ -939,6 +963,20 @@ __global__ void __launch_bounds__(kGatherThreads)
     report_bad(bad);
 }
 
+// The 16-bit copy alone, four indices a thread.
+__global__ void __launch_bounds__(kGatherThreads)
+    narrow_idx_kernel(long long fours, int n, const int64_t* __restrict__ idx, uint16_t* __restrict__ idx16)
+{
+    const long long t = static_cast<long long>(blockIdx.x) * kGatherThreads + threadIdx.x;
+    if (t >= fours) return;
+    bool bad = false;
+    int i0, i1, i2, i3;
+    load_four(idx + 4 * t, n, bad, i0, i1, i2, i3);
+    reinterpret_cast<ushort4*>(idx16)[t] =
+        make_ushort4(static_cast<uint16_t>(i0), static_cast<uint16_t>(i1), static_cast<uint16_t>(i2), static_cast<uint16_t>(i3));
+    report_bad(bad);
+}
+
 __global__ void __launch_bounds__(kGatherThreads)
     gather_centres_kernel(long long total, int n, int m, const float* __restrict__ xyz, const int32_t* __restrict__ fps_idx,
                           float* __restrict__ new_xyz)
@@ -965,6 +1003,44 @@ extern "C" int tpk_grouping(int b, int c, int n, int npoint, int nsample, const 
     if (b == 0 || c == 0 || ps == 0) return TPK_OK;
     TPK_REQUIRE(features && idx && out && n > 0, "grouping: NULL pointer or empty feature row");
     return grouping_forward(b, c, n, ps, c, 0, features, idx, nullptr, out, static_cast<cudaStream_t>(stream));
+}
+
+extern "C" int64_t tpk_grouping_scratch_bytes(int b, int c, int n, int npoint, int nsample)
+{
+    using namespace tpk;
+    if (b <= 0 || c <= 0 || n <= 0 || npoint <= 0 || nsample <= 0) return 0;
+    const int64_t ps = static_cast<int64_t>(npoint) * nsample, total = ps * b;
+    // (what the rows of grouping_forward ask, and enough values that the pass over the indices comes back, us without and with it:
+    // 16 x 64 x 16384 -> 4096 x 32 161, 111; 2 x 32 x 50000 -> 12500 x 32 35, 23; 1 x 64 x 16384 -> 4096 x 32 11.6, 10.7;
+    // but 1 x 128 x 4096 -> 1024 x 32 7.0, 7.7 and 16 x 512 x 256 -> 64 x 32 15.3, 16.4)
+    const bool pays = n >= 1024 && n < kBadIdx16 && static_cast<size_t>(n) * sizeof(float) <= kRowSmemBudget && ps % 4 == 0 &&
+                      ps >= 4096 && static_cast<int64_t>(b) * c <= 65535 && total <= (1ll << 38) &&
+                      total * c >= (1ll << 23) && c >= 16;
+    return pays ? total * static_cast<int64_t>(sizeof(uint16_t)) : 0;
+}
+
+extern "C" int tpk_grouping_ws(int b, int c, int n, int npoint, int nsample, const float* features, const int64_t* idx,
+                               float* out, void* scratch, int64_t scratch_bytes, void* stream)
+{
+    using namespace tpk;
+    const int64_t need = tpk_grouping_scratch_bytes(b, c, n, npoint, nsample);
+    if (need == 0 || !aligned16(idx) || !aligned16(out) || test_path("gather_direct"))
+        return tpk_grouping(b, c, n, npoint, nsample, features, idx, out, stream);
+    TPK_REQUIRE(features && idx && out, "grouping: NULL pointer or empty feature row");
+    if (scratch == nullptr || scratch_bytes < need)
+    {
+        set_error("grouping: scratch of %lld bytes given, %lld needed", static_cast<long long>(scratch ? scratch_bytes : 0),
+                  static_cast<long long>(need));
+        return TPK_ERR_SCRATCH;
+    }
+    TPK_REQUIRE(aligned16(scratch), "grouping: scratch must be 16-byte aligned");
+    const long long ps = static_cast<long long>(npoint) * nsample, fours = ps * b / 4;
+    cudaStream_t s = static_cast<cudaStream_t>(stream);
+    uint16_t* idx16 = static_cast<uint16_t*>(scratch);
+    count_launches(1), narrow_idx_kernel<<<static_cast<unsigned>((fours + kGatherThreads - 1) / kGatherThreads), kGatherThreads, 0, s>>>(fours, n, idx, idx16);
+    const int rc = check_launch("grouping");
+    if (rc != TPK_OK) return rc;
+    return grouping_forward(b, c, n, ps, c, 0, features, idx, idx16, out, s);
 }
 
 extern "C" int64_t tpk_sa_group_scratch_bytes(int b, int n, int m, int nsample)
@@ -1091,18 +1167,26 @@ extern "C" int tpk_three_interpolate(int b, int c, int m, int n, const float* po
         static_cast<size_t>(m) * 4 * 4 <= kRowSmemBudget && static_cast<long long>(b) * c <= 65535 &&
         !test_path("gather_direct"))
     {
-        if (c >= 8 && static_cast<size_t>(m) * 4 * 8 <= 128 * 1024)
-            return launch_interp_fwd_rows<8>(b, c, m, n, points, idx, weight, out, s);
-        return launch_interp_fwd_rows<4>(b, c, m, n, points, idx, weight, out, s);
+        // 8 rows share the indices and weights where that leaves enough CTAs, 4 otherwise (us: 1 x 64 x 16384 6.1 -> 5.6,
+        // 4 x 90 x 8192 9.3 -> 8.6; but 16 x 64 x 16384 37 -> 39, 16 x 256 x 1024 10.0 -> 11.1).  Where two CTAs do not fit
+        // an SM, 512 threads (16 x 64 x 16384 of 4096: 37 -> 32; 16 x 128 x 4096 of 1024: 17.8 -> 18.4).
+        if (c >= 8 && static_cast<size_t>(m) * 4 * 8 <= 128 * 1024 && static_cast<long long>(b) * c * n >= (1ll << 22))
+        {
+            if (2 * (static_cast<size_t>(m) * 4 * 8 + 2048) > kRowSmemPerSm)
+                return launch_interp_fwd_rows<8, 512>(b, c, m, n, points, idx, weight, out, s);
+            return launch_interp_fwd_rows<8, 256>(b, c, m, n, points, idx, weight, out, s);
+        }
+        return launch_interp_fwd_rows<4, 256>(b, c, m, n, points, idx, weight, out, s);
     }
     const int gx = (n + kGatherThreads * 4 - 1) / (kGatherThreads * 4);
-    const int gy = (c + kChanChunk - 1) / kChanChunk;
+    const int chan = channels_per_cta(static_cast<long long>(gx) * b, c), gy = (c + chan - 1) / chan;
     TPK_REQUIRE(gy <= 65535 && b <= 65535, "three_interpolate: grid too large");
     const dim3 g(gx, gy, b);
+    const auto launch = [&](auto kernel) { count_launches(1), kernel<<<g, kGatherThreads, 0, s>>>(c, m, n, points, idx, weight, out); };
     if (n % 4 == 0 && aligned16(out))
-        count_launches(1), interp_fwd_kernel<true><<<g, kGatherThreads, 0, s>>>(c, m, n, points, idx, weight, out);
+        launch(chan == kChanChunk ? interp_fwd_kernel<true, kChanChunk> : interp_fwd_kernel<true, kChanChunk / 4>);
     else
-        count_launches(1), interp_fwd_kernel<false><<<g, kGatherThreads, 0, s>>>(c, m, n, points, idx, weight, out);
+        launch(chan == kChanChunk ? interp_fwd_kernel<false, kChanChunk> : interp_fwd_kernel<false, kChanChunk / 4>);
     return check_launch("three_interpolate");
 }
 

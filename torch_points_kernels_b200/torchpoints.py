@@ -220,8 +220,15 @@ class GroupingOperation(Function):
         ctx.grouping_for_backward = (idx, n)
         out = torch.empty((B, c, npoint, nsample), dtype=torch.float32, device=features.device)
         with _lib.on_device(features):
-            _lib.call("tpk_grouping", B, c, n, npoint, nsample, _lib.ptr(features), _lib.ptr(idx),
-                      _lib.ptr(out), _lib.stream_of(features))
+            need = _lib.lib().tpk_grouping_scratch_bytes(B, c, n, npoint, nsample)
+            if need > 0:
+                # many values from long rows: by a 16-bit copy of the indices
+                scratch = torch.empty((need,), dtype=torch.uint8, device=features.device)
+                _lib.call("tpk_grouping_ws", B, c, n, npoint, nsample, _lib.ptr(features), _lib.ptr(idx),
+                          _lib.ptr(out), _lib.ptr(scratch), need, _lib.stream_of(features))
+            else:
+                _lib.call("tpk_grouping", B, c, n, npoint, nsample, _lib.ptr(features), _lib.ptr(idx),
+                          _lib.ptr(out), _lib.stream_of(features))
             if _lib.debug_checks():
                 _lib.raise_on_device_status("grouping_operation")
         return out
