@@ -521,6 +521,27 @@ TPK_API int tpk_grow_labels_step(int64_t n, int nsample, const int64_t* neighbou
                                  int32_t* changed, int rounds, void* stream);
 
 /*
+ * The same labels with fewer rounds: points that list each other are one tree, and labels go along the lists between
+ * trees.  _begin prepares `scratch` (tpk_grow_labels_scratch_bytes bytes, 256-byte aligned) from the lists; _push does
+ * `rounds` rounds and writes the labels reached so far (n int32); *changed == 0 afterwards: they are final.
+ */
+TPK_API int64_t tpk_grow_labels_scratch_bytes(int64_t n, int nsample);
+TPK_API int tpk_grow_labels_begin(int64_t n, int nsample, const int64_t* neighbours, void* scratch,
+                                  int64_t scratch_bytes, void* stream);
+TPK_API int tpk_grow_labels_push(int64_t n, int rounds, int32_t* labels, int32_t* changed, void* scratch, void* stream);
+
+/*
+ * Ground truth of the instance IoU.  batch, instance_labels: n_points int64 each, 0 <= batch < samples.
+ * num_gt_instances (samples): largest label of a sample, 0 if it has none.  offsets (samples + 2): their exclusive sums,
+ * their sum, their largest.  sizes (total_gt_instances): points of instance l >= 1 of sample b at offsets[b] + l - 1.
+ * Points of other samples are left out and recorded in the status word.
+ */
+TPK_API int tpk_instance_counts(int64_t n_points, int64_t samples, const int64_t* batch, const int64_t* instance_labels,
+                                int64_t* num_gt_instances, int64_t* offsets, void* stream);
+TPK_API int tpk_instance_sizes(int64_t n_points, int64_t samples, int64_t total_gt_instances, const int64_t* batch,
+                               const int64_t* instance_labels, const int64_t* offsets, int64_t* sizes, void* stream);
+
+/*
  * IoU of every proposal with every ground-truth instance of its sample; proposals_iou
  * (n_proposals,total_gt_instances) f32 is fully written (0 for other samples' instances).
  * Arguments as instance_iou_kernel_wrapper, cuda/src/metrics_gpu.cu:50-62 (kernel :9-43), plus

@@ -232,6 +232,89 @@ def test_grow_proximity_matches_sequential_traversal(nsample, radius):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("nsample", [1, 4, 8, 9, 16, 17, 33, 40])
+@pytest.mark.parametrize("kind", ["path", "random", "mutual"])
+def test_cluster_labels_of_any_lists(nsample, kind):
+    """Labels of lists that are no radius search (one way only, both ways, long chains, ends at every slot, entries
+    that address nothing) against the sequential traversal, by trees and by the entry point without scratch."""
+    from torch_points_kernels_b200 import _lib, cluster
+
+    g = data.gen(nsample)
+    n = 1237
+    lists = torch.full((n, nsample), -1, dtype=torch.int64)
+    ends = torch.randint(0, nsample + 1, (n,), generator=g)
+    at = torch.randperm(n, generator=g)
+    if kind == "path":  # in random order, so that labels go up and down along it
+        lists[at[:-1], 0] = at[1:]
+        lists[at[::100], 0] = -1
+    else:
+        near = torch.arange(n).unsqueeze(1) + torch.randint(-6, 7, (n, nsample), generator=g)
+        lists = torch.where(torch.arange(nsample) < ends.unsqueeze(1), at[near.clamp(0, n - 1)][torch.argsort(at)], lists)
+        if kind == "mutual":  # first slot: the answer of a partner
+            lists[at[:600], 0], lists[at[600:1200], 0] = at[600:1200], at[:600]
+    want = np.full(n, -1, np.int64)
+    for c in orc.grow_proximity(lists.numpy(), 1):
+        want[c] = c[0]
+    np.testing.assert_array_equal(cluster.cluster_labels(_cu(lists)).cpu().numpy(), want)
+    nb, labels = _cu(lists), torch.arange(n, dtype=torch.int32, device="cuda")
+    changed = torch.ones(1, dtype=torch.int32, device="cuda")
+    for _ in range(n):
+        changed.zero_()
+        _lib.call("tpk_grow_labels_step", n, nsample, _lib.ptr(nb), _lib.ptr(labels), _lib.ptr(changed), 8, _lib.stream_of(nb))
+        if not int(changed):
+            break
+    np.testing.assert_array_equal(labels.cpu().numpy(), want)
+    lists[lists == 5] = n + 3  # addresses nothing: neither an end nor an edge
+    np.testing.assert_array_equal(cluster.cluster_labels(_cu(lists)).cpu().numpy(), _reached(lists.numpy()))
+
+
+def _reached(lists):
+    """Smallest index that reaches a point along lists whose entries outside [0, n) are passed over."""
+    n = lists.shape[0]
+    label = np.full(n, -1, np.int64)
+    for seed in range(n):
+        todo = [seed] if label[seed] < 0 else []
+        while todo:
+            u = todo.pop()
+            if label[u] >= 0:
+                continue
+            label[u] = seed
+            for v in lists[u]:
+                if v == -1:
+                    break
+                if 0 <= v < n and label[v] < 0:
+                    todo.append(int(v))
+    return label
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n,samples,high,order", [(1, 1, 1, "sorted"), (5000, 1, 40, "sorted"), (5003, 70, 9, "sorted"),
+                                                  (4097, 5, 300, "mixed"), (300, 3, 0, "sorted")])
+def test_instance_counts_of_the_ground_truth(n, samples, high, order):
+    """Largest label, first instance and sizes of every sample, with labels below 1 and samples without any."""
+    from torch_points_kernels_b200 import _lib
+
+    g = data.gen(n + samples)
+    batch = torch.randint(0, samples, (n,), generator=g)
+    batch = torch.sort(batch).values if order == "sorted" else batch
+    gt = torch.randint(-3, high + 1, (n,), generator=g)
+    gt[batch == samples // 2] = 0
+    most = torch.zeros(samples, dtype=torch.int64).scatter_reduce_(0, batch, gt.clamp(min=0), "amax")
+    first = torch.cat([torch.zeros(1, dtype=torch.int64), most.cumsum(0)])
+    total = int(first[-1])
+    sizes = torch.bincount((first[batch] + gt - 1)[gt >= 1], minlength=total)[:total]
+    b, l = _cu(batch), _cu(gt)
+    counts = torch.empty(2 * samples + 2, dtype=torch.int64, device="cuda")
+    got = torch.empty(total, dtype=torch.int64, device="cuda")
+    _lib.call("tpk_instance_counts", n, samples, _lib.ptr(b), _lib.ptr(l), _lib.ptr(counts), _lib.ptr(counts[samples:]),
+              _lib.stream_of(b))
+    assert counts.tolist() == most.tolist() + first.tolist() + [int(most.max())]
+    _lib.call("tpk_instance_sizes", n, samples, total, _lib.ptr(b), _lib.ptr(l), _lib.ptr(counts[samples:]), _lib.ptr(got),
+              _lib.stream_of(b))
+    assert got.tolist() == sizes.tolist()
+
+
+@pytest.mark.gpu
 def test_instance_iou_known_answers_and_reference(known_answers, ref_cuda):
     import torch_points_kernels_b200 as tpk
 

@@ -65,6 +65,10 @@ _SIGNATURES = {
     "tpk_cubic_feature_sampling_grad_ws_f64": [_c_int, _c_int, _c_int, _c_int, _c_int, _ptr, _ptr, _ptr, _ptr, _ptr, _c_i64, _ptr],
     "tpk_sa_group": [_c_int, _c_int, _c_int, _c_int, _c_f32, _c_int, _ptr, _ptr, _ptr, _ptr, _ptr, _ptr, _ptr, _c_i64, _ptr],
     "tpk_grow_labels_step": [_c_i64, _c_int, _ptr, _ptr, _ptr, _c_int, _ptr],
+    "tpk_grow_labels_begin": [_c_i64, _c_int, _ptr, _ptr, _c_i64, _ptr],
+    "tpk_grow_labels_push": [_c_i64, _c_int, _ptr, _ptr, _ptr, _ptr],
+    "tpk_instance_counts": [_c_i64, _c_i64, _ptr, _ptr, _ptr, _ptr, _ptr],
+    "tpk_instance_sizes": [_c_i64, _c_i64, _c_i64, _ptr, _ptr, _ptr, _ptr, _ptr],
     "tpk_instance_iou": [_c_int, _c_i64, _c_i64, _c_i64, _ptr, _ptr, _ptr, _ptr, _ptr, _ptr, _ptr, _ptr, _ptr],
 }
 
@@ -73,7 +77,7 @@ EXPORTS = sorted(list(_SIGNATURES) + ["tpk_version", "tpk_last_error", "tpk_devi
                                        "tpk_three_nn_scratch_bytes", "tpk_chamfer_dist_scratch_bytes",
                                        "tpk_ball_query_partial_dense_scratch_bytes", "tpk_knn_dense_scratch_bytes", "tpk_sa_group_scratch_bytes",
                                        "tpk_knn_partial_dense_scratch_bytes", "tpk_cubic_feature_sampling_scratch_bytes",
-                                       "tpk_grouping_scratch_bytes", "tpk_grouping_grad_scratch_bytes",
+                                       "tpk_grouping_scratch_bytes", "tpk_grouping_grad_scratch_bytes", "tpk_grow_labels_scratch_bytes",
                                        "tpk_grouping_grad_cols_scratch_bytes",
                                        "tpk_three_interpolate_grad_cols_scratch_bytes",
                                        "tpk_three_nn_sorted_scratch_bytes", "tpk_chamfer_dist_sorted_scratch_bytes"])
@@ -119,6 +123,8 @@ def lib():
         handle.tpk_knn_partial_dense_scratch_bytes.restype = _c_i64
         handle.tpk_sa_group_scratch_bytes.argtypes = [_c_int, _c_int, _c_int, _c_int]
         handle.tpk_sa_group_scratch_bytes.restype = _c_i64
+        handle.tpk_grow_labels_scratch_bytes.argtypes = [_c_i64, _c_int]
+        handle.tpk_grow_labels_scratch_bytes.restype = _c_i64
         handle.tpk_grouping_scratch_bytes.argtypes = [_c_int, _c_int, _c_int, _c_int, _c_int]
         handle.tpk_grouping_scratch_bytes.restype = _c_i64
         handle.tpk_grouping_grad_cols_scratch_bytes.argtypes = [_c_int, _c_int, _c_int, _c_int, _c_int]

@@ -1,6 +1,6 @@
 """Region growing on the GPU (reference: torch_points_kernels/cluster.py, a numba traversal on
 the CPU there).  The neighbour search is the packed ball query; the clusters come from label
-propagation on the device (tpk_grow_labels_step) instead of a sequential traversal."""
+propagation on the device (tpk_grow_labels_begin, _push) instead of a sequential traversal."""
 import ctypes
 from typing import List
 
@@ -19,15 +19,19 @@ def cluster_labels(neighbours):
         raise RuntimeError("neighbours must be an int64 tensor")
     neighbours = neighbours.contiguous()
     n, nsample = neighbours.shape
-    labels = torch.arange(n, dtype=torch.int32, device=neighbours.device)
-    changed = torch.zeros(1, dtype=torch.int32, device=neighbours.device)
+    labels = torch.empty(n, dtype=torch.int32, device=neighbours.device)
+    if n == 0:
+        return labels
+    changed = torch.empty(1, dtype=torch.int32, device=neighbours.device)
     with _lib.on_device(neighbours):
-        # chains shorten geometrically; a handful of launches per host check keeps the number of
-        # device-to-host reads small
-        for _ in range(max(1, n)):
-            changed.zero_()
-            _lib.call("tpk_grow_labels_step", n, nsample, _lib.ptr(neighbours), _lib.ptr(labels), _lib.ptr(changed),
-                      8, _lib.stream_of(neighbours))
+        need = _lib.lib().tpk_grow_labels_scratch_bytes(n, nsample)
+        scratch = torch.empty((need,), dtype=torch.uint8, device=neighbours.device)
+        stream = _lib.stream_of(neighbours)
+        _lib.call("tpk_grow_labels_begin", n, nsample, _lib.ptr(neighbours), _lib.ptr(scratch), need, stream)
+        # labels go along the lists between trees of points that list each other: a few rounds as a rule; a
+        # handful of launches per host check keeps the number of device-to-host reads small
+        for _ in range(n):
+            _lib.call("tpk_grow_labels_push", n, 8, _lib.ptr(labels), _lib.ptr(changed), _lib.ptr(scratch), stream)
             if int(changed.item()) == 0:
                 break
     return labels

@@ -7,17 +7,21 @@
 //   first nsample hits of a radius search, so the graph is directed (a crowded point may
 //   not list a neighbour that lists it).  The traversal assigns point v to the smallest
 //   index that can reach v along directed edges, which is a fixed point of "push the
-//   smallest label seen so far along every edge": a few lanes own a point, push its
-//   label to the points it lists (atomicMin) and shorten its own label chain (the label of
-//   my label is also an ancestor of mine).  The host repeats launches until nothing changes.
+//   smallest label seen so far along every edge": labels are pushed (atomicMin), and chains of
+//   labels shortened (the label of my label is also an ancestor of mine), until nothing changes.  The Python
+//   wrapper unites points that list each other first (tpk_grow_labels_begin, _push); tpk_grow_labels_step needs no
+//   scratch and pushes along all lists, a few lanes to a point.
 // instance_iou:   cuda/src/metrics_gpu.cu:9-43: the reference compares every point of a proposal
 //   with every ground-truth instance; here a CTA histograms the proposal's labels once.
 #include <climits>
+#include <type_traits>
 
 #include "tpk_common.cuh"
 
 namespace tpk
 {
+TPK_DEFINE_STATUS_WORD()
+
 namespace
 {
 
@@ -80,6 +84,266 @@ __global__ void __launch_bounds__(kClThreads)
         if (__all_sync(kFullMask, ended)) break;
     }
     if (moved) *changed = 1;
+}
+
+// ---- the same labels by contraction
+//
+// Two points that list each other reach each other and share a label, so they are united first (a forest of
+// parents, the larger root always under the smaller: a root is the smallest index of its tree); only lists that are not
+// answered are left as edges between trees, and labels are pushed along those alone, tree by tree.  A round
+// over all lists is bound by its chain of dependent loads, 15 us for 160000 points and 16 slots, and a label moves a
+// few hops in it: 38 rounds, 565 us; uniting takes 100 us (chains of dependent loads too, of
+// roots and of lists that may answer), the edges 17, and eight rounds of 1.5 us end it.
+struct GrowScratch
+{
+    unsigned long long* count;  // edges
+    int32_t* parent;            // of a point; its root from grow_edges_kernel on
+    int32_t* tree;              // label of a root
+    int2* edges;
+};
+
+GrowScratch grow_layout(void* scratch, long long n)
+{
+    GrowScratch g;
+    unsigned char* p = static_cast<unsigned char*>(scratch);
+    g.count = reinterpret_cast<unsigned long long*>(p);
+    g.parent = reinterpret_cast<int32_t*>(p + 256);
+    g.tree = g.parent + (n + 63) / 64 * 64;
+    g.edges = reinterpret_cast<int2*>(g.tree + (n + 63) / 64 * 64);
+    return g;
+}
+
+__global__ void __launch_bounds__(kClThreads) grow_init_kernel(long long n, GrowScratch g)
+{
+    const long long v = static_cast<long long>(blockIdx.x) * kClThreads + threadIdx.x;
+    if (v == 0) *g.count = 0;
+    if (v < n) g.parent[v] = static_cast<int32_t>(v), g.tree[v] = static_cast<int32_t>(v);
+}
+
+// Root of v: parents are smaller than their children, so this ends.  Halves the path behind it.
+__device__ __forceinline__ int grow_root(int32_t* parent, int v)
+{
+    int p = __ldcg(parent + v);
+    while (p != v)
+    {
+        const int q = __ldcg(parent + p);
+        if (q != p) atomicMin(parent + v, q);
+        v = p;
+        p = q;
+    }
+    return v;
+}
+
+__device__ __forceinline__ bool grow_lists(const int64_t* row, int nsample, long long u)
+{
+    // (four slots at a time: 120 us for 100 of grow_unite_kernel; most lists are answered early)
+    for (int s = 0; s < nsample; ++s)
+    {
+        const long long v = __ldg(row + s);
+        if (v == u) return true;
+        if (v == -1) return false;
+    }
+    return false;
+}
+
+// What the lanes of a point take at a time: four slots each, v < 0 where there is none.  True: the list goes on.
+template <int LANES>
+__device__ __forceinline__ bool grow_slots(const int64_t* row, long long n, int nsample, int s, bool& ended, long long (&v)[4])
+{
+    const int lane = threadIdx.x & 31;
+    const uint32_t group = ((1u << LANES) - 1u) << (lane & ~(LANES - 1));
+#pragma unroll
+    for (int i = 0; i < 4; ++i) v[i] = !ended && s + i < nsample ? __ldg(row + s + i) : -1;
+    const bool end_here = v[0] == -1 || v[1] == -1 || v[2] == -1 || v[3] == -1;
+    const uint32_t end = __ballot_sync(kFullMask, end_here) & group;
+    bool listed = end == 0u || lane <= __ffs(end) - 1;
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+    {
+        listed = listed && v[i] != -1;
+        if (!listed || v[i] < 0 || v[i] >= n) v[i] = -1;
+    }
+    ended |= end != 0u;
+    return !__all_sync(kFullMask, ended);
+}
+
+// Unites the pairs that list each other, from the smaller index; pairs of one tree are done.
+template <int LANES>
+__global__ void __launch_bounds__(kClThreads)
+    grow_unite_kernel(long long n, int nsample, const int64_t* __restrict__ neighbours, GrowScratch g)
+{
+    const long long u = (static_cast<long long>(blockIdx.x) * kClThreads + threadIdx.x) / LANES;
+    const int slot = threadIdx.x & (LANES - 1);
+    bool ended = u >= n, more = true;
+    const int64_t* row = neighbours + (ended ? 0 : u) * nsample;
+    for (int s0 = 0; s0 < nsample && more; s0 += LANES * 4)
+    {
+        long long v[4];
+        more = grow_slots<LANES>(row, n, nsample, s0 + slot * 4, ended, v);
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+        {
+            if (v[i] <= u) continue;
+            int a = grow_root(g.parent, static_cast<int>(u)), b = grow_root(g.parent, static_cast<int>(v[i]));
+            if (a == b || !grow_lists(neighbours + v[i] * nsample, nsample, u)) continue;
+            while (a != b)
+            {
+                const int hi = max(a, b), lo = min(a, b);
+                const int old = atomicCAS(g.parent + hi, hi, lo);
+                if (old == hi) break;
+                a = old, b = lo;  // (hi has a parent by now, smaller than itself)
+            }
+        }
+    }
+}
+
+// Roots of all points, and the lists between trees as edges (from, to).
+template <int LANES>
+__global__ void __launch_bounds__(kClThreads)
+    grow_edges_kernel(long long n, int nsample, const int64_t* __restrict__ neighbours, GrowScratch g)
+{
+    const long long u = (static_cast<long long>(blockIdx.x) * kClThreads + threadIdx.x) / LANES;
+    const int lane = threadIdx.x & 31, slot = lane & (LANES - 1);
+    bool ended = u >= n, more = true;
+    const int a = ended ? 0 : grow_root(g.parent, static_cast<int>(u));
+    if (!ended && slot == 0) atomicMin(g.parent + u, a);
+    const int64_t* row = neighbours + (ended ? 0 : u) * nsample;
+    for (int s0 = 0; s0 < nsample && more; s0 += LANES * 4)
+    {
+        long long v[4];
+        int b[4], k = 0;
+        more = grow_slots<LANES>(row, n, nsample, s0 + slot * 4, ended, v);
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+        {
+            b[i] = v[i] < 0 ? a : grow_root(g.parent, static_cast<int>(v[i]));
+            k += b[i] != a;
+        }
+        int before = k;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1)
+        {
+            const int t = __shfl_up_sync(kFullMask, before, o);
+            if (lane >= o) before += t;
+        }
+        const int all = __shfl_sync(kFullMask, before, 31);
+        unsigned long long at = 0;
+        if (lane == 0 && all > 0) at = atomicAdd(g.count, static_cast<unsigned long long>(all));
+        at = __shfl_sync(kFullMask, at, 0) + (before - k);
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+            if (b[i] != a) g.edges[at++] = make_int2(a, b[i]);
+    }
+}
+
+__global__ void __launch_bounds__(kClThreads) grow_push_kernel(GrowScratch g, int32_t* __restrict__ changed)
+{
+    const long long edges = static_cast<long long>(*g.count), step = static_cast<long long>(gridDim.x) * kClThreads;
+    bool moved = false;
+    for (long long e = static_cast<long long>(blockIdx.x) * kClThreads + threadIdx.x; e < edges; e += step)
+    {
+        const int2 ab = __ldg(g.edges + e);
+        int la = __ldcg(g.tree + ab.x);
+        const int lb = __ldcg(g.tree + ab.y), ll = __ldcg(g.tree + la);
+        if (ll < la)
+        {
+            atomicMin(g.tree + ab.x, ll);
+            la = ll;
+            moved = true;
+        }
+        if (lb > la && atomicMin(g.tree + ab.y, la) > la) moved = true;
+    }
+    if (moved) *changed = 1;
+}
+
+__global__ void __launch_bounds__(kClThreads) grow_result_kernel(long long n, GrowScratch g, int32_t* __restrict__ labels)
+{
+    const long long v = static_cast<long long>(blockIdx.x) * kClThreads + threadIdx.x;
+    if (v < n) labels[v] = g.tree[g.parent[v]];
+}
+
+// ---- ground truth of the IoU: largest label of every sample, points of every instance
+
+// A thread takes kCountRun points and adds up what stays the same among them: samples lie together, and one atomic
+// a point goes to a few addresses (scatter_reduce, 240000 points in 4 samples: 231 us; this: 4.9).
+constexpr int kCountRun = 4;
+
+__global__ void __launch_bounds__(kClThreads)
+    instance_max_kernel(long long n, long long samples, const int64_t* __restrict__ batch, const int64_t* __restrict__ labels,
+                        int64_t* __restrict__ most)
+{
+    const long long t = static_cast<long long>(blockIdx.x) * kClThreads + threadIdx.x;
+    const int lane = threadIdx.x & 31;
+    long long b = -1, m = 0;
+    bool bad = false;
+    for (int i = 0; i < kCountRun; ++i)
+    {
+        // (neighbouring lanes read neighbouring points)
+        const long long k = (t - lane) * kCountRun + i * 32 + lane;
+        if (k >= n) break;
+        const long long bk = batch[k], l = labels[k];
+        if (bk < 0 || bk >= samples)
+        {
+            bad = true;
+            continue;
+        }
+        if (bk != b)
+        {
+            if (m > 0) atomicMax(reinterpret_cast<long long*>(most) + b, m);
+            b = bk, m = 0;
+        }
+        m = max(m, l);
+    }
+    const uint32_t same = __match_any_sync(kFullMask, b);
+    if (same == kFullMask)
+    {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(kFullMask, m, o));
+        if (lane != 0) m = 0;
+    }
+    if (m > 0 && m > *reinterpret_cast<volatile int64_t*>(most + b)) atomicMax(reinterpret_cast<long long*>(most) + b, m);
+    if (bad) atomicOr(&g_dev_status, kStatusBadIndex);
+}
+
+// First instance of every sample, the number of all, and the largest sample's, behind each other.
+__global__ void __launch_bounds__(32) instance_offsets_kernel(long long samples, const int64_t* __restrict__ most, int64_t* __restrict__ offsets)
+{
+    const int lane = threadIdx.x;
+    long long base = 0, top = 0;
+    for (long long s0 = 0; s0 < samples; s0 += 32)
+    {
+        const long long v = s0 + lane < samples ? most[s0 + lane] : 0;
+        long long incl = v;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1)
+        {
+            const long long t = __shfl_up_sync(kFullMask, incl, o);
+            if (lane >= o) incl += t;
+        }
+        if (s0 + lane < samples) offsets[s0 + lane] = base + incl - v;
+        base += __shfl_sync(kFullMask, incl, 31);
+        top = max(top, v);
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) top = max(top, __shfl_xor_sync(kFullMask, top, o));
+    if (lane == 0) offsets[samples] = base, offsets[samples + 1] = top;
+}
+
+__global__ void __launch_bounds__(kClThreads)
+    instance_sizes_kernel(long long n, long long samples, const int64_t* __restrict__ batch, const int64_t* __restrict__ labels,
+                          const int64_t* __restrict__ offsets, int64_t* __restrict__ sizes)
+{
+    const long long k = static_cast<long long>(blockIdx.x) * kClThreads + threadIdx.x;
+    const int lane = threadIdx.x & 31;
+    long long key = -1;
+    if (k < n)
+    {
+        const long long b = batch[k], l = labels[k];
+        if (l >= 1 && b >= 0 && b < samples) key = offsets[b] + l - 1;
+    }
+    const uint32_t same = __match_any_sync(kFullMask, key);
+    if (key >= 0 && lane == __ffs(same) - 1)
+        atomicAdd(reinterpret_cast<unsigned long long*>(sizes) + key, static_cast<unsigned long long>(__popc(same)));
 }
 
 // One CTA per proposal: histogram of the ground-truth instance ids of its points, then one
@@ -148,6 +412,120 @@ extern "C" int tpk_grow_labels_step(int64_t n, int nsample, const int64_t* neigh
             grow_labels_kernel<8><<<g, kClThreads, 0, st>>>(n, nsample, neighbours, labels, changed);
     }
     return check_launch("grow_labels");
+}
+
+extern "C" int64_t tpk_grow_labels_scratch_bytes(int64_t n, int nsample)
+{
+    if (n <= 0 || nsample < 0) return 0;
+    return 256 + (n + 63) / 64 * 64 * 2 * static_cast<int64_t>(sizeof(int32_t)) + n * nsample * static_cast<int64_t>(sizeof(int2));
+}
+
+extern "C" int tpk_grow_labels_begin(int64_t n, int nsample, const int64_t* neighbours, void* scratch, int64_t scratch_bytes,
+                                     void* stream)
+{
+    using namespace tpk;
+    TPK_REQUIRE(n >= 0 && nsample >= 0, "grow_labels: negative size");
+    TPK_REQUIRE(n < (1ll << 31), "grow_labels: too many points");
+    if (n == 0) return TPK_OK;
+    TPK_REQUIRE(neighbours || nsample == 0, "grow_labels: NULL pointer");
+    const int64_t need = tpk_grow_labels_scratch_bytes(n, nsample);
+    if (scratch == nullptr || scratch_bytes < need)
+    {
+        set_error("grow_labels: scratch of %lld bytes given, %lld needed", static_cast<long long>(scratch ? scratch_bytes : 0),
+                  static_cast<long long>(need));
+        return TPK_ERR_SCRATCH;
+    }
+    TPK_REQUIRE((reinterpret_cast<uintptr_t>(scratch) & 255u) == 0, "grow_labels: scratch must be 256-byte aligned");
+    const GrowScratch g = grow_layout(scratch, n);
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    const unsigned points = static_cast<unsigned>((n + kClThreads - 1) / kClThreads);
+    count_launches(1), grow_init_kernel<<<points, kClThreads, 0, st>>>(n, g);
+    const auto lists = [&](auto lanes) {
+        constexpr int L = decltype(lanes)::value;
+        const unsigned grid = static_cast<unsigned>((n * L + kClThreads - 1) / kClThreads);
+        count_launches(1), grow_unite_kernel<L><<<grid, kClThreads, 0, st>>>(n, nsample, neighbours, g);
+        count_launches(1), grow_edges_kernel<L><<<grid, kClThreads, 0, st>>>(n, nsample, neighbours, g);
+    };
+    if (nsample <= 8)
+        lists(std::integral_constant<int, 2>());
+    else if (nsample <= 16)
+        lists(std::integral_constant<int, 4>());
+    else
+        lists(std::integral_constant<int, 8>());
+    return check_launch("grow_labels");
+}
+
+extern "C" int tpk_grow_labels_push(int64_t n, int rounds, int32_t* labels, int32_t* changed, void* scratch, void* stream)
+{
+    using namespace tpk;
+    TPK_REQUIRE(n >= 0 && rounds >= 1, "grow_labels: bad size");
+    TPK_REQUIRE(n < (1ll << 31), "grow_labels: too many points");
+    if (n == 0) return TPK_OK;
+    TPK_REQUIRE(labels && changed && scratch, "grow_labels: NULL pointer");
+    const GrowScratch g = grow_layout(scratch, n);
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    // (the edges are counted on the device: as many CTAs as the SMs hold at most)
+    const long long most = 8ll * num_sms(), points = (n + kClThreads - 1) / kClThreads;
+    const unsigned grid = static_cast<unsigned>(points < most ? points : most);
+    for (int r = 0; r < rounds; ++r)
+    {
+        if (r == rounds - 1)
+        {
+            const cudaError_t err = cudaMemsetAsync(changed, 0, sizeof(int32_t), st);
+            if (err != cudaSuccess)
+            {
+                set_error("grow_labels: memset: %s", cudaGetErrorString(err));
+                return TPK_ERR_CUDA;
+            }
+        }
+        count_launches(1), grow_push_kernel<<<grid, kClThreads, 0, st>>>(g, changed);
+    }
+    count_launches(1), grow_result_kernel<<<static_cast<unsigned>(points), kClThreads, 0, st>>>(n, g, labels);
+    return check_launch("grow_labels");
+}
+
+extern "C" int tpk_instance_counts(int64_t n_points, int64_t samples, const int64_t* batch, const int64_t* instance_labels,
+                                   int64_t* num_gt_instances, int64_t* offsets, void* stream)
+{
+    using namespace tpk;
+    TPK_REQUIRE(n_points >= 0 && samples >= 1, "instance_counts: bad size");
+    TPK_REQUIRE(num_gt_instances && offsets && (n_points == 0 || (batch && instance_labels)), "instance_counts: NULL pointer");
+    const long long per = static_cast<long long>(kClThreads) * kCountRun, grid = (n_points + per - 1) / per;
+    TPK_REQUIRE(grid < (1ll << 31), "instance_counts: too many points");
+    cudaStream_t s = static_cast<cudaStream_t>(stream);
+    const cudaError_t err = cudaMemsetAsync(num_gt_instances, 0, sizeof(int64_t) * static_cast<size_t>(samples), s);
+    if (err != cudaSuccess)
+    {
+        set_error("instance_counts: memset: %s", cudaGetErrorString(err));
+        return TPK_ERR_CUDA;
+    }
+    if (grid > 0)
+        count_launches(1), instance_max_kernel<<<static_cast<unsigned>(grid), kClThreads, 0, s>>>(n_points, samples, batch, instance_labels,
+                                                                                                num_gt_instances);
+    count_launches(1), instance_offsets_kernel<<<1, 32, 0, s>>>(samples, num_gt_instances, offsets);
+    return check_launch("instance_counts");
+}
+
+extern "C" int tpk_instance_sizes(int64_t n_points, int64_t samples, int64_t total_gt_instances, const int64_t* batch,
+                                  const int64_t* instance_labels, const int64_t* offsets, int64_t* sizes, void* stream)
+{
+    using namespace tpk;
+    TPK_REQUIRE(n_points >= 0 && samples >= 1 && total_gt_instances >= 0, "instance_sizes: bad size");
+    if (total_gt_instances == 0) return TPK_OK;
+    TPK_REQUIRE(offsets && sizes && (n_points == 0 || (batch && instance_labels)), "instance_sizes: NULL pointer");
+    const long long grid = (n_points + kClThreads - 1) / kClThreads;
+    TPK_REQUIRE(grid < (1ll << 31), "instance_sizes: too many points");
+    cudaStream_t s = static_cast<cudaStream_t>(stream);
+    const cudaError_t err = cudaMemsetAsync(sizes, 0, sizeof(int64_t) * static_cast<size_t>(total_gt_instances), s);
+    if (err != cudaSuccess)
+    {
+        set_error("instance_sizes: memset: %s", cudaGetErrorString(err));
+        return TPK_ERR_CUDA;
+    }
+    if (grid > 0)
+        count_launches(1), instance_sizes_kernel<<<static_cast<unsigned>(grid), kClThreads, 0, s>>>(n_points, samples, batch,
+                                                                                                  instance_labels, offsets, sizes);
+    return check_launch("instance_sizes");
 }
 
 extern "C" int tpk_instance_iou(int n_proposals, int64_t total_gt_instances, int64_t max_gt_instances, int64_t n_points,

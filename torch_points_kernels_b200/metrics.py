@@ -34,17 +34,23 @@ def instance_iou(
         batch = torch.zeros_like(gt_instances)
     batch = batch.long().to(dev).contiguous()
 
+    if gt_instances.dim() != 1 or batch.shape != gt_instances.shape:
+        raise IndexError("batch of shape %s does not match gt_instances of shape %s"
+                         % (tuple(batch.shape), tuple(gt_instances.shape)))
+
     # Number of gt instances per sample (the largest label of the sample) and their sizes, on the
     # device: the reference loops over samples and instances in Python (metrics.py:63-74)
     batch_size = int(batch[-1].item()) + 1
-    num_gt_instances = torch.zeros(batch_size, dtype=torch.long, device=dev).scatter_reduce_(
-        0, batch, gt_instances.clamp(min=0), reduce="amax", include_self=True)
-    offset_num_gt = torch.cat([torch.zeros(1, dtype=torch.long, device=dev), num_gt_instances.cumsum(0)])
-    total_gt = int(offset_num_gt[-1].item())
-    max_gt = int(num_gt_instances.max().item()) if batch_size else 0
-    is_inst = gt_instances >= 1
-    key = offset_num_gt[batch[is_inst]] + gt_instances[is_inst] - 1
-    gt_instance_sizes = torch.bincount(key, minlength=max(total_gt, 1))[:total_gt].contiguous()
+    n = gt_instances.shape[0]
+    counts = torch.empty(2 * batch_size + 2, dtype=torch.long, device=dev)
+    num_gt_instances, offset_num_gt = counts[:batch_size], counts[batch_size:]
+    with _lib.on_device(gt_instances):
+        _lib.call("tpk_instance_counts", n, batch_size, _lib.ptr(batch), _lib.ptr(gt_instances),
+                  _lib.ptr(num_gt_instances), _lib.ptr(offset_num_gt), _lib.stream_of(gt_instances))
+        total_gt, max_gt = counts[-2:].tolist()
+        gt_instance_sizes = torch.empty(total_gt, dtype=torch.long, device=dev)
+        _lib.call("tpk_instance_sizes", n, batch_size, total_gt, _lib.ptr(batch), _lib.ptr(gt_instances),
+                  _lib.ptr(offset_num_gt), _lib.ptr(gt_instance_sizes), _lib.stream_of(gt_instances))
 
     offsets = [0]
     for instance in instance_idx:
