@@ -14,8 +14,8 @@
 // in shared memory first.  A tiled transposition writes the result.
 //
 // Bound by the rate of the reductions in L2 and the gradient's bytes: 16 clouds of 16384 points, 64 channels,
-// 4096 x 32 positions (537 MB, 82 us at the copy bandwidth) 204 us, 297 through the inverted index of
-// scatter_sorted.cu; all four levels of the benchmark's step 395 and 582; interpolation 112 and 187.
+// 4096 x 32 positions (537 MB, 82 us at the copy bandwidth) 180 us, 297 through the inverted index of
+// scatter_sorted.cu; all four levels of the benchmark's step 352 and 582; interpolation 110 and 187.
 //
 // semantics: autograd's scatter-add backward of the gather at torch_points_kernels/torchpoints.py:129-146,
 // and cuda/src/interpolate_gpu.cu:122-152.
@@ -84,12 +84,22 @@ __global__ void __launch_bounds__(kColsThreads)
     }
     const float* g = grad_out + static_cast<size_t>(cloud) * gbs + static_cast<size_t>(c0) * ps + p0 + (in ? lane : 0);
     float v[kColsMax];
+    if (nc == kColsMax)
+    {
 #pragma unroll
-    for (int r = 0; r < kColsMax; ++r)
-        if (r < nc) v[r] = __ldcs(g + static_cast<size_t>(r) * ps);
+        for (int r = 0; r < kColsMax; ++r) v[r] = __ldcs(g), g += ps;
 #pragma unroll
-    for (int r = 0; r < kColsMax; ++r)
-        if (r < nc4) s.v[r * kColsPitch + lane] = r < nc ? v[r] : 0.f;
+        for (int r = 0; r < kColsMax; ++r) s.v[r * kColsPitch + lane] = v[r];
+    }
+    else
+    {
+#pragma unroll
+        for (int r = 0; r < kColsMax; ++r)
+            if (r < nc) v[r] = __ldcs(g + static_cast<size_t>(r) * ps);
+#pragma unroll
+        for (int r = 0; r < kColsMax; ++r)
+            if (r < nc4) s.v[r * kColsPitch + lane] = r < nc ? v[r] : 0.f;
+    }
     __syncwarp();
 
     const int quads = nc4 >> 2;         // 16-byte pieces of a position's channels
@@ -112,6 +122,24 @@ __global__ void __launch_bounds__(kColsThreads)
             left &= ~others;
             float* row = s.v + lane * kColsPitch;  // lane = channel
             float a = row[first], b = 0.f;
+            const int low = __ffs(others) - 1;
+            if ((others + (1u << low) & others) == 0u)
+            {
+                // a run, as padding is: four words for what one takes below (with the loads of a full tile without
+                // their conditions 204 us -> 180 at 16 x 64 x 16384, 4096 x 32 positions; 561 -> 449 at 8 x 96 x 32768)
+                const float* run = row + low;
+                int k = __popc(others);
+                for (; k >= 4; k -= 4, run += 4)
+                {
+                    a += run[0];
+                    b += run[1];
+                    a += run[2];
+                    b += run[3];
+                }
+                if (k & 2) a += run[0], b += run[1], run += 2;
+                if (k & 1) a += run[0];
+                others = 0u;
+            }
             while (others != 0u)
             {
                 const int p = __ffs(others) - 1;
@@ -216,9 +244,9 @@ bool cols_fit(int b, int c, int n, long long ps)
     return warps < 1.0e9 && tiles < 1.0e9 && !test_path("scatter_atomic") && !test_path("scatter_global") && !test_path("scatter_sorted");
 }
 
-// Where three launches (zeros, sums, transposition; 8 us at least) pay.  us, rows of atomics or inverted index
-// and columns: 16 clouds of 16384 points, 64 channels, 4096 x 32 positions 297 and 204, 4096 points x 128 channels
-// 165 and 104, 256 x 512 46 and 31; one cloud 59 and 19; 8 x 32768 x 96, 8192 x 64 positions 1199 and 561; but 16 x
+// Where three launches (zeros, sums, transposition; 7.8 us at least) pay.  us, rows of atomics or inverted index
+// and columns: 16 clouds of 16384 points, 64 channels, 4096 x 32 positions 297 and 180, 4096 points x 128 channels
+// 165 and 95, 256 x 512 46 and 28; one cloud 59 and 14; 8 x 32768 x 96, 8192 x 64 positions 1199 and 449; but 16 x
 // 256 x 64, 64 x 32 positions 9.2 and 10.2, 4 x 2048 x 180, 512 x 16 16.3 and 18.1.  The rows cost the positions times
 // the rows that an SM has; neighbourhoods of a size that is no power of two, whose padding the rows do not
 // sum first, up to several times that (8 x 64 x 192, 16 x 48 positions 31 and 8.4; 3 x 625 x 140, 156 x 24
@@ -229,7 +257,7 @@ bool cols_pay_grouping(int b, int c, long long ps, int nsample)
     const long long rows = static_cast<long long>(b) * c, rows_sm = (rows + num_sms() - 1) / num_sms();
     const double per = (nsample & (nsample - 1)) == 0 ? 0.33e-3 : 1.2e-3;
     const double by_rows = 4.5 + per * static_cast<double>(ps) * static_cast<double>(rows_sm);
-    return 8.2 + 1.5e-6 * static_cast<double>(rows) * static_cast<double>(ps) < by_rows;
+    return 7.8 + 1.3e-6 * static_cast<double>(rows) * static_cast<double>(ps) < by_rows;
 }
 
 // us, rows of atomics and columns: 16 clouds of 16384 points from 4096, 64 channels 86 and 49; one cloud 42 and
