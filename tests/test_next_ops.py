@@ -234,10 +234,10 @@ def test_grow_proximity_matches_sequential_traversal(nsample, radius):
 @pytest.mark.gpu
 @pytest.mark.parametrize("nsample", [1, 4, 8, 9, 16, 17, 33, 40])
 @pytest.mark.parametrize("kind", ["path", "random", "mutual"])
-def test_cluster_labels_of_any_lists(nsample, kind):
+def test_cluster_labels_of_any_lists(nsample, kind, monkeypatch):
     """Labels of lists that are no radius search (one way only, both ways, long chains, ends at every slot, entries
-    that address nothing) against the sequential traversal, by trees and by the entry point without scratch."""
-    from torch_points_kernels_b200 import _lib, cluster
+    that address nothing) against the sequential traversal, by trees and without their scratch."""
+    from torch_points_kernels_b200 import cluster
 
     g = data.gen(nsample)
     n = 1237
@@ -256,14 +256,9 @@ def test_cluster_labels_of_any_lists(nsample, kind):
     for c in orc.grow_proximity(lists.numpy(), 1):
         want[c] = c[0]
     np.testing.assert_array_equal(cluster.cluster_labels(_cu(lists)).cpu().numpy(), want)
-    nb, labels = _cu(lists), torch.arange(n, dtype=torch.int32, device="cuda")
-    changed = torch.ones(1, dtype=torch.int32, device="cuda")
-    for _ in range(n):
-        changed.zero_()
-        _lib.call("tpk_grow_labels_step", n, nsample, _lib.ptr(nb), _lib.ptr(labels), _lib.ptr(changed), 8, _lib.stream_of(nb))
-        if not int(changed):
-            break
-    np.testing.assert_array_equal(labels.cpu().numpy(), want)
+    with monkeypatch.context() as m:
+        m.setattr(cluster, "_MOST_SCRATCH", 0)
+        np.testing.assert_array_equal(cluster.cluster_labels(_cu(lists)).cpu().numpy(), want)
     lists[lists == 5] = n + 3  # addresses nothing: neither an end nor an edge
     np.testing.assert_array_equal(cluster.cluster_labels(_cu(lists)).cpu().numpy(), _reached(lists.numpy()))
 

@@ -9,6 +9,10 @@ import torch
 from . import _lib
 from .torchpoints import ball_query_partial_dense
 
+# Scratch of the labels by trees is as large as the lists: beyond this the lists are walked in every round instead, so
+# that lists which fill half of the memory still get labels (160000 points, 16 slots: 38 rounds of 15 us for 130 us).
+_MOST_SCRATCH = 8 << 30
+
 
 def cluster_labels(neighbours):
     """neighbours: (N, nsample) int64 CUDA tensor of neighbour lists (-1 ends a list).  Returns
@@ -19,19 +23,29 @@ def cluster_labels(neighbours):
         raise RuntimeError("neighbours must be an int64 tensor")
     neighbours = neighbours.contiguous()
     n, nsample = neighbours.shape
-    labels = torch.empty(n, dtype=torch.int32, device=neighbours.device)
     if n == 0:
-        return labels
-    changed = torch.empty(1, dtype=torch.int32, device=neighbours.device)
+        return torch.empty(0, dtype=torch.int32, device=neighbours.device)
     with _lib.on_device(neighbours):
-        need = _lib.lib().tpk_grow_labels_scratch_bytes(n, nsample)
-        scratch = torch.empty((need,), dtype=torch.uint8, device=neighbours.device)
         stream = _lib.stream_of(neighbours)
-        _lib.call("tpk_grow_labels_begin", n, nsample, _lib.ptr(neighbours), _lib.ptr(scratch), need, stream)
-        # labels go along the lists between trees of points that list each other: a few rounds as a rule; a
-        # handful of launches per host check keeps the number of device-to-host reads small
+        need = _lib.lib().tpk_grow_labels_scratch_bytes(n, nsample)
+        if need <= _MOST_SCRATCH:
+            # labels go along the lists between trees of points that list each other: a few rounds as a rule
+            labels = torch.empty(n, dtype=torch.int32, device=neighbours.device)
+            changed = torch.empty(1, dtype=torch.int32, device=neighbours.device)
+            scratch = torch.empty((need,), dtype=torch.uint8, device=neighbours.device)
+            _lib.call("tpk_grow_labels_begin", n, nsample, _lib.ptr(neighbours), _lib.ptr(scratch), need, stream)
+        else:
+            labels = torch.arange(n, dtype=torch.int32, device=neighbours.device)
+            changed = torch.zeros(1, dtype=torch.int32, device=neighbours.device)
+            scratch = None
+        # a handful of launches per host check keeps the number of device-to-host reads small
         for _ in range(n):
-            _lib.call("tpk_grow_labels_push", n, 8, _lib.ptr(labels), _lib.ptr(changed), _lib.ptr(scratch), stream)
+            if scratch is not None:
+                _lib.call("tpk_grow_labels_push", n, 8, _lib.ptr(labels), _lib.ptr(changed), _lib.ptr(scratch), stream)
+            else:
+                changed.zero_()
+                _lib.call("tpk_grow_labels_step", n, nsample, _lib.ptr(neighbours), _lib.ptr(labels),
+                          _lib.ptr(changed), 8, stream)
             if int(changed.item()) == 0:
                 break
     return labels
