@@ -521,10 +521,11 @@ def pipeline_work(B, N):
 # (16 clouds), from one-launch ncu captures of dram__bytes_read.sum and dram__bytes_write.sum;
 # the commands and figures are in the summaries under profiles/.
 NCU_TRAFFIC_BYTES = {
-    "grouping_bwd_l1": (16794368 + 0) + (546299904 + 52450304),  # sort kernel + summing kernel
-    "grouping_fwd_l1": 84018432 + 476870912,
-    "interp_fwd_l1": 23094784 + 9831680,
-    "interp_bwd_l1": 73415168 + 2494976,
+    # dram__bytes.sum.per_second x gpu__time_duration.sum
+    "grouping_bwd_l1": 649316000 + 81156000,  # sums by columns + transposition
+    "grouping_fwd_l1": 16780000 + 548478000,  # 16-bit indices + gather
+    "interp_fwd_l1": 32734000,
+    "interp_bwd_l1": 93699000 + 16784000,
 }
 
 
