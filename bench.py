@@ -518,10 +518,9 @@ def pipeline_work(B, N):
 
 
 # DRAM bytes (read + write) of one launch of the HBM-bound kernels at the bench's own shape
-# (16 clouds), from one-launch ncu captures of dram__bytes_read.sum and dram__bytes_write.sum;
-# the commands and figures are in the summaries under profiles/.
+# (16 clouds), from one-launch ncu captures: dram__bytes.sum.per_second x gpu__time_duration.sum;
+# the command and figures are in profiles/gather_scatter_l1_B16.md.
 NCU_TRAFFIC_BYTES = {
-    # dram__bytes.sum.per_second x gpu__time_duration.sum
     "grouping_bwd_l1": 649316000 + 81156000,  # sums by columns + transposition
     "grouping_fwd_l1": 16780000 + 548478000,  # 16-bit indices + gather
     "interp_fwd_l1": 32734000,
